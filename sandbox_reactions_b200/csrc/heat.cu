@@ -28,10 +28,10 @@ constexpr int MAX_PART = 1184;    // most CTAs of a grid-stride heat kernel: one
 constexpr int PART_CAP = 16384;   // partials per reduced value (the level-0 smoother's CTAs included)
 // Device scalars. The kernels read Δt, the refinement's scale, δ and the PCG round's state from here (never from
 // launch arguments), so a captured graph of the implicit step replays for any step. The fused MG/Jacobi rounds keep
-// <r, z> of this round (S_RZC), of the last (S_RZP) and from the next preconditioner application (S_RZN), and which
+// <r, z> of this round (S_RZN, from the preconditioner application that opens it) and of the last (S_RZP), and which
 // direction buffer is current (S_PAR); the flexible (learned) rounds use S_RZ0/S_RZ1.
 enum Slot { S_HEAT0, S_NGAS, S_DT, S_RR, S_BB, S_GAM, S_HM, S_MOVED, S_VIOL, S_UB, S_TB, S_R32, S_PQ, S_RRI, S_RZ0, S_RZ1,
-            S_ZRO, S_MGRZ, S_BETA, S_RAD, S_GAIN, S_HELD, S_RZC, S_RZP, S_RZN, S_PAR, S_SCALE, S_ISCALE, S_DELTA,
+            S_ZRO, S_MGRZ, S_BETA, S_RAD, S_GAIN, S_HELD, S_RZP, S_RZN, S_PAR, S_SCALE, S_ISCALE, S_DELTA,
             S_COUNT };
 
 // Where a kernel's grid sum goes: the partials buffer, the ticket counter and the device scalar(s).
@@ -474,7 +474,7 @@ __global__ void pcg_direction_kernel(size_t n, const double* __restrict__ scal, 
     }
 }
 
-// The fused round head of (non-flexible) PCG: the search direction p_new = z + β p (β = <r,z>_cur / <r,z>_prev, or
+// After a (non-flexible) round's preconditioner: the search direction p_new = z + β p (β = <r,z> / <r,z>_prev, or
 // p_new = z while the S_BETA flag is 0: the first round) and q = A p_new in difference form, with partials of
 // <p_new, q>; the last CTA sets the flag. Four consecutive cells of a row per thread with 16-byte loads (W is a
 // multiple of 8); the neighbours' p_new are formed from their z and old p, so p_new goes to the other of the two
@@ -482,7 +482,7 @@ __global__ void pcg_direction_kernel(size_t n, const double* __restrict__ scal, 
 __global__ void spmv_dir_kernel(MgLevel L, const double* __restrict__ scal, const float* __restrict__ z, float* pa,
                                 float* pb, float* __restrict__ q, Red R, double* beta_flag) {
     const bool first = scal[S_BETA] == 0.0;  // p = z: the old direction is not read (it may hold anything)
-    const float beta = first ? 0.0f : (float)(scal[S_RZC] / scal[S_RZP]);
+    const float beta = first ? 0.0f : (float)(scal[S_RZN] / scal[S_RZP]);
     const bool par = scal[S_PAR] != 0.0;
     const float* __restrict__ p = par ? pb : pa;
     float* __restrict__ pnew = par ? pa : pb;
@@ -536,7 +536,7 @@ __global__ void spmv_dir_kernel(MgLevel L, const double* __restrict__ scal, cons
 // e += α p, r -= α q with 16-byte accesses (four cells per thread), p the round's new direction; partials of <r, r>.
 __global__ void pcg_update4_kernel(size_t n, const double* __restrict__ scal, const float* pa, const float* pb,
                                    const float* __restrict__ q, float* __restrict__ e, float* __restrict__ r, Red R) {
-    const float alpha = (float)(scal[S_RZC] / scal[S_PQ]);
+    const float alpha = (float)(scal[S_RZN] / scal[S_PQ]);
     const float* __restrict__ p = scal[S_PAR] != 0.0 ? pa : pb;
     const size_t n4 = n / 4, stride = (size_t)gridDim.x * blockDim.x;
     double acc = 0.0;
@@ -875,20 +875,17 @@ __global__ void set_scalar_kernel(double* scal, int slot, double value) {
     if (threadIdx.x == 0 && blockIdx.x == 0) scal[slot] = value;
 }
 
-// A fused PCG solve's start, after its first preconditioner application: that <r, z> is the current one, the first
-// direction is z, the direction buffers start at pa.
+// A fused PCG solve's start: the first direction is z, the direction buffers start at pa.
 __global__ void pcg_start_kernel(double* scal) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    scal[S_RZC] = scal[S_RZN];
     scal[S_BETA] = 0.0;
     scal[S_PAR] = 0.0;
 }
 
-// A fused PCG round's end: the new <r, z> becomes the current one and the new direction buffer the old.
+// A fused PCG round's end: its <r, z> becomes the last one and the new direction buffer the old.
 __global__ void pcg_rotate_kernel(double* scal) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    scal[S_RZP] = scal[S_RZC];
-    scal[S_RZC] = scal[S_RZN];
+    scal[S_RZP] = scal[S_RZN];
     scal[S_PAR] = scal[S_PAR] != 0.0 ? 0.0 : 1.0;
 }
 
@@ -985,8 +982,7 @@ __global__ void heat_ctl_kernel(HeatCtl* c, double* scal, int phase, CtlHandles 
             if (!go) ctl_set(hd, c, B_REFINE, false, false);
             break;
         }
-        case C_INNER_BEGIN: {  // after the scaled residual and its first preconditioner application
-            scal[S_RZC] = scal[S_RZN];
+        case C_INNER_BEGIN: {  // after the scaled residual
             scal[S_BETA] = 0.0;
             scal[S_PAR] = 0.0;
             c->rr0 = scal[S_R32];
@@ -998,8 +994,7 @@ __global__ void heat_ctl_kernel(HeatCtl* c, double* scal, int phase, CtlHandles 
         case C_ROUND: {  // after a round: rotate its state, test the residual
             c->runs[B_ROUND]++;
             c->it++;
-            scal[S_RZP] = scal[S_RZC];
-            scal[S_RZC] = scal[S_RZN];
+            scal[S_RZP] = scal[S_RZN];
             scal[S_PAR] = scal[S_PAR] != 0.0 ? 0.0 : 1.0;
             const double pq = scal[S_PQ], rr = scal[S_RRI];
             bool more = true;
@@ -1181,7 +1176,10 @@ void precondition(HeatSolver* H, uint32_t precond, int rz_slot, cudaStream_t s) 
     }
 }
 
-// One PCG round: q = A p, α, e += α p, r -= α q, z = M r, β, p = z + β p. `parity` picks the <r,z> slots.
+// One PCG round. MG and Jacobi: z = M r, β, p = z + β p, q = A p, α, e += α p, r -= α q — a round opens with its
+// preconditioner, so the solve's last round ends on the residual it tests and applies none in vain (a V-cycle less per
+// inner solve: 17 of 140 over three 2048² steps of the full world). Flexible CG: q = A p, α, e, r, z = M r, β, p;
+// `parity` picks its <r,z> slots.
 void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s) {
     const int rz_old = parity ? S_RZ1 : S_RZ0, rz_new = parity ? S_RZ0 : S_RZ1;
     if (precond == SR_PRECOND_LEARNED) {
@@ -1201,13 +1199,13 @@ void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s)
     // one captured graph serves every round
     (void)rz_old;
     (void)rz_new;
+    precondition(H, precond, S_RZN, s);
     spmv_dir_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2, H->q32,
                                                     H->red(S_PQ), H->scal + S_BETA);
     sr_note_launch();
     pcg_update4_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, H->p32, H->p2, H->q32, H->e32, H->r32,
                                                        H->red(S_RRI));
     sr_note_launch();
-    precondition(H, precond, S_RZN, s);
     pcg_rotate_kernel<<<1, 32, 0, s>>>(H->scal);
     sr_note_launch();
 }
@@ -1255,7 +1253,6 @@ int inner_pcg(HeatSolver* H, uint32_t precond, double eta, int max_it, cudaStrea
         pcg_direction_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, -1, S_RZ0, H->z32, H->p32);
         sr_note_launch();
     } else {  // the first round's fused direction is p = z
-        precondition(H, precond, S_RZN, s);
         pcg_start_kernel<<<1, 32, 0, s>>>(H->scal);
         sr_note_launch();
     }
@@ -1432,17 +1429,16 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                                            [&](cudaStream_t s3) {
                     scale_kernel<<<H->grid, RED_THREADS, 0, s3>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32));
                     sr_note_launch();
-                    precondition(H, precond, S_RZN, s3);
                     ctl_launch(H, C_INNER_BEGIN, hd, s3);
                     nb[B_ROUND] = capture_body(capture_conditional(s3, hd.h[B_ROUND], cudaGraphCondTypeWhile), H->cap[4],
                                                [&](cudaStream_t s4) {
+                        precondition(H, precond, S_RZN, s4);
                         spmv_dir_kernel<<<H->grid, RED_THREADS, 0, s4>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2,
                                                                           H->q32, H->red(S_PQ), H->scal + S_BETA);
                         sr_note_launch();
                         pcg_update4_kernel<<<H->grid, RED_THREADS, 0, s4>>>(H->n, H->scal, H->p32, H->p2, H->q32,
                                                                              H->e32, H->r32, H->red(S_RRI));
                         sr_note_launch();
-                        precondition(H, precond, S_RZN, s4);
                         ctl_launch(H, C_ROUND, hd, s4);
                     });
                     correction_kernel<<<H->grid, RED_THREADS, 0, s3>>>(H->n, H->gas, H->e32, H->scal, H->x);
