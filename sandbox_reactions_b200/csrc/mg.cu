@@ -17,26 +17,30 @@ namespace {
 // small levels are bound by one CTA's latency).
 constexpr int BIG_SX = 64, BIG_SY = 32, BIG_NT = 512;
 constexpr int SMALL_SX = 32, SMALL_SY = 16, SMALL_NT = 256;
-constexpr int TAIL_THREADS = 1024;
-constexpr int TAIL_ROWS = TAIL_THREADS / 32;  // the tail's threads as 32 columns x TAIL_ROWS rows
+constexpr int TAIL_THREADS = 512;
 
-// A tail level's arrays as offsets into the tail's shared memory (floats for the seven arrays, bytes for the mask).
+// A tail level's arrays as offsets (floats) into the tail's image, rows padded to an even pitch p and height hp.
 struct TailLevel {
-    int w, h;
-    int c, dx, dy, b, x, inv, t;  // float offsets; inv: the inverse diagonal (0 on masked cells); t: the weights towards
-                                  // the next coarser level
-    int m;                        // byte offset of the mask
+    int w, h, p, hp;
+    int dx, dy, inv, t, c, b, x;  // inv: the inverse diagonal (0 on masked cells); t: the weights towards the next
+                                  // coarser level; b and x: the lower levels' right-hand side and iterate
 };
 
 struct TailArgs {
     int t, nl, pre, post;
     float omega;
-    int sinv;                 // float offset of the coarsest level's inverse (nc x nc)
-    const float4* img;        // the tail's shared memory image (everything but the top level's b), per Newton pass
-    int img_f4;               // its size in 16-byte words
+    int sinv;                 // offset of the coarsest level's inverse (nc x nc)
+    int img_f4;               // the lower levels' part of the image in 16-byte words
+    const float* img;
+    const float* b;           // the top level's right-hand side and result
+    float* x2;
     double* out;              // non-null when the tail's top level is level 0: <b, x2> written here
-    MgLevel L[kMgMaxLevels];
     TailLevel T[kMgMaxLevels];
+};
+
+constexpr int kTailLevels = 6;  // 64 x 64 down to 2 x 2
+struct TailPack {
+    MgLevel L[kTailLevels];  // the tail's levels, the top first
 };
 
 // Level 0's couplings to the +x / +y neighbours from the f64 faces, zero unless both cells are gas.
@@ -841,283 +845,429 @@ __global__ void mg_coarse_inverse_kernel(MgLevel C, float* inv) {
     for (int k = threadIdx.x; k < n * n; k += blockDim.x) inv[k] = (float)fin[(k / n) * m + n + (k % n)];
 }
 
-// ---- the coarse tail: every level from t on, inside one CTA
-// The tail's levels live in its dynamic shared memory at the offsets of TailLevel: indexing the extern shared array
-// itself keeps every access a shared-memory access.
+// ---- the coarse tail: every level of at most 64 x 64 cells, inside one CTA
+//
+// What bounds it is latency: sixteen dependent half-sweeps a level under V(4,4), a few hundred cells each. So a level
+// is held in registers by no more warps than it fills, each thread a band of 4 rows of one column pair (as in the
+// row-band smoother), and synchronises only those: the top level by up to 16 warps, lanes = 32 column pairs, band edges
+// through shared memory; the next level (at most 32 x 32) by up to 4 warps of two 16-pair row groups; every level of at
+// most 16 x 16 by warp 0 alone, 8 pairs x 4 row groups, neighbours by shuffles and no barrier at all. The top level's
+// coefficients stay in registers from its pre- to its post-smoother; the lower levels are read from the image
+// mg_tail_pack_kernel writes once per Newton pass, whose rows are padded to even pitches and heights so that no access
+// has an edge case. 64 x 64 top under V(4,4): 27 -> 19 us a V-cycle against the whole CTA of 1,024 threads meeting at
+// every half-sweep of every level.
 extern __shared__ __align__(16) unsigned char tail_smem_raw[];
-__device__ __forceinline__ float* tsf() { return reinterpret_cast<float*>(tail_smem_raw); }
 
-// Threads of the tail run as 32 columns x TAIL_ROWS rows: thread (tx, ty) takes rows ty, ty + TAIL_ROWS, ... and, of
-// a sweep's colour, the columns 2 tx + parity, 2 (tx + 32) + parity, ... (no index divisions).
-__device__ __forceinline__ void tail_sweep(const TailLevel T, int color) {
-    float* f = tsf();
-    const float *b = f + T.b, *dx = f + T.dx, *dy = f + T.dy, *inv = f + T.inv;
-    float* x = f + T.x;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int y = ty; y < T.h; y += TAIL_ROWS) {
-        const int par = (y + color) & 1;
-        for (int xx = 2 * tx + par; xx < T.w; xx += 64) {
-            // masked cells: b = 0, no couplings, inv = 0, so they stay 0; couplings past the edges are 0
-            const int i = y * T.w + xx;
-            float s = b[i];
-            if (xx > 0) s += dx[i - 1] * x[i - 1];
-            if (xx + 1 < T.w) s += dx[i] * x[i + 1];
-            if (y > 0) s += dy[i - T.w] * x[i - T.w];
-            if (y + 1 < T.h) s += dy[i] * x[i + T.w];
-            x[i] = s * inv[i];
-        }
-    }
-    __syncthreads();
+struct TailBand {
+    float bA[RB_R], bB[RB_R], iA[RB_R], iB[RB_R], dl[RB_R], dm[RB_R], dr[RB_R], dA[RB_R], dB[RB_R], xA[RB_R], xB[RB_R];
+    float uA, uB;  // the couplings of row 0 to the row above
+};
+
+using TailEdge = float2[2][RB_WARPS][32];  // [top row / bottom row][warp][lane]: (x of 2j, x of 2j + 1)
+
+__device__ __forceinline__ void tail_bar(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// `count` half-sweeps from colour `color` of a tail level of at most 64 x 64 cells, each thread holding one 2 x 2 block
-// (warp v's rows 2v, 2v + 1, lane j's columns 2j, 2j + 1) with its coefficients and iterate in registers: a cell's
-// neighbours inside the block are registers, across a column edge a shuffle, across a row edge one shared-memory load
-// of the level's x (kept current after every half-sweep). Same arithmetic as tail_sweep.
-__device__ __forceinline__ void tail_sweeps_reg(const TailLevel T, int color, int count) {
-    float* f = tsf();
-    const float *b = f + T.b, *dx = f + T.dx, *dy = f + T.dy, *inv = f + T.inv;
-    float* x = f + T.x;
-    const int lane = threadIdx.x & 31, x0 = 2 * lane, y0 = 2 * (threadIdx.x >> 5);
-    float bb[4], iv[4], cl[4], cr[4], cu[4], cd[4], xv[4];
-    bool ok[4];
+// The band's coefficients from arrays of pitch p and hp rows (both even): column pair j of LC, rows row0 .. row0 + 3.
+template <int LC>
+__device__ __forceinline__ void tail_load(TailBand& B, const float* inv, const float* dx, const float* dy, int p, int hp,
+                                          int j, int row0) {
+    const bool in = 2 * j < p;
+    const float2 z = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const int xx = x0 + (k & 1), yy = y0 + (k >> 1);
-        ok[k] = xx < T.w && yy < T.h;
-        const int i = ok[k] ? yy * T.w + xx : 0;
-        bb[k] = ok[k] ? b[i] : 0.0f;
-        iv[k] = ok[k] ? inv[i] : 0.0f;
-        cl[k] = ok[k] && xx > 0 ? dx[i - 1] : 0.0f;
-        cr[k] = ok[k] && xx + 1 < T.w ? dx[i] : 0.0f;
-        cu[k] = ok[k] && yy > 0 ? dy[i - T.w] : 0.0f;
-        cd[k] = ok[k] && yy + 1 < T.h ? dy[i] : 0.0f;
-        xv[k] = ok[k] ? x[i] : 0.0f;
+    for (int r = 0; r < RB_R; r++) {
+        const int row = row0 + r, q = row * p + 2 * j;
+        const bool ok = in && row < hp;
+        const float2 i2 = ok ? *reinterpret_cast<const float2*>(inv + q) : z;
+        const float2 x2 = ok ? *reinterpret_cast<const float2*>(dx + q) : z;
+        const float2 y2 = ok ? *reinterpret_cast<const float2*>(dy + q) : z;
+        B.iA[r] = i2.x;
+        B.iB[r] = i2.y;
+        B.dm[r] = x2.x;
+        B.dr[r] = x2.y;
+        B.dA[r] = y2.x;
+        B.dB[r] = y2.y;
+        const float l = __shfl_up_sync(0xffffffffu, x2.y, 1);
+        B.dl[r] = j ? l : 0.0f;
     }
-    const int iu = y0 > 0 ? (y0 - 1) * T.w : 0, id = y0 + 2 < T.h ? (y0 + 2) * T.w : 0;
-    const bool hu = y0 > 0 && ok[0], hd = y0 + 2 < T.h && ok[2];
-    for (int s = 0; s < count; s++) {
-        if (((color + s) & 1) == 0) {  // cells (2j, 2v) and (2j + 1, 2v + 1)
-            const float left = __shfl_up_sync(0xffffffffu, xv[1], 1);
-            const float right = __shfl_down_sync(0xffffffffu, xv[2], 1);
-            const float up = hu ? x[iu + x0] : 0.0f;
-            const float down = hd && ok[3] ? x[id + x0 + 1] : 0.0f;
-            xv[0] = (bb[0] + cl[0] * left + cr[0] * xv[1] + cu[0] * up + cd[0] * xv[2]) * iv[0];
-            xv[3] = (bb[3] + cl[3] * xv[2] + cr[3] * right + cu[3] * xv[1] + cd[3] * down) * iv[3];
-            if (ok[0]) x[y0 * T.w + x0] = xv[0];
-            if (ok[3]) x[(y0 + 1) * T.w + x0 + 1] = xv[3];
-        } else {  // cells (2j + 1, 2v) and (2j, 2v + 1)
-            const float right = __shfl_down_sync(0xffffffffu, xv[0], 1);
-            const float left = __shfl_up_sync(0xffffffffu, xv[3], 1);
-            const float up = hu && ok[1] ? x[iu + x0 + 1] : 0.0f;
-            const float down = hd ? x[id + x0] : 0.0f;
-            xv[1] = (bb[1] + cl[1] * xv[0] + cr[1] * right + cu[1] * up + cd[1] * xv[3]) * iv[1];
-            xv[2] = (bb[2] + cl[2] * left + cr[2] * xv[3] + cu[2] * xv[0] + cd[2] * down) * iv[2];
-            if (ok[1]) x[y0 * T.w + x0 + 1] = xv[1];
-            if (ok[2]) x[(y0 + 1) * T.w + x0] = xv[2];
+    const float2 u2 = in && row0 > 0 && row0 - 1 < hp ? *reinterpret_cast<const float2*>(dy + (row0 - 1) * p + 2 * j) : z;
+    B.uA = u2.x;
+    B.uB = u2.y;
+}
+
+// The rows above and below the band, as the last half-sweep left them.
+template <int LC>
+__device__ __forceinline__ void tail_rows(const TailBand& B, const TailEdge& e, int warp, int lane, float2& above,
+                                          float2& below) {
+    if constexpr (LC == 32) {
+        above = e[1][warp > 0 ? warp - 1 : 0][lane];
+        below = e[0][warp + 1 < RB_WARPS ? warp + 1 : warp][lane];
+    } else {
+        above = make_float2(__shfl_up_sync(0xffffffffu, B.xA[RB_R - 1], LC), __shfl_up_sync(0xffffffffu, B.xB[RB_R - 1], LC));
+        below = make_float2(__shfl_down_sync(0xffffffffu, B.xA[0], LC), __shfl_down_sync(0xffffffffu, B.xB[0], LC));
+        if constexpr (LC == 16) {  // two row groups a warp: the outer rows belong to the next warps
+            const int j = lane & 15;
+            if (lane < 16) above = e[1][warp > 0 ? warp - 1 : 0][j];
+            else below = e[0][warp + 1 < RB_WARPS ? warp + 1 : warp][j];
         }
-        __syncthreads();
     }
 }
 
-__device__ __forceinline__ void tail_restrict(const TailLevel F, const TailLevel C) {
-    float* f = tsf();
-    const float *fc = f + F.c, *fdx = f + F.dx, *fdy = f + F.dy, *fb = f + F.b, *fx = f + F.x, *ft = f + F.t;
-    const uint8_t* fm = tail_smem_raw + F.m;
-    const uint8_t* cm = tail_smem_raw + C.m;
-    float *cb = f + C.b, *cx = f + C.x;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int Y = ty; Y < C.h; Y += TAIL_ROWS)
-        for (int X = tx; X < C.w; X += 32) {
-            const int I = Y * C.w + X;
-            float sum = 0.0f;
-            for (int bb = 0; bb < 2; bb++)
-                for (int a = 0; a < 2; a++) {
-                    const int x = 2 * X + a, y = 2 * Y + bb;
-                    if (x >= F.w || y >= F.h) continue;
-                    const int j = y * F.w + x;
-                    if (!fm[j]) continue;
-                    const float xj = fx[j];
-                    float ax = fc[j] * xj;
-                    if (x > 0) ax += fdx[j - 1] * (xj - fx[j - 1]);
-                    if (x + 1 < F.w) ax += fdx[j] * (xj - fx[j + 1]);
-                    if (y > 0) ax += fdy[j - F.w] * (xj - fx[j - F.w]);
-                    if (y + 1 < F.h) ax += fdy[j] * (xj - fx[j + F.w]);
-                    sum += ft[j] * (fb[j] - ax);
-                }
-            cb[I] = cm[I] ? sum : 0.0f;
-            cx[I] = 0.0f;
-        }
-    __syncthreads();
+template <int LC>
+__device__ __forceinline__ void tail_post_edges(const TailBand& B, TailEdge& e, int warp, int lane) {
+    if constexpr (LC == 32) {
+        e[0][warp][lane] = make_float2(B.xA[0], B.xB[0]);
+        e[1][warp][lane] = make_float2(B.xA[RB_R - 1], B.xB[RB_R - 1]);
+    } else if constexpr (LC == 16) {
+        if (lane < 16) e[0][warp][lane] = make_float2(B.xA[0], B.xB[0]);
+        else e[1][warp][lane - 16] = make_float2(B.xA[RB_R - 1], B.xB[RB_R - 1]);
+    }
 }
 
-__global__ void __launch_bounds__(TAIL_THREADS) mg_tail_kernel(TailArgs A) {
-    float* f = tsf();
-    __shared__ TailLevel T[kMgMaxLevels];  // indexed by a run-time level
-    if (threadIdx.x < kMgMaxLevels) T[threadIdx.x] = A.T[threadIdx.x];
-    // every level's coefficients, weights, inverse diagonal and mask, the iterates at 0 and the coarsest inverse, as
-    // packed once per Newton pass: one 16-byte copy per word, all in flight together
-    float4* dst = reinterpret_cast<float4*>(tail_smem_raw);
-    for (int k = threadIdx.x; k < A.img_f4; k += TAIL_THREADS) dst[k] = A.img[k];
-    __syncthreads();
-    {
-        const int n = T[A.t].w * T[A.t].h;
-        const float* b = A.L[A.t].b;
-        for (int i = threadIdx.x; i < n; i += TAIL_THREADS) f[T[A.t].b + i] = b[i];
-    }
-    const int nc = T[A.nl - 1].w * T[A.nl - 1].h;
-    const float* sinv = f + A.sinv;
-    __syncthreads();
-    for (int l = A.t; l < A.nl - 1; l++) {
-        const TailLevel Tl = T[l];
-        if (Tl.w <= 64 && Tl.h <= 64) {
-            tail_sweeps_reg(Tl, 0, 2 * A.pre);
+template <int LC, int COL>
+__device__ __forceinline__ void tail_half_sweep(TailBand& B, const TailEdge& e, int warp, int lane) {
+    float2 above, below;
+    tail_rows<LC>(B, e, warp, lane, above, below);
+#pragma unroll
+    for (int r = 0; r < RB_R; r++) {
+        if ((r & 1) == COL) {
+            const float left = __shfl_up_sync(0xffffffffu, B.xB[r], 1);
+            const float up = r ? B.xA[r - 1] : above.x, down = r + 1 < RB_R ? B.xA[r + 1] : below.x;
+            const float cu = r ? B.dA[r - 1] : B.uA;
+            B.xA[r] = (B.bA[r] + B.dl[r] * left + B.dm[r] * B.xB[r] + cu * up + B.dA[r] * down) * B.iA[r];
         } else {
-            for (int s = 0; s < A.pre; s++) {
-                tail_sweep(Tl, 0);
-                tail_sweep(Tl, 1);
+            const float right = __shfl_down_sync(0xffffffffu, B.xA[r], 1);
+            const float up = r ? B.xB[r - 1] : above.y, down = r + 1 < RB_R ? B.xB[r + 1] : below.y;
+            const float cu = r ? B.dB[r - 1] : B.uB;
+            B.xB[r] = (B.bB[r] + B.dm[r] * B.xA[r] + B.dr[r] * right + cu * up + B.dB[r] * down) * B.iB[r];
+        }
+    }
+}
+
+// `sweeps` sweeps, colour FIRST before the other; the edges in e[0] on entry and on return.
+template <int LC, int FIRST>
+__device__ __forceinline__ void tail_sweeps(TailBand& B, TailEdge* e, int sweeps, int warp, int lane, int bar,
+                                            int threads) {
+    for (int s = 0; s < sweeps; s++) {
+        tail_half_sweep<LC, FIRST>(B, e[0], warp, lane);
+        if constexpr (LC > 8) {
+            tail_post_edges<LC>(B, e[1], warp, lane);
+            tail_bar(bar, threads);
+        }
+        tail_half_sweep<LC, 1 - FIRST>(B, e[1], warp, lane);
+        if constexpr (LC > 8) {
+            tail_post_edges<LC>(B, e[0], warp, lane);
+            tail_bar(bar, threads);
+        }
+    }
+}
+
+// One array's cells of the band (0 outside).
+__device__ __forceinline__ void tail_cells(float2 (&v)[RB_R], const float* a, int p, int hp, int j, int row0) {
+#pragma unroll
+    for (int r = 0; r < RB_R; r++)
+        v[r] = 2 * j < p && row0 + r < hp ? *reinterpret_cast<const float2*>(a + (row0 + r) * p + 2 * j)
+                                          : make_float2(0.f, 0.f);
+}
+
+// The residual in difference form, weighted and summed over each 2 x 2 aggregate, into the next level's b.
+template <int LC>
+__device__ __forceinline__ void tail_restrict(const TailBand& B, const TailEdge* e, const float2 (&cc)[RB_R],
+                                              const float2 (&tt)[RB_R], int j, int row0, int warp, int lane, float* cb,
+                                              int cp, int cw, int ch) {
+    float2 above, below;
+    tail_rows<LC>(B, e[0], warp, lane, above, below);
+    float ragg[RB_R / 2] = {};
+#pragma unroll
+    for (int r = 0; r < RB_R; r++) {
+        const float2 c2 = cc[r], t2 = tt[r];
+        const float left = __shfl_up_sync(0xffffffffu, B.xB[r], 1);
+        const float right = __shfl_down_sync(0xffffffffu, B.xA[r], 1);
+        const float upA = r ? B.xA[r - 1] : above.x, dnA = r + 1 < RB_R ? B.xA[r + 1] : below.x;
+        const float upB = r ? B.xB[r - 1] : above.y, dnB = r + 1 < RB_R ? B.xB[r + 1] : below.y;
+        const float cuA = r ? B.dA[r - 1] : B.uA, cuB = r ? B.dB[r - 1] : B.uB;
+        float axA = c2.x * B.xA[r];
+        axA += B.dl[r] * (B.xA[r] - left);
+        axA += B.dm[r] * (B.xA[r] - B.xB[r]);
+        axA += cuA * (B.xA[r] - upA);
+        axA += B.dA[r] * (B.xA[r] - dnA);
+        float axB = c2.y * B.xB[r];
+        axB += B.dm[r] * (B.xB[r] - B.xA[r]);
+        axB += B.dr[r] * (B.xB[r] - right);
+        axB += cuB * (B.xB[r] - upB);
+        axB += B.dB[r] * (B.xB[r] - dnB);
+        // masked and padding cells: b = 0, x = 0 and no couplings, so their residual is 0
+        ragg[r >> 1] += t2.x * (B.bA[r] - axA) + t2.y * (B.bB[r] - axB);
+    }
+#pragma unroll
+    for (int k = 0; k < RB_R / 2; k++) {
+        const int Y = (row0 >> 1) + k;
+        if (j < cw && Y < ch) cb[Y * cp + j] = ragg[k];
+    }
+}
+
+// x += ω t x_c
+__device__ __forceinline__ void tail_correct(TailBand& B, const float2 (&tt)[RB_R], int j, int row0, float omega,
+                                             const float* cx, int cp, int cw, int ch) {
+#pragma unroll
+    for (int r = 0; r < RB_R; r++) {
+        const int Y = (row0 + r) >> 1;
+        if (j < cw && Y < ch) {
+            const float v = omega * cx[Y * cp + j];
+            B.xA[r] += v * tt[r].x;
+            B.xB[r] += v * tt[r].y;
+        }
+    }
+}
+
+// A lower level's pre-smoother from x = 0, its restriction, and its iterate left in shared memory.
+template <int LC>
+__device__ __forceinline__ void tail_down(const TailLevel& T, const TailLevel& C, float* f, TailEdge* e, int pre,
+                                          int warp, int lane, int bar, int threads) {
+    const int j = lane & (LC - 1), row0 = RB_R * ((32 / LC) * warp + lane / LC);
+    TailBand B;
+    tail_load<LC>(B, f + T.inv, f + T.dx, f + T.dy, T.p, T.hp, j, row0);
+    const bool in = 2 * j < T.p;
+#pragma unroll
+    for (int r = 0; r < RB_R; r++) {
+        const bool ok = in && row0 + r < T.hp;
+        const float2 b2 = ok ? *reinterpret_cast<const float2*>(f + T.b + (row0 + r) * T.p + 2 * j) : make_float2(0.f, 0.f);
+        B.bA[r] = b2.x;
+        B.bB[r] = b2.y;
+        B.xA[r] = B.xB[r] = 0.0f;
+    }
+    if constexpr (LC > 8) {
+        tail_post_edges<LC>(B, e[0], warp, lane);
+        tail_bar(bar, threads);
+    }
+    tail_sweeps<LC, 0>(B, e, pre, warp, lane, bar, threads);
+    float2 c2[RB_R], t2[RB_R];
+    tail_cells(c2, f + T.c, T.p, T.hp, j, row0);
+    tail_cells(t2, f + T.t, T.p, T.hp, j, row0);
+    tail_restrict<LC>(B, e, c2, t2, j, row0, warp, lane, f + C.b, C.p, C.w, C.h);
+#pragma unroll
+    for (int r = 0; r < RB_R; r++)
+        if (in && row0 + r < T.hp)
+            *reinterpret_cast<float2*>(f + T.x + (row0 + r) * T.p + 2 * j) = make_float2(B.xA[r], B.xB[r]);
+}
+
+// A lower level's coarse correction and post-smoother, its result left in shared memory.
+template <int LC>
+__device__ __forceinline__ void tail_up(const TailLevel& T, const TailLevel& C, float* f, TailEdge* e, int post,
+                                        float omega, int warp, int lane, int bar, int threads) {
+    const int j = lane & (LC - 1), row0 = RB_R * ((32 / LC) * warp + lane / LC);
+    TailBand B;
+    tail_load<LC>(B, f + T.inv, f + T.dx, f + T.dy, T.p, T.hp, j, row0);
+    const bool in = 2 * j < T.p;
+#pragma unroll
+    for (int r = 0; r < RB_R; r++) {
+        const int q = (row0 + r) * T.p + 2 * j;
+        const bool ok = in && row0 + r < T.hp;
+        const float2 z = make_float2(0.f, 0.f);
+        const float2 b2 = ok ? *reinterpret_cast<const float2*>(f + T.b + q) : z;
+        const float2 x2 = ok ? *reinterpret_cast<const float2*>(f + T.x + q) : z;
+        B.bA[r] = b2.x;
+        B.bB[r] = b2.y;
+        B.xA[r] = x2.x;
+        B.xB[r] = x2.y;
+    }
+    float2 t2[RB_R];
+    tail_cells(t2, f + T.t, T.p, T.hp, j, row0);
+    tail_correct(B, t2, j, row0, omega, f + C.x, C.p, C.w, C.h);
+    if constexpr (LC > 8) {
+        tail_post_edges<LC>(B, e[0], warp, lane);
+        tail_bar(bar, threads);
+    }
+    tail_sweeps<LC, 1>(B, e, post, warp, lane, bar, threads);
+#pragma unroll
+    for (int r = 0; r < RB_R; r++)
+        if (in && row0 + r < T.hp)
+            *reinterpret_cast<float2*>(f + T.x + (row0 + r) * T.p + 2 * j) = make_float2(B.xA[r], B.xB[r]);
+}
+
+// The coarsest level exactly, by warp 0: x = A⁻¹ b with the inverse built once per Newton pass (at most 4 x 4 cells).
+__device__ __forceinline__ void tail_coarsest(const TailLevel& T, float* f, const float* sinv, int lane) {
+    const int nc = T.w * T.h;
+    if (lane < nc) {
+        float s = 0.0f;
+        for (int y = 0, k = 0; y < T.h; y++)
+            for (int x = 0; x < T.w; x++, k++) s += sinv[lane * nc + k] * f[T.b + y * T.p + x];
+        f[T.x + (lane / T.w) * T.p + lane % T.w] = s;  // a masked cell: an identity row and b = 0
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(TAIL_THREADS, 1) mg_tail_kernel(const __grid_constant__ TailArgs A) {
+    float* f = reinterpret_cast<float*>(tail_smem_raw + 2 * sizeof(TailEdge));
+    TailEdge* e = reinterpret_cast<TailEdge*>(tail_smem_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const TailLevel& T = A.T[A.t];
+    const TailLevel& T1 = A.T[A.t + 1];
+    const int nw = (T.h + RB_R - 1) / RB_R, nw1 = (T1.h + 2 * RB_R - 1) / (2 * RB_R);
+    const int row0 = RB_R * warp;
+    // the lower levels' image (b and x 0) into shared memory, while the top level's loads are in flight
+    for (int k = threadIdx.x; k < A.img_f4; k += TAIL_THREADS)
+        reinterpret_cast<float4*>(f)[k] = reinterpret_cast<const float4*>(A.img)[k];
+    TailBand B;
+    float2 c2[RB_R], t2[RB_R];
+    tail_load<32>(B, A.img + T.inv, A.img + T.dx, A.img + T.dy, T.p, T.hp, lane, row0);
+    {
+        const float* b = A.b;
+        const bool two = 2 * lane + 1 < T.w;
+#pragma unroll
+        for (int r = 0; r < RB_R; r++) {
+            const bool ok = 2 * lane < T.w && row0 + r < T.h;
+            const int q = (row0 + r) * T.w + 2 * lane;
+            B.bA[r] = ok ? b[q] : 0.0f;
+            B.bB[r] = ok && two ? b[q + 1] : 0.0f;
+            B.xA[r] = B.xB[r] = 0.0f;
+        }
+    }
+    tail_cells(c2, A.img + T.c, T.p, T.hp, lane, row0);
+    tail_cells(t2, A.img + T.t, T.p, T.hp, lane, row0);
+    // every warp's rows in both edge buffers: a band past the level's last row reads 0 (times no coupling)
+    tail_post_edges<32>(B, e[0], warp, lane);
+    tail_post_edges<32>(B, e[1], warp, lane);
+    __syncthreads();
+    if (warp < nw) {
+        tail_sweeps<32, 0>(B, e, A.pre, warp, lane, 1, 32 * nw);
+        tail_restrict<32>(B, e, c2, t2, lane, row0, warp, lane, f + T1.b, T1.p, T1.w, T1.h);
+    }
+    __syncthreads();
+    if (warp < nw1) {
+        tail_down<16>(T1, A.T[A.t + 2], f, e, A.pre, warp, lane, 2, 32 * nw1);
+        tail_bar(2, 32 * nw1);
+        if (warp == 0) {
+            for (int l = A.t + 2; l < A.nl - 1; l++) {
+                tail_down<8>(A.T[l], A.T[l + 1], f, e, A.pre, 0, lane, 0, 0);
+                __syncwarp();
+            }
+            tail_coarsest(A.T[A.nl - 1], f, f + A.sinv, lane);
+            for (int l = A.nl - 2; l >= A.t + 2; l--) {
+                tail_up<8>(A.T[l], A.T[l + 1], f, e, A.post, A.omega, 0, lane, 0, 0);
+                __syncwarp();
             }
         }
-        tail_restrict(Tl, T[l + 1]);
+        tail_bar(2, 32 * nw1);
+        tail_up<16>(T1, A.T[A.t + 2], f, e, A.post, A.omega, warp, lane, 2, 32 * nw1);
     }
-    {
-        // the coarsest level exactly: x = A⁻¹ b with the inverse built once per Newton pass (mg_coarse_inverse_kernel)
-        // one warp per row, the lanes splitting the row and summing by shuffles
-        const TailLevel Cs = T[A.nl - 1];
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (int i = warp; i < nc; i += TAIL_THREADS / 32) {
-            float s = 0.0f;
-            for (int k = lane; k < nc; k += 32) s += sinv[i * nc + k] * f[Cs.b + k];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-            if (lane == 0) f[Cs.x + i] = tail_smem_raw[Cs.m + i] ? s : 0.0f;
-        }
-        __syncthreads();
-    }
-    for (int l = A.nl - 2; l >= A.t; l--) {
-        const TailLevel F = T[l];
-        const TailLevel Cs = T[l + 1];
-        {
-            const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-            for (int y = ty; y < F.h; y += TAIL_ROWS)
-                for (int x = tx; x < F.w; x += 32) {
-                    const int i = y * F.w + x;
-                    if (tail_smem_raw[F.m + i])
-                        f[F.x + i] += A.omega * f[F.t + i] * f[Cs.x + (y >> 1) * Cs.w + (x >> 1)];
-                }
-        }
-        __syncthreads();
-        if (F.w <= 64 && F.h <= 64) {
-            tail_sweeps_reg(F, 1, 2 * A.post);
-        } else {
-            for (int s = 0; s < A.post; s++) {
-                tail_sweep(F, 1);
-                tail_sweep(F, 0);
-            }
-        }
-    }
-    const TailLevel top = T[A.t];
-    const int n = top.w * top.h;
+    __syncthreads();
     double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += TAIL_THREADS) {
-        const float xv = f[top.x + i];
-        A.L[A.t].x2[i] = xv;
-        acc += (double)f[top.b + i] * (double)xv;
+    tail_correct(B, t2, lane, row0, A.omega, f + T1.x, T1.p, T1.w, T1.h);
+    tail_post_edges<32>(B, e[0], warp, lane);
+    __syncthreads();
+    if (warp < nw) {
+        tail_sweeps<32, 1>(B, e, A.post, warp, lane, 1, 32 * nw);
+        const bool two = 2 * lane + 1 < T.w;
+#pragma unroll
+        for (int r = 0; r < RB_R; r++) {
+            if (!(2 * lane < T.w && row0 + r < T.h)) continue;
+            const int q = (row0 + r) * T.w + 2 * lane;
+            A.x2[q] = B.xA[r];
+            if (two) A.x2[q + 1] = B.xB[r];
+            acc += (double)B.bA[r] * (double)B.xA[r] + (double)B.bB[r] * (double)B.xB[r];
+        }
     }
     if (A.out) {
-        __shared__ double red[TAIL_THREADS / 32];
+        __shared__ double red[RB_WARPS];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+        if (lane == 0) red[warp] = acc;
         __syncthreads();
         if (threadIdx.x == 0) {
             double t = 0.0;
-            for (int q = 0; q < TAIL_THREADS / 32; q++) t += red[q];
+            for (int q = 0; q < RB_WARPS; q++) t += red[q];
             *A.out = t;
         }
     }
 }
 
-// The tail's shared-memory layout: seven float arrays per level, the coarsest inverse, then the masks; the byte size
-// rounded up to 16. Fills A.T, A.sinv and A.img_f4.
-size_t tail_layout(const Multigrid& M, TailArgs& A) {
-    int off = 0;  // floats
-    for (int l = M.tail; l < M.nlevels; l++) {
-        const int n = M.L[l].w * M.L[l].h;
+// The image's layout, in floats: the lower levels' seven arrays and the coarsest inverse (the part the tail copies to
+// shared memory, a multiple of 16 bytes), then the top level's five coefficient arrays. Every array has an even pitch
+// and an even number of rows. Fills A.T, A.sinv and A.img_f4; returns the image's size in floats.
+int tail_layout(const Multigrid& M, TailArgs& A) {
+    int off = 0;
+    for (int k = 1; k <= M.nlevels - M.tail; k++) {
+        const int l = k < M.nlevels - M.tail ? M.tail + k : M.tail;  // the top level last
+        if (l == M.tail) {
+            const int nc = M.L[M.nlevels - 1].w * M.L[M.nlevels - 1].h;
+            A.sinv = off;
+            off = (off + nc * nc + 3) & ~3;
+            A.img_f4 = off / 4;
+        }
         TailLevel& T = A.T[l];
         T.w = M.L[l].w;
         T.h = M.L[l].h;
-        T.c = off;
-        T.dx = off + n;
-        T.dy = off + 2 * n;
-        T.b = off + 3 * n;
-        T.x = off + 4 * n;
-        T.inv = off + 5 * n;
-        T.t = off + 6 * n;
-        off += 7 * n;
+        T.p = (T.w + 1) & ~1;
+        T.hp = (T.h + 1) & ~1;
+        const int n = T.p * T.hp;
+        T.dx = off;
+        T.dy = off + n;
+        T.inv = off + 2 * n;
+        T.t = off + 3 * n;
+        T.c = off + 4 * n;
+        T.b = off + 5 * n;
+        T.x = off + 6 * n;
+        off += (l == M.tail ? 5 : 7) * n;
     }
-    const int nc = M.L[M.nlevels - 1].w * M.L[M.nlevels - 1].h;
-    A.sinv = off;
-    off += nc * nc;
-    int moff = off * (int)sizeof(float);
-    for (int l = M.tail; l < M.nlevels; l++) {
-        A.T[l].m = moff;
-        moff += M.L[l].w * M.L[l].h;
-    }
-    const size_t bytes = ((size_t)moff + 15) & ~(size_t)15;
-    A.img_f4 = (int)(bytes / 16);
-    return bytes;
+    return off;
 }
 
-size_t tail_smem(const Multigrid& M) {
-    TailArgs A;
-    return tail_layout(M, A);
-}
+// The tail's shared memory at most: 32 x 32, 16 x 16, 8 x 8 and 4 x 4 levels of seven arrays, a 16 x 16 inverse, edges.
+constexpr size_t kTailSmem = 2 * sizeof(TailEdge) + (7 * (1024 + 256 + 64 + 16) + 256) * sizeof(float);
 
-// Everything the tail kernel and its packing need but the output slot.
+// Everything the tail kernel and its packing need but the output slot; returns the launch's shared memory.
 size_t tail_args(const Multigrid& M, TailArgs& T) {
-    const size_t bytes = tail_layout(M, T);
+    tail_layout(M, T);
     T.t = M.tail;
     T.nl = M.nlevels;
     T.pre = M.pre;
     T.post = M.post;
     T.omega = M.omega;
-    T.img = reinterpret_cast<const float4*>(M.tail_img);
+    T.img = M.tail_img;
     T.out = nullptr;
-    for (int l = 0; l < M.nlevels; l++) T.L[l] = M.L[l];
-    return bytes;
+    T.b = M.L[M.tail].b;
+    T.x2 = M.L[M.tail].x2;
+    return 2 * sizeof(TailEdge) + (size_t)T.img_f4 * 16;
 }
 
-// The tail's image for the next V-cycles (once per Newton pass, after the coarsening): each tail level's c, dx, dy,
-// inverse diagonal, weights and mask at their offsets, b and x at 0, the coarsest inverse, and the padding after the
-// masks at 0. Every byte of the image is written by exactly one thread.
-__global__ void mg_tail_pack_kernel(TailArgs A, const float* __restrict__ coarse_inv, float* img) {
-    unsigned char* bytes = reinterpret_cast<unsigned char*>(img);
+// The tail's image for the next V-cycles (once per Newton pass, after the coarsening): each level's couplings, inverse
+// diagonal, weights and c (0 on the padding), the lower levels' b and x at 0, and the coarsest inverse.
+__global__ void mg_tail_pack_kernel(const __grid_constant__ TailArgs A, const __grid_constant__ TailPack K,
+                                    const float* __restrict__ coarse_inv, float* img) {
     const int stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
     for (int l = A.t; l < A.nl; l++) {
-        const TailLevel T = A.T[l];
-        const MgLevel& L = A.L[l];
-        const int n = T.w * T.h;
-        for (int i = tid; i < n; i += stride) {
-            const int x = i % T.w, y = i / T.w;
-            const float c = L.c[i], dx = L.dx[i], dy = L.dy[i];
-            const float d = c + dx + dy + (x > 0 ? L.dx[i - 1] : 0.0f) + (y > 0 ? L.dy[i - T.w] : 0.0f);
-            const uint8_t m = L.mask[i];
-            img[T.c + i] = c;
-            img[T.dx + i] = dx;
-            img[T.dy + i] = dy;
-            img[T.b + i] = 0.0f;
-            img[T.x + i] = 0.0f;
-            img[T.inv + i] = m ? 1.0f / d : 0.0f;
-            img[T.t + i] = l + 1 < A.nl ? (L.t ? L.t[i] : 1.0f) : 0.0f;
-            bytes[T.m + i] = m;
+        const TailLevel& T = A.T[l];
+        const MgLevel& L = K.L[l - A.t];
+        for (int q = tid; q < T.p * T.hp; q += stride) {
+            const int x = q % T.p, y = q / T.p, i = y * T.w + x;
+            const bool ok = x < T.w && y < T.h;
+            float c = 1.0f, dx = 0.0f, dy = 0.0f, inv = 0.0f, t = 0.0f;
+            if (ok) {
+                c = L.c[i];
+                dx = L.dx[i];
+                dy = L.dy[i];
+                const float d = c + dx + dy + (x > 0 ? L.dx[i - 1] : 0.0f) + (y > 0 ? L.dy[i - T.w] : 0.0f);
+                if (L.mask[i]) {
+                    inv = 1.0f / d;
+                    t = l + 1 < A.nl ? (L.t ? L.t[i] : 1.0f) : 0.0f;
+                }
+            }
+            img[T.dx + q] = dx;
+            img[T.dy + q] = dy;
+            img[T.inv + q] = inv;
+            img[T.t + q] = t;
+            img[T.c + q] = c;
+            if (l > A.t) {
+                img[T.b + q] = 0.0f;
+                img[T.x + q] = 0.0f;
+            }
         }
     }
-    const TailLevel last = A.T[A.nl - 1];
+    const TailLevel& last = A.T[A.nl - 1];
     const int nc = last.w * last.h;
-    for (int k = tid; k < nc * nc; k += stride) img[A.sinv + k] = coarse_inv[k];
-    const int end = last.m + nc;
-    for (int k = end + tid; k < A.img_f4 * 16; k += stride) bytes[k] = 0;
+    for (int k = tid; k < 4 * A.img_f4 - A.sinv; k += stride) img[A.sinv + k] = k < nc * nc ? coarse_inv[k] : 0.0f;
 }
 
 template <int NS, bool PRE, int SX, int SY, int NT, bool VEC, bool WT>
@@ -1300,14 +1450,15 @@ void Multigrid::create(int w, int h, int pre_, int post_) {
         lh = (lh + 1) / 2;
     }
     tail = 0;
-    while ((size_t)L[tail].w * L[tail].h > (size_t)kMgTailCells) tail++;
-    size_t ts = tail_smem(*this);
-    SR_REQUIRE(ts <= 200 * 1024, "the coarse tail does not fit in shared memory");
-    SR_CUDA_TRY(cudaFuncSetAttribute(mg_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts));
+    while (L[tail].w > kMgTailSide || L[tail].h > kMgTailSide) tail++;
+    TailArgs layout;
+    const size_t img = (size_t)tail_layout(*this, layout);
+    SR_REQUIRE(nlevels - tail >= 3 && nlevels - tail <= kTailLevels, "the coarse tail's levels");
+    SR_CUDA_TRY(cudaFuncSetAttribute(mg_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
     const size_t nc = (size_t)L[nlevels - 1].w * L[nlevels - 1].h;
-    SR_REQUIRE(nc <= 64, "the coarsest level holds more than 64 cells");
+    SR_REQUIRE(nc <= 16, "the coarsest level holds more than 16 cells");
     SR_CUDA_TRY(cudaMalloc(&coarse_inv, sizeof(float) * nc * nc));
-    SR_CUDA_TRY(cudaMalloc(&tail_img, ts));
+    SR_CUDA_TRY(cudaMalloc(&tail_img, img * sizeof(float)));
     SR_CUDA_TRY(cudaMalloc(&err, sizeof(int)));
     SR_CUDA_TRY(cudaMemset(err, 0, sizeof(int)));
     for (int l = 0; l < nlevels; l++) L[l].err = err;
@@ -1430,7 +1581,9 @@ void Multigrid::coarsen(cudaStream_t s) {
     sr_note_launch();
     TailArgs T;
     tail_args(*this, T);
-    mg_tail_pack_kernel<<<8, 256, 0, s>>>(T, coarse_inv, tail_img);
+    TailPack K;
+    for (int l = tail; l < nlevels; l++) K.L[l - tail] = L[l];
+    mg_tail_pack_kernel<<<8, 256, 0, s>>>(T, K, coarse_inv, tail_img);
     sr_note_launch();
     if (!tuned) autotune(s);
 }

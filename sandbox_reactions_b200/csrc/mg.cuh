@@ -10,14 +10,14 @@
 // Restriction is P^T (r_c = sum t_j r_j), prolongation P (x_j += t_j x_c). Smoothing is red-black Gauss-Seidel
 // (global parity), V(pre, post), the post-smoother sweeping the colours in reverse so the cycle is symmetric. Big
 // levels run as tile kernels that do all of a smoother's half-sweeps in shared memory (temporal blocking: the tile's
-// halo is as deep as the half-sweeps); every level of at most kMgTailCells cells runs inside one CTA (the coarse tail,
-// the reference's mg_coarse), and the coarsest level (at most 4 x 4) is solved exactly by its inverse, built once per
+// halo is as deep as the half-sweeps); every level of at most kMgTailSide cells a side runs inside one CTA (the coarse
+// tail, the reference's mg_coarse), and the coarsest level (at most 4 x 4) is solved exactly by its inverse, built once per
 // Newton pass.
 #pragma once
 
 #include "common.cuh"
 
-constexpr int kMgTailCells = 4096;   // levels at most this large are solved inside one CTA
+constexpr int kMgTailSide = 64;      // levels at most this large on both axes are solved inside one CTA
 constexpr int kMgMaxLevels = 16;
 
 struct MgLevel {
@@ -42,9 +42,9 @@ struct Multigrid {
     int pre = 2, post = 2;
     float omega = 1.0f;  // coarse-correction weight
     MgLevel L[kMgMaxLevels];
-    float* coarse_inv = nullptr;  // the coarsest level's operator inverted (at most 64 x 64), per Newton pass
-    float* tail_img = nullptr;    // the coarse tail's shared-memory image (coefficients, inverse diagonals, weights,
-                                  // masks, the coarsest inverse), packed once per Newton pass
+    float* coarse_inv = nullptr;  // the coarsest level's operator inverted (at most 16 x 16), per Newton pass
+    float* tail_img = nullptr;    // the coarse tail's image (coefficients, inverse diagonals, weights, the coarsest
+                                  // inverse), packed once per Newton pass
     int* err = nullptr;           // the smoothers' error flag (MgLevel::err of every level)
 
     void create(int w, int h, int pre, int post);
