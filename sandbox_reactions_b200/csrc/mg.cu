@@ -38,11 +38,6 @@ struct TailArgs {
     TailLevel T[kMgMaxLevels];
 };
 
-constexpr int kTailLevels = 6;  // 64 x 64 down to 2 x 2
-struct TailPack {
-    MgLevel L[kTailLevels];  // the tail's levels, the top first
-};
-
 // Level 0's couplings to the +x / +y neighbours from the f64 faces, zero unless both cells are gas.
 __global__ void mg_couplings0_kernel(MgLevel L, const double* __restrict__ kx, const double* __restrict__ ky,
                                      const uint8_t* __restrict__ gas) {
@@ -790,61 +785,6 @@ __global__ void __launch_bounds__(RB_NT, 2)
     }
 }
 
-// The coarsest level's operator inverted by Gauss-Jordan elimination in f64 in one CTA (n <= 64 cells), masked-out
-// cells as identity rows; stored f32. The operator is SPD, so no pivoting is needed. The augmented matrix [A | I] is
-// kept twice and each elimination step reads one copy and writes the other, so a step is one pass and one barrier;
-// at step p only columns p .. n + p change (to the left the pivot row is already 0, to the right of n + p it is still
-// 0: untouched identity columns, the same in both copies).
-__global__ void mg_coarse_inverse_kernel(MgLevel C, float* inv) {
-    extern __shared__ double aug[];  // two n x 2n copies
-    const int w = C.w, h = C.h, n = w * h, m = 2 * n;
-    for (int k = threadIdx.x; k < n * m; k += blockDim.x) {
-        const int i = k / m, j = k % m;
-        double v = 0.0;
-        if (j >= n) {
-            v = (j - n == i) ? 1.0 : 0.0;
-        } else if (!C.mask[i]) {
-            v = (i == j) ? 1.0 : 0.0;
-        } else {
-            const int xi = i % w, yi = i / w;
-            const double dl = xi > 0 ? C.dx[i - 1] : 0.0, dr = C.dx[i];
-            const double du = yi > 0 ? C.dy[i - w] : 0.0, dd = C.dy[i];
-            if (j == i) v = (double)C.c[i] + dl + dr + du + dd;
-            else if (xi > 0 && j == i - 1) v = -dl;
-            else if (xi + 1 < w && j == i + 1) v = -dr;
-            else if (yi > 0 && j == i - w) v = -du;
-            else if (yi + 1 < h && j == i + w) v = -dd;
-        }
-        aug[k] = v;
-        aug[n * m + k] = v;
-    }
-    __syncthreads();
-    // threads as 64 rows x 16 column lanes: thread (i, c) updates row i's active columns p + c, p + c + 16, ...
-    // (n <= 64 rows; n + 1 <= 65 active columns), no index divisions in the loop; the thread that writes the next
-    // step's pivot also leaves its reciprocal for every thread to read
-    __shared__ double rpiv[2];
-    if (threadIdx.x == 0) rpiv[0] = 1.0 / aug[0];
-    __syncthreads();
-    const int i = threadIdx.x >> 4, c = threadIdx.x & 15;
-    for (int p = 0; p < n; p++) {
-        const double* src = aug + (p & 1) * n * m;
-        double* dst = aug + ((p + 1) & 1) * n * m;
-        if (i < n) {
-            const double rp = rpiv[p & 1];
-            const double aip = src[i * m + p];
-            for (int j = p + c; j <= n + p; j += 16) {
-                const double apj = src[p * m + j] * rp;
-                const double v = i == p ? apj : src[i * m + j] - aip * apj;
-                dst[i * m + j] = v;
-                if (i == p + 1 && j == p + 1) rpiv[(p + 1) & 1] = 1.0 / v;
-            }
-        }
-        __syncthreads();
-    }
-    const double* fin = aug + (n & 1) * n * m;
-    for (int k = threadIdx.x; k < n * n; k += blockDim.x) inv[k] = (float)fin[(k / n) * m + n + (k % n)];
-}
-
 // ---- the coarse tail: every level of at most 64 x 64 cells, inside one CTA
 //
 // What bounds it is latency: sixteen dependent half-sweeps a level under V(4,4), a few hundred cells each. So a level
@@ -1232,42 +1172,166 @@ size_t tail_args(const Multigrid& M, TailArgs& T) {
     return 2 * sizeof(TailEdge) + (size_t)T.img_f4 * 16;
 }
 
-// The tail's image for the next V-cycles (once per Newton pass, after the coarsening): each level's couplings, inverse
-// diagonal, weights and c (0 on the padding), the lower levels' b and x at 0, and the coarsest inverse.
-__global__ void mg_tail_pack_kernel(const __grid_constant__ TailArgs A, const __grid_constant__ TailPack K,
-                                    const float* __restrict__ coarse_inv, float* img) {
-    const int stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+// The tail's levels below its top, and its image for the next V-cycles, once per Newton pass: level by level in shared
+// memory, the weights (mg_coarsen_kernel's four half-sweeps and scaling; level 0 takes none), the Galerkin operator
+// (f64 sums) and the level's part of the image — couplings, inverse diagonal, weights and c, 0 (c: 1) on the padding, b
+// and x at 0 — then the coarsest operator's inverse. One CTA: the levels are a serial chain of a few thousand cells at
+// most, so launches and their ramps were what it cost (a coarsening a level, the inverse and the packing: 53 us for a
+// 64 x 64 top, in six launches; now one of 29 us).
+constexpr int TS_NT = 512, TS_P = kMgTailSide + 2, TS_N = TS_P * TS_P;  // a level with a rim of one cell around it
+
+
+struct TailSetupShared {
+    float c[2][TS_N], dx[2][TS_N], dy[2][TS_N], t[TS_N];  // this level and the next
+    uint8_t m[2][TS_N];
+    double aug[2][16 * 32];
+    double rpiv[2];
+};
+
+// The coarsest operator's inverse by Gauss-Jordan elimination in f64 (SPD: no pivoting; masked cells are identity rows),
+// one thread per element of [A | I]; the thread that writes the next pivot leaves its reciprocal. Stored f32.
+__device__ __forceinline__ void tail_inverse(TailSetupShared& S, int k, int w, int h, int p, float* inv, int room) {
+    const int n = w * h, i = threadIdx.x >> 5, j = threadIdx.x & 31;
+    if (i < n && j < 2 * n) {
+        double v = 0.0;
+        if (j >= n) {
+            v = j - n == i ? 1.0 : 0.0;
+        } else {
+            const int xi = i % w, yi = i / w, q = (yi + 1) * p + xi + 1;
+            if (!S.m[k][q]) {
+                v = i == j ? 1.0 : 0.0;
+            } else {
+                const double dl = S.dx[k][q - 1], dr = S.dx[k][q], du = S.dy[k][q - p], dd = S.dy[k][q];
+                if (j == i) v = (double)S.c[k][q] + dl + dr + du + dd;
+                else if (xi > 0 && j == i - 1) v = -dl;
+                else if (xi + 1 < w && j == i + 1) v = -dr;
+                else if (yi > 0 && j == i - w) v = -du;
+                else if (yi + 1 < h && j == i + w) v = -dd;
+            }
+        }
+        S.aug[0][i * 32 + j] = v;
+        if (i == 0 && j == 0) S.rpiv[0] = 1.0 / v;
+    }
+    __syncthreads();
+    for (int s = 0; s < n; s++) {
+        if (i < n && j < 2 * n) {
+            const double* src = S.aug[s & 1];
+            const double pj = src[s * 32 + j] * S.rpiv[s & 1];
+            const double v = i == s ? pj : src[i * 32 + j] - src[i * 32 + s] * pj;
+            S.aug[(s + 1) & 1][i * 32 + j] = v;
+            if (i == s + 1 && j == s + 1) S.rpiv[(s + 1) & 1] = 1.0 / v;
+        }
+        __syncthreads();
+    }
+    for (int e = threadIdx.x; e < room; e += TS_NT) inv[e] = e < n * n ? (float)S.aug[n & 1][(e / n) * 32 + n + e % n] : 0.0f;
+}
+
+__global__ void __launch_bounds__(TS_NT) mg_tail_setup_kernel(const __grid_constant__ TailArgs A, MgLevel top, float* img) {
+    extern __shared__ __align__(16) unsigned char setup_smem[];
+    TailSetupShared& S = *reinterpret_cast<TailSetupShared*>(setup_smem);
+    const int tid = threadIdx.x;
+    {
+        const int w = top.w, h = top.h, p = w + 2;
+        constexpr int PER = (TS_N + TS_NT - 1) / TS_NT;
+#pragma unroll
+        for (int u = 0; u < PER; u++) {
+            const int q = tid + u * TS_NT;
+            if (q >= p * (h + 2)) break;
+            const int x = q % p - 1, y = q / p - 1;
+            const bool in = x >= 0 && x < w && y >= 0 && y < h;
+            const int i = y * w + x;
+            S.c[0][q] = in ? top.c[i] : 1.0f;
+            S.dx[0][q] = in ? top.dx[i] : 0.0f;
+            S.dy[0][q] = in ? top.dy[i] : 0.0f;
+            S.m[0][q] = in ? top.mask[i] : 0;
+        }
+    }
     for (int l = A.t; l < A.nl; l++) {
         const TailLevel& T = A.T[l];
-        const MgLevel& L = K.L[l - A.t];
-        for (int q = tid; q < T.p * T.hp; q += stride) {
-            const int x = q % T.p, y = q / T.p, i = y * T.w + x;
-            const bool ok = x < T.w && y < T.h;
-            float c = 1.0f, dx = 0.0f, dy = 0.0f, inv = 0.0f, t = 0.0f;
-            if (ok) {
-                c = L.c[i];
-                dx = L.dx[i];
-                dy = L.dy[i];
-                const float d = c + dx + dy + (x > 0 ? L.dx[i - 1] : 0.0f) + (y > 0 ? L.dy[i - T.w] : 0.0f);
-                if (L.mask[i]) {
-                    inv = 1.0f / d;
-                    t = l + 1 < A.nl ? (L.t ? L.t[i] : 1.0f) : 0.0f;
+        const int k = (l - A.t) & 1, w = T.w, h = T.h, p = w + 2;
+        const float *c = S.c[k], *dx = S.dx[k], *dy = S.dy[k];
+        const uint8_t* m = S.m[k];
+        float* t = S.t;
+        __syncthreads();
+        for (int q = tid; q < p * (h + 2); q += TS_NT) t[q] = m[q] ? 1.0f : 0.0f;
+        __syncthreads();
+        const bool coarsest = l + 1 == A.nl;
+        if (l > 0 && !coarsest) {
+            const int half = (w + 1) / 2;
+            for (int sweep = 0; sweep < 4; sweep++) {
+                for (int e = tid; e < half * h; e += TS_NT) {
+                    const int y = e / half, x = 2 * (e - y * half) + ((y + sweep) & 1);
+                    if (x >= w) continue;
+                    // a masked cell has c = 1 and no couplings (nor do its neighbours towards it): it stays 0
+                    const int q = (y + 1) * p + x + 1;
+                    const float dl = dx[q - 1], dr = dx[q], du = dy[q - p], dd = dy[q];
+                    const float num = dl * t[q - 1] + dr * t[q + 1] + du * t[q - p] + dd * t[q + p];
+                    t[q] = num / (c[q] + dl + dr + du + dd);
                 }
+                __syncthreads();
             }
-            img[T.dx + q] = dx;
-            img[T.dy + q] = dy;
-            img[T.inv + q] = inv;
-            img[T.t + q] = t;
-            img[T.c + q] = c;
+        }
+        if (!coarsest) {
+            // each aggregate scaled to a largest weight of 1 (1 on its system cells where all weights vanished), then
+            // the Galerkin operator, whose couplings read the neighbouring aggregates' scaled weights
+            const TailLevel& C = A.T[l + 1];
+            const int cw = C.w, ch = C.h, cp = cw + 2;
+            for (int e = tid; e < cw * ch; e += TS_NT) {
+                const int Y = e / cw, X = e - Y * cw, q = (2 * Y + 1) * p + 2 * X + 1;
+                const bool x1 = 2 * X + 1 < w, y1 = 2 * Y + 1 < h;
+                const int at[4] = {q, x1 ? q + 1 : q, y1 ? q + p : q, x1 && y1 ? q + p + 1 : q};
+                float big = 0.0f;
+                for (int a = 0; a < 4; a++) big = fmaxf(big, t[at[a]]);
+                float v[4];
+                for (int a = 0; a < 4; a++) v[a] = !m[at[a]] ? 0.0f : (big > 1e-30f ? t[at[a]] / big : 1.0f);
+                for (int a = 3; a >= 0; a--) t[at[a]] = v[a];
+            }
+            __syncthreads();
+            for (int q = tid; q < cp * (ch + 2); q += TS_NT) {
+                const int X = q % cp - 1, Y = q / cp - 1;
+                float cc = 1.0f, dxc = 0.0f, dyc = 0.0f;
+                bool any = false;
+                if (X >= 0 && X < cw && Y >= 0 && Y < ch) {
+                    double csum = 0.0, sx = 0.0, sy = 0.0;
+                    for (int b = 0; b < 2; b++)
+                        for (int a = 0; a < 2; a++) {
+                            const int x = 2 * X + a, y = 2 * Y + b, j = (y + 1) * p + x + 1;
+                            if (x >= w || y >= h || !m[j]) continue;
+                            any = true;
+                            const double tj = t[j];
+                            csum += tj * ((double)c[j] * tj + (double)dx[j - 1] * (tj - t[j - 1]) +
+                                          (double)dx[j] * (tj - t[j + 1]) + (double)dy[j - p] * (tj - t[j - p]) +
+                                          (double)dy[j] * (tj - t[j + p]));
+                            if (a) sx += tj * t[j + 1] * dx[j];
+                            if (b) sy += tj * t[j + p] * dy[j];
+                        }
+                    if (any) {
+                        cc = (float)csum;
+                        dxc = (float)sx;
+                        dyc = (float)sy;
+                    }
+                }
+                S.c[1 - k][q] = cc;
+                S.dx[1 - k][q] = dxc;
+                S.dy[1 - k][q] = dyc;
+                S.m[1 - k][q] = any;
+            }
+        }
+        for (int q = tid; q < T.p * T.hp; q += TS_NT) {
+            const int x = q % T.p, y = q / T.p, j = (y + 1) * p + x + 1;
+            const bool ok = x < w && y < h;
+            img[T.dx + q] = ok ? dx[j] : 0.0f;
+            img[T.dy + q] = ok ? dy[j] : 0.0f;
+            img[T.inv + q] = ok && m[j] ? 1.0f / (c[j] + dx[j] + dy[j] + dx[j - 1] + dy[j - p]) : 0.0f;
+            img[T.t + q] = ok && !coarsest ? t[j] : 0.0f;
+            img[T.c + q] = ok ? c[j] : 1.0f;
             if (l > A.t) {
                 img[T.b + q] = 0.0f;
                 img[T.x + q] = 0.0f;
             }
         }
+        if (coarsest) tail_inverse(S, k, w, h, p, img + A.sinv, 4 * A.img_f4 - A.sinv);
     }
-    const TailLevel& last = A.T[A.nl - 1];
-    const int nc = last.w * last.h;
-    for (int k = tid; k < 4 * A.img_f4 - A.sinv; k += stride) img[A.sinv + k] = k < nc * nc ? coarse_inv[k] : 0.0f;
 }
 
 template <int NS, bool PRE, int SX, int SY, int NT, bool VEC, bool WT>
@@ -1433,17 +1497,6 @@ void Multigrid::create(int w, int h, int pre_, int post_) {
         MgLevel& L = this->L[nlevels];
         L.w = lw;
         L.h = lh;
-        const size_t n = (size_t)lw * lh;
-        SR_CUDA_TRY(cudaMalloc(&L.c, n * sizeof(float)));
-        SR_CUDA_TRY(cudaMalloc(&L.dx, n * sizeof(float)));
-        SR_CUDA_TRY(cudaMalloc(&L.dy, n * sizeof(float)));
-        SR_CUDA_TRY(cudaMalloc(&L.mask, n));
-        SR_CUDA_TRY(cudaMalloc(&L.x, n * sizeof(float)));
-        if (nlevels > 0) {
-            SR_CUDA_TRY(cudaMalloc(&L.t, n * sizeof(float)));
-            SR_CUDA_TRY(cudaMalloc(&L.b, n * sizeof(float)));
-            SR_CUDA_TRY(cudaMalloc(&L.x2, n * sizeof(float)));
-        }
         nlevels++;
         if ((lw <= 4 && lh <= 4) || nlevels == kMgMaxLevels) break;
         lw = (lw + 1) / 2;
@@ -1451,19 +1504,31 @@ void Multigrid::create(int w, int h, int pre_, int post_) {
     }
     tail = 0;
     while (L[tail].w > kMgTailSide || L[tail].h > kMgTailSide) tail++;
+    SR_REQUIRE(nlevels - tail >= 3 && (size_t)L[nlevels - 1].w * L[nlevels - 1].h <= 16, "the coarse tail's levels");
+    // the levels down to the tail's top; those below it live in the tail's image
+    for (int l = 0; l <= tail; l++) {
+        MgLevel& L = this->L[l];
+        const size_t n = (size_t)L.w * L.h;
+        SR_CUDA_TRY(cudaMalloc(&L.c, n * sizeof(float)));
+        SR_CUDA_TRY(cudaMalloc(&L.dx, n * sizeof(float)));
+        SR_CUDA_TRY(cudaMalloc(&L.dy, n * sizeof(float)));
+        SR_CUDA_TRY(cudaMalloc(&L.mask, n));
+        SR_CUDA_TRY(cudaMalloc(&L.x, n * sizeof(float)));
+        if (l > 0) {
+            SR_CUDA_TRY(cudaMalloc(&L.t, n * sizeof(float)));
+            SR_CUDA_TRY(cudaMalloc(&L.b, n * sizeof(float)));
+            SR_CUDA_TRY(cudaMalloc(&L.x2, n * sizeof(float)));
+        }
+    }
     TailArgs layout;
-    const size_t img = (size_t)tail_layout(*this, layout);
-    SR_REQUIRE(nlevels - tail >= 3 && nlevels - tail <= kTailLevels, "the coarse tail's levels");
-    SR_CUDA_TRY(cudaFuncSetAttribute(mg_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
-    const size_t nc = (size_t)L[nlevels - 1].w * L[nlevels - 1].h;
-    SR_REQUIRE(nc <= 16, "the coarsest level holds more than 16 cells");
-    SR_CUDA_TRY(cudaMalloc(&coarse_inv, sizeof(float) * nc * nc));
-    SR_CUDA_TRY(cudaMalloc(&tail_img, img * sizeof(float)));
+    SR_CUDA_TRY(cudaMalloc(&tail_img, (size_t)tail_layout(*this, layout) * sizeof(float)));
     SR_CUDA_TRY(cudaMalloc(&err, sizeof(int)));
     SR_CUDA_TRY(cudaMemset(err, 0, sizeof(int)));
     for (int l = 0; l < nlevels; l++) L[l].err = err;
-    SR_CUDA_TRY(cudaFuncSetAttribute(mg_coarse_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(2 * nc * 2 * nc * sizeof(double))));
+    // the same for every world: a world's creation leaves the launches of the others' tails as they were
+    SR_CUDA_TRY(cudaFuncSetAttribute(mg_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
+    SR_CUDA_TRY(cudaFuncSetAttribute(mg_tail_setup_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(TailSetupShared)));
     set_attributes_ns<2>();
     set_attributes_ns<4>();
     set_attributes_ns<6>();
@@ -1484,8 +1549,6 @@ void Multigrid::destroy() {
         }
         L[l] = MgLevel();
     }
-    cudaFree(coarse_inv);
-    coarse_inv = nullptr;
     cudaFree(tail_img);
     tail_img = nullptr;
     cudaFree(err);
@@ -1504,7 +1567,7 @@ bool Multigrid::error(cudaStream_t s) {
 
 size_t Multigrid::bytes() const {
     size_t s = 0;
-    for (int l = 0; l < nlevels; l++)
+    for (int l = 0; l <= tail; l++)
         s += (size_t)L[l].w * L[l].h * (l ? 7 * sizeof(float) + 1 : 4 * sizeof(float) + 1);
     return s;
 }
@@ -1566,7 +1629,7 @@ void Multigrid::autotune(cudaStream_t s) {
 }
 
 void Multigrid::coarsen(cudaStream_t s) {
-    for (int l = 1; l < nlevels; l++) {
+    for (int l = 1; l <= tail; l++) {
         if (l == 1) {
             mg_aggregate_kernel<<<grid_for((size_t)L[1].w * L[1].h), 256, 0, s>>>(L[0], L[1]);
         } else {
@@ -1575,15 +1638,9 @@ void Multigrid::coarsen(cudaStream_t s) {
         }
         sr_note_launch();
     }
-    const MgLevel& C = L[nlevels - 1];
-    const size_t nc = (size_t)C.w * C.h;
-    mg_coarse_inverse_kernel<<<1, 1024, 2 * nc * 2 * nc * sizeof(double), s>>>(C, coarse_inv);
-    sr_note_launch();
     TailArgs T;
     tail_args(*this, T);
-    TailPack K;
-    for (int l = tail; l < nlevels; l++) K.L[l - tail] = L[l];
-    mg_tail_pack_kernel<<<8, 256, 0, s>>>(T, K, coarse_inv, tail_img);
+    mg_tail_setup_kernel<<<1, TS_NT, sizeof(TailSetupShared), s>>>(T, L[tail], tail_img);
     sr_note_launch();
     if (!tuned) autotune(s);
 }

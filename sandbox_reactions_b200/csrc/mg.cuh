@@ -42,9 +42,8 @@ struct Multigrid {
     int pre = 2, post = 2;
     float omega = 1.0f;  // coarse-correction weight
     MgLevel L[kMgMaxLevels];
-    float* coarse_inv = nullptr;  // the coarsest level's operator inverted (at most 16 x 16), per Newton pass
     float* tail_img = nullptr;    // the coarse tail's image (coefficients, inverse diagonals, weights, the coarsest
-                                  // inverse), packed once per Newton pass
+                                  // inverse), built once per Newton pass
     int* err = nullptr;           // the smoothers' error flag (MgLevel::err of every level)
 
     void create(int w, int h, int pre, int post);
