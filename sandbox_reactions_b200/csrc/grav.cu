@@ -10,9 +10,13 @@
 //   3. inverse rows: two output rows packed through Hermitian symmetry into one complex inverse FFT, the world's
 //      columns and the ring columns kept;
 //   4. gradient: φ and g = -∇φ.
-// The FFT is a Stockham autosort over radix-16 stages (a radix-2/4/8 stage last when log2 N is not a multiple of 4),
-// each thread holding 16 points in registers between shared-memory exchanges; inter-stage twiddles come from a table
-// built in f64 on the host.
+// The FFT is a Stockham autosort over radix-16 stages and one radix-2/4/8 stage when log2 N is not a multiple of 4 (last
+// in a forward transform, first in an inverse one), each thread holding 16 points in registers. A transform's first
+// stage takes its points straight from global memory and its last leaves them in natural order in registers, so the
+// column pass multiplies by K̂ between the forward's last and the inverse's first stage without leaving registers, and
+// shared memory only carries the exchanges between stages: 4 of them for a 4096-point column, where staging every
+// stage through shared memory took 16 passes over it. Stage twiddles come from a table built in f64 on the host, laid
+// out so that neighbouring threads read neighbouring entries.
 #include <math.h>
 
 #include <functional>
@@ -26,15 +30,6 @@
 
 namespace {
 
-__device__ __constant__ float kCos16[16] = {1.0f, 9.238795325e-01f, 7.071067812e-01f, 3.826834324e-01f, 0.0f,
-                                             -3.826834324e-01f, -7.071067812e-01f, -9.238795325e-01f, -1.0f,
-                                             -9.238795325e-01f, -7.071067812e-01f, -3.826834324e-01f, 0.0f,
-                                             3.826834324e-01f, 7.071067812e-01f, 9.238795325e-01f};
-__device__ __constant__ float kSin16[16] = {0.0f, 3.826834324e-01f, 7.071067812e-01f, 9.238795325e-01f, 1.0f,
-                                             9.238795325e-01f, 7.071067812e-01f, 3.826834324e-01f, 0.0f,
-                                             -3.826834324e-01f, -7.071067812e-01f, -9.238795325e-01f, -1.0f,
-                                             -9.238795325e-01f, -7.071067812e-01f, -3.826834324e-01f};
-
 // Shared-memory FFT buffers hold one float2 of padding after every 16 points: the radix-16 stages' scattered writes
 // (stride Ns·16 elements in the first stage) and strided reads then fall on different banks.
 __device__ __forceinline__ int fpad(int i) { return i + (i >> 4); }
@@ -45,6 +40,15 @@ constexpr int fft_len() {
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
+// e^{-2πi m/16} for 0 < m < 8, m != 4
+__host__ __device__ constexpr float cos16(int m) {
+    return m == 1 ? 9.238795325e-01f : m == 2 ? 7.071067812e-01f : m == 3 ? 3.826834324e-01f
+         : m == 5 ? -3.826834324e-01f : m == 6 ? -7.071067812e-01f : -9.238795325e-01f;
+}
+__host__ __device__ constexpr float sin16(int m) {
+    return m == 1 || m == 7 ? 3.826834324e-01f : m == 2 || m == 6 ? 7.071067812e-01f : 9.238795325e-01f;
 }
 
 // In-register DFT of R (<= 16) points, natural order in and out, by recursive decimation in time. Forward uses
@@ -63,8 +67,10 @@ struct Dft {
 #pragma unroll
         for (int k = 0; k < R / 2; k++) {
             const int m = k * (16 / R);
-            float2 wk = make_float2(kCos16[m], INV ? kSin16[m] : -kSin16[m]);
-            float2 t = k == 0 ? o[k] : cmul(o[k], wk);
+            float2 t;
+            if (m == 0) t = o[k];
+            else if (m == 4) t = INV ? make_float2(-o[k].y, o[k].x) : make_float2(o[k].y, -o[k].x);
+            else t = cmul(o[k], make_float2(cos16(m), INV ? sin16(m) : -sin16(m)));
             v[k] = make_float2(e[k].x + t.x, e[k].y + t.y);
             v[k + R / 2] = make_float2(e[k].x - t.x, e[k].y - t.y);
         }
@@ -75,203 +81,264 @@ struct Dft<1, INV> {
     __device__ __forceinline__ static void run(float2*) {}
 };
 
-// One Stockham stage of radix R over an N-point sequence in shared memory, in place: every participating thread
-// reads its butterflies' inputs into registers, the CTA synchronises, then every thread writes its outputs.
-// `t` in [0, N/16) is the thread's index within this FFT; each thread owns N/(16 R) ... (16/R) butterflies so that it
-// always holds 16 points.
-template <int N, int R, bool INV>
-__device__ __forceinline__ void stockham_stage(float2* buf, const float2* __restrict__ tw, int t, int Ns, bool active) {
-    constexpr int B = 16 / R;  // butterflies per thread
-    float2 v[B][R];
-    if (active) {
-#pragma unroll
-        for (int b = 0; b < B; b++) {
-            const int j = t + b * (N / 16);
-            const int k = j % Ns;
-#pragma unroll
-            for (int r = 0; r < R; r++) v[b][r] = buf[fpad(j + r * (N / R))];
-            if (Ns > 1) {
-                const int step = N / (Ns * R);
-#pragma unroll
-                for (int r = 1; r < R; r++) {
-                    float2 wv = tw[(r * k * step) & (N - 1)];
-                    if (INV) wv.y = -wv.y;
-                    v[b][r] = cmul(v[b][r], wv);
-                }
-            }
-            Dft<R, INV>::run(v[b]);
-        }
+// The stages of an N-point transform: their radices, the product Ns of the radices before each, and where each one's
+// twiddles (R x Ns entries, e^{-2πi r k/(Ns R)} at r Ns + k) begin in the axis's table, the forward's before the
+// inverse's. Evaluated by the kernels at compile time and by the host when it builds the table.
+struct FftPlan {
+    int full, rest, stages;
+    __host__ __device__ constexpr explicit FftPlan(int n) : full(0), rest(1), stages(0) {
+        int l = 0;
+        while ((1 << l) < n) l++;
+        full = l / 4;
+        rest = 1 << (l % 4);
+        stages = full + (rest > 1 ? 1 : 0);
     }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-        for (int b = 0; b < B; b++) {
-            const int j = t + b * (N / 16);
-            const int k = j % Ns;
-            const int base = (j / Ns) * Ns * R + k;
-#pragma unroll
-            for (int r = 0; r < R; r++) buf[fpad(base + r * Ns)] = v[b][r];
-        }
+    __host__ __device__ constexpr int radix(bool inv, int s) const {
+        return rest == 1 ? 16 : (s == (inv ? 0 : full) ? rest : 16);
     }
-    __syncthreads();
-}
-
-template <int N>
-struct Log2 {
-    static constexpr int value = 1 + Log2<N / 2>::value;
+    __host__ __device__ constexpr int ns(bool inv, int s) const {
+        int p = 1;
+        for (int q = 0; q < s; q++) p *= radix(inv, q);
+        return p;
+    }
+    __host__ __device__ constexpr int offset(bool inv, int s) const {
+        int o = 0;
+        for (int q = 1; q < (inv ? stages : s); q++) o += radix(false, q) * ns(false, q);
+        if (inv)
+            for (int q = 1; q < s; q++) o += radix(true, q) * ns(true, q);
+        return o;
+    }
+    __host__ __device__ constexpr int entries() const { return offset(true, stages); }
 };
-template <>
-struct Log2<1> {
-    static constexpr int value = 0;
-};
-
-// A full N-point FFT in shared memory by N/16 threads (`t` their index; `active` false for spare threads, which still
-// take every barrier).
-template <int N, bool INV>
-__device__ __forceinline__ void fft_smem(float2* buf, const float2* __restrict__ tw, int t, bool active) {
-    constexpr int L = Log2<N>::value;
-    constexpr int full = L / 4, rest = L % 4;
-    int Ns = 1;
-#pragma unroll
-    for (int s = 0; s < full; s++) {
-        stockham_stage<N, 16, INV>(buf, tw, t, Ns, active);
-        Ns *= 16;
-    }
-    if (rest == 1) stockham_stage<N, 2, INV>(buf, tw, t, Ns, active);
-    if (rest == 2) stockham_stage<N, 4, INV>(buf, tw, t, Ns, active);
-    if (rest == 3) stockham_stage<N, 8, INV>(buf, tw, t, Ns, active);
-}
 
 template <int N>
 constexpr int fft_threads() {
-    return N / 16 < 32 ? 32 : N / 16;
+    return N / 16;
 }
 
-// ---- pass 1: two real rows per complex FFT, two FFTs per CTA (four rows)
+// A barrier of one transform's threads: a warp's (or less) in lockstep, or `N / 16` threads on barrier `bar`.
 template <int N>
-__global__ void __launch_bounds__(2 * fft_threads<N>()) grav_rows_kernel(GravArgs A) {
-    extern __shared__ float2 sm[];
-    constexpr int T = fft_threads<N>();
-    const int f = threadIdx.x / T, t = threadIdx.x % T;
-    float2* buf = sm + f * fft_len<N>();
-    const int ya = blockIdx.x * 4 + 2 * f, yb = ya + 1;
-    const int w = A.w, h = A.h;
-    const float sv = A.sigma_vac;
-    for (int x = t; x < N; x += T) {
-        float a = 0.0f, b = 0.0f;
-        if (x < w) {
-            if (ya < h) {
-                float s = A.src[(size_t)ya * w + x];
-                a = s >= sv ? s : 0.0f;
-            }
-            if (yb < h) {
-                float s = A.src[(size_t)yb * w + x];
-                b = s >= sv ? s : 0.0f;
+__device__ __forceinline__ void fft_sync(int bar) {
+    if constexpr (N / 16 <= 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(N / 16) : "memory");
+}
+
+// The points of stage S's butterflies of thread t: v[b R + r] = x[j + r N/R], j = t + b N/16.
+template <int N, bool INV, int S>
+__device__ __forceinline__ void fft_gather(float2 (&v)[16], const float2* buf, int t) {
+    constexpr int R = FftPlan(N).radix(INV, S);
+#pragma unroll
+    for (int b = 0; b < 16 / R; b++)
+#pragma unroll
+        for (int r = 0; r < R; r++) v[b * R + r] = buf[fpad(t + b * (N / 16) + r * (N / R))];
+}
+
+// Stages S and on of an N-point transform by its N/16 threads, `v` gathered for stage S on entry; on return v holds
+// the last stage's outputs, X[j + r N/R] at b R + r, in natural order. `buf` is free to be written on entry.
+template <int N, bool INV, int S>
+__device__ __forceinline__ void fft_stages(float2 (&v)[16], float2* buf, const float2* __restrict__ tw, int t, int bar) {
+    constexpr FftPlan P(N);
+    constexpr int R = P.radix(INV, S), Ns = P.ns(INV, S);
+    if constexpr (S > 0) {
+        constexpr int OFF = P.offset(INV, S);
+        const float2* w = tw + OFF;
+#pragma unroll
+        for (int b = 0; b < 16 / R; b++) {
+            const int k = (t + b * (N / 16)) & (Ns - 1);
+#pragma unroll
+            for (int r = 1; r < R; r++) {
+                float2 wv = __ldg(w + r * Ns + k);
+                if (INV) wv.y = -wv.y;
+                v[b * R + r] = cmul(v[b * R + r], wv);
             }
         }
-        buf[fpad(x)] = make_float2(a, b);
     }
-    __syncthreads();
-    fft_smem<N, false>(buf, A.tw_x, t, t < N / 16);
-    // unpack: X_a[k] = (Z[k] + conj Z[N-k]) / 2, X_b[k] = (Z[k] - conj Z[N-k]) / 2i, k = 0..N/2; column-major out
-    const size_t ld = A.ld;
-    for (int k = t; k <= N / 2; k += T) {
-        float2 z = buf[fpad(k)], zc = buf[fpad((N - k) & (N - 1))];
-        float2 xa = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
-        float2 xb = make_float2(0.5f * (z.y + zc.y), 0.5f * (zc.x - z.x));
-        if (ya < h) A.spec[(size_t)k * ld + 1 + ya] = xa;
-        if (yb < h) A.spec[(size_t)k * ld + 1 + yb] = xb;
+#pragma unroll
+    for (int b = 0; b < 16 / R; b++) Dft<R, INV>::run(v + b * R);
+    if constexpr (S + 1 < P.stages) {
+#pragma unroll
+        for (int b = 0; b < 16 / R; b++) {
+            const int j = t + b * (N / 16), k = j & (Ns - 1), base = (j - k) * R + k;
+#pragma unroll
+            for (int r = 0; r < R; r++) buf[fpad(base + r * Ns)] = v[b * R + r];
+        }
+        fft_sync<N>(bar);
+        fft_gather<N, INV, S + 1>(v, buf, t);
+        fft_sync<N>(bar);
+        fft_stages<N, INV, S + 1>(v, buf, tw, t, bar);
     }
 }
 
-// ---- pass 2: one spectrum column per CTA: forward, × K̂, inverse, rows -1..h kept
+// ---- pass 1: two real rows per complex FFT, two FFTs per CTA (four rows: 32-byte runs of the column-major spectrum),
+// or as many as fill a warp
 template <int N>
-__global__ void __launch_bounds__(fft_threads<N>()) grav_columns_kernel(GravArgs A) {
+constexpr int rows_group() {
+    return fft_threads<N>() < 16 ? 32 / fft_threads<N>() : 2;
+}
+
+template <int N>
+__global__ void __launch_bounds__(rows_group<N>() * fft_threads<N>()) grav_rows_kernel(GravArgs A) {
     extern __shared__ float2 sm[];
-    constexpr int T = fft_threads<N>();
-    const int t = threadIdx.x;
-    const int kx = blockIdx.x;
+    constexpr int T = fft_threads<N>(), G = rows_group<N>();
+    const int f = threadIdx.x / T, t = threadIdx.x % T;
+    const int w = A.w, h = A.h, y0 = blockIdx.x * 2 * G;
+    const float sv = A.sigma_vac;
+    float2* buf = sm + f * fft_len<N>();
+    {
+        const int ya = y0 + 2 * f;
+        const float* ra = A.src + (size_t)ya * w;
+        float2 v[16];
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+            const int x = t + r * T;
+            float a = 0.0f, b = 0.0f;
+            if (x < w) {
+                if (ya < h) a = ra[x];
+                if (ya + 1 < h) b = ra[w + x];
+            }
+            v[r] = make_float2(a >= sv ? a : 0.0f, b >= sv ? b : 0.0f);
+        }
+        fft_stages<N, false, 0>(v, buf, A.tw_x, t, 1 + f);
+        constexpr int R = FftPlan(N).radix(false, FftPlan(N).stages - 1);
+#pragma unroll
+        for (int b = 0; b < 16 / R; b++)
+#pragma unroll
+            for (int r = 0; r < R; r++) buf[fpad(t + b * T + r * (N / R))] = v[b * R + r];
+    }
+    __syncthreads();
+    // unpack: X_a[k] = (Z[k] + conj Z[N-k]) / 2, X_b[k] = (Z[k] - conj Z[N-k]) / 2i, k = 0..N/2; column-major out, the
+    // CTA's rows of a column by neighbouring threads
+    const size_t ld = A.ld;
+    for (int e = threadIdx.x; e < 2 * G * (N / 2 + 1); e += G * T) {
+        const int q = e % (2 * G), k = e / (2 * G);
+        if (y0 + q >= h) continue;
+        const float2* bq = sm + (q >> 1) * fft_len<N>();
+        const float2 z = bq[fpad(k)], zc = bq[fpad((N - k) & (N - 1))];
+        A.spec[(size_t)k * ld + y0 + q] = q & 1 ? make_float2(0.5f * (z.y + zc.y), 0.5f * (zc.x - z.x))
+                                                : make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));
+    }
+}
+
+// ---- pass 2: spectrum columns, one per N/16 threads: forward, × K̂, inverse, rows -1..h kept
+template <int N>
+constexpr int column_group() {
+    return fft_threads<N>() < 32 ? 32 / fft_threads<N>() : 1;
+}
+
+template <int N>
+__global__ void __launch_bounds__(column_group<N>() * fft_threads<N>(), N == 4096 ? 3 : 1) grav_columns_kernel(GravArgs A) {
+    extern __shared__ float2 sm[];
+    constexpr int T = fft_threads<N>(), G = column_group<N>();
+    constexpr FftPlan P(N);
+    constexpr int R = P.radix(true, 0);
+    const int f = threadIdx.x / T, t = threadIdx.x % T;
+    const int kx = blockIdx.x * G + f;
+    const bool on = G == 1 || kx <= A.px / 2;
     const int h = A.h;
-    const size_t ld = A.ld;
-    float2* col = A.spec + (size_t)kx * ld;
-    for (int y = t; y < N; y += T) sm[fpad(y)] = y < h ? col[1 + y] : make_float2(0.0f, 0.0f);
-    __syncthreads();
-    fft_smem<N, false>(sm, A.tw_y, t, t < N / 16);
-    const float* kq = A.khat + (size_t)kx * (N / 2 + 1);
-    for (int ky = t; ky < N; ky += T) {
-        float k = kq[ky <= N / 2 ? ky : N - ky];
-        float2 z = sm[fpad(ky)];
-        sm[fpad(ky)] = make_float2(z.x * k, z.y * k);
+    float2* buf = sm + f * fft_len<N>();
+    float2* col = A.spec + (size_t)(on ? kx : 0) * A.ld;
+    float2 v[16];
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+        const int y = t + r * T;
+        v[r] = on && y < h ? col[y] : make_float2(0.0f, 0.0f);
     }
-    __syncthreads();
-    fft_smem<N, true>(sm, A.tw_y, t, t < N / 16);
-    for (int r = t; r < h + 2; r += T) col[r] = sm[fpad((r - 1 + N) & (N - 1))];
+    fft_stages<N, false, 0>(v, buf, A.tw_y, t, 0);
+    const float* kq = A.khat + (size_t)(on ? kx : 0) * (N / 2 + 1);
+#pragma unroll
+    for (int b = 0; b < 16 / R; b++)
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int ky = t + b * T + r * (N / R);
+            const float k = kq[ky <= N / 2 ? ky : N - ky];
+            v[b * R + r].x *= k;
+            v[b * R + r].y *= k;
+        }
+    fft_stages<N, true, 0>(v, buf, A.tw_y, t, 0);
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+        const int row = (t + r * T + 1) & (N - 1);  // the world's row y at y + 1, row -1 (the last point) at 0
+        if (on && row < h + 2) col[row] = v[r];
+    }
 }
 
-// ---- pass 3: two output rows per complex inverse FFT, two FFTs per CTA; columns -1..w kept into φ_ring
+// ---- pass 3: two output rows per complex inverse FFT, grouped as in pass 1; columns -1..w kept into φ_ring
 template <int N>
-__global__ void __launch_bounds__(2 * fft_threads<N>()) grav_rows_inverse_kernel(GravArgs A) {
+__global__ void __launch_bounds__(rows_group<N>() * fft_threads<N>()) grav_rows_inverse_kernel(GravArgs A) {
     extern __shared__ float2 sm[];
-    constexpr int T = fft_threads<N>();
+    constexpr int T = fft_threads<N>(), G = rows_group<N>();
+    const int rows = A.h + 2, r0 = blockIdx.x * 2 * G;  // rows is even (the world's height is)
+    const size_t ld = A.ld;
+    for (int e = threadIdx.x; e < G * (N / 2 + 1); e += G * T) {
+        const int f = e % G, k = e / G, ra = r0 + 2 * f;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);  // X_a[k], X_b[k]
+        if (ra < rows) x = *reinterpret_cast<const float4*>(A.spec + (size_t)k * ld + ra);
+        // Z[k] = X_a[k] + i X_b[k]; Z[N-k] = conj X_a[k] + i conj X_b[k]
+        float2* buf = sm + f * fft_len<N>();
+        buf[fpad(k)] = make_float2(x.x - x.w, x.y + x.z);
+        if (k > 0 && k < N / 2) buf[fpad(N - k)] = make_float2(x.x + x.w, x.z - x.y);
+    }
+    __syncthreads();
     const int f = threadIdx.x / T, t = threadIdx.x % T;
     float2* buf = sm + f * fft_len<N>();
-    const int rows = A.h + 2;
-    const int ra = blockIdx.x * 4 + 2 * f, rb = ra + 1;
-    const size_t ld = A.ld;
-    for (int k = t; k <= N / 2; k += T) {
-        float2 xa = ra < rows ? A.spec[(size_t)k * ld + ra] : make_float2(0.0f, 0.0f);
-        float2 xb = rb < rows ? A.spec[(size_t)k * ld + rb] : make_float2(0.0f, 0.0f);
-        // Z[k] = X_a[k] + i X_b[k]; Z[N-k] = conj X_a[k] + i conj X_b[k]
-        buf[fpad(k)] = make_float2(xa.x - xb.y, xa.y + xb.x);
-        if (k > 0 && k < N / 2) buf[fpad(N - k)] = make_float2(xa.x + xb.y, xb.x - xa.y);
-    }
-    __syncthreads();
-    fft_smem<N, true>(buf, A.tw_x, t, t < N / 16);
-    const int w = A.w, rw = w + 2;
-    for (int c = t; c < rw; c += T) {
-        float2 z = buf[fpad((c - 1 + N) & (N - 1))];
-        if (ra < rows) A.phi_ring[(size_t)ra * rw + c] = z.x;
-        if (rb < rows) A.phi_ring[(size_t)rb * rw + c] = z.y;
+    float2 v[16];
+    fft_gather<N, true, 0>(v, buf, t);
+    fft_sync<N>(1 + f);
+    fft_stages<N, true, 0>(v, buf, A.tw_x, t, 1 + f);
+    const int rw = A.w + 2, ra = r0 + 2 * f;
+    if (ra >= rows) return;
+    float* ring = A.phi_ring + (size_t)ra * A.rp + kRingPad;
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+        const int c = (t + r * T + 1) & (N - 1);
+        if (c < rw) {
+            ring[c] = v[r].x;
+            ring[A.rp + c] = v[r].y;
+        }
     }
 }
 
-// ---- pass 4: φ and g = -∇φ by central differences over the ringed potential (grav.rs:55-70)
+// ---- pass 4: φ and g = -∇φ by central differences over the ringed potential (grav.rs:55-70), four cells a thread (the
+// world's width is a multiple of 8 and the ring's rows are padded so that its cells lie on 16-byte boundaries)
 __global__ void grav_gradient_kernel(GravArgs A) {
-    const int w = A.w, h = A.h, rw = w + 2;
-    const size_t n = (size_t)w * h;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const int w = A.w, h = A.h, rp = A.rp;
+    const int n4 = w * h / 4;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += gridDim.x * blockDim.x) {
         int x, y;
-        split_index(i, w, x, y);
-        const float* r0 = A.phi_ring + (size_t)y * rw;
-        const float* r1 = r0 + rw;
-        const float* r2 = r1 + rw;
-        A.gx[i] = -(r1[x + 2] - r1[x]) / 2.0f;
-        A.gy[i] = -(r2[x + 1] - r0[x + 1]) / 2.0f;
-        A.phi[i] = r1[x + 1];
+        split_index((size_t)q * 4, w, x, y);
+        const float* r1 = A.phi_ring + (size_t)(y + 1) * rp + kRingPad + 1 + x;
+        const float4 c = *reinterpret_cast<const float4*>(r1);
+        const float l = r1[-1], r = r1[4];
+        const float4 u = *reinterpret_cast<const float4*>(r1 - rp), d = *reinterpret_cast<const float4*>(r1 + rp);
+        reinterpret_cast<float4*>(A.gx)[q] = make_float4(-(c.y - l) / 2.0f, -(c.z - c.x) / 2.0f, -(c.w - c.y) / 2.0f,
+                                                         -(r - c.z) / 2.0f);
+        reinterpret_cast<float4*>(A.gy)[q] = make_float4(-(d.x - u.x) / 2.0f, -(d.y - u.y) / 2.0f, -(d.z - u.z) / 2.0f,
+                                                         -(d.w - u.w) / 2.0f);
+        reinterpret_cast<float4*>(A.phi)[q] = c;
     }
 }
 
 template <int N>
 void launch_rows(const GravArgs& A, cudaStream_t s) {
-    size_t smem = 2 * fft_len<N>() * sizeof(float2);
+    size_t smem = rows_group<N>() * fft_len<N>() * sizeof(float2);
     cudaFuncSetAttribute(grav_rows_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    grav_rows_kernel<N><<<div_up(A.h, 4), 2 * fft_threads<N>(), smem, s>>>(A);
+    grav_rows_kernel<N><<<div_up(A.h, 2 * rows_group<N>()), rows_group<N>() * fft_threads<N>(), smem, s>>>(A);
     sr_note_launch();
 }
 
 template <int N>
 void launch_columns(const GravArgs& A, cudaStream_t s) {
-    size_t smem = fft_len<N>() * sizeof(float2);
+    size_t smem = column_group<N>() * fft_len<N>() * sizeof(float2);
     cudaFuncSetAttribute(grav_columns_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    grav_columns_kernel<N><<<A.px / 2 + 1, fft_threads<N>(), smem, s>>>(A);
+    grav_columns_kernel<N><<<div_up(A.px / 2 + 1, column_group<N>()), column_group<N>() * fft_threads<N>(), smem, s>>>(A);
     sr_note_launch();
 }
 
 template <int N>
 void launch_rows_inverse(const GravArgs& A, cudaStream_t s) {
-    size_t smem = 2 * fft_len<N>() * sizeof(float2);
+    size_t smem = rows_group<N>() * fft_len<N>() * sizeof(float2);
     cudaFuncSetAttribute(grav_rows_inverse_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    grav_rows_inverse_kernel<N><<<div_up(A.h + 2, 4), 2 * fft_threads<N>(), smem, s>>>(A);
+    grav_rows_inverse_kernel<N><<<div_up(A.h + 2, 2 * rows_group<N>()), rows_group<N>() * fft_threads<N>(), smem, s>>>(A);
     sr_note_launch();
 }
 
@@ -389,15 +456,6 @@ const std::vector<float>& khat_quarter(int px, int py, int kind, double G, doubl
     return g_khat_cache.emplace(key, std::move(q)).first->second;
 }
 
-std::vector<float2> twiddle_table(int n) {
-    std::vector<float2> t(n);
-    for (int k = 0; k < n; k++) {
-        double a = -2.0 * M_PI * (double)k / (double)n;
-        t[k] = make_float2((float)cos(a), (float)sin(a));
-    }
-    return t;
-}
-
 }  // namespace
 
 int grav_padded_size(int len) {
@@ -409,6 +467,21 @@ int grav_padded_size(int len) {
     return n > 8192 ? 0 : n;
 }
 
+size_t grav_twiddle_count(int n) { return (size_t)FftPlan(n).entries(); }
+
+void grav_twiddles(int n, float2* out) {
+    const FftPlan P(n);
+    for (int inv = 0; inv < 2; inv++)
+        for (int s = 1; s < P.stages; s++) {
+            const int R = P.radix(inv != 0, s), Ns = P.ns(inv != 0, s);
+            for (int r = 0; r < R; r++)
+                for (int k = 0; k < Ns; k++) {
+                    const double a = -2.0 * M_PI * (double)r * (double)k / ((double)Ns * R);
+                    out[P.offset(inv != 0, s) + r * Ns + k] = make_float2((float)cos(a), (float)sin(a));
+                }
+        }
+}
+
 void GravPlan::create(int w_, int h_, int kernel, double G, double eps, float sigma_vac_) {
     w = w_;
     h = h_;
@@ -416,17 +489,19 @@ void GravPlan::create(int w_, int h_, int kernel, double G, double eps, float si
     py = grav_padded_size(h);
     SR_REQUIRE(px && py, "a world axis pads past the FFT's 8192 points");
     sigma_vac = sigma_vac_;
-    ld = (size_t)h + 2;
+    ld = grav_column_stride(h);
     SR_CUDA_TRY(cudaMalloc(&spec, sizeof(float2) * (size_t)(px / 2 + 1) * ld));
-    SR_CUDA_TRY(cudaMalloc(&phi_ring, sizeof(float) * (size_t)(w + 2) * (h + 2)));
+    SR_CUDA_TRY(cudaMalloc(&phi_ring, sizeof(float) * (size_t)grav_ring_stride(w) * (h + 2)));
     const std::vector<float>& q = khat_quarter(px, py, kernel, G, eps);
     SR_CUDA_TRY(cudaMalloc(&khat, sizeof(float) * q.size()));
     SR_CUDA_TRY(cudaMemcpy(khat, q.data(), sizeof(float) * q.size(), cudaMemcpyHostToDevice));
-    std::vector<float2> tx = twiddle_table(px), ty = twiddle_table(py);
-    SR_CUDA_TRY(cudaMalloc(&tw_x, sizeof(float2) * px));
-    SR_CUDA_TRY(cudaMalloc(&tw_y, sizeof(float2) * py));
-    SR_CUDA_TRY(cudaMemcpy(tw_x, tx.data(), sizeof(float2) * px, cudaMemcpyHostToDevice));
-    SR_CUDA_TRY(cudaMemcpy(tw_y, ty.data(), sizeof(float2) * py, cudaMemcpyHostToDevice));
+    std::vector<float2> tx(grav_twiddle_count(px)), ty(grav_twiddle_count(py));
+    grav_twiddles(px, tx.data());
+    grav_twiddles(py, ty.data());
+    SR_CUDA_TRY(cudaMalloc(&tw_x, sizeof(float2) * tx.size()));
+    SR_CUDA_TRY(cudaMalloc(&tw_y, sizeof(float2) * ty.size()));
+    SR_CUDA_TRY(cudaMemcpy(tw_x, tx.data(), sizeof(float2) * tx.size(), cudaMemcpyHostToDevice));
+    SR_CUDA_TRY(cudaMemcpy(tw_y, ty.data(), sizeof(float2) * ty.size(), cudaMemcpyHostToDevice));
 }
 
 void GravPlan::destroy() {
@@ -442,8 +517,9 @@ void GravPlan::destroy() {
 }
 
 size_t GravPlan::bytes() const {
-    return sizeof(float2) * (size_t)(px / 2 + 1) * ld + sizeof(float) * (size_t)(w + 2) * (h + 2) +
-           sizeof(float) * (size_t)(px / 2 + 1) * (py / 2 + 1) + sizeof(float2) * (px + py);
+    return sizeof(float2) * (size_t)(px / 2 + 1) * ld + sizeof(float) * (size_t)grav_ring_stride(w) * (h + 2) +
+           sizeof(float) * (size_t)(px / 2 + 1) * (py / 2 + 1) +
+           sizeof(float2) * (grav_twiddle_count(px) + grav_twiddle_count(py));
 }
 
 void GravPlan::solve(const float* src, float* phi, float* gx, float* gy, cudaStream_t s) const {
@@ -453,6 +529,7 @@ void GravPlan::solve(const float* src, float* phi, float* gx, float* gy, cudaStr
     A.px = px;
     A.py = py;
     A.ld = ld;
+    A.rp = grav_ring_stride(w);
     A.sigma_vac = sigma_vac;
     A.src = src;
     A.spec = spec;

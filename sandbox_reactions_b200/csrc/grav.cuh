@@ -5,7 +5,8 @@
 
 struct GravArgs {
     int w, h, px, py;
-    size_t ld;  // column stride of the spectrum buffer, in complex values (h + 2)
+    size_t ld;  // column stride of the spectrum buffer, in complex values
+    int rp;     // row stride of the ringed potential
     float sigma_vac;
     const float* src;
     float2* spec;
@@ -20,6 +21,14 @@ struct GravArgs {
 
 // The smallest power of two >= 2 len, at least 32, at most 8192 (0: refused).
 int grav_padded_size(int len);
+// An axis's twiddle table for n-point transforms: its entries, and their values (built in f64).
+size_t grav_twiddle_count(int n);
+void grav_twiddles(int n, float2* out);
+// A spectrum column holds the world's h rows, then the ring's h + 2 in their place; columns begin on 32 bytes.
+constexpr int grav_column_stride(int h) { return (h + 2 + 3) & ~3; }
+// A row of the ringed potential: column c of -1..w at kRingPad + 1 + c, so that the world's cells begin on 16 bytes.
+constexpr int kRingPad = 3;
+constexpr int grav_ring_stride(int w) { return w + 8; }
 
 // One world's solve: its spectrum work buffer, ringed potential, K̂ quarter and twiddle tables.
 struct GravPlan {

@@ -28,21 +28,22 @@ namespace {
 
 constexpr int kStaticMaxWorld = 256;                // world axes up to 256 cells
 constexpr int kStaticMaxPadded = 2 * kStaticMaxWorld;  // their padded FFT length
-constexpr size_t kSpecCount = (size_t)(kStaticMaxPadded / 2 + 1) * (kStaticMaxWorld + 2);
-constexpr size_t kRingCount = (size_t)(kStaticMaxWorld + 2) * (kStaticMaxWorld + 2);
+constexpr size_t kSpecCount = (size_t)(kStaticMaxPadded / 2 + 1) * grav_column_stride(kStaticMaxWorld);
+constexpr size_t kRingCount = (size_t)grav_ring_stride(kStaticMaxWorld) * (kStaticMaxWorld + 2);
 constexpr size_t kKhatCount = (size_t)(kStaticMaxPadded / 2 + 1) * (kStaticMaxPadded / 2 + 1);
 
 static __device__ __align__(256) float2 g_spec[kSpecCount];
 static __device__ __align__(256) float g_ring[kRingCount];
 static __device__ __align__(256) float g_khat[kKhatCount];
-static __device__ __align__(256) float2 g_tw[2 * kStaticMaxPadded];
+constexpr size_t kTwiddleMax = 3 * kStaticMaxPadded;  // an axis's twiddle table at most (grav_twiddle_count)
+static __device__ __align__(256) float2 g_tw[2 * kTwiddleMax];
 
 // Host-side staging, static too: the f64 work of the kernel's spectrum and the f32 tables copied up.
 static double h_re[(size_t)kStaticMaxPadded * kStaticMaxPadded];
 static double h_im[(size_t)kStaticMaxPadded * kStaticMaxPadded];
 static double h_cos[kStaticMaxPadded / 2], h_sin[kStaticMaxPadded / 2];
 static float h_khat[kKhatCount];
-static float2 h_tw[2 * kStaticMaxPadded];
+static float2 h_tw[2 * kTwiddleMax];
 
 constexpr int kMaxDevices = 64;
 struct DeviceSlot {
@@ -121,20 +122,15 @@ void upload_tables(DeviceSlot& d, int px, int py, int kind, double G, double eps
     const double scale = 1.0 / ((double)px * (double)py);
     for (int i = 0; i <= px / 2; i++)
         for (int j = 0; j <= py / 2; j++) h_khat[(size_t)i * (py / 2 + 1) + j] = (float)(h_re[(size_t)j * px + i] * scale);
-    for (int k = 0; k < px; k++) {
-        const double a = -2.0 * M_PI * (double)k / (double)px;
-        h_tw[k] = make_float2((float)cos(a), (float)sin(a));
-    }
-    for (int k = 0; k < py; k++) {
-        const double a = -2.0 * M_PI * (double)k / (double)py;
-        h_tw[kStaticMaxPadded + k] = make_float2((float)cos(a), (float)sin(a));
-    }
+    SR_REQUIRE(grav_twiddle_count(px) <= kTwiddleMax && grav_twiddle_count(py) <= kTwiddleMax, "the twiddle tables");
+    grav_twiddles(px, h_tw);
+    grav_twiddles(py, h_tw + kTwiddleMax);
     const size_t kq = (size_t)(px / 2 + 1) * (py / 2 + 1);
     // forget what the arrays held before the copies start: if one of them fails, the next call uploads again
     d.kind = -1;
     d.px = d.py = 0;
     check(cudaMemcpyAsync(d.khat, h_khat, sizeof(float) * kq, cudaMemcpyHostToDevice, s), "copy K̂ to the static array");
-    check(cudaMemcpyAsync(d.tw, h_tw, sizeof(float2) * 2 * kStaticMaxPadded, cudaMemcpyHostToDevice, s),
+    check(cudaMemcpyAsync(d.tw, h_tw, sizeof(float2) * 2 * kTwiddleMax, cudaMemcpyHostToDevice, s),
           "copy the twiddles to the static array");
     check(cudaStreamSynchronize(s), "wait for the table upload");  // the host staging is reused by the next call
     d.px = px;
@@ -186,13 +182,13 @@ extern "C" sr_status sr_gravity_solve_static(const sr_config* cfg, const float* 
         plan.h = h;
         plan.px = px;
         plan.py = py;
-        plan.ld = (size_t)h + 2;
+        plan.ld = grav_column_stride(h);
         plan.sigma_vac = (float)cfg->sigma_vac;
         plan.spec = d.spec;
         plan.phi_ring = d.ring;
         plan.khat = d.khat;
         plan.tw_x = d.tw;
-        plan.tw_y = d.tw + kStaticMaxPadded;
+        plan.tw_y = d.tw + kTwiddleMax;
         plan.solve(sigma, phi, gx, gy, s);
         check(cudaGetLastError(), "gravity kernels");
         return SR_OK;
