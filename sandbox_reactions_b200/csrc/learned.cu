@@ -318,72 +318,140 @@ __global__ void pack_weights_kernel(const float* __restrict__ theta, int cin, in
     }
 }
 
-// ---- weight gradient on the CUDA cores: dW[co][k] = Σ_p g[p][co] x[p][k], g the output gradient under the ReLU mask
-// and x the convolution's input (through the input transform), per chunk of pixels; partials summed in chunk order.
-constexpr int DW_PIX = 2048;  // pixels per CTA
-constexpr int DW_SUB = 32;    // pixels staged at once
+// ---- weight and bias gradients on the CUDA cores, in FP32: dW[co][tap][ci] = Σ_p g[p][co] x[p + tap][ci] and
+// db[co] = Σ_p g[p][co], g the output gradient under the ReLU mask and x the convolution's input (through the input
+// transform). A CTA takes tiles of 16 x 8 pixels, staging g and the input's halo in shared memory; a thread holds
+// 4 output channels x 4 input channels x the 3 taps of one row of the kernel (48 sums) and slides along its pixel rows,
+// so that a pixel costs two 16-byte shared-memory loads for 48 multiply-adds. Few channels leave few such threads:
+// `PG` groups then share the tile's rows and are summed in order at the end. Tiles are dealt to the CTAs in order and
+// the CTAs' partials summed in order (dw_reduce_kernel): the result does not depend on the launch. A 16 x 64² batch's
+// fifteen layers: 2.8 -> 0.2 ms against one output channel's 2,048 pixels per thread with a shared-memory load for
+// nearly every multiply-add, and 8 threads a channel for the bias.
+constexpr int DW_W = 16, DW_H = 8, DW_HW = DW_W + 2, DW_HH = DW_H + 2, DW_NT = 192;
+constexpr int DW_CHUNKS = 128;  // partials at most
+
 template <int CIN_P, int COUT_P>
-__global__ void __launch_bounds__(256) dw_kernel(ConvArgs A, const float* __restrict__ gy, const float* __restrict__ y,
-                                                 int relu, float* part) {
-    constexpr int KT = 9 * CIN_P;
-    __shared__ float sg[DW_SUB][COUT_P];
-    __shared__ float sx[DW_SUB][64];
+struct DwShape {
+    static constexpr int TILES = (CIN_P / 4) * (COUT_P / 4) * 3;        // 48-sum threads for all of dW
+    static constexpr int NB = TILES <= DW_NT ? 1 : TILES / DW_NT;       // CTAs that share them (over output channels)
+    static constexpr int PG = DW_NT * NB / TILES;                       // pixel groups
+    static constexpr int CO = COUT_P / NB;                              // output channels of a CTA
+    static constexpr int SPAN = PG <= DW_H ? DW_W : DW_W * DW_H / PG;   // pixels of a row that one thread takes
+    static constexpr size_t SMEM = sizeof(float) * std::max((size_t)DW_HW * DW_HH * CIN_P + (size_t)DW_W * DW_H * CO,
+                                                            (size_t)(PG > 1 ? DW_NT * 52 : 0));
+    static_assert(PG * TILES == DW_NT * NB && PG <= 2 * DW_H, "whole groups of threads");
+};
+
+int dw_chunks(int B, int H, int W) {
+    const long long tiles = (long long)B * ((H + DW_H - 1) / DW_H) * ((W + DW_W - 1) / DW_W);
+    return (int)std::min<long long>(tiles, DW_CHUNKS);
+}
+
+template <int CIN_P, int COUT_P>
+__global__ void __launch_bounds__(DW_NT) dw_kernel(ConvArgs A, const float* __restrict__ gy, const float* __restrict__ y,
+                                                   int relu, float* part, float* bpart) {
+    using S = DwShape<CIN_P, COUT_P>;
+    constexpr int KT = 9 * CIN_P, CQ = CIN_P / 4, OQ = S::CO / 4;
+    extern __shared__ __align__(16) float sdw[];
+    float* sx = sdw;                             // [DW_HH][DW_HW][CIN_P]
+    float* sg = sdw + DW_HW * DW_HH * CIN_P;     // [DW_H][DW_W][CO]
     const int tid = threadIdx.x;
-    const int k0 = blockIdx.y * 64;
-    const int kl = tid % 64, cg = tid / 64;  // this thread: k = k0 + kl, channels cg, cg + 4, ...
-    constexpr int CPT = (COUT_P + 3) / 4;
-    float acc[CPT];
+    const int tt = tid % (S::TILES / S::NB), pg = tid / (S::TILES / S::NB);
+    const int ciq = tt % CQ, coq = (tt / CQ) % OQ, dy = tt / (CQ * OQ);
+    const int co0 = blockIdx.y * S::CO;
+    float acc[3][4][4], accb[4];
 #pragma unroll
-    for (int j = 0; j < CPT; j++) acc[j] = 0.0f;
-    const long long P = (long long)A.B * A.H * A.W;
-    const long long p0 = (long long)blockIdx.x * DW_PIX;
-    for (long long ps = p0; ps < p0 + DW_PIX && ps < P; ps += DW_SUB) {
-        for (int e = tid; e < DW_SUB * COUT_P; e += 256) {
-            const int q = e / COUT_P, co = e % COUT_P;
-            const long long p = ps + q;
-            float v = 0.0f;
-            if (p < P) {
-                v = gy[(size_t)p * COUT_P + co];
-                if (relu && !(y[(size_t)p * COUT_P + co] > 0.0f)) v = 0.0f;
-            }
-            sg[q][co] = v;
-        }
-        for (int e = tid; e < DW_SUB * 8; e += 256) {  // 8 groups of 8 k per pixel
-            const int q = e / 8, grp = e % 8;
-            const long long p = ps + q;
-            const int k = k0 + grp * 8;
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[a][i][j] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) accb[i] = 0.0f;
+    const int tw = (A.W + DW_W - 1) / DW_W, th = (A.H + DW_H - 1) / DW_H;
+    const int tiles = A.B * th * tw;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int img = tile / (th * tw), rem = tile - img * th * tw;
+        const int Y0 = (rem / tw) * DW_H, X0 = (rem % tw) * DW_W;
+        __syncthreads();
+        for (int e = tid; e < DW_HW * DW_HH * (CIN_P / 8); e += DW_NT) {
+            const int g = e % (CIN_P / 8), px = e / (CIN_P / 8), hy = px / DW_HW, hx = px - hy * DW_HW;
             float v[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) v[j] = 0.0f;
-            if (p < P && k < KT) {
-                const int tap = k / CIN_P, ci = k % CIN_P;
-                const int img = (int)(p / ((long long)A.H * A.W));
-                const int r = (int)(p - (long long)img * A.H * A.W);
-                const int yy = r / A.W, xx = r - (r / A.W) * A.W;
-                conv_input<CIN_P>(A, img, yy + tap / 3 - 1, xx + tap % 3 - 1, ci, v);
+            conv_input<CIN_P>(A, img, Y0 + hy - 1, X0 + hx - 1, 8 * g, v);
+            float4* d = reinterpret_cast<float4*>(sx + px * CIN_P + 8 * g);
+            d[0] = make_float4(v[0], v[1], v[2], v[3]);
+            d[1] = make_float4(v[4], v[5], v[6], v[7]);
+        }
+        for (int e = tid; e < DW_W * DW_H * OQ; e += DW_NT) {
+            const int q = e % OQ, px = e / OQ, yy = Y0 + px / DW_W, xx = X0 + px % DW_W;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (yy < A.H && xx < A.W) {
+                const size_t i = (((size_t)img * A.H + yy) * A.W + xx) * COUT_P + co0 + 4 * q;
+                v = *reinterpret_cast<const float4*>(gy + i);
+                if (relu) {
+                    const float4 m = *reinterpret_cast<const float4*>(y + i);
+                    if (!(m.x > 0.0f)) v.x = 0.0f;
+                    if (!(m.y > 0.0f)) v.y = 0.0f;
+                    if (!(m.z > 0.0f)) v.z = 0.0f;
+                    if (!(m.w > 0.0f)) v.w = 0.0f;
+                }
             }
-#pragma unroll
-            for (int j = 0; j < 8; j++) sx[q][grp * 8 + j] = v[j];
+            *reinterpret_cast<float4*>(sg + px * S::CO + 4 * q) = v;
         }
         __syncthreads();
+        // this thread's pixels: whole rows pg, pg + PG, ..., or the pg-th part of the rows
+        constexpr int PARTS = DW_W / S::SPAN, GROUPS = S::PG / PARTS;
+        const int x0 = (pg % PARTS) * S::SPAN;
+        for (int row = pg / PARTS; row < DW_H; row += GROUPS) {
+            const float* xr = sx + ((row + dy) * DW_HW + x0) * CIN_P + 4 * ciq;
+            const float* gr = sg + (row * DW_W + x0) * S::CO + 4 * coq;
+            float4 w0 = *reinterpret_cast<const float4*>(xr), w1 = *reinterpret_cast<const float4*>(xr + CIN_P);
 #pragma unroll 4
-        for (int q = 0; q < DW_SUB; q++) {
-            const float xv = sx[q][kl];
+            for (int x = 0; x < S::SPAN; x++) {
+                const float4 w2 = *reinterpret_cast<const float4*>(xr + (x + 2) * CIN_P);
+                const float4 g4 = *reinterpret_cast<const float4*>(gr + x * S::CO);
+                const float g[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
-            for (int j = 0; j < CPT; j++) {
-                const int co = cg + 4 * j;
-                if (co < COUT_P) acc[j] += sg[q][co] * xv;
+                for (int i = 0; i < 4; i++) {
+                    acc[0][i][0] += g[i] * w0.x; acc[0][i][1] += g[i] * w0.y;
+                    acc[0][i][2] += g[i] * w0.z; acc[0][i][3] += g[i] * w0.w;
+                    acc[1][i][0] += g[i] * w1.x; acc[1][i][1] += g[i] * w1.y;
+                    acc[1][i][2] += g[i] * w1.z; acc[1][i][3] += g[i] * w1.w;
+                    acc[2][i][0] += g[i] * w2.x; acc[2][i][1] += g[i] * w2.y;
+                    acc[2][i][2] += g[i] * w2.z; acc[2][i][3] += g[i] * w2.w;
+                    accb[i] += g[i];
+                }
+                w0 = w1;
+                w1 = w2;
             }
         }
-        __syncthreads();
     }
-    const int k = k0 + kl;
-    if (k < KT)
+    if constexpr (S::PG > 1) {  // the pixel groups' sums in group order, by the first group's threads
+        __syncthreads();
+        if (pg > 0) {
 #pragma unroll
-        for (int j = 0; j < CPT; j++) {
-            const int co = cg + 4 * j;
-            if (co < COUT_P) part[((size_t)blockIdx.x * COUT_P + co) * KT + k] = acc[j];
+            for (int q = 0; q < 48; q++) sdw[q * DW_NT + tid] = acc[q / 16][(q / 4) % 4][q % 4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) sdw[(48 + i) * DW_NT + tid] = accb[i];
         }
+        __syncthreads();
+        if (pg > 0) return;
+        for (int p = 1; p < S::PG; p++) {
+            const int o = tid + p * (S::TILES / S::NB);
+#pragma unroll
+            for (int q = 0; q < 48; q++) acc[q / 16][(q / 4) % 4][q % 4] += sdw[q * DW_NT + o];
+#pragma unroll
+            for (int i = 0; i < 4; i++) accb[i] += sdw[(48 + i) * DW_NT + o];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float* d = part + ((size_t)blockIdx.x * COUT_P + co0 + 4 * coq + i) * KT + 3 * dy * CIN_P + 4 * ciq;
+#pragma unroll
+        for (int a = 0; a < 3; a++)
+            *reinterpret_cast<float4*>(d + a * CIN_P) = make_float4(acc[a][i][0], acc[a][i][1], acc[a][i][2], acc[a][i][3]);
+        if (dy == 0 && ciq == 0) bpart[(size_t)blockIdx.x * COUT_P + co0 + 4 * coq + i] = accb[i];
+    }
 }
 
 // dW and db from the partials into the gradient vector (the parameter layout W[cout][3][3][cin], b[cout]).
@@ -404,28 +472,6 @@ __global__ void dw_reduce_kernel(const float* __restrict__ part, int chunks, int
             for (int c = 0; c < chunks; c++) s += bpart[(size_t)c * cout_p + co];
             gb[co] = (float)s;
         }
-    }
-}
-
-// Bias gradient partials: Σ over a chunk of pixels of the masked output gradient.
-template <int COUT_P>
-__global__ void db_kernel(long long P, const float* __restrict__ gy, const float* __restrict__ y, int relu,
-                          float* bpart) {
-    __shared__ float red[COUT_P][8];
-    const int co = threadIdx.x % COUT_P, lane = threadIdx.x / COUT_P;  // blockDim = COUT_P * 8
-    const long long p0 = (long long)blockIdx.x * DW_PIX;
-    float s = 0.0f;
-    for (long long p = p0 + lane; p < p0 + DW_PIX && p < P; p += 8) {
-        float v = gy[(size_t)p * COUT_P + co];
-        if (relu && !(y[(size_t)p * COUT_P + co] > 0.0f)) v = 0.0f;
-        s += v;
-    }
-    red[co][lane] = s;
-    __syncthreads();
-    if (lane == 0) {
-        float t = 0.0f;
-        for (int q = 0; q < 8; q++) t += red[co][q];
-        bpart[(size_t)blockIdx.x * COUT_P + co] = t;
     }
 }
 
@@ -732,9 +778,14 @@ struct Net {
         if (train) {
             SR_CUDA_TRY(cudaMalloc(&gx, sizeof(float) * maxin));
             SR_CUDA_TRY(cudaMalloc(&energy, sizeof(float) * B));
-            const size_t chunks = (pix(0) + DW_PIX - 1) / DW_PIX;
-            SR_CUDA_TRY(cudaMalloc(&wpart, sizeof(float) * chunks * 64 * 9 * 64));
-            SR_CUDA_TRY(cudaMalloc(&bpart, sizeof(float) * chunks * 64));
+            size_t wmax = 0, bmax = 0;  // the largest layer's partials
+            for (int l = 0; l < NL; l++) {
+                const size_t co = (size_t)dw_chunks(B, lh[kL[l].level], lw[kL[l].level]) * pad8(kL[l].cout);
+                wmax = std::max(wmax, co * 9 * pad8(kL[l].cin));
+                bmax = std::max(bmax, co);
+            }
+            SR_CUDA_TRY(cudaMalloc(&wpart, sizeof(float) * wmax));
+            SR_CUDA_TRY(cudaMalloc(&bpart, sizeof(float) * bmax));
         }
     }
     void destroy() {
@@ -832,12 +883,9 @@ void forward(const Learner* Lr, const Net& N, cudaStream_t s) {
 template <int CI, int CO>
 void launch_dw_t(const ConvArgs& A, const float* gy, const float* y, int relu, float* wpart, float* bpart,
                  cudaStream_t s) {
-    const long long P = (long long)A.B * A.H * A.W;
-    const int chunks = (int)((P + DW_PIX - 1) / DW_PIX);
-    dim3 grid(chunks, (9 * CI + 63) / 64);
-    dw_kernel<CI, CO><<<grid, 256, 0, s>>>(A, gy, y, relu, wpart);
-    sr_note_launch();
-    db_kernel<CO><<<chunks, CO * 8, 0, s>>>(P, gy, y, relu, bpart);
+    using S = DwShape<CI, CO>;
+    const dim3 grid(dw_chunks(A.B, A.H, A.W), S::NB);
+    dw_kernel<CI, CO><<<grid, DW_NT, S::SMEM, s>>>(A, gy, y, relu, wpart, bpart);
     sr_note_launch();
 }
 
@@ -851,6 +899,16 @@ void launch_dw(int ci, int co, const ConvArgs& A, const float* gy, const float* 
     throw SrError{SR_E_INVALID, "no weight gradient for these channel counts"};
 }
 
+// Shared-memory opt-in of every weight gradient, with the convolutions'.
+void dw_attributes() {
+#define SR_DW_CASE(CI, CO)                                                                                        \
+    SR_CUDA_TRY(cudaFuncSetAttribute(dw_kernel<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,              \
+                                     (int)DwShape<CI, CO>::SMEM));
+    SR_DW_CASE(8, 8) SR_DW_CASE(8, 16) SR_DW_CASE(16, 16) SR_DW_CASE(16, 32) SR_DW_CASE(32, 32) SR_DW_CASE(32, 64)
+    SR_DW_CASE(64, 64) SR_DW_CASE(64, 32) SR_DW_CASE(32, 16) SR_DW_CASE(16, 8)
+#undef SR_DW_CASE
+}
+
 // Loss gradient already in gact[NL-1]: every layer's weight gradient and the input gradients, last layer first.
 void backward(Learner* Lr, Net& N, cudaStream_t s) {
     for (int l = 0; l < NL - 1; l++)
@@ -860,7 +918,7 @@ void backward(Learner* Lr, Net& N, cudaStream_t s) {
         const int ci = pad8(d.cin), co = pad8(d.cout);
         ConvArgs A = layer_args(Lr, N, l);
         const long long P = (long long)A.B * A.H * A.W;
-        const int chunks = (int)((P + DW_PIX - 1) / DW_PIX);
+        const int chunks = dw_chunks(A.B, A.H, A.W);
         launch_dw(ci, co, A, N.gact[l], N.act[l], d.relu, N.wpart, N.bpart, s);
         dw_reduce_kernel<<<grid_of((size_t)d.cout * 9 * d.cin + d.cout), RT, 0, s>>>(
             N.wpart, chunks, d.cin, d.cout, ci, co, Lr->grad + Lr->woff[l], Lr->grad + Lr->boff[l], N.bpart);
@@ -919,6 +977,7 @@ Learner* learned_create(int crop, int capacity, uint64_t seed) {
     Learner* L = new Learner();
     try {
         conv_attributes();
+        dw_attributes();
         L->crop = crop;
         L->capacity = capacity;
         L->rng.seed(seed);
