@@ -60,10 +60,8 @@ struct sr_ctx {
     double* rfin = nullptr;
     GravPlan grav;
     bool grav_ready = false;
-    double* part_d = nullptr;
-    float* part_best = nullptr;
-    int* part_idx = nullptr;
-    double* hreport = nullptr;  // 7 doubles
+    void* hpart = nullptr;        // the hydro kernels' partials and tickets, and the floors kernel's ticket
+    unsigned* tickets = nullptr;
     int* herr = nullptr;        // the hydro kernels' error flag (a bounded wait gave up)
     DtRecord* rec = nullptr;
     float *part_rate = nullptr, *part_g = nullptr;
@@ -167,7 +165,7 @@ static void ctx_free(sr_ctx* c) {
     cudaFree(c->table); cudaFree(c->held); cudaFree(c->src_free); cudaFree(c->phip); cudaFree(c->gxp);
     cudaFree(c->gyp); cudaFree(c->push); cudaFree(c->radx); cudaFree(c->rady); cudaFree(c->rpart); cudaFree(c->rbest); cudaFree(c->ridx); cudaFree(c->rfin);
     if (c->grav_ready) c->grav.destroy();
-    cudaFree(c->part_d); cudaFree(c->part_best); cudaFree(c->part_idx); cudaFree(c->hreport); cudaFree(c->herr);
+    cudaFree(c->hpart); cudaFree(c->tickets); cudaFree(c->herr);
     cudaFree(c->rec); cudaFree(c->part_rate); cudaFree(c->part_g); cudaFree(c->part_nf);
     drop_step_graphs(c);
     if (c->heat) heat_destroy(c->heat);
@@ -265,7 +263,7 @@ static void ref_setup(sr_ctx* c) {
 static RefArgs ref_args(sr_ctx* c, int cur) {
     RefArgs A{};
     A.R = c->R;
-    A.dt = &c->rec->dt;
+    A.dt = &c->rec->dt_next;  // P1: the step runs on the last P9's Δt_{n+1}; its P9 books it
     A.U = c->U[cur];
     A.Uout = c->U[1 - cur];
     A.held = c->held;
@@ -288,26 +286,29 @@ static RefArgs ref_args(sr_ctx* c, int cur) {
     return A;
 }
 
+static DtRule dt_rule(sr_ctx* c, int advance) {
+    const sr_config& k = c->cfg;
+    return DtRule{k.cfl, k.eta_g, k.dt_fixed, k.dt_cap, c->rec, advance};
+}
+
 // P2 on the current state, then P9 (no floors) — what Twin::new does before step 0 (reference/mod.rs:129-177).
 static void initial_reductions(sr_ctx* c) {
     DtRecord rec{};
     SR_CUDA_TRY(cudaMemcpyAsync(c->rec, &rec, sizeof rec, cudaMemcpyHostToDevice, c->stream));
-    SR_CUDA_TRY(cudaMemsetAsync(c->hreport, 0, 7 * sizeof(double), c->stream));
     const sr_config& k = c->cfg;
     if (ref_mode(c)) {
         // reference/mod.rs:129-177: the hold's rule on the initial state, P2, then Δt_0
         ref_hold_dt_launch(c->R, planes(c), c->held, nullptr, nullptr, 1, 0, c->part_rate, c->part_g, c->part_nf,
-                           k.cfl, k.eta_g, k.dt_fixed, k.dt_cap, c->rec, c->stream);
+                           dt_rule(c, 0), c->stream);
         if (k.gravity) c->grav.solve(planes(c), c->phi, c->gx, c->gy, c->stream);
         ref_hold_dt_launch(c->R, planes(c), c->held, k.gravity ? c->gx : nullptr, k.gravity ? c->gy : nullptr, 0, 1,
-                           c->part_rate, c->part_g, c->part_nf, k.cfl, k.eta_g, k.dt_fixed, k.dt_cap, c->rec,
-                           c->stream);
+                           c->part_rate, c->part_g, c->part_nf, dt_rule(c, 0), c->stream);
         SR_CUDA_TRY(cudaGetLastError());
         return;
     }
     if (c->cfg.gravity) c->grav.solve(planes(c), c->phi, c->gx, c->gy, c->stream);
     floors_dt_launch(c->H, planes(c), k.gravity ? c->gx : nullptr, k.gravity ? c->gy : nullptr, 0, c->part_rate,
-                     c->part_g, c->part_nf, k.cfl, k.eta_g, k.dt_fixed, k.dt_cap, c->rec, c->stream);
+                     c->part_g, c->part_nf, c->tickets, dt_rule(c, 0), c->stream);
     SR_CUDA_TRY(cudaGetLastError());
 }
 
@@ -323,7 +324,7 @@ static cudaEvent_t event_at(sr_ctx* c, size_t i) {
 static HydroArgs hydro_args(sr_ctx* c, int cur) {
     HydroArgs A{};
     A.H = c->H;
-    A.dt = &c->rec->dt;
+    A.dt = &c->rec->dt_next;  // P1: the step runs on the last P9's Δt_{n+1}; its P9 books it
     A.U = c->U[cur];
     A.Uout = c->U[1 - cur];
     A.gx = c->cfg.gravity ? c->gx : nullptr;
@@ -332,10 +333,9 @@ static HydroArgs hydro_args(sr_ctx* c, int cur) {
     A.phim = c->phim;
     A.gxm = c->gxm;
     A.gym = c->gym;
-    A.part_d = c->part_d;
-    A.part_best = c->part_best;
-    A.part_idx = c->part_idx;
-    A.report = c->hreport;
+    A.part = c->hpart;
+    A.tickets = c->tickets + 1;
+    A.rule = dt_rule(c, 1);
     A.err = c->herr;
     return A;
 }
@@ -350,7 +350,6 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
     const sr_config& k = c->cfg;
     float* U = c->U[cur];
     mark(0);
-    dt_advance_launch(c->rec, s);
     if (k.gravity) c->grav.solve(U, c->phi, c->gx, c->gy, s);
     mark(1);
     if (ref_mode(c)) {
@@ -373,8 +372,8 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
         }
         mark(4);
         if (k.heat) {
-            if (root) heat_top = heat_capture_step(c->heat, U, nullptr, &c->rec->dt, s, root);
-            else heat_step(c->heat, U, nullptr, &c->rec->dt, s, &c->heat_report);
+            if (root) heat_top = heat_capture_step(c->heat, U, nullptr, &c->rec->dt_next, s, root);
+            else heat_step(c->heat, U, nullptr, &c->rec->dt_next, s, &c->heat_report);
             const float *fx, *fy;
             heat_flux_planes(c->heat, &fx, &fy);
             ref_cell_flux_launch(fx, fy, c->radx, c->rady, c->w, c->h, s);
@@ -382,7 +381,7 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
         mark(5);
         ref_floors_launch(c->R, U, s);
         ref_hold_dt_launch(c->R, U, c->held, k.gravity ? c->gx : nullptr, k.gravity ? c->gy : nullptr, 1, 1,
-                           c->part_rate, c->part_g, c->part_nf, k.cfl, k.eta_g, k.dt_fixed, k.dt_cap, c->rec, s);
+                           c->part_rate, c->part_g, c->part_nf, dt_rule(c, 1), s);
         mark(6);
         return heat_top;
     }
@@ -394,12 +393,16 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
             mark(2);
             hydro_launch(kHydroUpdateGrav, A, s);
             mark(3);
-            hydro_finalize_launch(A, 1, s);
         } else {
             mark(2);
-            hydro_launch(kHydroUpdate, A, s);
+            hydro_launch(k.heat ? kHydroUpdate : kHydroStep, A, s);
             mark(3);
-            hydro_finalize_launch(A, 0, s);
+            if (!k.heat) {  // the floors and Δt rode along: the step is done
+                mark(4);
+                mark(5);
+                mark(6);
+                return 0;
+            }
         }
         U = c->U[1 - cur];
     } else {
@@ -409,12 +412,12 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
     mark(4);
     if (k.heat) {
         const float* kappa = k.opacity_plane ? c->kappa : nullptr;
-        if (root) heat_top = heat_capture_step(c->heat, U, kappa, &c->rec->dt, s, root);
-        else heat_step(c->heat, U, kappa, &c->rec->dt, s, &c->heat_report);
+        if (root) heat_top = heat_capture_step(c->heat, U, kappa, &c->rec->dt_next, s, root);
+        else heat_step(c->heat, U, kappa, &c->rec->dt_next, s, &c->heat_report);
     }
     mark(5);
     floors_dt_launch(c->H, U, k.gravity ? c->gx : nullptr, k.gravity ? c->gy : nullptr, 1, c->part_rate, c->part_g,
-                     c->part_nf, k.cfl, k.eta_g, k.dt_fixed, k.dt_cap, c->rec, s);
+                     c->part_nf, c->tickets, dt_rule(c, 1), s);
     mark(6);
     return heat_top;
 }
@@ -773,11 +776,8 @@ sr_status sr_create(const sr_config* cfg, sr_ctx** out) {
             c->grav_ready = true;
         }
         if (cfg->opacity_plane) dalloc(&c->kappa, n);
-        int hb = hydro_blocks(c->w, c->h);
-        dalloc(&c->part_d, (size_t)hb * 6);
-        dalloc(&c->part_best, (size_t)hb);
-        dalloc(&c->part_idx, (size_t)hb);
-        dalloc(&c->hreport, 7);
+        dalloc((unsigned char**)&c->hpart, hydro_part_count(c->w, c->h) * kHydroPartBytes);
+        dalloc(&c->tickets, 1 + hydro_ticket_count(c->h));
         dalloc(&c->herr, 1);
         dalloc(&c->rec, 1);
         int fb = floors_dt_blocks(c->w, c->h);

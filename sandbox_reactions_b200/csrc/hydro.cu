@@ -4,9 +4,11 @@
 // memory by one TMA box, the world's ghosts are formed there, every lane runs the Hancock predictor for one cell (the
 // tile's and the one-cell ring around it), the faces meet for the HLL fluxes by warp shuffles (x) and shared memory
 // (y), and the per-cell epilogue of the pass finishes:
-//   - kHydroUpdate:     U' = U - Δt ΔF (no gravity);
+//   - kHydroStep:       U' = U - Δt ΔF, then P8's floors and P9's Δt on U' (no gravity, no heat: the whole step);
+//   - kHydroUpdate:     U' = U - Δt ΔF (no gravity; heat follows);
 //   - kHydroSource:     the half step's gravity source ½(Σⁿ + Σⁿ⁺¹), masked (reference hydro.rs:815-836);
-//   - kHydroUpdateGrav: U' with gravity's half-step kick and the faces' work across φ_mid (hydro.rs:871-947).
+//   - kHydroUpdateGrav: U' with gravity's half-step kick and the faces' work across φ_mid (hydro.rs:871-947), the net
+//                       kick taken back from the densest cell.
 // The scheme follows crates/sr-physics/src/reference/hydro.rs (step_held without held cells, sinks or radiation).
 #include "hydro.cuh"
 
@@ -111,6 +113,90 @@ struct FaceS {
     float U0, U1, U2, U3, u, v, P;
 };
 
+// What the CTAs sum: gravity's net kick (FP64) and the densest cell (the lowest index on a tie), or the largest wave
+// rate and the first non-finite value (cell * 4 + channel).
+struct KickPart {
+    double kx, ky;
+    float best;
+    int idx;
+    __device__ __forceinline__ static KickPart none() { return KickPart{0.0, 0.0, 0.0f, -1}; }
+    __device__ __forceinline__ void merge(const KickPart& o) {
+        kx += o.kx;
+        ky += o.ky;
+        if (o.idx >= 0 && (idx < 0 || o.best > best || (o.best == best && o.idx < idx))) {
+            best = o.best;
+            idx = o.idx;
+        }
+    }
+    __device__ __forceinline__ KickPart down(int o) const {
+        return KickPart{__shfl_down_sync(0xffffffffu, kx, o), __shfl_down_sync(0xffffffffu, ky, o),
+                        __shfl_down_sync(0xffffffffu, best, o), __shfl_down_sync(0xffffffffu, idx, o)};
+    }
+};
+struct RatePart {
+    long long nf;
+    float rate;
+    __device__ __forceinline__ static RatePart none() { return RatePart{LLONG_MAX, 0.0f}; }
+    __device__ __forceinline__ void merge(const RatePart& o) {
+        nf = o.nf < nf ? o.nf : nf;
+        rate = fmaxf(rate, o.rate);
+    }
+    __device__ __forceinline__ RatePart down(int o) const {
+        return RatePart{__shfl_down_sync(0xffffffffu, nf, o), __shfl_down_sync(0xffffffffu, rate, o)};
+    }
+};
+union Part {
+    double align[3];
+    __device__ __forceinline__ KickPart& kick() { return *reinterpret_cast<KickPart*>(this); }
+    __device__ __forceinline__ RatePart& rate() { return *reinterpret_cast<RatePart*>(this); }
+};
+static_assert(sizeof(KickPart) == sizeof(Part) && sizeof(RatePart) <= sizeof(Part), "a partial's slot");
+static_assert(sizeof(Part) == kHydroPartBytes, "the partials' buffer");
+
+template <class P>
+__device__ __forceinline__ P warp_merge(P v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v.merge(v.down(o));
+    return v;
+}
+
+// The grid's total of the CTAs' partials `v` (lane 0's), by warp 0 of every CTA: the last CTA of a grid row to arrive
+// merges the row's partials and the last row to arrive the rows', each in a fixed order (two short tickets instead of
+// one CTA walking all partials: at 2048² 10,143 of them took a kernel of their own 52 us). True, with the total in
+// lane 0, in the one warp that arrives last; the tickets are left at 0 for the next launch.
+template <class P>
+__device__ __forceinline__ bool grid_total(P& v, void* parts, unsigned* tickets) {
+    P* part = reinterpret_cast<P*>(parts);
+    P* rows = part + (size_t)gridDim.x * gridDim.y;
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int level = 0; level < 2; level++) {
+        P* slot = level ? rows + blockIdx.y : part + (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+        unsigned* ticket = tickets + (level ? gridDim.y : blockIdx.y);
+        const unsigned count = level ? gridDim.y : gridDim.x;
+        const P* from = level ? rows : part + (size_t)blockIdx.y * gridDim.x;
+        bool last = false;
+        if (lane == 0) {
+            *slot = v;
+            __threadfence();
+            last = atomicAdd(ticket, 1u) == count - 1;
+            if (last) *ticket = 0u;
+            __threadfence();
+        }
+        if (!__shfl_sync(0xffffffffu, last, 0)) return false;
+        P t = P::none();
+        for (unsigned k = lane; k < count; k += 32) {
+            P o;
+            const double* src = reinterpret_cast<const double*>(from + k);
+#pragma unroll
+            for (int q = 0; q < (int)(sizeof(P) / sizeof(double)); q++) reinterpret_cast<double*>(&o)[q] = __ldcg(src + q);
+            t.merge(o);
+        }
+        v = warp_merge(t);
+    }
+    return true;
+}
+
 struct __align__(128) BandShared {
     float raw[4][HB_BY][HB_BX];  // the TMA box of Σ, Σu, Σv, E (first: 128-byte aligned)
     float4 P[HB_SY][HB_SX];      // primitives (Σ, u, v, Π) of the staged region, ghosts included
@@ -119,9 +205,7 @@ struct __align__(128) BandShared {
     float M[3][HB_W][32];        // half-step (Σ, Σu, Σv) of each lane's cell
     float YF[7][HB_W][32];       // each lane's y+ face
     float FY[4][HB_W][32];       // the flux through each lane's top face
-    double red_d[6][HB_W];
-    float red_best[HB_W];
-    int red_idx[HB_W];
+    Part red[HB_W];              // the rows' partials
     uint64_t mbar;
 };
 
@@ -235,6 +319,60 @@ __device__ __forceinline__ void face_flux_at(const HydroConst& H, const FaceS& L
         }
     } else {
         hll_s(H, L, R, dir, f);
+    }
+}
+
+// P8 on one cell: the vacuum reset and the thermal floor (reference/floors.rs:124-196, Σ_vac and Σ_floor as the planes'
+// f32); returns which values changed (1: E alone, 2: all).
+__device__ __forceinline__ int floor_cell(const HydroConst& H, float& s, float& mx, float& my, float& e) {
+    if (s < H.sigma_vac) {
+        s = H.sigma_floor;
+        mx = 0.0f;
+        my = 0.0f;
+        e = H.sigma_floor * H.eps_floor;
+        return 2;
+    }
+    const float kinetic = 0.5f * (mx * mx + my * my) / (s * s);
+    const float raw = e / s - kinetic;
+    if (raw < H.eps_floor) {
+        e = e + s * (H.eps_floor - raw);
+        return 1;
+    }
+    return 0;
+}
+
+// P9's terms of one floored cell: its wave rate (|u|+c)+(|v|+c) (hydro.rs:618-634) and the non-finite guard's code.
+__device__ __forceinline__ void rate_cell(const HydroConst& H, float s, float mx, float my, float e, size_t i,
+                                          float& rate, long long& nf) {
+    if (!(isfinite(s) && isfinite(mx) && isfinite(my) && isfinite(e))) {
+        const int c = !isfinite(s) ? 0 : (!isfinite(mx) ? 1 : (!isfinite(my) ? 2 : 3));
+        const long long code = (long long)i * 4 + c;
+        nf = code < nf ? code : nf;
+    }
+    const Prim p = eos_read(H, s, mx, my, e);
+    const float c = eos_sound(H, p);
+    rate = fmaxf(rate, (fabsf(p.u) + c) + (fabsf(p.v) + c));
+}
+
+// Δt_{n+1} = min(C / max rate, η_g / sqrt(max |g|)) (hydro.rs:618-634), the configured fixed Δt or cap, and the guard;
+// with `advance` the step that ends here is booked first (P1: it ran on Δt_n = the last Δt_{n+1}, f64 sim time).
+__device__ void dt_close(const DtRule& R, float rate, float gmax, long long nf, int channels) {
+    DtRecord* rec = R.rec;
+    if (R.advance) {
+        rec->dt = rec->dt_next;
+        rec->sim_time += rec->dt;
+        rec->steps += 1;
+    }
+    double dt = R.cfl / (double)rate;
+    if (gmax > 0.0f) dt = fmin(dt, R.eta_g / sqrt((double)gmax));
+    if (R.dt_fixed > 0.0) dt = R.dt_fixed;
+    if (R.dt_cap > 0.0) dt = fmin(dt, R.dt_cap);
+    rec->dt_next = dt;
+    if (nf != LLONG_MAX && !rec->non_finite) {
+        rec->non_finite = 1;
+        rec->nf_cell = nf / channels;
+        rec->nf_channel = (int)(nf % channels);
+        rec->nf_step = rec->steps;
     }
 }
 
@@ -412,10 +550,8 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
         return;
     }
 
-    double kick_acc[2] = {0.0, 0.0};
-    float best = 0.0f;
-    int best_i = -1;
-    double esc[4] = {0.0, 0.0, 0.0, 0.0};
+    KickPart kp = KickPart::none();
+    RatePart rp = RatePart::none();
     if (inside) {
         const int bx = X - xs, by = Y - ys;
         float u[4];
@@ -431,11 +567,11 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
                 const float m[3] = {sh.M[0][row][lane], sh.M[1][row][lane], sh.M[2][row][lane]};
                 const float src = A.src[i];
                 float kick[2] = {dt * src * A.gxm[i], dt * src * A.gym[i]};
-                kick_acc[0] = (double)kick[0];
-                kick_acc[1] = (double)kick[1];
+                kp.kx = (double)kick[0];
+                kp.ky = (double)kick[1];
                 if (src > 0.0f) {
-                    best = src;
-                    best_i = (int)i;
+                    kp.best = src;
+                    kp.idx = (int)i;
                 }
                 const float p = A.phim[i];
                 float pr = p, pl = p, pd = p, pu = p;
@@ -472,12 +608,10 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
                 u[2] += kick[1];
                 u[3] += r[1] + l[2] + dn[1] + up[2];
             }
-            // escaped (hydro.rs:948-973): the boundary faces' fluxes as the cell took them
-            const float phi_edge = MODE == kHydroUpdateGrav ? A.phim[i] : 0.0f;
-            if (X == 0) { for (int q = 0; q < 4; q++) esc[q] -= (double)(dt * fl[q]); esc[3] -= (double)(dt * fl[0] * phi_edge); }
-            if (X + 1 == w) { for (int q = 0; q < 4; q++) esc[q] += (double)(dt * fr[q]); esc[3] += (double)(dt * fr[0] * phi_edge); }
-            if (Y == 0) { for (int q = 0; q < 4; q++) esc[q] -= (double)(dt * fu[q]); esc[3] -= (double)(dt * fu[0] * phi_edge); }
-            if (Y + 1 == h) { for (int q = 0; q < 4; q++) esc[q] += (double)(dt * fd[q]); esc[3] += (double)(dt * fd[0] * phi_edge); }
+        }
+        if (MODE == kHydroStep) {
+            floor_cell(H, u[0], u[1], u[2], u[3]);
+            rate_cell(H, u[0], u[1], u[2], u[3], i, rp.rate, rp.nf);
         }
         A.Uout[i] = u[0];
         A.Uout[n + i] = u[1];
@@ -485,104 +619,26 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
         A.Uout[3 * n + i] = u[3];
     }
 
-    // ---- per-CTA partials in a fixed order: Σ kicks (FP64), the densest cell (max src, lowest index), Σ escaped
-    // a warp whose lanes hold no term skips its tree (interior rows hold no escaped flux; only the gravity pass kicks)
-    double vals[6] = {kick_acc[0], kick_acc[1], esc[0], esc[1], esc[2], esc[3]};
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        double v = vals[q];
-        if (__any_sync(0xffffffffu, v != 0.0)) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    // ---- the grid's sums, in a fixed order: the rows of the tile, the CTAs of a grid row, the grid rows
+    if (MODE == kHydroUpdate) return;
+    if (MODE == kHydroUpdateGrav) {
+        kp = warp_merge(kp);
+        if (lane == 0) sh.red[row].kick() = kp;
+        __syncthreads();
+        if (row > 0) return;
+        kp = warp_merge(lane < HB_W ? sh.red[lane].kick() : KickPart::none());
+        // the net kick on the gas's own field taken back from the densest cell (hydro.rs:1004-1012)
+        if (grid_total(kp, A.part, A.tickets) && lane == 0 && kp.idx >= 0) {
+            A.Uout[n + kp.idx] = __ldcg(A.Uout + n + kp.idx) - (float)kp.kx;
+            A.Uout[2 * n + kp.idx] = __ldcg(A.Uout + 2 * n + kp.idx) - (float)kp.ky;
         }
-        if (lane == 0) sh.red_d[q][row] = v;
-    }
-    if (__any_sync(0xffffffffu, best_i >= 0)) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_down_sync(0xffffffffu, best, o);
-            const int oi = __shfl_down_sync(0xffffffffu, best_i, o);
-            if (oi >= 0 && (best_i < 0 || ob > best || (ob == best && oi < best_i))) {
-                best = ob;
-                best_i = oi;
-            }
-        }
-    }
-    if (lane == 0) {
-        sh.red_best[row] = best;
-        sh.red_idx[row] = best_i;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        const int b = blockIdx.y * gridDim.x + blockIdx.x;
-        for (int q = 0; q < 6; q++) {
-            double t = 0.0;
-            for (int k = 0; k < HB_W; k++) t += sh.red_d[q][k];
-            A.part_d[(size_t)b * 6 + q] = t;
-        }
-        float bb = 0.0f;
-        int bi = -1;
-        for (int k = 0; k < HB_W; k++) {
-            const int oi = sh.red_idx[k];
-            const float ob = sh.red_best[k];
-            if (oi >= 0 && (bi < 0 || ob > bb || (ob == bb && oi < bi))) {
-                bb = ob;
-                bi = oi;
-            }
-        }
-        A.part_best[b] = bb;
-        A.part_idx[b] = bi;
-    }
-}
-
-// The net kick on the gas's own field taken back from the densest cell (hydro.rs:1004-1012), and the escaped totals,
-// summed over the CTAs' partials in CTA order by one CTA.
-__global__ void hydro_finalize_kernel(HydroArgs A, int nblocks, int take_back) {
-    __shared__ double sd[6][256];
-    __shared__ float sb[256];
-    __shared__ int si[256];
-    const int tid = threadIdx.x;
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    float best = 0.0f;
-    int bi = -1;
-    // each thread sums a contiguous run of CTAs, so the order is fixed
-    int per = (nblocks + 255) / 256;
-    for (int b = tid * per; b < min(nblocks, (tid + 1) * per); b++) {
-        for (int q = 0; q < 6; q++) acc[q] += A.part_d[(size_t)b * 6 + q];
-        int oi = A.part_idx[b];
-        float ob = A.part_best[b];
-        if (oi >= 0 && (bi < 0 || ob > best || (ob == best && oi < bi))) {
-            best = ob;
-            bi = oi;
-        }
-    }
-    for (int q = 0; q < 6; q++) sd[q][tid] = acc[q];
-    sb[tid] = best;
-    si[tid] = bi;
-    __syncthreads();
-    if (tid == 0) {
-        double t[6] = {0, 0, 0, 0, 0, 0};
-        for (int k = 0; k < 256; k++)
-            for (int q = 0; q < 6; q++) t[q] += sd[q][k];
-        float bb = 0.0f;
-        int idx = -1;
-        for (int k = 0; k < 256; k++) {
-            int oi = si[k];
-            float ob = sb[k];
-            if (oi >= 0 && (idx < 0 || ob > bb || (ob == bb && oi < idx))) {
-                bb = ob;
-                idx = oi;
-            }
-        }
-        const size_t n = (size_t)A.H.w * A.H.h;
-        if (take_back && idx >= 0) {
-            A.Uout[n + idx] -= (float)t[0];
-            A.Uout[2 * n + idx] -= (float)t[1];
-        }
-        A.report[0] = t[0];
-        A.report[1] = t[1];
-        A.report[2] = (double)idx;
-        for (int q = 0; q < 4; q++) A.report[3 + q] += t[2 + q];  // escaped accumulates over steps
+    } else {
+        rp = warp_merge(rp);
+        if (lane == 0) sh.red[row].rate() = rp;
+        __syncthreads();
+        if (row > 0) return;
+        rp = warp_merge(lane < HB_W ? sh.red[lane].rate() : RatePart::none());
+        if (grid_total(rp, A.part, A.tickets) && lane == 0) dt_close(A.rule, rp.rate, 0.0f, rp.nf, 4);
     }
 }
 
@@ -591,7 +647,9 @@ __global__ void hydro_finalize_kernel(HydroArgs A, int nblocks, int take_back) {
 
 size_t hydro_smem_bytes() { return sizeof(BandShared); }
 
-int hydro_blocks(int w, int h) { return (int)(div_up(w, HB_TX) * div_up(h, HB_TY)); }
+size_t hydro_part_count(int w, int h) { return (size_t)(div_up(w, HB_TX) + 1) * div_up(h, HB_TY); }
+
+size_t hydro_ticket_count(int h) { return (size_t)div_up(h, HB_TY) + 1; }
 
 void tma_encode_planes(CUtensorMap* map, const float* base, int w, int h, int planes, int bx, int by) {
     // encoded maps are kept by their arguments: a launch on the same planes (every launch of a step, every smoother
@@ -654,89 +712,88 @@ void hydro_launch_m(const CUtensorMap& map, const HydroArgs& A, cudaStream_t s) 
 void hydro_launch(int mode, const HydroArgs& A, cudaStream_t s) {
     CUtensorMap map;
     tma_encode_planes(&map, A.U, A.H.w, A.H.h, 4, HB_BX, HB_BY);
-    if (mode == kHydroUpdate) hydro_launch_m<kHydroUpdate>(map, A, s);
+    if (mode == kHydroStep) hydro_launch_m<kHydroStep>(map, A, s);
+    else if (mode == kHydroUpdate) hydro_launch_m<kHydroUpdate>(map, A, s);
     else if (mode == kHydroSource) hydro_launch_m<kHydroSource>(map, A, s);
     else hydro_launch_m<kHydroUpdateGrav>(map, A, s);
 }
 
-void hydro_finalize_launch(const HydroArgs& A, int take_back, cudaStream_t s) {
-    hydro_finalize_kernel<<<1, 256, 0, s>>>(A, hydro_blocks(A.H.w, A.H.h), take_back);
-    sr_note_launch();
-}
-
 // ------------------------------------------------------------------------------------------------ P8 + P9
-// P8's vacuum reset and thermal floor (reference/floors.rs:124-196, Σ_vac and Σ_floor as the planes' f32), then P9's
-// per-cell Δt terms (hydro.rs:618-634): the wave rate (|u|+c)+(|v|+c) of the floored state and |g| of the step's P2
-// field, reduced per CTA with the non-finite guard (reduce.wgsl's exit-5 scan: the first (cell, channel) not finite).
+// P8's floors, then P9's per-cell Δt terms of the floored state and |g| of the step's P2 field; per-CTA partials, the
+// last CTA to arrive (a ticket) reduces them (max and min are exact in any order) and closes the step's Δt record.
 __global__ void floors_dt_kernel(HydroConst H, float* __restrict__ U, const float* __restrict__ gx,
                                  const float* __restrict__ gy, int do_floors, float* part_rate, float* part_g,
-                                 long long* part_nf) {
+                                 long long* part_nf, unsigned* ticket, DtRule rule) {
     const size_t n = (size_t)H.w * H.h;
     float rate = 0.0f, gmax = 0.0f;
     long long nf = LLONG_MAX;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float s = U[i], mx = U[n + i], my = U[2 * n + i], e = U[3 * n + i];
         if (do_floors) {
-            if (s < H.sigma_vac) {
-                s = H.sigma_floor;
-                mx = 0.0f;
-                my = 0.0f;
-                e = H.sigma_floor * H.eps_floor;
-                U[i] = s; U[n + i] = mx; U[2 * n + i] = my; U[3 * n + i] = e;
-            } else {
-                float kinetic = 0.5f * (mx * mx + my * my) / (s * s);
-                float raw = e / s - kinetic;
-                if (raw < H.eps_floor) {
-                    e = e + s * (H.eps_floor - raw);
-                    U[3 * n + i] = e;
-                }
+            const int changed = floor_cell(H, s, mx, my, e);
+            if (changed == 2) {
+                U[i] = s;
+                U[n + i] = mx;
+                U[2 * n + i] = my;
             }
+            if (changed) U[3 * n + i] = e;
         }
-        if (!(isfinite(s) && isfinite(mx) && isfinite(my) && isfinite(e))) {
-            int c = !isfinite(s) ? 0 : (!isfinite(mx) ? 1 : (!isfinite(my) ? 2 : 3));
-            long long code = (long long)i * 4 + c;
-            nf = code < nf ? code : nf;
-        }
-        Prim p = eos_read(H, s, mx, my, e);
-        float c = eos_sound(H, p);
-        float r = (fabsf(p.u) + c) + (fabsf(p.v) + c);
-        rate = fmaxf(rate, r);
+        rate_cell(H, s, mx, my, e, i, rate, nf);
         if (gx) gmax = fmaxf(gmax, hypotf(gx[i], gy[i]));
     }
     __shared__ float sr[32], sg[32];
     __shared__ long long sn[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x / 32;
+    for (int level = 0; level < 2; level++) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        rate = fmaxf(rate, __shfl_down_sync(0xffffffffu, rate, o));
-        gmax = fmaxf(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
-        long long on = __shfl_down_sync(0xffffffffu, nf, o);
-        nf = on < nf ? on : nf;
-    }
-    if (lane == 0) {
-        sr[warp] = rate;
-        sg[warp] = gmax;
-        sn[warp] = nf;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < (int)(blockDim.x / 32); k++) {
-            rate = fmaxf(rate, sr[k]);
-            gmax = fmaxf(gmax, sg[k]);
-            nf = sn[k] < nf ? sn[k] : nf;
+        for (int o = 16; o > 0; o >>= 1) {
+            rate = fmaxf(rate, __shfl_down_sync(0xffffffffu, rate, o));
+            gmax = fmaxf(gmax, __shfl_down_sync(0xffffffffu, gmax, o));
+            const long long on = __shfl_down_sync(0xffffffffu, nf, o);
+            nf = on < nf ? on : nf;
         }
-        part_rate[blockIdx.x] = rate;
-        part_g[blockIdx.x] = gmax;
-        part_nf[blockIdx.x] = nf;
+        if (lane == 0) {
+            sr[warp] = rate;
+            sg[warp] = gmax;
+            sn[warp] = nf;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < warps; k++) {
+                rate = fmaxf(rate, sr[k]);
+                gmax = fmaxf(gmax, sg[k]);
+                nf = sn[k] < nf ? sn[k] : nf;
+            }
+            if (level == 0) {
+                part_rate[blockIdx.x] = rate;
+                part_g[blockIdx.x] = gmax;
+                part_nf[blockIdx.x] = nf;
+                __threadfence();
+                last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+                if (last) *ticket = 0u;
+                __threadfence();
+            } else {
+                dt_close(rule, rate, gmax, nf, 4);
+            }
+        }
+        __syncthreads();
+        if (level == 1 || !last) return;
+        rate = gmax = 0.0f;
+        nf = LLONG_MAX;
+        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+            rate = fmaxf(rate, __ldcg(part_rate + b));
+            gmax = fmaxf(gmax, __ldcg(part_g + b));
+            const long long o = __ldcg(part_nf + b);
+            nf = o < nf ? o : nf;
+        }
     }
 }
 
-// Δt_{n+1} = min(C / max rate, η_g / sqrt(max |g|)) (hydro.rs:618-634), the configured fixed Δt or cap, and the guard.
-// One CTA: each thread takes a strided share of the partials, then a shuffle and shared-memory tree (max and min are
-// exact in any order, so the result does not depend on the split).
+// The same from partials another kernel left. One CTA: each thread takes a strided share of them, then a shuffle and
+// shared-memory tree.
 __global__ void dt_finalize_kernel(int nblocks, int channels, const float* part_rate, const float* part_g,
-                                   const long long* part_nf, double cfl, double eta_g, double dt_fixed, double dt_cap,
-                                   DtRecord* rec) {
+                                   const long long* part_nf, DtRule rule) {
     float rate = 0.0f, gmax = 0.0f;
     long long nf = LLONG_MAX;
     for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
@@ -766,25 +823,7 @@ __global__ void dt_finalize_kernel(int nblocks, int channels, const float* part_
         gmax = fmaxf(gmax, sg[k]);
         nf = sn[k] < nf ? sn[k] : nf;
     }
-    double dt = cfl / (double)rate;
-    if (gmax > 0.0f) dt = fmin(dt, eta_g / sqrt((double)gmax));
-    if (dt_fixed > 0.0) dt = dt_fixed;
-    if (dt_cap > 0.0) dt = fmin(dt, dt_cap);
-    rec->dt_next = dt;
-    if (nf != LLONG_MAX && !rec->non_finite) {
-        rec->non_finite = 1;
-        rec->nf_cell = nf / channels;
-        rec->nf_channel = (int)(nf % channels);
-        rec->nf_step = rec->steps;
-    }
-}
-
-// P1: this step runs on Δt_n = the last P9's Δt_{n+1} and adds it to the sim time (f64).
-__global__ void dt_advance_kernel(DtRecord* rec) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    rec->dt = rec->dt_next;
-    rec->sim_time += rec->dt;
-    rec->steps += 1;
+    dt_close(rule, rate, gmax, nf, channels);
 }
 
 int floors_dt_blocks(int w, int h) {
@@ -794,21 +833,14 @@ int floors_dt_blocks(int w, int h) {
 }
 
 void floors_dt_launch(const HydroConst& H, float* U, const float* gx, const float* gy, int do_floors, float* part_rate,
-                      float* part_g, long long* part_nf, double cfl, double eta_g, double dt_fixed, double dt_cap,
-                      DtRecord* rec, cudaStream_t s) {
-    int nb = floors_dt_blocks(H.w, H.h);
-    floors_dt_kernel<<<nb, 256, 0, s>>>(H, U, gx, gy, do_floors, part_rate, part_g, part_nf);
+                      float* part_g, long long* part_nf, unsigned* ticket, const DtRule& rule, cudaStream_t s) {
+    floors_dt_kernel<<<floors_dt_blocks(H.w, H.h), 256, 0, s>>>(H, U, gx, gy, do_floors, part_rate, part_g, part_nf,
+                                                                ticket, rule);
     sr_note_launch();
-    dt_finalize_launch(nb, 4, part_rate, part_g, part_nf, cfl, eta_g, dt_fixed, dt_cap, rec, s);
 }
 
 void dt_finalize_launch(int nblocks, int channels, const float* part_rate, const float* part_g,
-                        const long long* part_nf, double cfl, double eta_g, double dt_fixed, double dt_cap,
-                        DtRecord* rec, cudaStream_t s) {
-    dt_finalize_kernel<<<1, 256, 0, s>>>(nblocks, channels, part_rate, part_g, part_nf, cfl, eta_g, dt_fixed, dt_cap,
-                                         rec);
+                        const long long* part_nf, const DtRule& rule, cudaStream_t s) {
+    dt_finalize_kernel<<<1, 256, 0, s>>>(nblocks, channels, part_rate, part_g, part_nf, rule);
     sr_note_launch();
 }
-
-void dt_advance_launch(DtRecord* rec, cudaStream_t s) { dt_advance_kernel<<<1, 32, 0, s>>>(rec);
-    sr_note_launch(); }

@@ -3,7 +3,7 @@
 
 #include "common.cuh"
 
-enum { kHydroUpdate = 0, kHydroSource = 1, kHydroUpdateGrav = 2 };
+enum { kHydroUpdate = 0, kHydroSource = 1, kHydroUpdateGrav = 2, kHydroStep = 3 };
 
 // The Δt record kept on the device (crates/sr-engine/src/step/dt.rs:51-61): steps never wait on the host for it.
 struct DtRecord {
@@ -17,6 +17,13 @@ struct DtRecord {
     unsigned long long nf_step;
 };
 
+// P9's rule for the next Δt, and where the step's Δt record lives.
+struct DtRule {
+    double cfl, eta_g, dt_fixed, dt_cap;
+    DtRecord* rec;
+    int advance;  // 1: a step ends here (its Δt, the sim time and the step count are booked)
+};
+
 struct HydroArgs {
     HydroConst H;
     const double* dt;          // device Δt_n
@@ -28,24 +35,21 @@ struct HydroArgs {
     const float* phim;         // the half step's φ, g (kHydroUpdateGrav)
     const float* gxm;
     const float* gym;
-    double* part_d;            // per-CTA partials: 6 doubles (kick x, y, escaped Σ, Σu, Σv, E)
-    float* part_best;          // per-CTA densest Σ_src,mid and its cell
-    int* part_idx;
-    double* report;            // [kick x, kick y, densest, escaped Σ, Σu, Σv, E]
+    void* part;                // partials of the grid's sums (hydro_part_count x kHydroPartBytes)
+    unsigned* tickets;         // hydro_ticket_count counters, 0 between launches
+    DtRule rule;               // kHydroStep
     int* err;                  // set to 1 when a bounded wait of the kernel gave up (its TMA box never landed)
 };
 
 size_t hydro_smem_bytes();
-int hydro_blocks(int w, int h);
+constexpr size_t kHydroPartBytes = 24;
+size_t hydro_part_count(int w, int h);
+size_t hydro_ticket_count(int h);
 void hydro_launch(int mode, const HydroArgs& A, cudaStream_t s);
-void hydro_finalize_launch(const HydroArgs& A, int take_back, cudaStream_t s);
 
 int floors_dt_blocks(int w, int h);
 void floors_dt_launch(const HydroConst& H, float* U, const float* gx, const float* gy, int do_floors, float* part_rate,
-                      float* part_g, long long* part_nf, double cfl, double eta_g, double dt_fixed, double dt_cap,
-                      DtRecord* rec, cudaStream_t s);
-void dt_advance_launch(DtRecord* rec, cudaStream_t s);
+                      float* part_g, long long* part_nf, unsigned* ticket, const DtRule& rule, cudaStream_t s);
 // Δt_{n+1} and the guard from per-CTA partials (the guard's codes are cell * channels + channel).
 void dt_finalize_launch(int nblocks, int channels, const float* part_rate, const float* part_g,
-                        const long long* part_nf, double cfl, double eta_g, double dt_fixed, double dt_cap,
-                        DtRecord* rec, cudaStream_t s);
+                        const long long* part_nf, const DtRule& rule, cudaStream_t s);

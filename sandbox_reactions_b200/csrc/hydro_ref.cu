@@ -1133,10 +1133,10 @@ void ref_floors_launch(const RefConst& R, float* U, cudaStream_t s) {
 }
 
 void ref_hold_dt_launch(const RefConst& R, float* U, uint8_t* held, const float* gx, const float* gy, int do_hold,
-                        int do_dt, float* part_rate, float* part_g, long long* part_nf, double cfl, double eta_g,
-                        double dt_fixed, double dt_cap, DtRecord* rec, cudaStream_t s) {
+                        int do_dt, float* part_rate, float* part_g, long long* part_nf, const DtRule& rule,
+                        cudaStream_t s) {
     const int nb = ref_grid((size_t)R.w * R.h);
     ref_hold_dt_kernel<<<nb, 256, 0, s>>>(R, U, held, gx, gy, do_hold, do_dt, part_rate, part_g, part_nf);
     sr_note_launch();
-    if (do_dt) dt_finalize_launch(nb, kRefChannels, part_rate, part_g, part_nf, cfl, eta_g, dt_fixed, dt_cap, rec, s);
+    if (do_dt) dt_finalize_launch(nb, kRefChannels, part_rate, part_g, part_nf, rule, s);
 }

@@ -63,5 +63,5 @@ void ref_floors_launch(const RefConst& R, float* U, cudaStream_t s);
 // The hold (floors.rs:196-243) and/or P9's per-CTA Δt terms with the 14-channel guard; then, with `do_dt`, the
 // finalize into `rec`.
 void ref_hold_dt_launch(const RefConst& R, float* U, uint8_t* held, const float* gx, const float* gy, int do_hold,
-                        int do_dt, float* part_rate, float* part_g, long long* part_nf, double cfl, double eta_g,
-                        double dt_fixed, double dt_cap, DtRecord* rec, cudaStream_t s);
+                        int do_dt, float* part_rate, float* part_g, long long* part_nf, const DtRule& rule,
+                        cudaStream_t s);
