@@ -1,6 +1,6 @@
 // batch.cu — many independent worlds advanced together on one GPU, each with its own context.
 //
-// After the worlds' first step (which tunes each world's multigrid), a batch step is ONE captured CUDA graph: from the
+// A batch step is ONE captured CUDA graph (a world with the learned preconditioner keeps the batch on the pool): from the
 // batch's stream it forks to every world's stream, each branch holds that world's whole step — P1 to P9, the implicit
 // step under device control with its conditional loops — and the branches join again. The graph is captured once per
 // combination of the worlds' state buffers (two, as the worlds alternate them in step) and replayed; the worlds'
@@ -209,7 +209,7 @@ sr_status sr_batch_step(sr_batch* b, uint32_t steps, double* device_ms) {
     try {
         while (done < steps) {
             BatchGraph* g = batch_graph(b);
-            if (!g) {  // a world not ready for capture (its first step tunes its multigrid): one step on the pool
+            if (!g) {  // a world that cannot be captured (the learned preconditioner): one step on the pool
                 pool_steps(b, 1, status);
                 done++;
                 bool bad = false;

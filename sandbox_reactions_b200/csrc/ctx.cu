@@ -617,7 +617,7 @@ static void run_steps(sr_ctx* c, uint32_t steps) {
         return;
     }
     const unsigned long long launches0 = sr_launches();
-    // after the first step (which tunes the multigrid) every step is one captured graph, unless the per-pass timing
+    // every step is one captured graph (not under the learned preconditioner), unless the per-pass timing
     // (2) asks for the passes launched one by one; timing 1 records the device time of each step's graph
     if (c->timing != 2 && steps && capturable(c)) {
         for (uint32_t s = 0; s < steps; s++) {

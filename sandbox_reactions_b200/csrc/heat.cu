@@ -1759,7 +1759,7 @@ void heat_sync_report(HeatSolver* H, cudaStream_t s) {
 
 void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev, cudaStream_t s,
                sr_heat_report* rep) {
-    if (H->precond != SR_PRECOND_LEARNED && H->use_graphs && H->mg.tuned) {
+    if (H->precond != SR_PRECOND_LEARNED && H->use_graphs) {
         // the device-controlled step: captured once per state buffer, then replayed with no host round trip
         auto it = H->step_graphs.find(U);
         if (it == H->step_graphs.end()) {
@@ -1897,7 +1897,7 @@ void heat_report(HeatSolver* H, cudaStream_t s, sr_heat_report* rep) {
 void heat_account_launches(HeatSolver* H, cudaStream_t s) { heat_sync_report(H, s); }
 
 bool heat_capturable(const HeatSolver* H) {
-    return H->precond != SR_PRECOND_LEARNED && H->use_graphs && H->mg.tuned;
+    return H->precond != SR_PRECOND_LEARNED && H->use_graphs;
 }
 
 void heat_prepare_capture(HeatSolver* H, cudaStream_t s) {

@@ -220,7 +220,7 @@ constexpr size_t smooth_smem() {
     return (size_t)RN * (PRE ? 6 : 5) * sizeof(float);
 }
 
-template <int NS, bool PRE, int SX, int SY, int NT, bool VEC, bool WT>
+template <int NS, bool PRE, int SX, int SY, int NT>
 __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, const float* __restrict__ xc,
                                                                     float omega, double* part, unsigned* counter,
                                                                     double* out) {
@@ -232,59 +232,6 @@ __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, con
     const int w = L.w, h = L.h;
     const int X0 = blockIdx.x * SX - H, Y0 = blockIdx.y * SY - H;  // X0 + Y0 even: local colour = global colour
     const int tid = threadIdx.x;
-    if constexpr (VEC) {
-        // rows in 16-byte chunks from the 4-aligned column at or left of X0 (the level's width is a multiple of 4, so a
-        // chunk lies wholly inside or wholly outside the level): 4 cells' b, c, dx, dy, the row above's dy, and for
-        // POST x and the two coarse corrections, in 6-7 loads
-        constexpr int OFF = (4 - H % 4) % 4, NCH = (OFF + RX + 3) / 4, NV = RY * NCH;
-        const int X0a = X0 - OFF;
-        constexpr int NVL = (NV + NT - 1) / NT;
-#pragma unroll
-        for (int it = 0; it < NVL; it++) {
-            const int k = tid + it * NT;
-            if (k >= NV) break;
-            const int ly = k / NCH, ch = k - ly * NCH;
-            const int gx0 = X0a + 4 * ch, gy = Y0 + ly;
-            float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f), c4 = make_float4(1.f, 1.f, 1.f, 1.f), dx4 = b4, dy4 = b4,
-                   dyu4 = b4, x4 = b4;
-            float dxl = 0.0f;
-            float2 xc2 = make_float2(0.f, 0.f);
-            float4 t4 = b4;
-            const bool in = gy >= 0 && gy < h && gx0 >= 0 && gx0 < w;
-            if (in) {
-                const size_t i = (size_t)gy * w + gx0;
-                b4 = *reinterpret_cast<const float4*>(L.b + i);
-                c4 = *reinterpret_cast<const float4*>(L.c + i);
-                dx4 = *reinterpret_cast<const float4*>(L.dx + i);
-                dy4 = *reinterpret_cast<const float4*>(L.dy + i);
-                if (gy > 0) dyu4 = *reinterpret_cast<const float4*>(L.dy + i - w);
-                if (gx0 > 0) dxl = L.dx[i - 1];
-                if (!PRE) {
-                    x4 = *reinterpret_cast<const float4*>(L.x + i);
-                    if constexpr (WT) t4 = *reinterpret_cast<const float4*>(L.t + i);
-                    xc2 = *reinterpret_cast<const float2*>(xc + (size_t)(gy >> 1) * C.w + (gx0 >> 1));
-                }
-            }
-            const float bb[4] = {b4.x, b4.y, b4.z, b4.w}, cc[4] = {c4.x, c4.y, c4.z, c4.w};
-            const float dxa[5] = {dxl, dx4.x, dx4.y, dx4.z, dx4.w}, dya[4] = {dy4.x, dy4.y, dy4.z, dy4.w};
-            const float dyua[4] = {dyu4.x, dyu4.y, dyu4.z, dyu4.w}, xa[4] = {x4.x, x4.y, x4.z, x4.w};
-            const float xcv[2] = {xc2.x, xc2.y}, ta[4] = {t4.x, t4.y, t4.z, t4.w};
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int lx = 4 * ch + e - OFF;
-                if (lx < 0 || lx >= RX) continue;
-                const float inv = in ? __fdividef(1.0f, cc[e] + dxa[e + 1] + dxa[e] + dya[e] + dyua[e]) : 0.0f;
-                const float x = (!PRE && in) ? xa[e] + omega * (WT ? ta[e] : 1.0f) * xcv[e >> 1] : 0.0f;
-                const int col = (lx + ly) & 1, q = ly * HX + (lx >> 1);
-                arr(A_X, col)[q] = x;
-                arr(A_B, col)[q] = bb[e];
-                arr(A_INV, col)[q] = inv;
-                arr(A_DX, col)[q] = dxa[e + 1];
-                arr(A_DY, col)[q] = dya[e];
-                if (PRE) arr(A_C, col)[q] = cc[e];
-            }
-        }
-    } else {
     constexpr int NLOAD = (RN + NT - 1) / NT;
 #pragma unroll
     for (int it = 0; it < NLOAD; it++) {
@@ -300,7 +247,7 @@ __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, con
             dx = L.dx[i];
             dy = L.dy[i];
             const float dxl = gx > 0 ? L.dx[i - 1] : 0.0f, dyu = gy > 0 ? L.dy[i - w] : 0.0f;
-            if (!PRE) x = L.x[i] + omega * (WT ? L.t[i] : 1.0f) * xc[(size_t)(gy >> 1) * C.w + (gx >> 1)];
+            if (!PRE) x = L.x[i] + omega * L.t[i] * xc[(size_t)(gy >> 1) * C.w + (gx >> 1)];
             inv = __fdividef(1.0f, c + dx + dxl + dy + dyu);  // the smoother's diagonal: an approximate reciprocal
         }
         const int col = (lx + ly) & 1, q = ly * HX + (lx >> 1);
@@ -310,7 +257,6 @@ __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, con
         arr(A_DX, col)[q] = dx;
         arr(A_DY, col)[q] = dy;
         if (PRE) arr(A_C, col)[q] = c;
-    }
     }
     __syncthreads();
     constexpr int NSWEEP = (HN + NT - 1) / NT;
@@ -384,12 +330,8 @@ __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, con
                     ax += arr(A_DX, col)[q] * (xj - xo[right]);
                     ax += arr(A_DY, oth)[q - HX] * (xj - xo[q - HX]);
                     ax += arr(A_DY, col)[q] * (xj - xo[q + HX]);
-                    if constexpr (WT) {
-                        const int gx = X0 + lx, gy = Y0 + ly;
-                        sum += (gx < w && gy < h ? L.t[gy * w + gx] : 0.0f) * (arr(A_B, col)[q] - ax);
-                    } else {
-                        sum += arr(A_B, col)[q] - ax;
-                    }
+                    const int gx = X0 + lx, gy = Y0 + ly;
+                    sum += (gx < w && gy < h ? L.t[gy * w + gx] : 0.0f) * (arr(A_B, col)[q] - ax);
                 }
             C.b[(size_t)Y * C.w + X] = C.mask[(size_t)Y * C.w + X] ? sum : 0.0f;
         }
@@ -406,13 +348,15 @@ __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, con
 // neighbours the same lane's rows above and below (registers), except across a band edge, whose rows go through shared
 // memory once per half-sweep (double-buffered: one barrier per half-sweep). Which cell of a pair a colour updates is
 // fixed by the row's parity (the region starts on an even column and row, so local parity = global parity), so the
-// sweeps unroll into straight-line code. The halo is NS + 2 for the pre-smoother (NS + 1 keeps the restriction's
-// neighbours exact; one more keeps the region on even columns, so pairs load as 8-byte words and sit inside one 2 x 2
-// aggregate) and NS for the post-smoother. Cells outside the level: b = 0, c = 1, no couplings, inverse diagonal 0.
+// sweeps unroll into straight-line code. The halo is NS for both: the post-smoother's first half-sweep reads
+// neighbours and its last result none beyond; the pre-smoother's first half-sweep starts from x = 0 and reads none, and
+// the residual after the last one reads them. (NS + 2 for the pre-smoother, as if its first half-sweep read
+// neighbours, took 19 % more CTAs under V(4,4).) An even halo keeps pairs on 8-byte words inside one aggregate. Cells
+// outside the level: b = 0, c = 1, no couplings, inverse diagonal 0.
 constexpr int RB_R = 4, RB_WARPS = 16, RB_NT = 32 * RB_WARPS, RB_RX = 64, RB_RY = RB_R * RB_WARPS;
 
 template <int NS, bool PRE>
-constexpr int rb_halo() { return PRE ? NS + 2 : NS; }
+constexpr int rb_halo() { return NS; }
 
 template <int NS, bool PRE, bool WT>
 __global__ void __launch_bounds__(RB_NT, 2) mg_rowband_kernel(MgLevel L, MgLevel C, const float* __restrict__ xc,
@@ -1334,30 +1278,13 @@ __global__ void __launch_bounds__(TS_NT) mg_tail_setup_kernel(const __grid_const
     }
 }
 
-template <int NS, bool PRE, int SX, int SY, int NT, bool VEC, bool WT>
-void launch_one(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, unsigned* counter,
-                double* out, cudaStream_t s) {
-    const dim3 grid(div_up(L.w, SX), div_up(L.h, SY));
-    mg_smooth_kernel<NS, PRE, SX, SY, NT, VEC, WT><<<grid, NT, smooth_smem<NS, PRE, SX, SY>(), s>>>(
-        L, C, xc, omega, part, counter, out);
-}
-
+// Level 0's width is even, so every level that comes here has weights.
 template <int NS, bool PRE, int SX, int SY, int NT>
 void launch_smooth_t(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, unsigned* counter,
                      double* out, cudaStream_t s) {
-    // 16-byte rows (and 8-byte coarse pairs) stay aligned; the pre-smoother's odd halo would load 8 % more columns, and
-    // measured slower, so it keeps the per-cell loads. Level 0 has no weights (its kernels read none).
-    const bool wt = L.t != nullptr;
-    if constexpr (!PRE) {
-        if (L.w % 4 == 0 && C.w % 2 == 0) {
-            if (wt) launch_one<NS, PRE, SX, SY, NT, true, true>(L, C, xc, omega, part, counter, out, s);
-            else launch_one<NS, PRE, SX, SY, NT, true, false>(L, C, xc, omega, part, counter, out, s);
-            sr_note_launch();
-            return;
-        }
-    }
-    if (wt) launch_one<NS, PRE, SX, SY, NT, false, true>(L, C, xc, omega, part, counter, out, s);
-    else launch_one<NS, PRE, SX, SY, NT, false, false>(L, C, xc, omega, part, counter, out, s);
+    const dim3 grid(div_up(L.w, SX), div_up(L.h, SY));
+    mg_smooth_kernel<NS, PRE, SX, SY, NT><<<grid, NT, smooth_smem<NS, PRE, SX, SY>(), s>>>(L, C, xc, omega, part,
+                                                                                        counter, out);
     sr_note_launch();
 }
 
@@ -1418,50 +1345,48 @@ void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float o
     sr_note_launch();
 }
 
+// The row-band kernel wherever the level's width is even (it loads cell pairs as 8-byte words): its registers beat the
+// shared-memory tiles at every size (level 0 of a 512² world under V(4,4): pre 11.9 -> 4.7 us, post 12.5 -> 7.0). Levels
+// of odd width take the shared-memory tiles, the small one where the big one leaves fewer than 2 CTAs per SM.
 template <int NS, bool PRE>
 void launch_smooth(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, unsigned* counter,
-                   double* out, int tile, cudaStream_t s) {
-    if (tile < 0 ? small_tiles(L) : tile == 1)
+                   double* out, cudaStream_t s) {
+    if (L.w % 2 == 0)
+        launch_rowband<NS, PRE>(L, C, xc, omega, part, counter, out, s);
+    else if (small_tiles(L))
         launch_smooth_t<NS, PRE, SMALL_SX, tile_sy<NS, PRE, SMALL_SX, SMALL_SY, SMALL_NT>(), SMALL_NT>(
             L, C, xc, omega, part, counter, out, s);
-    else if (L.w % 2 == 0)  // the row-band kernel loads cell pairs as 8-byte words
-        launch_rowband<NS, PRE>(L, C, xc, omega, part, counter, out, s);
     else
         launch_smooth_t<NS, PRE, BIG_SX, tile_sy<NS, PRE, BIG_SX, BIG_SY, BIG_NT>(), BIG_NT>(L, C, xc, omega, part,
                                                                                            counter, out, s);
 }
 
-// `tile`: 0 the big tile, 1 the small one, -1 by the CTA-count rule (small_tiles).
 void smooth(int nu, bool pre, const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part,
-            unsigned* counter, double* out, cudaStream_t s, int tile = -1) {
+            unsigned* counter, double* out, cudaStream_t s) {
     if (pre) {
-        if (nu == 1) launch_smooth<2, true>(L, C, xc, omega, part, counter, out, tile, s);
-        else if (nu == 2) launch_smooth<4, true>(L, C, xc, omega, part, counter, out, tile, s);
-        else if (nu == 3) launch_smooth<6, true>(L, C, xc, omega, part, counter, out, tile, s);
-        else launch_smooth<8, true>(L, C, xc, omega, part, counter, out, tile, s);
+        if (nu == 1) launch_smooth<2, true>(L, C, xc, omega, part, counter, out, s);
+        else if (nu == 2) launch_smooth<4, true>(L, C, xc, omega, part, counter, out, s);
+        else if (nu == 3) launch_smooth<6, true>(L, C, xc, omega, part, counter, out, s);
+        else launch_smooth<8, true>(L, C, xc, omega, part, counter, out, s);
     } else {
-        if (nu == 1) launch_smooth<2, false>(L, C, xc, omega, part, counter, out, tile, s);
-        else if (nu == 2) launch_smooth<4, false>(L, C, xc, omega, part, counter, out, tile, s);
-        else if (nu == 3) launch_smooth<6, false>(L, C, xc, omega, part, counter, out, tile, s);
-        else launch_smooth<8, false>(L, C, xc, omega, part, counter, out, tile, s);
+        if (nu == 1) launch_smooth<2, false>(L, C, xc, omega, part, counter, out, s);
+        else if (nu == 2) launch_smooth<4, false>(L, C, xc, omega, part, counter, out, s);
+        else if (nu == 3) launch_smooth<6, false>(L, C, xc, omega, part, counter, out, s);
+        else launch_smooth<8, false>(L, C, xc, omega, part, counter, out, s);
     }
 }
 
-template <int NS, bool PRE, int SX, int SY, int NT, bool VEC, bool WT>
+template <int NS, bool PRE, int SX, int SY, int NT>
 void set_attribute_one() {
-    SR_CUDA_TRY(cudaFuncSetAttribute(mg_smooth_kernel<NS, PRE, SX, SY, NT, VEC, WT>,
+    SR_CUDA_TRY(cudaFuncSetAttribute(mg_smooth_kernel<NS, PRE, SX, SY, NT>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smooth_smem<NS, PRE, SX, SY>()));
 }
 
 template <int NS, int SX, int SY, int NT>
 void set_attributes_tile() {
     constexpr int PSY = tile_sy<NS, true, SX, SY, NT>(), QSY = tile_sy<NS, false, SX, SY, NT>();
-    set_attribute_one<NS, true, SX, PSY, NT, false, false>();
-    set_attribute_one<NS, true, SX, PSY, NT, false, true>();
-    set_attribute_one<NS, false, SX, QSY, NT, false, false>();
-    set_attribute_one<NS, false, SX, QSY, NT, false, true>();
-    set_attribute_one<NS, false, SX, QSY, NT, true, false>();
-    set_attribute_one<NS, false, SX, QSY, NT, true, true>();
+    set_attribute_one<NS, true, SX, PSY, NT>();
+    set_attribute_one<NS, false, SX, QSY, NT>();
 }
 
 template <int NS>
@@ -1577,57 +1502,6 @@ void Multigrid::set_couplings(const double* kx, const double* ky, const uint8_t*
     sr_note_launch();
 }
 
-// The smoother tile of each level below 0 (level 0 keeps the CTA-count rule, which bounds its grid-sum partials),
-// chosen by timing on the level's first operator: per candidate (the big and the small tile) one warm-up pre- and
-// post-smoother, then the median of kTuneReps timed pairs; the rule's tile is kept unless the other is at least
-// kTuneMargin faster, so that run-to-run noise does not flip a choice. Choices are kept per level size for the process
-// (a batch's worlds of one size tune once).
-constexpr int kTuneReps = 7;
-constexpr float kTuneMargin = 0.95f;
-
-void Multigrid::autotune(cudaStream_t s) {
-    static std::mutex mu;
-    static std::map<std::tuple<int, int, int, int>, int> chosen;  // (w, h, sweeps before, after) -> tile
-    tuned = true;
-    cudaEvent_t a, b;
-    SR_CUDA_TRY(cudaEventCreate(&a));
-    SR_CUDA_TRY(cudaEventCreate(&b));
-    for (int l = 1; l < tail; l++) {
-        const std::tuple<int, int, int, int> key(L[l].w, L[l].h, pre, post);
-        {
-            std::lock_guard<std::mutex> g(mu);
-            auto it = chosen.find(key);
-            if (it != chosen.end()) {
-                tile[l] = it->second;
-                continue;
-            }
-        }
-        float med[2];
-        for (int cand = 0; cand < 2; cand++) {
-            float t[kTuneReps];
-            for (int rep = -1; rep < kTuneReps; rep++) {  // rep -1 warms up
-                SR_CUDA_TRY(cudaEventRecord(a, s));
-                smooth(pre, true, L[l], L[l + 1], nullptr, omega, nullptr, nullptr, nullptr, s, cand);
-                smooth(post, false, L[l], L[l + 1], L[l + 1].x2, omega, nullptr, nullptr, nullptr, s, cand);
-                SR_CUDA_TRY(cudaEventRecord(b, s));
-                SR_CUDA_TRY(cudaEventSynchronize(b));
-                float ms = 0.0f;
-                SR_CUDA_TRY(cudaEventElapsedTime(&ms, a, b));
-                if (rep >= 0) t[rep] = ms;
-            }
-            std::sort(t, t + kTuneReps);
-            med[cand] = t[kTuneReps / 2];
-        }
-        const int rule = small_tiles(L[l]) ? 1 : 0, other = 1 - rule;
-        const int pick = med[other] < kTuneMargin * med[rule] ? other : rule;
-        tile[l] = pick;
-        std::lock_guard<std::mutex> g(mu);
-        chosen[key] = pick;
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-}
-
 void Multigrid::coarsen(cudaStream_t s) {
     for (int l = 1; l <= tail; l++) {
         if (l == 1) {
@@ -1642,14 +1516,13 @@ void Multigrid::coarsen(cudaStream_t s) {
     tail_args(*this, T);
     mg_tail_setup_kernel<<<1, TS_NT, sizeof(TailSetupShared), s>>>(T, L[tail], tail_img);
     sr_note_launch();
-    if (!tuned) autotune(s);
 }
 
 void Multigrid::apply(const float* r, float* z, double* part, unsigned* counter, double* rz_out, cudaStream_t s) {
     L[0].b = const_cast<float*>(r);
     L[0].x2 = z;
     for (int l = 0; l < tail; l++)
-        smooth(pre, true, L[l], L[l + 1], nullptr, omega, nullptr, nullptr, nullptr, s, tile[l]);
+        smooth(pre, true, L[l], L[l + 1], nullptr, omega, nullptr, nullptr, nullptr, s);
     TailArgs T;
     const size_t ts = tail_args(*this, T);
     T.out = tail == 0 ? rz_out : nullptr;
@@ -1657,7 +1530,7 @@ void Multigrid::apply(const float* r, float* z, double* part, unsigned* counter,
     sr_note_launch();
     for (int l = tail - 1; l >= 0; l--)
         smooth(post, false, L[l], L[l + 1], L[l + 1].x2, omega, l == 0 ? part : nullptr, l == 0 ? counter : nullptr,
-               l == 0 ? rz_out : nullptr, s, tile[l]);
+               l == 0 ? rz_out : nullptr, s);
 }
 
 void Multigrid::time_level0(int reps, void* flush, size_t flush_bytes, cudaStream_t s, double* pre_ms,
