@@ -45,6 +45,7 @@ struct sr_ctx {
     int cur = 0;
     float *phi = nullptr, *gx = nullptr, *gy = nullptr;             // P2's field of the step's start state
     float *src = nullptr, *phim = nullptr, *gxm = nullptr, *gym = nullptr;  // the half step's source and field
+    float* mid = nullptr;                                           // 4 channels: the half step's Σ, Σu, Σv and mass fluxes
     float* kappa = nullptr;
     // reference mode (14 channels)
     int nc = 4;                   // channels of the state
@@ -159,6 +160,7 @@ static void ctx_free(sr_ctx* c) {
     cudaFree(c->U[1]);
     cudaFree(c->phi); cudaFree(c->gx); cudaFree(c->gy);
     cudaFree(c->src); cudaFree(c->phim); cudaFree(c->gxm); cudaFree(c->gym);
+    cudaFree(c->mid);
     cudaFree(c->kappa);
     for (sr_ctx* s : c->subs) ctx_free(s);
     cudaFree(c->box_part); cudaFree(c->box_rec); cudaFree(c->plane32);
@@ -330,6 +332,9 @@ static HydroArgs hydro_args(sr_ctx* c, int cur) {
     A.gx = c->cfg.gravity ? c->gx : nullptr;
     A.gy = c->cfg.gravity ? c->gy : nullptr;
     A.src = c->src;
+    A.mid = c->mid;
+    A.mfx = c->mid ? c->mid + 3 * c->n : nullptr;
+    A.mfy = c->mid ? c->mid + 4 * c->n : nullptr;
     A.phim = c->phim;
     A.gxm = c->gxm;
     A.gym = c->gym;
@@ -388,11 +393,11 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
     if (k.hydro) {
         HydroArgs A = hydro_args(c, cur);
         if (k.gravity) {
-            hydro_launch(kHydroSource, A, s);
-            c->grav.solve(c->src, c->phim, c->gxm, c->gym, s);
             mark(2);
-            hydro_launch(kHydroUpdateGrav, A, s);
+            hydro_launch(kHydroPredict, A, s);
             mark(3);
+            c->grav.solve(c->src, c->phim, c->gxm, c->gym, s);
+            hydro_gravity_launch(A, s);
         } else {
             mark(2);
             hydro_launch(k.heat ? kHydroUpdate : kHydroStep, A, s);
@@ -772,6 +777,7 @@ sr_status sr_create(const sr_config* cfg, sr_ctx** out) {
             dalloc(&c->phim, n);
             dalloc(&c->gxm, n);
             dalloc(&c->gym, n);
+            if (c->nc == 4 && cfg->hydro) dalloc(&c->mid, 5 * n);
             c->grav.create(c->w, c->h, (int)cfg->kernel, cfg->G, cfg->softening, (float)cfg->sigma_vac);
             c->grav_ready = true;
         }

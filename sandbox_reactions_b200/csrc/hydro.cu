@@ -6,9 +6,12 @@
 // (y), and the per-cell epilogue of the pass finishes:
 //   - kHydroStep:       U' = U - Δt ΔF, then P8's floors and P9's Δt on U' (no gravity, no heat: the whole step);
 //   - kHydroUpdate:     U' = U - Δt ΔF (no gravity; heat follows);
-//   - kHydroSource:     the half step's gravity source ½(Σⁿ + Σⁿ⁺¹), masked (reference hydro.rs:815-836);
-//   - kHydroUpdateGrav: U' with gravity's half-step kick and the faces' work across φ_mid (hydro.rs:871-947), the net
-//                       kick taken back from the densest cell.
+//   - kHydroPredict:    with gravity: U - Δt ΔF, the half step's source ½(Σⁿ + Σⁿ⁺¹), masked (reference
+//                       hydro.rs:815-836), and what gravity's work reads — the half-step (Σ, Σu, Σv) and the faces'
+//                       mass fluxes. Once φ_mid is solved, hydro_gravity_kernel adds the half-step kick and the faces'
+//                       work across it (hydro.rs:871-947) and takes the net kick back from the densest cell.
+// The predictor runs once a step: it is what the step costs (FP32 issue), and a second run of it after the solve, to
+// recompute fluxes that 20 B a cell can carry over, took 172 + 331 us at 2048² where predict and gravity take 198 + 90.
 // The scheme follows crates/sr-physics/src/reference/hydro.rs (step_held without held cells, sinks or radiation).
 #include "hydro.cuh"
 
@@ -145,13 +148,7 @@ struct RatePart {
         return RatePart{__shfl_down_sync(0xffffffffu, nf, o), __shfl_down_sync(0xffffffffu, rate, o)};
     }
 };
-union Part {
-    double align[3];
-    __device__ __forceinline__ KickPart& kick() { return *reinterpret_cast<KickPart*>(this); }
-    __device__ __forceinline__ RatePart& rate() { return *reinterpret_cast<RatePart*>(this); }
-};
-static_assert(sizeof(KickPart) == sizeof(Part) && sizeof(RatePart) <= sizeof(Part), "a partial's slot");
-static_assert(sizeof(Part) == kHydroPartBytes, "the partials' buffer");
+static_assert(sizeof(KickPart) == kHydroPartBytes && sizeof(RatePart) <= kHydroPartBytes, "a partial's slot");
 
 template <class P>
 __device__ __forceinline__ P warp_merge(P v) {
@@ -205,7 +202,7 @@ struct __align__(128) BandShared {
     float M[3][HB_W][32];        // half-step (Σ, Σu, Σv) of each lane's cell
     float YF[7][HB_W][32];       // each lane's y+ face
     float FY[4][HB_W][32];       // the flux through each lane's top face
-    Part red[HB_W];              // the rows' partials
+    RatePart red[HB_W];          // the rows' partials
     uint64_t mbar;
 };
 
@@ -376,6 +373,148 @@ __device__ void dt_close(const DtRule& R, float rate, float gmax, long long nf, 
     }
 }
 
+// The CTA's last word on gravity's kick: its warps' partials merged, then the grid's; the warp that arrives last takes
+// the net kick on the gas's own field back from the densest cell (hydro.rs:1004-1012).
+template <int WARPS>
+__device__ __forceinline__ void take_back(KickPart kp, KickPart* red, const HydroArgs& A) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const size_t n = (size_t)A.H.w * A.H.h;
+    kp = warp_merge(kp);
+    if (lane == 0) red[warp] = kp;
+    __syncthreads();
+    if (warp > 0) return;
+    kp = warp_merge(lane < WARPS ? red[lane] : KickPart::none());
+    if (grid_total(kp, A.part, A.tickets) && lane == 0 && kp.idx >= 0) {
+        A.Uout[n + kp.idx] = __ldcg(A.Uout + n + kp.idx) - (float)kp.kx;
+        A.Uout[2 * n + kp.idx] = __ldcg(A.Uout + 2 * n + kp.idx) - (float)kp.ky;
+    }
+}
+
+// Gravity's part of the step, after the half step's solve: each cell's kick Δt Σ_src g_mid and its four faces' work.
+// A thread takes four neighbouring columns (16-byte accesses: the world's width is a multiple of 8) of HG_R rows,
+// works out the faces to the right of and below each of its cells once, and hands the right one to the next lane; a
+// cell with no gas around it (its source stored as -0) takes nothing but lends its faces. Bound by HBM: 68 B a cell.
+constexpr int HG_R = 4, HG_WARPS = 4;
+
+__global__ void __launch_bounds__(32 * HG_WARPS) hydro_gravity_kernel(HydroArgs A) {
+    __shared__ KickPart red[HG_WARPS];
+    const int w = A.H.w, h = A.H.h;
+    const size_t n = (size_t)w * h;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x = blockIdx.x * 128 + 4 * lane, y0 = (blockIdx.y * HG_WARPS + warp) * HG_R;
+    const float dt = (float)(*A.dt);
+    const bool on = x < w;
+    struct Row {
+        float m[3][4], p[4];
+    };
+    auto load4 = [&](const float* a, size_t i, float* v) {
+        const float4 q = *reinterpret_cast<const float4*>(a + i);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    };
+    auto load_row = [&](int y, Row& r) {
+        const bool ok = on && y >= 0 && y < h;
+        const size_t i = ok ? (size_t)y * w + x : 0;
+#pragma unroll
+        for (int k = 0; k < 3; k++) load4(A.mid + k * n, i, r.m[k]);
+        load4(A.phim, i, r.p);
+    };
+    KickPart kp = KickPart::none();
+    Row c, d;
+    float upk[4], upe[4];  // the face above each cell: impulse to the cell above, energy to this one
+    load_row(y0, c);
+    {
+        Row a;
+        float f[4];
+        load_row(y0 - 1, a);
+        const bool ok = on && y0 > 0 && y0 < h;
+        load4(A.mfy, ok ? (size_t)(y0 - 1) * w + x : 0, f);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float o[3] = {0.0f, 0.0f, 0.0f};
+            if (ok) face_work(f[k], a.m[0][k], c.m[0][k], a.m[2][k], c.m[2][k], a.p[k] - c.p[k], dt, o);
+            upk[k] = o[0];
+            upe[k] = o[2];
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < HG_R; r++) {
+        const int y = y0 + r;
+        const bool row = y < h;
+        const bool ok = on && row;
+        const size_t i = ok ? (size_t)y * w + x : 0;
+        load_row(y + 1, d);
+        float fx[4], fy[4], src[4], gx[4], gy[4], u1[4], u2[4], u3[4];
+        load4(A.mfx, i, fx);
+        load4(A.mfy, i, fy);
+        load4(A.src, i, src);
+        load4(A.gxm, i, gx);
+        load4(A.gym, i, gy);
+        load4(A.Uout + n, i, u1);
+        load4(A.Uout + 2 * n, i, u2);
+        load4(A.Uout + 3 * n, i, u3);
+        // the next column's mids and potential
+        float mn[2], pn;
+        mn[0] = __shfl_down_sync(0xffffffffu, c.m[0][0], 1);
+        mn[1] = __shfl_down_sync(0xffffffffu, c.m[1][0], 1);
+        pn = __shfl_down_sync(0xffffffffu, c.p[0], 1);
+        const bool has_right = ok && x + 4 < w;
+        if (lane == 31 && has_right) {
+            mn[0] = A.mid[i + 4];
+            mn[1] = A.mid[n + i + 4];
+            pn = A.phim[i + 4];
+        }
+        float rk[4], rl[4], rh[4];  // the face right of each cell: impulse and energy to the cell, energy to the next
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float o[3] = {0.0f, 0.0f, 0.0f};
+            if (k < 3 ? ok : has_right)
+                face_work(fx[k], c.m[0][k], k < 3 ? c.m[0][k < 3 ? k + 1 : 3] : mn[0], c.m[1][k],
+                          k < 3 ? c.m[1][k < 3 ? k + 1 : 3] : mn[1], c.p[k] - (k < 3 ? c.p[k < 3 ? k + 1 : 3] : pn), dt, o);
+            rk[k] = o[0];
+            rl[k] = o[1];
+            rh[k] = o[2];
+        }
+        float lk = __shfl_up_sync(0xffffffffu, rk[3], 1), lh = __shfl_up_sync(0xffffffffu, rh[3], 1);
+        if (lane == 0) {
+            float o[3] = {0.0f, 0.0f, 0.0f};
+            if (ok && x > 0)
+                face_work(A.mfx[i - 1], A.mid[i - 1], c.m[0][0], A.mid[n + i - 1], c.m[1][0], A.phim[i - 1] - c.p[0], dt, o);
+            lk = o[0];
+            lh = o[2];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float o[3] = {0.0f, 0.0f, 0.0f};
+            if (ok && y + 1 < h)
+                face_work(fy[k], c.m[0][k], d.m[0][k], c.m[2][k], d.m[2][k], c.p[k] - d.p[k], dt, o);
+            const bool empty = src[k] == 0.0f && signbit(src[k]);
+            if (ok && !empty) {
+                float kick[2] = {dt * src[k] * gx[k], dt * src[k] * gy[k]};
+                KickPart one{(double)kick[0], (double)kick[1], 0.0f, -1};
+                if (src[k] > 0.0f) {
+                    one.best = src[k];
+                    one.idx = (int)i + k;
+                }
+                kp.merge(one);
+                kick[0] += rk[k] - (k ? rk[k ? k - 1 : 0] : lk);
+                kick[1] += o[0] - upk[k];
+                u1[k] += kick[0];
+                u2[k] += kick[1];
+                u3[k] += rl[k] + (k ? rh[k ? k - 1 : 0] : lh) + o[1] + upe[k];
+            }
+            upk[k] = o[0];
+            upe[k] = o[2];
+        }
+        if (ok) {
+            *reinterpret_cast<float4*>(A.Uout + n + i) = make_float4(u1[0], u1[1], u1[2], u1[3]);
+            *reinterpret_cast<float4*>(A.Uout + 2 * n + i) = make_float4(u2[0], u2[1], u2[2], u2[3]);
+            *reinterpret_cast<float4*>(A.Uout + 3 * n + i) = make_float4(u3[0], u3[1], u3[2], u3[3]);
+        }
+        c = d;
+    }
+    take_back<HG_WARPS>(kp, red, A);
+}
+
 template <int MODE, int LIM, bool BRACKET>
 __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_constant__ CUtensorMap map, HydroArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -536,21 +675,6 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
     const bool empty = vac && sh.S[sy][sx - 1] < sv && sh.S[sy][sx + 1] < sv && sh.S[sy - 1][sx] < sv &&
                        sh.S[sy + 1][sx] < sv;
 
-    if (MODE == kHydroSource) {
-        if (!inside) return;
-        float s;
-        if (empty) {
-            s = 0.0f;
-        } else {
-            const float start = vac ? sh.P[sy][sx].x : sh.S[sy][sx];
-            const float div = (fr[0] - fl[0]) + (fd[0] - fu[0]);
-            s = 0.5f * (sh.S[sy][sx] + (start - dt * div));
-        }
-        A.src[i] = s >= sv ? s : 0.0f;
-        return;
-    }
-
-    KickPart kp = KickPart::none();
     RatePart rp = RatePart::none();
     if (inside) {
         const int bx = X - xs, by = Y - ys;
@@ -563,51 +687,22 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
         if (!empty) {
 #pragma unroll
             for (int q = 0; q < 4; q++) u[q] -= dt * ((fr[q] - fl[q]) + (fd[q] - fu[q]));
-            if (MODE == kHydroUpdateGrav) {
-                const float m[3] = {sh.M[0][row][lane], sh.M[1][row][lane], sh.M[2][row][lane]};
-                const float src = A.src[i];
-                float kick[2] = {dt * src * A.gxm[i], dt * src * A.gym[i]};
-                kp.kx = (double)kick[0];
-                kp.ky = (double)kick[1];
-                if (src > 0.0f) {
-                    kp.best = src;
-                    kp.idx = (int)i;
-                }
-                const float p = A.phim[i];
-                float pr = p, pl = p, pd = p, pu = p;
-                float mr[3] = {m[0], m[1], m[2]}, ml[3] = {m[0], m[1], m[2]}, md[3] = {m[0], m[1], m[2]},
-                      mu[3] = {m[0], m[1], m[2]};
-                if (X + 1 < w) {
-                    pr = A.phim[i + 1];
-#pragma unroll
-                    for (int q = 0; q < 3; q++) mr[q] = sh.M[q][row][lane + 1];
-                }
-                if (X > 0) {
-                    pl = A.phim[i - 1];
-#pragma unroll
-                    for (int q = 0; q < 3; q++) ml[q] = sh.M[q][row][lane - 1];
-                }
-                if (Y + 1 < h) {
-                    pd = A.phim[i + w];
-#pragma unroll
-                    for (int q = 0; q < 3; q++) md[q] = sh.M[q][row + 1][lane];
-                }
-                if (Y > 0) {
-                    pu = A.phim[i - w];
-#pragma unroll
-                    for (int q = 0; q < 3; q++) mu[q] = sh.M[q][row - 1][lane];
-                }
-                float r[3], l[3], dn[3], up[3];
-                face_work(fr[0], m[0], mr[0], m[1], mr[1], p - pr, dt, r);
-                face_work(fl[0], ml[0], m[0], ml[1], m[1], pl - p, dt, l);
-                face_work(fd[0], m[0], md[0], m[2], md[2], p - pd, dt, dn);
-                face_work(fu[0], mu[0], m[0], mu[2], m[2], pu - p, dt, up);
-                kick[0] += r[0] - l[0];
-                kick[1] += dn[0] - up[0];
-                u[1] += kick[0];
-                u[2] += kick[1];
-                u[3] += r[1] + l[2] + dn[1] + up[2];
+        }
+        if (MODE == kHydroPredict) {
+            // what follows the half step's solve: an empty cell's source is -0 (gravity leaves the cell as it is)
+            float src = -0.0f;
+            if (!empty) {
+                const float start = vac ? sh.P[sy][sx].x : sh.S[sy][sx];
+                const float div = (fr[0] - fl[0]) + (fd[0] - fu[0]);
+                src = 0.5f * (sh.S[sy][sx] + (start - dt * div));
+                src = src >= sv ? src : 0.0f;
             }
+            A.src[i] = src;
+            A.mid[i] = sh.M[0][row][lane];
+            A.mid[n + i] = sh.M[1][row][lane];
+            A.mid[2 * n + i] = sh.M[2][row][lane];
+            A.mfx[i] = fr[0];
+            A.mfy[i] = fd[0];
         }
         if (MODE == kHydroStep) {
             floor_cell(H, u[0], u[1], u[2], u[3]);
@@ -620,26 +715,13 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
     }
 
     // ---- the grid's sums, in a fixed order: the rows of the tile, the CTAs of a grid row, the grid rows
-    if (MODE == kHydroUpdate) return;
-    if (MODE == kHydroUpdateGrav) {
-        kp = warp_merge(kp);
-        if (lane == 0) sh.red[row].kick() = kp;
-        __syncthreads();
-        if (row > 0) return;
-        kp = warp_merge(lane < HB_W ? sh.red[lane].kick() : KickPart::none());
-        // the net kick on the gas's own field taken back from the densest cell (hydro.rs:1004-1012)
-        if (grid_total(kp, A.part, A.tickets) && lane == 0 && kp.idx >= 0) {
-            A.Uout[n + kp.idx] = __ldcg(A.Uout + n + kp.idx) - (float)kp.kx;
-            A.Uout[2 * n + kp.idx] = __ldcg(A.Uout + 2 * n + kp.idx) - (float)kp.ky;
-        }
-    } else {
-        rp = warp_merge(rp);
-        if (lane == 0) sh.red[row].rate() = rp;
-        __syncthreads();
-        if (row > 0) return;
-        rp = warp_merge(lane < HB_W ? sh.red[lane].rate() : RatePart::none());
-        if (grid_total(rp, A.part, A.tickets) && lane == 0) dt_close(A.rule, rp.rate, 0.0f, rp.nf, 4);
-    }
+    if (MODE != kHydroStep) return;
+    rp = warp_merge(rp);
+    if (lane == 0) sh.red[row] = rp;
+    __syncthreads();
+    if (row > 0) return;
+    rp = warp_merge(lane < HB_W ? sh.red[lane] : RatePart::none());
+    if (grid_total(rp, A.part, A.tickets) && lane == 0) dt_close(A.rule, rp.rate, 0.0f, rp.nf, 4);
 }
 
 }  // namespace
@@ -714,8 +796,13 @@ void hydro_launch(int mode, const HydroArgs& A, cudaStream_t s) {
     tma_encode_planes(&map, A.U, A.H.w, A.H.h, 4, HB_BX, HB_BY);
     if (mode == kHydroStep) hydro_launch_m<kHydroStep>(map, A, s);
     else if (mode == kHydroUpdate) hydro_launch_m<kHydroUpdate>(map, A, s);
-    else if (mode == kHydroSource) hydro_launch_m<kHydroSource>(map, A, s);
-    else hydro_launch_m<kHydroUpdateGrav>(map, A, s);
+    else hydro_launch_m<kHydroPredict>(map, A, s);
+}
+
+void hydro_gravity_launch(const HydroArgs& A, cudaStream_t s) {
+    const dim3 grid(div_up(A.H.w, 128), div_up(A.H.h, HG_WARPS * HG_R));
+    hydro_gravity_kernel<<<grid, 32 * HG_WARPS, 0, s>>>(A);
+    sr_note_launch();
 }
 
 // ------------------------------------------------------------------------------------------------ P8 + P9

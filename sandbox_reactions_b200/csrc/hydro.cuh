@@ -3,7 +3,7 @@
 
 #include "common.cuh"
 
-enum { kHydroUpdate = 0, kHydroSource = 1, kHydroUpdateGrav = 2, kHydroStep = 3 };
+enum { kHydroUpdate = 0, kHydroPredict = 1, kHydroStep = 2 };
 
 // The Δt record kept on the device (crates/sr-engine/src/step/dt.rs:51-61): steps never wait on the host for it.
 struct DtRecord {
@@ -28,11 +28,14 @@ struct HydroArgs {
     HydroConst H;
     const double* dt;          // device Δt_n
     const float* U;            // state in: 4 planes
-    float* Uout;               // state out: 4 planes (kHydroUpdate*)
+    float* Uout;               // state out: 4 planes
     const float* gx;           // P2's field of the start state (nullptr: no gravity)
     const float* gy;
-    float* src;                // kHydroSource: out; kHydroUpdateGrav: in (Σ_src,mid)
-    const float* phim;         // the half step's φ, g (kHydroUpdateGrav)
+    float* src;                // kHydroPredict: out; hydro_gravity: in (Σ_src,mid; -0 where the cell is empty)
+    float* mid;                // likewise: the half-step Σ, Σu, Σv (3 planes)
+    float* mfx;                // likewise: the mass flux through each cell's +x and +y face
+    float* mfy;
+    const float* phim;         // the half step's φ, g (hydro_gravity)
     const float* gxm;
     const float* gym;
     void* part;                // partials of the grid's sums (hydro_part_count x kHydroPartBytes)
@@ -46,6 +49,8 @@ constexpr size_t kHydroPartBytes = 24;
 size_t hydro_part_count(int w, int h);
 size_t hydro_ticket_count(int h);
 void hydro_launch(int mode, const HydroArgs& A, cudaStream_t s);
+// After kHydroPredict and the half step's solve: gravity's kick and work on Uout, the net kick taken back.
+void hydro_gravity_launch(const HydroArgs& A, cudaStream_t s);
 
 int floors_dt_blocks(int w, int h);
 void floors_dt_launch(const HydroConst& H, float* U, const float* gx, const float* gy, int do_floors, float* part_rate,
