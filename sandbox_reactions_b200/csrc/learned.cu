@@ -1,13 +1,12 @@
 // learned.cu — the learned preconditioner (see learned.cuh): network, tcgen05 convolutions, training and inference.
 //
 // Tensors are FP32 NHWC with channels padded to a multiple of 8, images stacked along N. A 3x3 convolution is an
-// implicit GEMM: M = 128 output pixels per CTA (a 16 x 8 tile, one TMEM lane each), N = the output channels, K = 9 taps
+// implicit GEMM: M = 128 output pixels per CTA (an 8 x 16 tile, one TMEM lane each), N = the output channels, K = 9 taps
 // x the input channels; the CTA stages its input halo once in shared memory as BF16 (applying the layer's input
-// transform: pooling, upsampling, the skip addition, or for the data gradient the ReLU mask), builds its im2col rows
-// from it in the canonical no-swizzle K-major layout, thread 0 issues tcgen05.mma (kind::f16, FP32 accumulator in
-// TMEM) per 16 of K, commits to an mbarrier, and the four warps read their 32 TMEM lanes back for the epilogue (bias,
-// ReLU, FP32 store). Every mbarrier wait is
-// bounded; a wait that gives up sets the learner's error flag and the CTA skips its store.
+// transform: pooling, upsampling, the skip addition, or for the data gradient the ReLU mask) so that the halo itself is
+// the A operand of every tap, thread 0 issues tcgen05.mma (kind::f16, FP32 accumulator in TMEM) per 16 of K, commits to
+// an mbarrier, and the four warps read their 32 TMEM lanes back for the epilogue (bias, ReLU, FP32 store). Every
+// mbarrier wait is bounded; a wait that gives up sets the learner's error flag and the CTA skips its store.
 #include <math.h>
 #include <string.h>
 
@@ -101,25 +100,25 @@ __device__ __forceinline__ void conv_input(const ConvArgs& A, int img, int yy, i
     }
 }
 
-// A CTA's output tile: 16 x 8 pixels of one image (thread t <-> pixel (t % 16, t / 16) <-> TMEM lane t), and its input
-// halo, 18 x 10 pixels, staged once in shared memory as BF16 (through the layer's input transform), from which each
-// thread builds its im2col row with 16-byte shared-memory copies (8 channels = one core-matrix row).
-constexpr int TW = 16, TH = 8, HW_ = TW + 2, HH_ = TH + 2, HP = HW_ * HH_;
+// A CTA's output tile: 8 x 16 pixels of one image (thread t <-> pixel (t % 8, t / 8) <-> TMEM lane t), and its input
+// halo, 10 x 18 pixels, in shared memory as planes of 8 channels: [channel group][pixel][8 BF16]. Eight neighbouring
+// pixels of a row are then 128 contiguous bytes, one core matrix of the no-swizzle K-major layout, whatever pixel they
+// start on: tap (dy, dx)'s A operand is the halo itself from pixel (dy, dx) on, its 16 groups of 8 rows one halo row
+// apart (the descriptor's stride along M) and its channel groups one plane apart (along K; with 8 channels, the next
+// tap's pixel). Building im2col rows in shared memory instead — nine copies of the halo — was most of a CTA's time and
+// shared memory: 512², 8 -> 8 channels, 13.3 -> 12.5 us; 32 -> 32 at 128², 12.7 -> 10.7.
+constexpr int TW = 8, TH = 16, HW_ = TW + 2, HH_ = TH + 2, HP = HW_ * HH_;
+constexpr int HPLANE = 16 * (HP + 1);  // a plane's bytes; the odd pixel spreads a pixel's planes over the banks
 
 template <int CIN_P, int COUT_P>
 struct ConvShape {
-    static constexpr int NC = CIN_P >= 32 ? 3 : 1;           // K chunks (3 taps each, or all 9 taps)
     static constexpr int KT = CIN_P == 8 ? 80 : 9 * CIN_P;   // K of the weight image (8 channels: 72 padded to 80)
-    static constexpr int KC = NC == 1 ? KT : 3 * CIN_P;      // K of a chunk
-    static constexpr int TAPS = NC == 1 ? 9 : 3;
-    static constexpr int NBUF = (NC == 1 || CIN_P == 64) ? 1 : 2;  // one A buffer for 64 channels: 2 CTAs per SM
     static constexpr int NM = COUT_P < 16 ? 16 : COUT_P;     // MMA N (M = 128 takes N in multiples of 16)
     static constexpr int NCOLS = NM <= 32 ? 32 : 64;         // TMEM columns (a power of two >= 32)
     static constexpr size_t SBG = (size_t)COUT_P * KT * 2;   // the weight image in global memory
     static constexpr size_t SB = (size_t)NM * KT * 2;        // in shared memory, zero rows up to NM
-    static constexpr size_t SA = (size_t)128 * KC * 2;
-    static constexpr size_t SI = (size_t)HP * CIN_P * 2;     // the BF16 halo tile
-    static constexpr size_t SMEM = SB + NBUF * SA + SI + 64;
+    static constexpr size_t SI = (size_t)(CIN_P / 8) * HPLANE;  // the BF16 halo tile
+    static constexpr size_t SMEM = SB + SI + 32;
 };
 
 template <int CIN_P, int COUT_P>
@@ -127,11 +126,10 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
     using S = ConvShape<CIN_P, COUT_P>;
     constexpr int G = CIN_P / 8;  // channel groups of 16 bytes (BF16)
     extern __shared__ __align__(1024) unsigned char smem[];
-    __nv_bfloat16* sB = reinterpret_cast<__nv_bfloat16*>(smem);
-    unsigned char* sA = smem + S::SB;
-    uint4* sIn = reinterpret_cast<uint4*>(sA + S::NBUF * S::SA);  // [HP][G]
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(sA + S::NBUF * S::SA + S::SI);
-    uint32_t* tbase = reinterpret_cast<uint32_t*>(mbar + 2);
+    unsigned char* sB = smem;
+    unsigned char* sIn = smem + S::SB;  // [G][HP] of 16 bytes, planes HPLANE apart
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + S::SB + S::SI);
+    uint32_t* tbase = reinterpret_cast<uint32_t*>(mbar + 1);
     const int tid = threadIdx.x, warp = tid >> 5;
     constexpr uint32_t IDESC = tc::idesc_bf16_f32(128, S::NM);
 
@@ -140,8 +138,7 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
         tc::tmem_relinquish();
     }
     if (tid == 0) {
-        tc::mbar_init(&mbar[0], 1);
-        tc::mbar_init(&mbar[1], 1);
+        tc::mbar_init(mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     {
@@ -169,6 +166,7 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
         for (int u = 0; u < NB; u++) {
             const int e = tid + (i0 + u) * 128;
             if (i0 + u < NI && e < HP * G) {
+                const int hp = e / G, g = e - hp * G;
                 uint4 packed;
                 __nv_bfloat162 h0 = __floats2bfloat162_rn(v[u][0], v[u][1]), h1 = __floats2bfloat162_rn(v[u][2], v[u][3]);
                 __nv_bfloat162 h2 = __floats2bfloat162_rn(v[u][4], v[u][5]), h3 = __floats2bfloat162_rn(v[u][6], v[u][7]);
@@ -176,61 +174,41 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
                 packed.y = *reinterpret_cast<uint32_t*>(&h1);
                 packed.z = *reinterpret_cast<uint32_t*>(&h2);
                 packed.w = *reinterpret_cast<uint32_t*>(&h3);
-                sIn[e] = packed;
+                *reinterpret_cast<uint4*>(sIn + g * HPLANE + hp * 16) = packed;
             }
         }
     }
+    tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tbase;
-
-    const int px = tid % TW, py = tid / TW;
-    const int x = X0 + px, y = Y0 + py;
-    const bool valid = x < A.W && y < A.H;
-    uint32_t par0 = 0u, par1 = 0u;
-    bool ok = true;
-    for (int c = 0; c < S::NC; c++) {
-        const int buf = c % S::NBUF;
-        if (c >= S::NBUF) {  // this buffer's previous MMAs must be done before it is rewritten
-            const uint32_t par = buf ? par1 : par0;
-            if (!tc::mbar_wait(&mbar[buf], par, kWaitLimit)) ok = false;
-            if (buf) par1 ^= 1u; else par0 ^= 1u;
-        }
-        unsigned char* a = sA + buf * S::SA;
+    if (tid == 0) {
+        const uint32_t a0 = tc::smem_addr(sIn), b0 = tc::smem_addr(sB);
 #pragma unroll
-        for (int t = 0; t < S::TAPS; t++) {
-            const int tap = S::NC == 1 ? t : c * 3 + t;
-            const int hp = (py + tap / 3) * HW_ + px + tap % 3;  // the halo pixel of (x + dx, y + dy)
-#pragma unroll
-            for (int g = 0; g < G; g++) {
-                const int k = t * CIN_P + g * 8;
-                *reinterpret_cast<uint4*>(a + ((tid / 8) * (S::KC / 8) + k / 8) * 128 + (tid % 8) * 16) =
-                    sIn[hp * G + g];
+        for (int ks = 0; ks < S::KT / 16; ks++) {
+            uint32_t at, lbo;  // the A operand's first core matrix, and the distance to the one 8 of K on
+            if constexpr (CIN_P == 8) {
+                // taps 2 ks and 2 ks + 1; the last MMA is tap 7 again, against zero weights, and tap 8
+                const int t0 = ks < 4 ? 2 * ks : 7, t1 = t0 + 1;
+                const int p0 = (t0 / 3) * HW_ + t0 % 3, p1 = (t1 / 3) * HW_ + t1 % 3;
+                at = a0 + 16 * p0;
+                lbo = 16 * (p1 - p0);
+            } else {
+                const int tap = ks / (CIN_P / 16), g = 2 * (ks % (CIN_P / 16));
+                at = a0 + g * HPLANE + 16 * ((tap / 3) * HW_ + tap % 3);
+                lbo = HPLANE;
             }
+            const uint64_t ad = tc::desc_kmajor(at, lbo, 16 * HW_);
+            const uint64_t bd = tc::desc_kmajor(b0 + 2 * ks * 128, 128, S::KT * 16);
+            tc::mma_bf16(tmem, ad, bd, IDESC, ks > 0);
         }
-        if (CIN_P == 8)  // K 72..79: zero padding to a multiple of 16
-            *reinterpret_cast<uint4*>(a + ((tid / 8) * (S::KC / 8) + 9) * 128 + (tid % 8) * 16) = make_uint4(0, 0, 0, 0);
-        tc::fence_async_smem();
-        tc::fence_before_sync();
-        __syncthreads();
-        if (tid == 0) {
-            tc::fence_after_sync();
-            const uint32_t a0 = tc::smem_addr(a), b0 = tc::smem_addr(sB);
-#pragma unroll
-            for (int ks = 0; ks < S::KC / 16; ks++) {
-                const uint64_t ad = tc::desc_kmajor(a0 + ks * 256, 128, S::KC * 16);
-                const uint64_t bd = tc::desc_kmajor(b0 + (c * (S::KC / 8) + 2 * ks) * 128, 128, S::KT * 16);
-                tc::mma_bf16(tmem, ad, bd, IDESC, c > 0 || ks > 0);
-            }
-            tc::mma_commit(&mbar[buf]);
-        }
+        tc::mma_commit(mbar);
     }
-    {
-        const int buf = (S::NC - 1) % S::NBUF;
-        if (!tc::mbar_wait(&mbar[buf], buf ? par1 : par0, kWaitLimit)) ok = false;
-    }
+    const bool ok = tc::mbar_wait(mbar, 0u, kWaitLimit);
     tc::fence_after_sync();
+    const int x = X0 + tid % TW, y = Y0 + tid / TW;
+    const bool valid = x < A.W && y < A.H;
     float acc[COUT_P];
 #pragma unroll
     for (int c0 = 0; c0 < COUT_P; c0 += 8) tc::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc + c0);
@@ -295,7 +273,12 @@ void launch_conv(int cin_p, int cout_p, const ConvArgs& A, cudaStream_t s) {
 }
 
 // ---- weight images: the forward B operand [cout_p/8][KT/8][8][8] with k = tap * cin_p + ci, and the data-gradient
-// one, the convolution with the taps flipped and the channels swapped: n = ci, k = tap' * cout_p + co.
+// one, the convolution with the taps flipped and the channels swapped: n = ci, k = tap' * cout_p + co. With 8 channels
+// the ten groups of 8 are taps 0..7, none (zeros) and tap 8.
+__device__ __forceinline__ int tap_of(int group, int channels) {
+    return channels > 8 || group < 8 ? group : (group == 8 ? 9 : 8);
+}
+
 __global__ void pack_weights_kernel(const float* __restrict__ theta, int cin, int cout, int cin_p, int cout_p,
                                     __nv_bfloat16* fwd, __nv_bfloat16* bwd) {
     const int ktf = cin_p == 8 ? 80 : 9 * cin_p, ktb = cout_p == 8 ? 80 : 9 * cout_p;
@@ -303,14 +286,14 @@ __global__ void pack_weights_kernel(const float* __restrict__ theta, int cin, in
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nf + nb; e += gridDim.x * blockDim.x) {
         if (e < nf) {
             const int n = e / ktf, k = e % ktf;
-            const int tap = k / cin_p, ci = k % cin_p;
+            const int tap = tap_of(k / cin_p, cin_p), ci = k % cin_p;
             float v = 0.0f;
             if (n < cout && tap < 9 && ci < cin) v = theta[((size_t)n * 9 + tap) * cin + ci];
             fwd[((n / 8) * (ktf / 8) + k / 8) * 64 + (n % 8) * 8 + (k % 8)] = __float2bfloat16_rn(v);
         } else {
             const int f = e - nf;
             const int n = f / ktb, k = f % ktb;  // n: forward input channel, k: flipped tap x forward output channel
-            const int tapf = k / cout_p, co = k % cout_p;
+            const int tapf = tap_of(k / cout_p, cout_p), co = k % cout_p;
             float v = 0.0f;
             if (n < cin && tapf < 9 && co < cout) v = theta[((size_t)co * 9 + (8 - tapf)) * cin + n];
             bwd[((n / 8) * (ktb / 8) + k / 8) * 64 + (n % 8) * 8 + (k % 8)] = __float2bfloat16_rn(v);
