@@ -49,6 +49,7 @@ struct ConvArgs {
     const float* bias;  // optional
     int cout_real;
     float* out;
+    float* out2;  // optional, a second copy of the output
     int relu;
     int* err;
 };
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
     tc::tmem_wait_ld();
     if (!ok) atomicExch(A.err, 1);
     if (valid && ok) {
-        float* o = A.out + ((((size_t)img * A.H + y) * A.W) + x) * COUT_P;
+        const size_t at = ((((size_t)img * A.H + y) * A.W) + x) * COUT_P;
 #pragma unroll
         for (int c0 = 0; c0 < COUT_P; c0 += 4) {
             float4 q;
@@ -227,7 +228,8 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
                 if (A.relu) v = fmaxf(v, 0.0f);
                 qq[j] = v;
             }
-            *reinterpret_cast<float4*>(o + c0) = q;
+            *reinterpret_cast<float4*>(A.out + at + c0) = q;
+            if (A.out2) *reinterpret_cast<float4*>(A.out2 + at + c0) = q;
         }
     }
     tc::fence_before_sync();
@@ -459,11 +461,6 @@ __global__ void dw_reduce_kernel(const float* __restrict__ part, int chunks, int
 }
 
 // ---- input-transform adjoints and the elementwise pieces
-__global__ void add_kernel(size_t n, const float* __restrict__ a, float* dst) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        dst[i] += a[i];
-}
-
 // g_fine[fy][fx] += g_coarse[fy/2][fx/2] / (cells of that block)
 __global__ void pool_adjoint_kernel(int B, int H, int W, int C, const float* __restrict__ gc, float* gf) {
     const int Hc = (H + 1) / 2, Wc = (W + 1) / 2;
@@ -478,7 +475,7 @@ __global__ void pool_adjoint_kernel(int B, int H, int W, int C, const float* __r
     }
 }
 
-// g_coarse[Y][X] += Σ over the fine cells of the block of g_fine
+// g_coarse[Y][X] = Σ over the fine cells of the block of g_fine
 __global__ void up_adjoint_kernel(int B, int H, int W, int C, const float* __restrict__ gf, float* gc) {
     const int Hc = (H + 1) / 2, Wc = (W + 1) / 2;
     const size_t n = (size_t)B * Hc * Wc * C;
@@ -492,7 +489,7 @@ __global__ void up_adjoint_kernel(int B, int H, int W, int C, const float* __res
                 const int y = 2 * Y + b, x = 2 * X + a;
                 if (y < H && x < W) s += gf[(((size_t)img * H + y) * W + x) * C + ch];
             }
-        gc[e] += s;
+        gc[e] = s;
     }
 }
 
@@ -593,6 +590,12 @@ __global__ void gather_kernel(int C, const int* __restrict__ idx, int batch, con
         reinterpret_cast<float4*>(bf)[e * 2 + 1] = reinterpret_cast<const float4*>(feats)[src * 2 + 1];
         bt[e] = targets[src];
     }
+}
+
+// The head's channel 0 of every pixel.
+__global__ void head_kernel(size_t n, const float* __restrict__ head, float* out) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        out[i] = head[i * 8];
 }
 
 // Host features (n, 4, C, C) -> NHWC 8-padded.
@@ -892,15 +895,15 @@ void dw_attributes() {
 #undef SR_DW_CASE
 }
 
-// Loss gradient already in gact[NL-1]: every layer's weight gradient and the input gradients, last layer first.
+// Loss gradient already in gact[NL-1]: every layer's weight gradient and the input gradients, last layer first. A
+// layer's input gradient goes straight to where it is wanted: an encoder output that a skip adds gets the skip's first
+// (the later layer's) and the pooling's added to it; every other gradient has one source. (Buffers cleared first and
+// added to by kernels of their own were 25 of the pass's 114 launches.)
 void backward(Learner* Lr, Net& N, cudaStream_t s) {
-    for (int l = 0; l < NL - 1; l++)
-        SR_CUDA_TRY(cudaMemsetAsync(N.gact[l], 0, sizeof(float) * N.pix(kL[l].level) * pad8(kL[l].cout), s));
     for (int l = NL - 1; l >= 0; l--) {
         const LayerDef& d = kL[l];
         const int ci = pad8(d.cin), co = pad8(d.cout);
         ConvArgs A = layer_args(Lr, N, l);
-        const long long P = (long long)A.B * A.H * A.W;
         const int chunks = dw_chunks(A.B, A.H, A.W);
         launch_dw(ci, co, A, N.gact[l], N.act[l], d.relu, N.wpart, N.bpart, s);
         dw_reduce_kernel<<<grid_of((size_t)d.cout * 9 * d.cin + d.cout), RT, 0, s>>>(
@@ -920,19 +923,13 @@ void backward(Learner* Lr, Net& N, cudaStream_t s) {
         G.wimg = Lr->wb[l];
         G.bias = nullptr;
         G.cout_real = ci;
-        G.out = N.gx;
+        const bool direct = d.mode == M_PREV || d.mode == M_SKIP;
+        G.out = direct ? N.gact[l - 1] : N.gx;
+        G.out2 = d.mode == M_SKIP ? N.gact[d.skip] : nullptr;
         G.relu = 0;
         G.err = Lr->err;
         launch_conv(co, ci, G, s);
-        const size_t nin = (size_t)P * ci;
-        if (d.mode == M_PREV || d.mode == M_SKIP) {
-            add_kernel<<<grid_of(nin), RT, 0, s>>>(nin, N.gx, N.gact[l - 1]);
-            sr_note_launch();
-            if (d.mode == M_SKIP) {
-                add_kernel<<<grid_of(nin), RT, 0, s>>>(nin, N.gx, N.gact[d.skip]);
-                sr_note_launch();
-            }
-        } else if (d.mode == M_POOL) {
+        if (d.mode == M_POOL) {
             const int lv = d.level - 1;
             const size_t nf = N.pix(lv) * ci;
             pool_adjoint_kernel<<<grid_of(nf), RT, 0, s>>>(N.B, N.lh[lv], N.lw[lv], ci, N.gx, N.gact[l - 1]);
@@ -1157,27 +1154,20 @@ double learned_loss_grad(Learner* L, const float* feats, const float* target, in
                          cudaStream_t s) {
     ensure_train_net(L, n);
     const size_t per = (size_t)L->crop * L->crop;
-    float* hin = nullptr;
-    SR_CUDA_TRY(cudaMalloc(&hin, sizeof(float) * per * 4 * n));
-    try {
-        SR_CUDA_TRY(cudaMemcpyAsync(hin, feats, sizeof(float) * per * 4 * n, cudaMemcpyHostToDevice, s));
-        nchw_to_feats_kernel<<<grid_of(per * n), RT, 0, s>>>(n, L->crop, hin, L->train_net.feats);
+    float* hin = L->train_net.gact[0];  // n x crop² x 8: free until the backward pass, and again after it
+    SR_CUDA_TRY(cudaMemcpyAsync(hin, feats, sizeof(float) * per * 4 * n, cudaMemcpyHostToDevice, s));
+    nchw_to_feats_kernel<<<grid_of(per * n), RT, 0, s>>>(n, L->crop, hin, L->train_net.feats);
+    sr_note_launch();
+    SR_CUDA_TRY(cudaMemcpyAsync(L->btarget, target, sizeof(float) * per * n, cudaMemcpyHostToDevice, s));
+    const double loss = loss_step(L, L->train_net, L->btarget, s);
+    if (grad) SR_CUDA_TRY(cudaMemcpyAsync(grad, L->grad, sizeof(float) * L->nparams, cudaMemcpyDeviceToHost, s));
+    if (out) {
+        head_kernel<<<grid_of(per * n), RT, 0, s>>>(per * n, L->train_net.act[NL - 1], hin);
         sr_note_launch();
-        SR_CUDA_TRY(cudaMemcpyAsync(L->btarget, target, sizeof(float) * per * n, cudaMemcpyHostToDevice, s));
-        const double loss = loss_step(L, L->train_net, L->btarget, s);
-        if (grad) SR_CUDA_TRY(cudaMemcpy(grad, L->grad, sizeof(float) * L->nparams, cudaMemcpyDeviceToHost));
-        if (out) {
-            std::vector<float> head(per * n * 8);
-            SR_CUDA_TRY(cudaMemcpy(head.data(), L->train_net.act[NL - 1], sizeof(float) * head.size(),
-                                   cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < per * n; i++) out[i] = head[i * 8];
-        }
-        cudaFree(hin);
-        return loss;
-    } catch (...) {
-        cudaFree(hin);
-        throw;
+        SR_CUDA_TRY(cudaMemcpyAsync(out, hin, sizeof(float) * per * n, cudaMemcpyDeviceToHost, s));
     }
+    SR_CUDA_TRY(cudaStreamSynchronize(s));
+    return loss;
 }
 
 LearnedApply* learned_apply_create(Learner* L, int w, int h) {
