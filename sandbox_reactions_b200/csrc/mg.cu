@@ -26,8 +26,9 @@ struct TailLevel {
                                   // coarser level; b and x: the lower levels' right-hand side and iterate
 };
 
+constexpr int kTailLevels = 5;  // 64 x 64 down to 4 x 4
 struct TailArgs {
-    int t, nl, pre, post;
+    int nl, pre, post;        // nl: the tail's levels
     float omega;
     int sinv;                 // offset of the coarsest level's inverse (nc x nc)
     int img_f4;               // the lower levels' part of the image in 16-byte words
@@ -35,7 +36,7 @@ struct TailArgs {
     const float* b;           // the top level's right-hand side and result
     float* x2;
     double* out;              // non-null when the tail's top level is level 0: <b, x2> written here
-    TailLevel T[kMgMaxLevels];
+    TailLevel T[kTailLevels];  // the top first
 };
 
 // Level 0's couplings to the +x / +y neighbours from the f64 faces, zero unless both cells are gas.
@@ -100,30 +101,40 @@ __global__ void mg_aggregate_kernel(MgLevel F, MgLevel C) {
 // restriction and prolongation use. One tile of CO_S x CO_S fine cells per CTA, all four half-sweeps in shared
 // memory: the tile's halo is as deep as the half-sweeps plus the two rings whose aggregates' scale the Galerkin sums
 // read (t of the cells next to the tile's aggregates).
-constexpr int CO_S = 32, CO_H = 6, CO_R = CO_S + 2 * CO_H, CO_N = CO_R * CO_R, CO_NT = 256;
+constexpr int CO_S = 32, CO_H = 6, CO_R = CO_S + 2 * CO_H, CO_N = CO_R * CO_R, CO_NT = 512;
 
 __global__ void __launch_bounds__(CO_NT) mg_coarsen_kernel(MgLevel F, MgLevel C) {
     __shared__ float sc[CO_N], sdx[CO_N], sdy[CO_N], st[CO_N];
     __shared__ uint8_t sm[CO_N];
     const int wf = F.w, hf = F.h;
     const int X0 = blockIdx.x * CO_S - CO_H, Y0 = blockIdx.y * CO_S - CO_H;  // even: local parity = global parity
-    for (int k = threadIdx.x; k < CO_N; k += CO_NT) {
-        const int gx = X0 + k % CO_R, gy = Y0 + k / CO_R;
-        float c = 1.0f, dx = 0.0f, dy = 0.0f, t = 0.0f;
-        uint8_t m = 0;
-        if (gx >= 0 && gx < wf && gy >= 0 && gy < hf) {
+    // all of a thread's loads in flight together: the launch is one CTA's latency on the coarse levels (11.2 -> 6.7 us)
+    constexpr int PER = (CO_N + CO_NT - 1) / CO_NT;
+    float lc[PER], ldx[PER], ldy[PER];
+    uint8_t lm[PER];
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const int k = threadIdx.x + u * CO_NT, gx = X0 + k % CO_R, gy = Y0 + k / CO_R;
+        lc[u] = 1.0f;
+        ldx[u] = ldy[u] = 0.0f;
+        lm[u] = 0;
+        if (k < CO_N && gx >= 0 && gx < wf && gy >= 0 && gy < hf) {
             const int i = gy * wf + gx;
-            c = F.c[i];
-            dx = F.dx[i];
-            dy = F.dy[i];
-            m = F.mask[i];
-            t = m ? 1.0f : 0.0f;
+            lc[u] = F.c[i];
+            ldx[u] = F.dx[i];
+            ldy[u] = F.dy[i];
+            lm[u] = F.mask[i];
         }
-        sm[k] = m;
-        sc[k] = c;
-        sdx[k] = dx;
-        sdy[k] = dy;
-        st[k] = t;
+    }
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+        const int k = threadIdx.x + u * CO_NT;
+        if (k >= CO_N) break;
+        sm[k] = lm[u];
+        sc[k] = lc[u];
+        sdx[k] = ldx[u];
+        sdy[k] = ldy[u];
+        st[k] = lm[u] ? 1.0f : 0.0f;
     }
     __syncthreads();
     // four half-sweeps, colour 0 first, over the region less its outermost ring (a cell's value is exact once it
@@ -738,7 +749,7 @@ __global__ void __launch_bounds__(RB_NT, 2)
 // most 16 x 16 by warp 0 alone, 8 pairs x 4 row groups, neighbours by shuffles and no barrier at all. The top level's
 // coefficients stay in registers from its pre- to its post-smoother; the lower levels are read from the image
 // mg_tail_pack_kernel writes once per Newton pass, whose rows are padded to even pitches and heights so that no access
-// has an edge case. 64 x 64 top under V(4,4): 27 -> 19 us a V-cycle against the whole CTA of 1,024 threads meeting at
+// has an edge case. 64 x 64 top under V(4,4): 27 -> 15.5 us a V-cycle against the whole CTA of 1,024 threads meeting at
 // every half-sweep of every level.
 extern __shared__ __align__(16) unsigned char tail_smem_raw[];
 
@@ -986,13 +997,17 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) mg_tail_kernel(const __grid_c
     float* f = reinterpret_cast<float*>(tail_smem_raw + 2 * sizeof(TailEdge));
     TailEdge* e = reinterpret_cast<TailEdge*>(tail_smem_raw);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const TailLevel& T = A.T[A.t];
-    const TailLevel& T1 = A.T[A.t + 1];
-    const int nw = (T.h + RB_R - 1) / RB_R, nw1 = (T1.h + 2 * RB_R - 1) / (2 * RB_R);
+    // the level table, read by run-time index below, out of the constant bank once; the lower levels' image (b and x 0)
+    // into shared memory while the top level's loads are in flight
+    __shared__ TailLevel sT[kTailLevels];
+    if (threadIdx.x < kTailLevels * (int)(sizeof(TailLevel) / 4))
+        reinterpret_cast<int*>(sT)[threadIdx.x] = reinterpret_cast<const int*>(A.T)[threadIdx.x];
+    for (int q = threadIdx.x; q < A.img_f4; q += TAIL_THREADS)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_addr(f + 4 * q)), "l"(A.img + 4 * q) : "memory");
+    const TailLevel& T = A.T[0];
+    const TailLevel& T1 = sT[1];
+    const int nw = (T.h + RB_R - 1) / RB_R, nw1 = (A.T[1].h + 2 * RB_R - 1) / (2 * RB_R);
     const int row0 = RB_R * warp;
-    // the lower levels' image (b and x 0) into shared memory, while the top level's loads are in flight
-    for (int k = threadIdx.x; k < A.img_f4; k += TAIL_THREADS)
-        reinterpret_cast<float4*>(f)[k] = reinterpret_cast<const float4*>(A.img)[k];
     TailBand B;
     float2 c2[RB_R], t2[RB_R];
     tail_load<32>(B, A.img + T.inv, A.img + T.dx, A.img + T.dy, T.p, T.hp, lane, row0);
@@ -1013,6 +1028,7 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) mg_tail_kernel(const __grid_c
     // every warp's rows in both edge buffers: a band past the level's last row reads 0 (times no coupling)
     tail_post_edges<32>(B, e[0], warp, lane);
     tail_post_edges<32>(B, e[1], warp, lane);
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (warp < nw) {
         tail_sweeps<32, 0>(B, e, A.pre, warp, lane, 1, 32 * nw);
@@ -1020,21 +1036,21 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) mg_tail_kernel(const __grid_c
     }
     __syncthreads();
     if (warp < nw1) {
-        tail_down<16>(T1, A.T[A.t + 2], f, e, A.pre, warp, lane, 2, 32 * nw1);
+        tail_down<16>(T1, sT[2], f, e, A.pre, warp, lane, 2, 32 * nw1);
         tail_bar(2, 32 * nw1);
         if (warp == 0) {
-            for (int l = A.t + 2; l < A.nl - 1; l++) {
-                tail_down<8>(A.T[l], A.T[l + 1], f, e, A.pre, 0, lane, 0, 0);
+            for (int l = 2; l < A.nl - 1; l++) {
+                tail_down<8>(sT[l], sT[l + 1], f, e, A.pre, 0, lane, 0, 0);
                 __syncwarp();
             }
-            tail_coarsest(A.T[A.nl - 1], f, f + A.sinv, lane);
-            for (int l = A.nl - 2; l >= A.t + 2; l--) {
-                tail_up<8>(A.T[l], A.T[l + 1], f, e, A.post, A.omega, 0, lane, 0, 0);
+            tail_coarsest(sT[A.nl - 1], f, f + A.sinv, lane);
+            for (int l = A.nl - 2; l >= 2; l--) {
+                tail_up<8>(sT[l], sT[l + 1], f, e, A.post, A.omega, 0, lane, 0, 0);
                 __syncwarp();
             }
         }
         tail_bar(2, 32 * nw1);
-        tail_up<16>(T1, A.T[A.t + 2], f, e, A.post, A.omega, warp, lane, 2, 32 * nw1);
+        tail_up<16>(T1, sT[2], f, e, A.post, A.omega, warp, lane, 2, 32 * nw1);
     }
     __syncthreads();
     double acc = 0.0;
@@ -1072,15 +1088,16 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) mg_tail_kernel(const __grid_c
 // and an even number of rows. Fills A.T, A.sinv and A.img_f4; returns the image's size in floats.
 int tail_layout(const Multigrid& M, TailArgs& A) {
     int off = 0;
-    for (int k = 1; k <= M.nlevels - M.tail; k++) {
-        const int l = k < M.nlevels - M.tail ? M.tail + k : M.tail;  // the top level last
-        if (l == M.tail) {
+    const int nl = M.nlevels - M.tail;
+    for (int q = 1; q <= nl; q++) {
+        const int k = q % nl, l = M.tail + k;  // the top level last
+        if (k == 0) {
             const int nc = M.L[M.nlevels - 1].w * M.L[M.nlevels - 1].h;
             A.sinv = off;
             off = (off + nc * nc + 3) & ~3;
             A.img_f4 = off / 4;
         }
-        TailLevel& T = A.T[l];
+        TailLevel& T = A.T[k];
         T.w = M.L[l].w;
         T.h = M.L[l].h;
         T.p = (T.w + 1) & ~1;
@@ -1093,7 +1110,7 @@ int tail_layout(const Multigrid& M, TailArgs& A) {
         T.c = off + 4 * n;
         T.b = off + 5 * n;
         T.x = off + 6 * n;
-        off += (l == M.tail ? 5 : 7) * n;
+        off += (k == 0 ? 5 : 7) * n;
     }
     return off;
 }
@@ -1104,8 +1121,7 @@ constexpr size_t kTailSmem = 2 * sizeof(TailEdge) + (7 * (1024 + 256 + 64 + 16) 
 // Everything the tail kernel and its packing need but the output slot; returns the launch's shared memory.
 size_t tail_args(const Multigrid& M, TailArgs& T) {
     tail_layout(M, T);
-    T.t = M.tail;
-    T.nl = M.nlevels;
+    T.nl = M.nlevels - M.tail;
     T.pre = M.pre;
     T.post = M.post;
     T.omega = M.omega;
@@ -1121,9 +1137,9 @@ size_t tail_args(const Multigrid& M, TailArgs& T) {
 // (f64 sums) and the level's part of the image — couplings, inverse diagonal, weights and c, 0 (c: 1) on the padding, b
 // and x at 0 — then the coarsest operator's inverse. One CTA: the levels are a serial chain of a few thousand cells at
 // most, so launches and their ramps were what it cost (a coarsening a level, the inverse and the packing: 53 us for a
-// 64 x 64 top, in six launches; now one of 29 us).
-constexpr int TS_NT = 512, TS_P = kMgTailSide + 2, TS_N = TS_P * TS_P;  // a level with a rim of one cell around it
-
+// 64 x 64 top, in six launches; now one of 23 us). Every level has the top's pitch, so that a thread's cell is its
+// index's bits and not a division, and the column before and the row above a level (couplings 0) are never written.
+constexpr int TS_NT = 1024, TS_P = kMgTailSide + 2, TS_N = TS_P * TS_P;  // a level with a rim of one cell around it
 
 struct TailSetupShared {
     float c[2][TS_N], dx[2][TS_N], dy[2][TS_N], t[TS_N];  // this level and the next
@@ -1134,7 +1150,8 @@ struct TailSetupShared {
 
 // The coarsest operator's inverse by Gauss-Jordan elimination in f64 (SPD: no pivoting; masked cells are identity rows),
 // one thread per element of [A | I]; the thread that writes the next pivot leaves its reciprocal. Stored f32.
-__device__ __forceinline__ void tail_inverse(TailSetupShared& S, int k, int w, int h, int p, float* inv, int room) {
+__device__ __forceinline__ void tail_inverse(TailSetupShared& S, int k, int w, int h, float* inv, int room) {
+    constexpr int p = TS_P;
     const int n = w * h, i = threadIdx.x >> 5, j = threadIdx.x & 31;
     if (i < n && j < 2 * n) {
         double v = 0.0;
@@ -1170,111 +1187,124 @@ __device__ __forceinline__ void tail_inverse(TailSetupShared& S, int k, int w, i
     for (int e = threadIdx.x; e < room; e += TS_NT) inv[e] = e < n * n ? (float)S.aug[n & 1][(e / n) * 32 + n + e % n] : 0.0f;
 }
 
-__global__ void __launch_bounds__(TS_NT) mg_tail_setup_kernel(const __grid_constant__ TailArgs A, MgLevel top, float* img) {
+__global__ void __launch_bounds__(TS_NT) mg_tail_setup_kernel(const __grid_constant__ TailArgs A, MgLevel top, bool level0,
+                                                              float* img) {
     extern __shared__ __align__(16) unsigned char setup_smem[];
     TailSetupShared& S = *reinterpret_cast<TailSetupShared*>(setup_smem);
-    const int tid = threadIdx.x;
+    constexpr int p = TS_P;
+    // cells by 64 columns x 16 rows of threads, aggregates and a sweep's pairs by 32 x 32
+    const int tid = threadIdx.x, x64 = tid & 63, y64 = tid >> 6, x32 = tid & 31, y32 = tid >> 5;
     {
-        const int w = top.w, h = top.h, p = w + 2;
-        constexpr int PER = (TS_N + TS_NT - 1) / TS_NT;
+        float lc[4], ldx[4], ldy[4];
+        uint8_t lm[4];
 #pragma unroll
-        for (int u = 0; u < PER; u++) {
-            const int q = tid + u * TS_NT;
-            if (q >= p * (h + 2)) break;
-            const int x = q % p - 1, y = q / p - 1;
-            const bool in = x >= 0 && x < w && y >= 0 && y < h;
-            const int i = y * w + x;
-            S.c[0][q] = in ? top.c[i] : 1.0f;
-            S.dx[0][q] = in ? top.dx[i] : 0.0f;
-            S.dy[0][q] = in ? top.dy[i] : 0.0f;
-            S.m[0][q] = in ? top.mask[i] : 0;
+        for (int u = 0; u < 4; u++) {
+            const int y = y64 + 16 * u, i = y * top.w + x64;
+            const bool in = x64 < top.w && y < top.h;
+            lc[u] = in ? top.c[i] : 1.0f;
+            ldx[u] = in ? top.dx[i] : 0.0f;
+            ldy[u] = in ? top.dy[i] : 0.0f;
+            lm[u] = in ? top.mask[i] : 0;
+        }
+        for (int q = tid; q < TS_N; q += TS_NT) S.t[q] = 0.0f;
+        if (tid < TS_P) {
+            S.dx[0][tid * p] = S.dx[1][tid * p] = 0.0f;
+            S.dy[0][tid] = S.dy[1][tid] = 0.0f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int q = (y64 + 16 * u + 1) * p + x64 + 1;
+            S.c[0][q] = lc[u];
+            S.dx[0][q] = ldx[u];
+            S.dy[0][q] = ldy[u];
+            S.m[0][q] = lm[u];
         }
     }
-    for (int l = A.t; l < A.nl; l++) {
+    for (int l = 0; l < A.nl; l++) {
         const TailLevel& T = A.T[l];
-        const int k = (l - A.t) & 1, w = T.w, h = T.h, p = w + 2;
+        const int k = l & 1, w = T.w, h = T.h;
         const float *c = S.c[k], *dx = S.dx[k], *dy = S.dy[k];
         const uint8_t* m = S.m[k];
         float* t = S.t;
-        __syncthreads();
-        for (int q = tid; q < p * (h + 2); q += TS_NT) t[q] = m[q] ? 1.0f : 0.0f;
-        __syncthreads();
         const bool coarsest = l + 1 == A.nl;
-        if (l > 0 && !coarsest) {
-            const int half = (w + 1) / 2;
-            for (int sweep = 0; sweep < 4; sweep++) {
-                for (int e = tid; e < half * h; e += TS_NT) {
-                    const int y = e / half, x = 2 * (e - y * half) + ((y + sweep) & 1);
-                    if (x >= w) continue;
-                    // a masked cell has c = 1 and no couplings (nor do its neighbours towards it): it stays 0
-                    const int q = (y + 1) * p + x + 1;
-                    const float dl = dx[q - 1], dr = dx[q], du = dy[q - p], dd = dy[q];
-                    const float num = dl * t[q - 1] + dr * t[q + 1] + du * t[q - p] + dd * t[q + p];
-                    t[q] = num / (c[q] + dl + dr + du + dd);
-                }
-                __syncthreads();
-            }
-        }
+        __syncthreads();
         if (!coarsest) {
+            if (x64 < w)
+                for (int y = y64; y < h; y += 16) {
+                    const int q = (y + 1) * p + x64 + 1;
+                    t[q] = m[q] ? 1.0f : 0.0f;
+                }
+            __syncthreads();
+            if (l > 0 || !level0) {
+                for (int sweep = 0; sweep < 4; sweep++) {
+                    for (int y = y32; y < h; y += 32) {
+                        const int x = 2 * x32 + ((y + sweep) & 1);
+                        if (x >= w) continue;
+                        // a masked cell has c = 1 and no couplings (nor do its neighbours towards it): it stays 0
+                        const int q = (y + 1) * p + x + 1;
+                        const float dl = dx[q - 1], dr = dx[q], du = dy[q - p], dd = dy[q];
+                        const float num = dl * t[q - 1] + dr * t[q + 1] + du * t[q - p] + dd * t[q + p];
+                        t[q] = num / (c[q] + dl + dr + du + dd);
+                    }
+                    __syncthreads();
+                }
+            }
             // each aggregate scaled to a largest weight of 1 (1 on its system cells where all weights vanished), then
             // the Galerkin operator, whose couplings read the neighbouring aggregates' scaled weights
-            const TailLevel& C = A.T[l + 1];
-            const int cw = C.w, ch = C.h, cp = cw + 2;
-            for (int e = tid; e < cw * ch; e += TS_NT) {
-                const int Y = e / cw, X = e - Y * cw, q = (2 * Y + 1) * p + 2 * X + 1;
-                const bool x1 = 2 * X + 1 < w, y1 = 2 * Y + 1 < h;
-                const int at[4] = {q, x1 ? q + 1 : q, y1 ? q + p : q, x1 && y1 ? q + p + 1 : q};
+            const int cw = A.T[l + 1].w, ch = A.T[l + 1].h;
+            const int X = x32, Y = y32;
+            const bool agg = X < cw && Y < ch;
+            const int q = (2 * Y + 1) * p + 2 * X + 1;
+            const bool x1 = 2 * X + 1 < w, y1 = 2 * Y + 1 < h;
+            const bool has[4] = {agg, agg && x1, agg && y1, agg && x1 && y1};
+            const int at[4] = {q, q + 1, q + p, q + p + 1};
+            if (agg) {
                 float big = 0.0f;
-                for (int a = 0; a < 4; a++) big = fmaxf(big, t[at[a]]);
-                float v[4];
-                for (int a = 0; a < 4; a++) v[a] = !m[at[a]] ? 0.0f : (big > 1e-30f ? t[at[a]] / big : 1.0f);
-                for (int a = 3; a >= 0; a--) t[at[a]] = v[a];
+#pragma unroll
+                for (int a = 0; a < 4; a++)
+                    if (has[a]) big = fmaxf(big, t[at[a]]);
+#pragma unroll
+                for (int a = 0; a < 4; a++)
+                    if (has[a]) t[at[a]] = !m[at[a]] ? 0.0f : (big > 1e-30f ? t[at[a]] / big : 1.0f);
             }
             __syncthreads();
-            for (int q = tid; q < cp * (ch + 2); q += TS_NT) {
-                const int X = q % cp - 1, Y = q / cp - 1;
-                float cc = 1.0f, dxc = 0.0f, dyc = 0.0f;
+            if (agg) {
+                double csum = 0.0, sx = 0.0, sy = 0.0;
                 bool any = false;
-                if (X >= 0 && X < cw && Y >= 0 && Y < ch) {
-                    double csum = 0.0, sx = 0.0, sy = 0.0;
-                    for (int b = 0; b < 2; b++)
-                        for (int a = 0; a < 2; a++) {
-                            const int x = 2 * X + a, y = 2 * Y + b, j = (y + 1) * p + x + 1;
-                            if (x >= w || y >= h || !m[j]) continue;
-                            any = true;
-                            const double tj = t[j];
-                            csum += tj * ((double)c[j] * tj + (double)dx[j - 1] * (tj - t[j - 1]) +
-                                          (double)dx[j] * (tj - t[j + 1]) + (double)dy[j - p] * (tj - t[j - p]) +
-                                          (double)dy[j] * (tj - t[j + p]));
-                            if (a) sx += tj * t[j + 1] * dx[j];
-                            if (b) sy += tj * t[j + p] * dy[j];
-                        }
-                    if (any) {
-                        cc = (float)csum;
-                        dxc = (float)sx;
-                        dyc = (float)sy;
-                    }
+#pragma unroll
+                for (int a = 0; a < 4; a++) {
+                    const int j = at[a];
+                    if (!has[a] || !m[j]) continue;
+                    any = true;
+                    const double tj = t[j];
+                    csum += tj * ((double)c[j] * tj + (double)dx[j - 1] * (tj - t[j - 1]) + (double)dx[j] * (tj - t[j + 1]) +
+                                  (double)dy[j - p] * (tj - t[j - p]) + (double)dy[j] * (tj - t[j + p]));
+                    if (a & 1) sx += tj * t[j + 1] * dx[j];
+                    if (a & 2) sy += tj * t[j + p] * dy[j];
                 }
-                S.c[1 - k][q] = cc;
-                S.dx[1 - k][q] = dxc;
-                S.dy[1 - k][q] = dyc;
-                S.m[1 - k][q] = any;
+                const int o = (Y + 1) * p + X + 1;
+                S.c[1 - k][o] = any ? (float)csum : 1.0f;
+                S.dx[1 - k][o] = any ? (float)sx : 0.0f;
+                S.dy[1 - k][o] = any ? (float)sy : 0.0f;
+                S.m[1 - k][o] = any;
             }
         }
-        for (int q = tid; q < T.p * T.hp; q += TS_NT) {
-            const int x = q % T.p, y = q / T.p, j = (y + 1) * p + x + 1;
-            const bool ok = x < w && y < h;
-            img[T.dx + q] = ok ? dx[j] : 0.0f;
-            img[T.dy + q] = ok ? dy[j] : 0.0f;
-            img[T.inv + q] = ok && m[j] ? 1.0f / (c[j] + dx[j] + dy[j] + dx[j - 1] + dy[j - p]) : 0.0f;
-            img[T.t + q] = ok && !coarsest ? t[j] : 0.0f;
-            img[T.c + q] = ok ? c[j] : 1.0f;
-            if (l > A.t) {
-                img[T.b + q] = 0.0f;
-                img[T.x + q] = 0.0f;
+        if (x64 < T.p)
+            for (int y = y64; y < T.hp; y += 16) {
+                const int q = y * T.p + x64, j = (y + 1) * p + x64 + 1;
+                const bool ok = x64 < w && y < h;
+                img[T.dx + q] = ok ? dx[j] : 0.0f;
+                img[T.dy + q] = ok ? dy[j] : 0.0f;
+                img[T.inv + q] = ok && m[j] ? 1.0f / (c[j] + dx[j] + dy[j] + dx[j - 1] + dy[j - p]) : 0.0f;
+                img[T.t + q] = ok && !coarsest ? t[j] : 0.0f;
+                img[T.c + q] = ok ? c[j] : 1.0f;
+                if (l > 0) {
+                    img[T.b + q] = 0.0f;
+                    img[T.x + q] = 0.0f;
+                }
             }
-        }
-        if (coarsest) tail_inverse(S, k, w, h, p, img + A.sinv, 4 * A.img_f4 - A.sinv);
+        if (coarsest) tail_inverse(S, k, w, h, img + A.sinv, 4 * A.img_f4 - A.sinv);
     }
 }
 
@@ -1429,7 +1459,7 @@ void Multigrid::create(int w, int h, int pre_, int post_) {
     }
     tail = 0;
     while (L[tail].w > kMgTailSide || L[tail].h > kMgTailSide) tail++;
-    SR_REQUIRE(nlevels - tail >= 3 && (size_t)L[nlevels - 1].w * L[nlevels - 1].h <= 16, "the coarse tail's levels");
+    SR_REQUIRE(nlevels - tail >= 3 && nlevels - tail <= kTailLevels && (size_t)L[nlevels - 1].w * L[nlevels - 1].h <= 16, "the coarse tail's levels");
     // the levels down to the tail's top; those below it live in the tail's image
     for (int l = 0; l <= tail; l++) {
         MgLevel& L = this->L[l];
@@ -1514,7 +1544,7 @@ void Multigrid::coarsen(cudaStream_t s) {
     }
     TailArgs T;
     tail_args(*this, T);
-    mg_tail_setup_kernel<<<1, TS_NT, sizeof(TailSetupShared), s>>>(T, L[tail], tail_img);
+    mg_tail_setup_kernel<<<1, TS_NT, sizeof(TailSetupShared), s>>>(T, L[tail], tail == 0, tail_img);
     sr_note_launch();
 }
 
