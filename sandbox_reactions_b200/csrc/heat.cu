@@ -474,15 +474,49 @@ __global__ void pcg_direction_kernel(size_t n, const double* __restrict__ scal, 
     }
 }
 
+// Σ v[0..n) by the block, in an order that depends on n and the block's size alone; valid in thread 0.
+__device__ __forceinline__ double block_sum_ordered(const double* __restrict__ v, int n) {
+    __shared__ double red[32];
+    double x = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) x += v[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
+    return t;
+}
+
+__global__ void sum_parts_kernel(const double* __restrict__ v, int n, double* out) {
+    const double t = block_sum_ordered(v, n);
+    if (threadIdx.x == 0) *out = t;
+}
+
 // After a (non-flexible) round's preconditioner: the search direction p_new = z + β p (β = <r,z> / <r,z>_prev, or
 // p_new = z while the S_BETA flag is 0: the first round) and q = A p_new in difference form, with partials of
 // <p_new, q>; the last CTA sets the flag. Four consecutive cells of a row per thread with 16-byte loads (W is a
 // multiple of 8); the neighbours' p_new are formed from their z and old p, so p_new goes to the other of the two
 // direction buffers (S_PAR says which holds the old one).
-__global__ void spmv_dir_kernel(MgLevel L, const double* __restrict__ scal, const float* __restrict__ z, float* pa,
-                                float* pb, float* __restrict__ q, Red R, double* beta_flag) {
+// <r, z> comes as the preconditioner's `parts` partials, which every CTA sums for itself in the same order (0: it is in
+// S_RZN already); the first CTA leaves it there.
+__global__ void spmv_dir_kernel(MgLevel L, double* scal, const float* __restrict__ z, float* pa, float* pb,
+                                float* __restrict__ q, Red R, double* beta_flag, const double* __restrict__ rz_part,
+                                int parts) {
+    __shared__ double s_rz;
+    if (parts > 0) {
+        const double v = block_sum_ordered(rz_part, parts);
+        if (threadIdx.x == 0) {
+            s_rz = v;
+            if (blockIdx.x == 0) scal[S_RZN] = v;
+        }
+    } else if (threadIdx.x == 0) {
+        s_rz = scal[S_RZN];
+    }
+    __syncthreads();
     const bool first = scal[S_BETA] == 0.0;  // p = z: the old direction is not read (it may hold anything)
-    const float beta = first ? 0.0f : (float)(scal[S_RZN] / scal[S_RZP]);
+    const float beta = first ? 0.0f : (float)(s_rz / scal[S_RZP]);
     const bool par = scal[S_PAR] != 0.0;
     const float* __restrict__ p = par ? pb : pa;
     float* __restrict__ pnew = par ? pa : pb;
@@ -1100,6 +1134,7 @@ struct HeatSolver {
     float* p2 = nullptr;  // the fused rounds' second direction buffer (rounds alternate p32 -> p2 -> p32)
     float *fx = nullptr, *fy = nullptr;
     double* part = nullptr;      // grid-sum partials: 4 x PART_CAP
+    double* rz_part = nullptr;   // the preconditioner's partials of <r, z>
     unsigned* counter = nullptr;  // grid-sum ticket
     double* scal = nullptr;       // S_COUNT device scalars
     double* hscal = nullptr;      // pinned host copy
@@ -1152,7 +1187,7 @@ void setup_step(HeatSolver* H, const float* U, const float* kappa, cudaStream_t 
     H->mg.set_couplings(H->kx, H->ky, H->gas, s);
 }
 
-// z = M r, and <r, z> into scalar `rz_slot`.
+// z = M r, and <r, z> into scalar `rz_slot` (into S_RZN, multigrid's: as partials, for spmv_dir_kernel to sum).
 void precondition(HeatSolver* H, uint32_t precond, int rz_slot, cudaStream_t s) {
     if (precond == SR_PRECOND_JACOBI) {
         jacobi_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->mg.L[0], H->r32, H->z32, H->red(rz_slot));
@@ -1162,17 +1197,21 @@ void precondition(HeatSolver* H, uint32_t precond, int rz_slot, cudaStream_t s) 
         // smooth error the first cycle leaves; the second cycle removes the rounding noise of its BF16 output (high
         // frequencies, which the smoothers take out) and what remains of the smooth error.
         const MgLevel& L0 = H->mg.L[0];
-        H->mg.apply(H->r32, H->z32, H->part, H->counter, H->scal + S_MGRZ, s);
+        H->mg.apply(H->r32, H->z32, nullptr, s);
         vcycle_residual_kernel<<<H->grid, RED_THREADS, 0, s>>>(L0, H->r32, H->z32, nullptr, H->q32, nullptr);
         sr_note_launch();
         learned_apply(H->lapply, L0, H->q32, H->z32, H->r32, H->z32, H->part, H->counter, H->scal + S_MGRZ, s);
         vcycle_residual_kernel<<<H->grid, RED_THREADS, 0, s>>>(L0, H->r32, H->z32, nullptr, H->q32, nullptr);
         sr_note_launch();
-        H->mg.apply(H->q32, H->vz, H->part, H->counter, H->scal + S_MGRZ, s);
+        H->mg.apply(H->q32, H->vz, nullptr, s);
         add_dot_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->r32, H->vz, H->z32, H->red(rz_slot));
         sr_note_launch();
     } else {
-        H->mg.apply(H->r32, H->z32, H->part, H->counter, H->scal + rz_slot, s);
+        H->mg.apply(H->r32, H->z32, H->rz_part, s);
+        if (rz_slot != S_RZN) {  // a round outside the fused loop: its kernels read the sum
+            sum_parts_kernel<<<1, RED_THREADS, 0, s>>>(H->rz_part, H->mg.parts(), H->scal + rz_slot);
+            sr_note_launch();
+        }
     }
 }
 
@@ -1201,7 +1240,8 @@ void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s)
     (void)rz_new;
     precondition(H, precond, S_RZN, s);
     spmv_dir_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2, H->q32,
-                                                    H->red(S_PQ), H->scal + S_BETA);
+                                                    H->red(S_PQ), H->scal + S_BETA, H->rz_part,
+                                                    precond == SR_PRECOND_MG ? H->mg.parts() : 0);
     sr_note_launch();
     pcg_update4_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, H->p32, H->p2, H->q32, H->e32, H->r32,
                                                        H->red(S_RRI));
@@ -1434,7 +1474,8 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                                                [&](cudaStream_t s4) {
                         precondition(H, precond, S_RZN, s4);
                         spmv_dir_kernel<<<H->grid, RED_THREADS, 0, s4>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2,
-                                                                          H->q32, H->red(S_PQ), H->scal + S_BETA);
+                                                                          H->q32, H->red(S_PQ), H->scal + S_BETA, H->rz_part,
+                                                    precond == SR_PRECOND_MG ? H->mg.parts() : 0);
                         sr_note_launch();
                         pcg_update4_kernel<<<H->grid, RED_THREADS, 0, s4>>>(H->n, H->scal, H->p32, H->p2, H->q32,
                                                                              H->e32, H->r32, H->red(S_RRI));
@@ -1561,6 +1602,7 @@ HeatSolver* heat_create(const sr_config& cfg, cudaStream_t s) {
         SR_CUDA_TRY(cudaMemset(H->fx, 0, sizeof(float) * nx));
         SR_CUDA_TRY(cudaMemset(H->fy, 0, sizeof(float) * ny));
         SR_CUDA_TRY(cudaMalloc(&H->part, sizeof(double) * 4 * PART_CAP));
+        SR_CUDA_TRY(cudaMalloc(&H->rz_part, sizeof(double) * PART_CAP));
         SR_CUDA_TRY(cudaMalloc(&H->counter, sizeof(unsigned)));
         SR_CUDA_TRY(cudaMemset(H->counter, 0, sizeof(unsigned)));
         SR_CUDA_TRY(cudaMalloc(&H->scal, sizeof(double) * S_COUNT));
@@ -1599,6 +1641,7 @@ void heat_destroy(HeatSolver* H) {
     float* d32[] = {H->kap, H->sig, H->r32, H->e32, H->p32, H->q32, H->z32, H->fx, H->fy, H->p2};
     for (float* p : d32) cudaFree(p);
     cudaFree(H->part);
+    cudaFree(H->rz_part);
     cudaFree(H->counter);
     cudaFree(H->scal);
     cudaFree(H->r_old);

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(CO_NT) mg_coarsen_kernel(MgLevel F, MgLevel C)
 // One smoother on a big level, all NS half-sweeps of a tile in shared memory (the tile's halo as deep as the
 // half-sweeps, so the tile's result is exactly the global red-black sweeps'). PRE: from x = 0, red first, into L.x,
 // then the residual summed over each 2x2 aggregate into the coarse level's b (one more halo ring keeps the residual's
-// neighbours exact). POST: from x = L.x + ω P xc, black first, into L.x2; at level 0 `out` gets <b, x2>.
+// neighbours exact). POST: from x = L.x + ω P xc, black first, into L.x2.
 //
 // The tile is stored split by colour (cell (lx, ly) of colour (lx + ly) & 1 at ly * HX + lx / 2 of its colour's
 // arrays), so that a half-sweep's consecutive threads update consecutive cells of one colour and read their
@@ -233,8 +233,7 @@ constexpr size_t smooth_smem() {
 
 template <int NS, bool PRE, int SX, int SY, int NT>
 __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, const float* __restrict__ xc,
-                                                                    float omega, double* part, unsigned* counter,
-                                                                    double* out) {
+                                                                    float omega) {
     constexpr int H = PRE ? NS + 1 : NS;
     constexpr int RX = SX + 2 * H, RY = SY + 2 * H, RN = RX * RY, HX = RX / 2, HN = HX * RY;
     static_assert(RX % 2 == 0, "the tile's rows split evenly by colour");
@@ -307,7 +306,6 @@ __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, con
         }
         __syncthreads();
     }
-    double acc = 0.0;
     float* dst = PRE ? L.x : L.x2;
     for (int k = tid; k < SX * SY; k += NT) {
         const int ox = k % SX, oy = k / SX;
@@ -316,7 +314,6 @@ __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, con
             const int lx = ox + H, ly = oy + H, col = (lx + ly) & 1, q = ly * HX + (lx >> 1);
             const float xv = arr(A_X, col)[q];
             dst[(size_t)gy * w + gx] = xv;
-            if (!PRE && out) acc += (double)arr(A_B, col)[q] * (double)xv;
         }
     }
     if (PRE) {
@@ -346,8 +343,6 @@ __global__ void __launch_bounds__(NT) mg_smooth_kernel(MgLevel L, MgLevel C, con
                 }
             C.b[(size_t)Y * C.w + X] = C.mask[(size_t)Y * C.w + X] ? sum : 0.0f;
         }
-    } else if (out) {
-        grid_sum_last1(acc, part, counter, out);
     }
 }
 
@@ -369,10 +364,25 @@ constexpr int RB_R = 4, RB_WARPS = 16, RB_NT = 32 * RB_WARPS, RB_RX = 64, RB_RY 
 template <int NS, bool PRE>
 constexpr int rb_halo() { return NS; }
 
+// The CTA's share of <b, x2>, left for the kernel that reads it to sum (Multigrid::apply). A ticket and a last CTA here
+// would hold every CTA's registers and shared memory for an atomic's round trip at its end.
+__device__ __forceinline__ void cta_partial(double acc, double* part) {
+    __shared__ double red[RB_WARPS];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < RB_WARPS; q++) t += red[q];
+        part[blockIdx.y * gridDim.x + blockIdx.x] = t;
+    }
+}
+
 template <int NS, bool PRE, bool WT>
 __global__ void __launch_bounds__(RB_NT, 2) mg_rowband_kernel(MgLevel L, MgLevel C, const float* __restrict__ xc,
-                                                            float omega, double* part, unsigned* counter,
-                                                            double* out) {
+                                                            float omega, double* part) {
     constexpr int H = rb_halo<NS, PRE>(), SX = RB_RX - 2 * H, SY = RB_RY - 2 * H;
     static_assert(H % 2 == 0 && NS % 2 == 0, "the region starts on an even column and row");
     __shared__ float2 edge[2][2][RB_WARPS][32];  // [buffer][top row / bottom row][warp][lane]: (x of 2j, x of 2j+1)
@@ -513,10 +523,10 @@ __global__ void __launch_bounds__(RB_NT, 2) mg_rowband_kernel(MgLevel L, MgLevel
             if (xout && ly >= H && ly < RB_RY - H && gy < h) {
                 const size_t i = (size_t)gy * w + gx;
                 *reinterpret_cast<float2*>(L.x2 + i) = make_float2(xA[r], xB[r]);
-                if (out) acc += (double)bA[r] * (double)xA[r] + (double)bB[r] * (double)xB[r];
+                if (part) acc += (double)bA[r] * (double)xA[r] + (double)bB[r] * (double)xB[r];
             }
         }
-        if (out) grid_sum_last1(acc, part, counter, out);
+        if (part) cta_partial(acc, part);
     }
     (void)SX;
     (void)SY;
@@ -545,7 +555,7 @@ __global__ void __launch_bounds__(RB_NT, 2)
     mg_rowband_tma_kernel(const __grid_constant__ CUtensorMap mb, const __grid_constant__ CUtensorMap mc,
                           const __grid_constant__ CUtensorMap mdx, const __grid_constant__ CUtensorMap mdy,
                           const __grid_constant__ CUtensorMap mx, MgLevel L, MgLevel C, const float* __restrict__ xc,
-                          float omega, double* part, unsigned* counter, double* out) {
+                          float omega, double* part) {
     constexpr int H = rb_halo<NS, PRE>(), SX = RB_RX - 2 * H;
     constexpr int XO = (H % 4 == 2) ? 2 : 4;  // the region's first column within the box (X0 - XO on a 16-byte boundary)
     constexpr int NA = rb_tma_arrays<PRE, WT>();
@@ -733,10 +743,10 @@ __global__ void __launch_bounds__(RB_NT, 2)
             if (xout && ly >= H && ly < RB_RY - H && gy < h) {
                 const size_t i = (size_t)gy * w + gx;
                 *reinterpret_cast<float2*>(L.x2 + i) = make_float2(xA[r], xB[r]);
-                if (out) acc += (double)bA[r] * (double)xA[r] + (double)bB[r] * (double)xB[r];
+                if (part) acc += (double)bA[r] * (double)xA[r] + (double)bB[r] * (double)xB[r];
             }
         }
-        if (out) grid_sum_last1(acc, part, counter, out);
+        if (part) cta_partial(acc, part);
     }
 }
 
@@ -1310,11 +1320,9 @@ __global__ void __launch_bounds__(TS_NT) mg_tail_setup_kernel(const __grid_const
 
 // Level 0's width is even, so every level that comes here has weights.
 template <int NS, bool PRE, int SX, int SY, int NT>
-void launch_smooth_t(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, unsigned* counter,
-                     double* out, cudaStream_t s) {
+void launch_smooth_t(const MgLevel& L, const MgLevel& C, const float* xc, float omega, cudaStream_t s) {
     const dim3 grid(div_up(L.w, SX), div_up(L.h, SY));
-    mg_smooth_kernel<NS, PRE, SX, SY, NT><<<grid, NT, smooth_smem<NS, PRE, SX, SY>(), s>>>(L, C, xc, omega, part,
-                                                                                        counter, out);
+    mg_smooth_kernel<NS, PRE, SX, SY, NT><<<grid, NT, smooth_smem<NS, PRE, SX, SY>(), s>>>(L, C, xc, omega);
     sr_note_launch();
 }
 
@@ -1341,8 +1349,7 @@ constexpr int tile_sy() {
 }
 
 template <int NS, bool PRE>
-void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, unsigned* counter,
-                    double* out, cudaStream_t s) {
+void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, cudaStream_t s) {
     constexpr int H = rb_halo<NS, PRE>();
     const dim3 grid(div_up(L.w, RB_RX - 2 * H), div_up(L.h, RB_RY - 2 * H));
     // rows of 16 bytes and 16-byte bases: the region staged by TMA
@@ -1362,7 +1369,7 @@ void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float o
                 SR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 attr = true;
             }
-            kernel<<<grid, RB_NT, smem, s>>>(mb, mc, mdx, mdy, mx, L, C, xc, omega, part, counter, out);
+            kernel<<<grid, RB_NT, smem, s>>>(mb, mc, mdx, mdy, mx, L, C, xc, omega, part);
         };
         static bool attr_w = false, attr_u = false;
         if (L.t) go(mg_rowband_tma_kernel<NS, PRE, true>, rb_tma_smem<PRE, true>(), attr_w);
@@ -1370,8 +1377,8 @@ void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float o
         sr_note_launch();
         return;
     }
-    if (L.t) mg_rowband_kernel<NS, PRE, true><<<grid, RB_NT, 0, s>>>(L, C, xc, omega, part, counter, out);
-    else mg_rowband_kernel<NS, PRE, false><<<grid, RB_NT, 0, s>>>(L, C, xc, omega, part, counter, out);
+    if (L.t) mg_rowband_kernel<NS, PRE, true><<<grid, RB_NT, 0, s>>>(L, C, xc, omega, part);
+    else mg_rowband_kernel<NS, PRE, false><<<grid, RB_NT, 0, s>>>(L, C, xc, omega, part);
     sr_note_launch();
 }
 
@@ -1379,30 +1386,28 @@ void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float o
 // shared-memory tiles at every size (level 0 of a 512² world under V(4,4): pre 11.9 -> 4.7 us, post 12.5 -> 7.0). Levels
 // of odd width take the shared-memory tiles, the small one where the big one leaves fewer than 2 CTAs per SM.
 template <int NS, bool PRE>
-void launch_smooth(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, unsigned* counter,
-                   double* out, cudaStream_t s) {
+void launch_smooth(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, cudaStream_t s) {
     if (L.w % 2 == 0)
-        launch_rowband<NS, PRE>(L, C, xc, omega, part, counter, out, s);
+        launch_rowband<NS, PRE>(L, C, xc, omega, part, s);
     else if (small_tiles(L))
         launch_smooth_t<NS, PRE, SMALL_SX, tile_sy<NS, PRE, SMALL_SX, SMALL_SY, SMALL_NT>(), SMALL_NT>(
-            L, C, xc, omega, part, counter, out, s);
+            L, C, xc, omega, s);
     else
-        launch_smooth_t<NS, PRE, BIG_SX, tile_sy<NS, PRE, BIG_SX, BIG_SY, BIG_NT>(), BIG_NT>(L, C, xc, omega, part,
-                                                                                           counter, out, s);
+        launch_smooth_t<NS, PRE, BIG_SX, tile_sy<NS, PRE, BIG_SX, BIG_SY, BIG_NT>(), BIG_NT>(L, C, xc, omega, s);
 }
 
 void smooth(int nu, bool pre, const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part,
-            unsigned* counter, double* out, cudaStream_t s) {
+            cudaStream_t s) {
     if (pre) {
-        if (nu == 1) launch_smooth<2, true>(L, C, xc, omega, part, counter, out, s);
-        else if (nu == 2) launch_smooth<4, true>(L, C, xc, omega, part, counter, out, s);
-        else if (nu == 3) launch_smooth<6, true>(L, C, xc, omega, part, counter, out, s);
-        else launch_smooth<8, true>(L, C, xc, omega, part, counter, out, s);
+        if (nu == 1) launch_smooth<2, true>(L, C, xc, omega, part, s);
+        else if (nu == 2) launch_smooth<4, true>(L, C, xc, omega, part, s);
+        else if (nu == 3) launch_smooth<6, true>(L, C, xc, omega, part, s);
+        else launch_smooth<8, true>(L, C, xc, omega, part, s);
     } else {
-        if (nu == 1) launch_smooth<2, false>(L, C, xc, omega, part, counter, out, s);
-        else if (nu == 2) launch_smooth<4, false>(L, C, xc, omega, part, counter, out, s);
-        else if (nu == 3) launch_smooth<6, false>(L, C, xc, omega, part, counter, out, s);
-        else launch_smooth<8, false>(L, C, xc, omega, part, counter, out, s);
+        if (nu == 1) launch_smooth<2, false>(L, C, xc, omega, part, s);
+        else if (nu == 2) launch_smooth<4, false>(L, C, xc, omega, part, s);
+        else if (nu == 3) launch_smooth<6, false>(L, C, xc, omega, part, s);
+        else launch_smooth<8, false>(L, C, xc, omega, part, s);
     }
 }
 
@@ -1433,13 +1438,8 @@ int grid_for(size_t n) {
 }  // namespace
 
 size_t mg_smooth_ctas(int w, int h) {
-    MgLevel L;
-    L.w = w;
-    L.h = h;
-    // a bound: the shortest tile tile_sy can pick, or the row-band kernel's smallest output tile (V(4,4)'s pre-smoother)
-    const size_t rb = (size_t)div_up(w, RB_RX - 2 * rb_halo<8, true>()) * div_up(h, RB_RY - 2 * rb_halo<8, true>());
-    return std::max(rb, small_tiles(L) ? (size_t)div_up(w, SMALL_SX) * div_up(h, SMALL_SY - 6)
-                                       : (size_t)div_up(w, BIG_SX) * div_up(h, BIG_SY - 6));
+    constexpr unsigned out = RB_RX - 2 * rb_halo<8, false>();  // the smallest output tile
+    return (size_t)div_up(w, out) * div_up(h, out);
 }
 
 void Multigrid::create(int w, int h, int pre_, int post_) {
@@ -1548,19 +1548,23 @@ void Multigrid::coarsen(cudaStream_t s) {
     sr_note_launch();
 }
 
-void Multigrid::apply(const float* r, float* z, double* part, unsigned* counter, double* rz_out, cudaStream_t s) {
+int Multigrid::parts() const {
+    if (tail == 0) return 1;
+    const unsigned out = RB_RX - 2 * (2 * post);  // the post-smoother's halo is its half-sweeps
+    return (int)(div_up(L[0].w, out) * div_up(L[0].h, out));
+}
+
+void Multigrid::apply(const float* r, float* z, double* rz_part, cudaStream_t s) {
     L[0].b = const_cast<float*>(r);
     L[0].x2 = z;
-    for (int l = 0; l < tail; l++)
-        smooth(pre, true, L[l], L[l + 1], nullptr, omega, nullptr, nullptr, nullptr, s);
+    for (int l = 0; l < tail; l++) smooth(pre, true, L[l], L[l + 1], nullptr, omega, nullptr, s);
     TailArgs T;
     const size_t ts = tail_args(*this, T);
-    T.out = tail == 0 ? rz_out : nullptr;
+    T.out = tail == 0 ? rz_part : nullptr;
     mg_tail_kernel<<<1, TAIL_THREADS, ts, s>>>(T);
     sr_note_launch();
     for (int l = tail - 1; l >= 0; l--)
-        smooth(post, false, L[l], L[l + 1], L[l + 1].x2, omega, l == 0 ? part : nullptr, l == 0 ? counter : nullptr,
-               l == 0 ? rz_out : nullptr, s);
+        smooth(post, false, L[l], L[l + 1], L[l + 1].x2, omega, l == 0 ? rz_part : nullptr, s);
 }
 
 void Multigrid::time_level0(int reps, void* flush, size_t flush_bytes, cudaStream_t s, double* pre_ms,
@@ -1576,9 +1580,9 @@ void Multigrid::time_level0(int reps, void* flush, size_t flush_bytes, cudaStrea
             SR_CUDA_TRY(cudaMemsetAsync(flush, k & 0xff, flush_bytes, s));
             SR_CUDA_TRY(cudaEventRecord(a, s));
             if (which == 0)
-                smooth(pre, true, L[0], L[1], nullptr, omega, nullptr, nullptr, nullptr, s);
+                smooth(pre, true, L[0], L[1], nullptr, omega, nullptr, s);
             else
-                smooth(post, false, L[0], L[1], L[1].x2, omega, nullptr, nullptr, nullptr, s);
+                smooth(post, false, L[0], L[1], L[1].x2, omega, nullptr, s);
             SR_CUDA_TRY(cudaEventRecord(b, s));
             SR_CUDA_TRY(cudaEventSynchronize(b));
             float t = 0.0f;

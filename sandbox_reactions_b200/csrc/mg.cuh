@@ -33,7 +33,7 @@ struct MgLevel {
     int* err = nullptr;   // set to 1 when a bounded wait of a smoother gave up (its TMA boxes never landed)
 };
 
-// At most this many CTAs in one smoother launch on a w x h level (each writes one grid-sum partial at level 0).
+// At most this many CTAs in a post-smoother launch on a w x h level 0 (each leaves one partial of <r, z>).
 size_t mg_smooth_ctas(int w, int h);
 
 struct Multigrid {
@@ -53,8 +53,9 @@ struct Multigrid {
     void set_couplings(const double* kx, const double* ky, const uint8_t* gas, cudaStream_t s);
     // Every coarse level's operator, once level 0's c (written by the caller, per Newton pass) is in place.
     void coarsen(cudaStream_t s);
-    // z = M r (level-0 b := r, x2 := z), and <r, z> into *rz_out (a one-launch grid sum over `part` and `counter`).
-    void apply(const float* r, float* z, double* part, unsigned* counter, double* rz_out, cudaStream_t s);
+    // z = M r (level-0 b := r, x2 := z), and (rz_part not null) <r, z> as parts() partials, to be summed in order.
+    void apply(const float* r, float* z, double* rz_part, cudaStream_t s);
+    int parts() const;
     // The device time (ms) of one launch of level 0's pre- and post-smoother on the last applied system, each
     // averaged over `reps` launches with `flush` (flush_bytes, larger than L2) rewritten before each: a timing hook.
     void time_level0(int reps, void* flush, size_t flush_bytes, cudaStream_t s, double* pre_ms, double* post_ms);
