@@ -17,6 +17,7 @@
 
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <string>
@@ -105,7 +106,10 @@ __device__ __forceinline__ void face_work(float q, float sl, float sh, float pl,
 // write nothing. The four planes of the tile grown by two cells (the reconstruction's reach) arrive in one TMA box;
 // the world's ghosts (hydro.rs:686-709) are formed from it in shared memory. Each lane predicts its cell's four faces
 // (hydro.rs:587-614); the x faces meet by warp shuffles (a lane's x+ face against the next lane's x- face), the y faces
-// through shared memory (a row's y+ faces against the next row's y- faces); the fluxes go back the same ways.
+// through shared memory (a row's y+ faces against the next row's y- faces); the fluxes go back the same ways. The kernel
+// is persistent, two CTAs per SM walking the tiles: a tile's box lands while the one before is worked on, and the grid's
+// sum takes one ticket a CTA (a CTA per tile held its SM for the box's and the ticket's latency: gas alone at 512²,
+// 23.6 -> 19.6 us a step).
 constexpr int HB_TX = 30, HB_TY = 14, HB_W = HB_TY + 2, HB_NT = 32 * HB_W;
 constexpr int HB_SX = HB_TX + 4, HB_SY = HB_TY + 4;  // the staged region: the tile grown by 2
 constexpr int HB_BX = 40, HB_BY = HB_SY;             // the TMA box: from a 16-byte aligned column, wide enough
@@ -167,7 +171,7 @@ __device__ __forceinline__ bool grid_total(P& v, void* parts, unsigned* tickets)
     P* rows = part + (size_t)gridDim.x * gridDim.y;
     const int lane = threadIdx.x & 31;
 #pragma unroll 1
-    for (int level = 0; level < 2; level++) {
+    for (int level = 0; level < (gridDim.y > 1 ? 2 : 1); level++) {
         P* slot = level ? rows + blockIdx.y : part + (size_t)blockIdx.y * gridDim.x + blockIdx.x;
         unsigned* ticket = tickets + (level ? gridDim.y : blockIdx.y);
         const unsigned count = level ? gridDim.y : gridDim.x;
@@ -195,7 +199,7 @@ __device__ __forceinline__ bool grid_total(P& v, void* parts, unsigned* tickets)
 }
 
 struct __align__(128) BandShared {
-    float raw[4][HB_BY][HB_BX];  // the TMA box of Σ, Σu, Σv, E (first: 128-byte aligned)
+    float raw2[2][4][HB_BY][HB_BX];  // the TMA boxes of Σ, Σu, Σv, E, this tile's and the next's (128-byte aligned)
     float4 P[HB_SY][HB_SX];      // primitives (Σ, u, v, Π) of the staged region, ghosts included
     float Q[HB_SY][HB_SX];       // Π/Σ (the thermal bracket's temperatures)
     float S[HB_SY][HB_SX];       // raw Σ (out of the world: -1, read as vacuum)
@@ -203,8 +207,9 @@ struct __align__(128) BandShared {
     float YF[7][HB_W][32];       // each lane's y+ face
     float FY[4][HB_W][32];       // the flux through each lane's top face
     RatePart red[HB_W];          // the rows' partials
-    uint64_t mbar;
+    uint64_t mbar[2];
 };
+static_assert(sizeof(float) * 4 * HB_BY * HB_BX % 128 == 0, "the second box is 128-byte aligned");
 
 __device__ __forceinline__ Prim prim_at(const BandShared& sh, int y, int x) {
     const float4 q = sh.P[y][x];
@@ -394,21 +399,22 @@ __device__ __forceinline__ void take_back(KickPart kp, KickPart* red, const Hydr
 // A thread takes four neighbouring columns (16-byte accesses: the world's width is a multiple of 8) of HG_R rows,
 // works out the faces to the right of and below each of its cells once, and hands the right one to the next lane; a
 // cell with no gas around it (its source stored as -0) takes nothing but lends its faces. Bound by HBM: 68 B a cell.
-constexpr int HG_R = 4, HG_WARPS = 4;
+constexpr int HG_R = 4, HG_WARPS = 4, HG_COLS = 128;
 
-__global__ void __launch_bounds__(32 * HG_WARPS) hydro_gravity_kernel(HydroArgs A) {
+__global__ void __launch_bounds__(32 * HG_WARPS, 4) hydro_gravity_kernel(HydroArgs A) {
     __shared__ KickPart red[HG_WARPS];
     const int w = A.H.w, h = A.H.h;
     const size_t n = (size_t)w * h;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int x = blockIdx.x * 128 + 4 * lane, y0 = (blockIdx.y * HG_WARPS + warp) * HG_R;
+    const int x = blockIdx.x * HG_COLS + 4 * lane, y0 = (blockIdx.y * HG_WARPS + warp) * HG_R;
     const float dt = (float)(*A.dt);
     const bool on = x < w;
     struct Row {
         float m[3][4], p[4];
     };
+    // what this kernel does not write, as read-only loads: the stores of one row hold back no load of the next
     auto load4 = [&](const float* a, size_t i, float* v) {
-        const float4 q = *reinterpret_cast<const float4*>(a + i);
+        const float4 q = __ldg(reinterpret_cast<const float4*>(a + i));
         v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
     };
     auto load_row = [&](int y, Row& r) {
@@ -449,9 +455,13 @@ __global__ void __launch_bounds__(32 * HG_WARPS) hydro_gravity_kernel(HydroArgs 
         load4(A.src, i, src);
         load4(A.gxm, i, gx);
         load4(A.gym, i, gy);
-        load4(A.Uout + n, i, u1);
-        load4(A.Uout + 2 * n, i, u2);
-        load4(A.Uout + 3 * n, i, u3);
+        auto load_own = [&](const float* a, float* v) {
+            const float4 q = *reinterpret_cast<const float4*>(a + i);
+            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        };
+        load_own(A.Uout + n, u1);
+        load_own(A.Uout + 2 * n, u2);
+        load_own(A.Uout + 3 * n, u3);
         // the next column's mids and potential
         float mn[2], pn;
         mn[0] = __shfl_down_sync(0xffffffffu, c.m[0][0], 1);
@@ -523,198 +533,210 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
     const int w = H.w, h = H.h;
     const size_t n = (size_t)w * h;
     const int tid = threadIdx.x, lane = tid & 31, row = tid >> 5;
-    const int x0 = blockIdx.x * HB_TX, y0 = blockIdx.y * HB_TY;
-    const int xs = (x0 - 2) & ~3, ys = y0 - 2;  // the box's origin: x on a 16-byte boundary
     const float dt = (float)(*A.dt);
     const float half = 0.5f * dt;
     const bool grav = A.gx != nullptr;
+    const int ntx = (w + HB_TX - 1) / HB_TX, tiles = ntx * ((h + HB_TY - 1) / HB_TY);
 
-    // ---- the four planes of the staged region by one TMA box; every wait is bounded
+    // ---- the four planes of a tile's staged region by one TMA box (x on a 16-byte boundary); every wait is bounded
     if (tid == 0) {
-        tc::mbar_init(&sh.mbar, 1);
+        tc::mbar_init(&sh.mbar[0], 1);
+        tc::mbar_init(&sh.mbar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (tid == 0) {
-        tma::expect_tx(&sh.mbar, (uint32_t)sizeof(sh.raw));
-        tma::load_3d(&sh.raw[0][0][0], &map, xs, ys, 0, &sh.mbar);
-    }
-    const bool landed = tc::mbar_wait(&sh.mbar, 0, kHydroWaitPolls);
-    if (__syncthreads_or(!landed)) {
-        if (tid == 0) atomicOr(A.err, 1);
-        tc::mbar_wait(&sh.mbar, 0, kHydroWaitPolls);  // the copy still in flight lands before the CTA leaves
-        return;
-    }
-
-    // ---- primitives of the staged region: world cells, or ghosts past the edges (bounce mirrors the cells beyond
-    // with the normal velocity negated, leave copies the edge cell with it clamped outward)
-    for (int k = tid; k < HB_SY * HB_SX; k += HB_NT) {
-        const int ly = k / HB_SX, lx = k - ly * HB_SX;
-        const int x = x0 - 2 + lx, y = y0 - 2 + ly;
-        Prim p;
-        float raw = -1.0f;
-        if (x >= -2 && x <= w + 1 && y >= -2 && y <= h + 1) {
-            const bool xo = x < 0 || x >= w, yo = y < 0 || y >= h;
-            int cx, cy;
-            if (H.edge == SR_EDGE_BOUNCE) {
-                cx = x < 0 ? -x - 1 : (x >= w ? 2 * w - 1 - x : x);
-                cy = y < 0 ? -y - 1 : (y >= h ? 2 * h - 1 - y : y);
-            } else {
-                cx = min(max(x, 0), w - 1);
-                cy = min(max(y, 0), h - 1);
-            }
-            const int bx = cx - xs, by = cy - ys;
-            const float s = sh.raw[0][by][bx];
-            p = eos_read(H, s, sh.raw[1][by][bx], sh.raw[2][by][bx], sh.raw[3][by][bx]);
-            raw = (xo || yo) ? -1.0f : s;
-            if (H.edge == SR_EDGE_BOUNCE) {
-                if (xo) p.u = -p.u;
-                if (yo) p.v = -p.v;
-            } else {
-                if (x < 0) p.u = fminf(p.u, 0.0f);
-                if (x >= w) p.u = fmaxf(p.u, 0.0f);
-                if (y < 0) p.v = fminf(p.v, 0.0f);
-                if (y >= h) p.v = fmaxf(p.v, 0.0f);
-            }
-        } else {
-            p.s = 1.0f; p.u = 0.0f; p.v = 0.0f; p.p = 1.0f;  // past every ghost: never reaches a kept cell
-        }
-        sh.P[ly][lx] = make_float4(p.s, p.u, p.v, p.p);
-        sh.Q[ly][lx] = sr_div(p.p, p.s);
-        sh.S[ly][lx] = raw;
-    }
-    __syncthreads();
-
-    // ---- this lane's cell: slopes, the Hancock increment and the half-step centre (hydro.rs:587-614)
-    const int sx = lane + 1, sy = row + 1;  // the cell in the staged region
-    const int X = x0 - 1 + lane, Y = y0 - 1 + row;
-    const Prim c = prim_at(sh, sy, sx);
-    const Prim slx = slope<LIM, BRACKET>(prim_at(sh, sy, sx - 1), c, prim_at(sh, sy, sx + 1), sh.Q[sy][sx - 1],
-                                         sh.Q[sy][sx], sh.Q[sy][sx + 1]);
-    const Prim sly = slope<LIM, BRACKET>(prim_at(sh, sy - 1, sx), c, prim_at(sh, sy + 1, sx), sh.Q[sy - 1][sx],
-                                         sh.Q[sy][sx], sh.Q[sy + 1][sx]);
-    float gxv = 0.0f, gyv = 0.0f;
-    if (grav) {  // a ghost takes its edge cell's g
-        const size_t gi = (size_t)min(max(Y, 0), h - 1) * w + min(max(X, 0), w - 1);
-        gxv = A.gx[gi];
-        gyv = A.gy[gi];
-    }
-    float delta[4];
-    {
-        float a[4], b[4], dxs[4];
-        face_flux(H, c, slx, -0.5f, 0, a);
-        face_flux(H, c, slx, 0.5f, 0, b);
-#pragma unroll
-        for (int k = 0; k < 4; k++) dxs[k] = a[k] - b[k];
-        face_flux(H, c, sly, -0.5f, 1, a);
-        face_flux(H, c, sly, 0.5f, 1, b);
-#pragma unroll
-        for (int k = 0; k < 4; k++) delta[k] = half * (dxs[k] + (a[k] - b[k]));
-    }
-    {
-        float m1 = c.s * c.u + delta[1], m2 = c.s * c.v + delta[2];
-        if (grav) {
-            m1 += half * c.s * gxv;
-            m2 += half * c.s * gyv;
-        }
-        sh.M[0][row][lane] = c.s + delta[0];
-        sh.M[1][row][lane] = m1;
-        sh.M[2][row][lane] = m2;
-    }
-
-    // ---- x faces: this lane's x+ face against the next lane's x- face; the left face's flux from the lane before
-    float fr[4], fl[4];
-    {
-        const FaceS R = shfl_face_down(face_state(H, c, slx, -0.5f, delta, half, grav, gxv, gyv));
-        const FaceS L = face_state(H, c, slx, 0.5f, delta, half, grav, gxv, gyv);
-        face_flux_at(H, L, R, 0, X + 1, w, Y >= 0 && Y < h, fr);
-#pragma unroll
-        for (int k = 0; k < 4; k++) fl[k] = __shfl_up_sync(0xffffffffu, fr[k], 1);
-    }
-    // ---- y faces: the row above's y+ faces against this row's y- faces, through shared memory
-    {
-        const FaceS T = face_state(H, c, sly, 0.5f, delta, half, grav, gxv, gyv);
-        sh.YF[0][row][lane] = T.U0;
-        sh.YF[1][row][lane] = T.U1;
-        sh.YF[2][row][lane] = T.U2;
-        sh.YF[3][row][lane] = T.U3;
-        sh.YF[4][row][lane] = T.u;
-        sh.YF[5][row][lane] = T.v;
-        sh.YF[6][row][lane] = T.P;
-    }
-    const FaceS B = face_state(H, c, sly, -0.5f, delta, half, grav, gxv, gyv);
-    __syncthreads();
-    if (row >= 1) {
-        FaceS L;
-        L.U0 = sh.YF[0][row - 1][lane];
-        L.U1 = sh.YF[1][row - 1][lane];
-        L.U2 = sh.YF[2][row - 1][lane];
-        L.U3 = sh.YF[3][row - 1][lane];
-        L.u = sh.YF[4][row - 1][lane];
-        L.v = sh.YF[5][row - 1][lane];
-        L.P = sh.YF[6][row - 1][lane];
-        float ft[4];
-        face_flux_at(H, L, B, 1, Y, h, X >= 0 && X < w, ft);
-#pragma unroll
-        for (int k = 0; k < 4; k++) sh.FY[k][row][lane] = ft[k];
-    }
-    __syncthreads();
-
-    // ---- epilogue: the tile's cells
-    const bool inside = lane >= 1 && lane <= HB_TX && row >= 1 && row <= HB_TY && X < w && Y < h;
-    const size_t i = inside ? (size_t)Y * w + X : 0;
-    float fu[4], fd[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        fu[k] = row >= 1 ? sh.FY[k][row][lane] : 0.0f;
-        fd[k] = row + 1 < HB_W ? sh.FY[k][row + 1][lane] : 0.0f;
-    }
-    // a cell with no gas around it stays empty (hydro.rs:733-742); out-of-world neighbours read as vacuum
-    const float sv = H.sigma_vac;
-    const bool vac = sh.S[sy][sx] < sv;
-    const bool empty = vac && sh.S[sy][sx - 1] < sv && sh.S[sy][sx + 1] < sv && sh.S[sy - 1][sx] < sv &&
-                       sh.S[sy + 1][sx] < sv;
-
+    auto request = [&](int tile, int buf) {
+        const int ty = tile / ntx, tx = tile - ty * ntx;
+        tma::expect_tx(&sh.mbar[buf], (uint32_t)sizeof(sh.raw2[0]));
+        tma::load_3d(&sh.raw2[buf][0][0][0], &map, (tx * HB_TX - 2) & ~3, ty * HB_TY - 2, 0, &sh.mbar[buf]);
+    };
+    if (tid == 0 && (int)blockIdx.x < tiles) request(blockIdx.x, 0);
     RatePart rp = RatePart::none();
-    if (inside) {
-        const int bx = X - xs, by = Y - ys;
-        float u[4];
-        if (empty || !vac) {
-            u[0] = sh.raw[0][by][bx]; u[1] = sh.raw[1][by][bx]; u[2] = sh.raw[2][by][bx]; u[3] = sh.raw[3][by][bx];
-        } else {
-            eos_cons(H, c, u);
+    int it = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, it++) {
+        const int buf = it & 1, next = tile + (int)gridDim.x;
+        const int x0 = (tile % ntx) * HB_TX, y0 = (tile / ntx) * HB_TY;
+        const int xs = (x0 - 2) & ~3, ys = y0 - 2;
+        float(&raw)[4][HB_BY][HB_BX] = sh.raw2[buf];
+        if (it > 0) __syncthreads();  // the tile before is done with the shared planes and with the other box
+        if (tid == 0 && next < tiles) request(next, 1 - buf);
+        const bool landed = tc::mbar_wait(&sh.mbar[buf], (it >> 1) & 1, kHydroWaitPolls);
+        if (__syncthreads_or(!landed)) {
+            if (tid == 0) atomicOr(A.err, 1);
+            tc::mbar_wait(&sh.mbar[buf], (it >> 1) & 1, kHydroWaitPolls);  // the copies still in flight land before the
+            if (next < tiles) tc::mbar_wait(&sh.mbar[1 - buf], ((it + 1) >> 1) & 1, kHydroWaitPolls);  // CTA leaves
+            break;  // its share of the grid's sum is still due
         }
-        if (!empty) {
-#pragma unroll
-            for (int q = 0; q < 4; q++) u[q] -= dt * ((fr[q] - fl[q]) + (fd[q] - fu[q]));
-        }
-        if (MODE == kHydroPredict) {
-            // what follows the half step's solve: an empty cell's source is -0 (gravity leaves the cell as it is)
-            float src = -0.0f;
-            if (!empty) {
-                const float start = vac ? sh.P[sy][sx].x : sh.S[sy][sx];
-                const float div = (fr[0] - fl[0]) + (fd[0] - fu[0]);
-                src = 0.5f * (sh.S[sy][sx] + (start - dt * div));
-                src = src >= sv ? src : 0.0f;
-            }
-            A.src[i] = src;
-            A.mid[i] = sh.M[0][row][lane];
-            A.mid[n + i] = sh.M[1][row][lane];
-            A.mid[2 * n + i] = sh.M[2][row][lane];
-            A.mfx[i] = fr[0];
-            A.mfy[i] = fd[0];
-        }
-        if (MODE == kHydroStep) {
-            floor_cell(H, u[0], u[1], u[2], u[3]);
-            rate_cell(H, u[0], u[1], u[2], u[3], i, rp.rate, rp.nf);
-        }
-        A.Uout[i] = u[0];
-        A.Uout[n + i] = u[1];
-        A.Uout[2 * n + i] = u[2];
-        A.Uout[3 * n + i] = u[3];
-    }
 
-    // ---- the grid's sums, in a fixed order: the rows of the tile, the CTAs of a grid row, the grid rows
+        // ---- primitives of the staged region: world cells, or ghosts past the edges (bounce mirrors the cells beyond
+        // with the normal velocity negated, leave copies the edge cell with it clamped outward)
+        for (int k = tid; k < HB_SY * HB_SX; k += HB_NT) {
+            const int ly = k / HB_SX, lx = k - ly * HB_SX;
+            const int x = x0 - 2 + lx, y = y0 - 2 + ly;
+            Prim p;
+            float solid = -1.0f;
+            if (x >= -2 && x <= w + 1 && y >= -2 && y <= h + 1) {
+                const bool xo = x < 0 || x >= w, yo = y < 0 || y >= h;
+                int cx, cy;
+                if (H.edge == SR_EDGE_BOUNCE) {
+                    cx = x < 0 ? -x - 1 : (x >= w ? 2 * w - 1 - x : x);
+                    cy = y < 0 ? -y - 1 : (y >= h ? 2 * h - 1 - y : y);
+                } else {
+                    cx = min(max(x, 0), w - 1);
+                    cy = min(max(y, 0), h - 1);
+                }
+                const int bx = cx - xs, by = cy - ys;
+                const float s = raw[0][by][bx];
+                p = eos_read(H, s, raw[1][by][bx], raw[2][by][bx], raw[3][by][bx]);
+                solid = (xo || yo) ? -1.0f : s;
+                if (H.edge == SR_EDGE_BOUNCE) {
+                    if (xo) p.u = -p.u;
+                    if (yo) p.v = -p.v;
+                } else {
+                    if (x < 0) p.u = fminf(p.u, 0.0f);
+                    if (x >= w) p.u = fmaxf(p.u, 0.0f);
+                    if (y < 0) p.v = fminf(p.v, 0.0f);
+                    if (y >= h) p.v = fmaxf(p.v, 0.0f);
+                }
+            } else {
+                p.s = 1.0f; p.u = 0.0f; p.v = 0.0f; p.p = 1.0f;  // past every ghost: never reaches a kept cell
+            }
+            sh.P[ly][lx] = make_float4(p.s, p.u, p.v, p.p);
+            sh.Q[ly][lx] = sr_div(p.p, p.s);
+            sh.S[ly][lx] = solid;
+        }
+        __syncthreads();
+
+        // ---- this lane's cell: slopes, the Hancock increment and the half-step centre (hydro.rs:587-614)
+        const int sx = lane + 1, sy = row + 1;  // the cell in the staged region
+        const int X = x0 - 1 + lane, Y = y0 - 1 + row;
+        const Prim c = prim_at(sh, sy, sx);
+        const Prim slx = slope<LIM, BRACKET>(prim_at(sh, sy, sx - 1), c, prim_at(sh, sy, sx + 1), sh.Q[sy][sx - 1],
+                                             sh.Q[sy][sx], sh.Q[sy][sx + 1]);
+        const Prim sly = slope<LIM, BRACKET>(prim_at(sh, sy - 1, sx), c, prim_at(sh, sy + 1, sx), sh.Q[sy - 1][sx],
+                                             sh.Q[sy][sx], sh.Q[sy + 1][sx]);
+        float gxv = 0.0f, gyv = 0.0f;
+        if (grav) {  // a ghost takes its edge cell's g
+            const size_t gi = (size_t)min(max(Y, 0), h - 1) * w + min(max(X, 0), w - 1);
+            gxv = A.gx[gi];
+            gyv = A.gy[gi];
+        }
+        float delta[4];
+        {
+            float a[4], b[4], dxs[4];
+            face_flux(H, c, slx, -0.5f, 0, a);
+            face_flux(H, c, slx, 0.5f, 0, b);
+#pragma unroll
+            for (int k = 0; k < 4; k++) dxs[k] = a[k] - b[k];
+            face_flux(H, c, sly, -0.5f, 1, a);
+            face_flux(H, c, sly, 0.5f, 1, b);
+#pragma unroll
+            for (int k = 0; k < 4; k++) delta[k] = half * (dxs[k] + (a[k] - b[k]));
+        }
+        {
+            float m1 = c.s * c.u + delta[1], m2 = c.s * c.v + delta[2];
+            if (grav) {
+                m1 += half * c.s * gxv;
+                m2 += half * c.s * gyv;
+            }
+            sh.M[0][row][lane] = c.s + delta[0];
+            sh.M[1][row][lane] = m1;
+            sh.M[2][row][lane] = m2;
+        }
+
+        // ---- x faces: this lane's x+ face against the next lane's x- face; the left face's flux from the lane before
+        float fr[4], fl[4];
+        {
+            const FaceS R = shfl_face_down(face_state(H, c, slx, -0.5f, delta, half, grav, gxv, gyv));
+            const FaceS L = face_state(H, c, slx, 0.5f, delta, half, grav, gxv, gyv);
+            face_flux_at(H, L, R, 0, X + 1, w, Y >= 0 && Y < h, fr);
+#pragma unroll
+            for (int k = 0; k < 4; k++) fl[k] = __shfl_up_sync(0xffffffffu, fr[k], 1);
+        }
+        // ---- y faces: the row above's y+ faces against this row's y- faces, through shared memory
+        {
+            const FaceS T = face_state(H, c, sly, 0.5f, delta, half, grav, gxv, gyv);
+            sh.YF[0][row][lane] = T.U0;
+            sh.YF[1][row][lane] = T.U1;
+            sh.YF[2][row][lane] = T.U2;
+            sh.YF[3][row][lane] = T.U3;
+            sh.YF[4][row][lane] = T.u;
+            sh.YF[5][row][lane] = T.v;
+            sh.YF[6][row][lane] = T.P;
+        }
+        const FaceS B = face_state(H, c, sly, -0.5f, delta, half, grav, gxv, gyv);
+        __syncthreads();
+        if (row >= 1) {
+            FaceS L;
+            L.U0 = sh.YF[0][row - 1][lane];
+            L.U1 = sh.YF[1][row - 1][lane];
+            L.U2 = sh.YF[2][row - 1][lane];
+            L.U3 = sh.YF[3][row - 1][lane];
+            L.u = sh.YF[4][row - 1][lane];
+            L.v = sh.YF[5][row - 1][lane];
+            L.P = sh.YF[6][row - 1][lane];
+            float ft[4];
+            face_flux_at(H, L, B, 1, Y, h, X >= 0 && X < w, ft);
+#pragma unroll
+            for (int k = 0; k < 4; k++) sh.FY[k][row][lane] = ft[k];
+        }
+        __syncthreads();
+
+        // ---- epilogue: the tile's cells
+        const bool inside = lane >= 1 && lane <= HB_TX && row >= 1 && row <= HB_TY && X < w && Y < h;
+        const size_t i = inside ? (size_t)Y * w + X : 0;
+        float fu[4], fd[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            fu[k] = row >= 1 ? sh.FY[k][row][lane] : 0.0f;
+            fd[k] = row + 1 < HB_W ? sh.FY[k][row + 1][lane] : 0.0f;
+        }
+        // a cell with no gas around it stays empty (hydro.rs:733-742); out-of-world neighbours read as vacuum
+        const float sv = H.sigma_vac;
+        const bool vac = sh.S[sy][sx] < sv;
+        const bool empty = vac && sh.S[sy][sx - 1] < sv && sh.S[sy][sx + 1] < sv && sh.S[sy - 1][sx] < sv &&
+                           sh.S[sy + 1][sx] < sv;
+
+        if (inside) {
+            const int bx = X - xs, by = Y - ys;
+            float u[4];
+            if (empty || !vac) {
+                u[0] = raw[0][by][bx]; u[1] = raw[1][by][bx]; u[2] = raw[2][by][bx]; u[3] = raw[3][by][bx];
+            } else {
+                eos_cons(H, c, u);
+            }
+            if (!empty) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) u[q] -= dt * ((fr[q] - fl[q]) + (fd[q] - fu[q]));
+            }
+            if (MODE == kHydroPredict) {
+                // what follows the half step's solve: an empty cell's source is -0 (gravity leaves the cell as it is)
+                float src = -0.0f;
+                if (!empty) {
+                    const float start = vac ? sh.P[sy][sx].x : sh.S[sy][sx];
+                    const float div = (fr[0] - fl[0]) + (fd[0] - fu[0]);
+                    src = 0.5f * (sh.S[sy][sx] + (start - dt * div));
+                    src = src >= sv ? src : 0.0f;
+                }
+                A.src[i] = src;
+                A.mid[i] = sh.M[0][row][lane];
+                A.mid[n + i] = sh.M[1][row][lane];
+                A.mid[2 * n + i] = sh.M[2][row][lane];
+                A.mfx[i] = fr[0];
+                A.mfy[i] = fd[0];
+            }
+            if (MODE == kHydroStep) {
+                floor_cell(H, u[0], u[1], u[2], u[3]);
+                rate_cell(H, u[0], u[1], u[2], u[3], i, rp.rate, rp.nf);
+            }
+            A.Uout[i] = u[0];
+            A.Uout[n + i] = u[1];
+            A.Uout[2 * n + i] = u[2];
+            A.Uout[3 * n + i] = u[3];
+        }
+
+    }
+    // ---- the grid's sums, in a fixed order: a thread's tiles, the CTA's rows, the CTAs
     if (MODE != kHydroStep) return;
     rp = warp_merge(rp);
     if (lane == 0) sh.red[row] = rp;
@@ -729,9 +751,11 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
 
 size_t hydro_smem_bytes() { return sizeof(BandShared); }
 
-size_t hydro_part_count(int w, int h) { return (size_t)(div_up(w, HB_TX) + 1) * div_up(h, HB_TY); }
+size_t hydro_part_count(int w, int h) {
+    return std::max((size_t)2 * 148, (size_t)(div_up(w, HG_COLS) + 1) * div_up(h, HG_WARPS * HG_R));
+}
 
-size_t hydro_ticket_count(int h) { return (size_t)div_up(h, HB_TY) + 1; }
+size_t hydro_ticket_count(int h) { return (size_t)div_up(h, HG_WARPS * HG_R) + 1; }
 
 void tma_encode_planes(CUtensorMap* map, const float* base, int w, int h, int planes, int bx, int by) {
     // encoded maps are kept by their arguments: a launch on the same planes (every launch of a step, every smoother
@@ -777,7 +801,7 @@ void hydro_launch_t(const CUtensorMap& map, const HydroArgs& A, cudaStream_t s) 
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BandShared)));
         attr = true;
     }
-    const dim3 grid(div_up(A.H.w, HB_TX), div_up(A.H.h, HB_TY));
+    const unsigned grid = std::min(div_up(A.H.w, HB_TX) * div_up(A.H.h, HB_TY), 2u * 148u);
     hydro_band_kernel<MODE, LIM, BRACKET><<<grid, HB_NT, sizeof(BandShared), s>>>(map, A);
     sr_note_launch();
 }
@@ -800,7 +824,7 @@ void hydro_launch(int mode, const HydroArgs& A, cudaStream_t s) {
 }
 
 void hydro_gravity_launch(const HydroArgs& A, cudaStream_t s) {
-    const dim3 grid(div_up(A.H.w, 128), div_up(A.H.h, HG_WARPS * HG_R));
+    const dim3 grid(div_up(A.H.w, HG_COLS), div_up(A.H.h, HG_WARPS * HG_R));
     hydro_gravity_kernel<<<grid, 32 * HG_WARPS, 0, s>>>(A);
     sr_note_launch();
 }
@@ -808,26 +832,41 @@ void hydro_gravity_launch(const HydroArgs& A, cudaStream_t s) {
 // ------------------------------------------------------------------------------------------------ P8 + P9
 // P8's floors, then P9's per-cell Δt terms of the floored state and |g| of the step's P2 field; per-CTA partials, the
 // last CTA to arrive (a ticket) reduces them (max and min are exact in any order) and closes the step's Δt record.
-__global__ void floors_dt_kernel(HydroConst H, float* __restrict__ U, const float* __restrict__ gx,
-                                 const float* __restrict__ gy, int do_floors, float* part_rate, float* part_g,
-                                 long long* part_nf, unsigned* ticket, DtRule rule) {
-    const size_t n = (size_t)H.w * H.h;
+__global__ void __launch_bounds__(256) floors_dt_kernel(HydroConst H, float* __restrict__ U, const float* __restrict__ gx,
+                                                        const float* __restrict__ gy, int do_floors, float* part_rate,
+                                                        float* part_g, long long* part_nf, unsigned* ticket, DtRule rule) {
+    const size_t n = (size_t)H.w * H.h, n4 = n / 4;  // the world's axes are multiples of 8
     float rate = 0.0f, gmax = 0.0f;
+    double g2 = 0.0;  // |g|²: no square of an f32 leaves f64's range
     long long nf = LLONG_MAX;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        float s = U[i], mx = U[n + i], my = U[2 * n + i], e = U[3 * n + i];
-        if (do_floors) {
-            const int changed = floor_cell(H, s, mx, my, e);
-            if (changed == 2) {
-                U[i] = s;
-                U[n + i] = mx;
-                U[2 * n + i] = my;
-            }
-            if (changed) U[3 * n + i] = e;
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += (size_t)gridDim.x * blockDim.x) {
+        float4 p[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) p[k] = reinterpret_cast<const float4*>(U + k * n)[q];
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+        if (gx) {
+            a = reinterpret_cast<const float4*>(gx)[q];
+            b = reinterpret_cast<const float4*>(gy)[q];
         }
-        rate_cell(H, s, mx, my, e, i, rate, nf);
-        if (gx) gmax = fmaxf(gmax, hypotf(gx[i], gy[i]));
+        float s[4] = {p[0].x, p[0].y, p[0].z, p[0].w}, mx[4] = {p[1].x, p[1].y, p[1].z, p[1].w};
+        float my[4] = {p[2].x, p[2].y, p[2].z, p[2].w}, e[4] = {p[3].x, p[3].y, p[3].z, p[3].w};
+        int changed = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (do_floors) changed = max(changed, floor_cell(H, s[k], mx[k], my[k], e[k]));
+            rate_cell(H, s[k], mx[k], my[k], e[k], 4 * q + k, rate, nf);
+        }
+        if (changed == 2) {
+            reinterpret_cast<float4*>(U)[q] = make_float4(s[0], s[1], s[2], s[3]);
+            reinterpret_cast<float4*>(U + n)[q] = make_float4(mx[0], mx[1], mx[2], mx[3]);
+            reinterpret_cast<float4*>(U + 2 * n)[q] = make_float4(my[0], my[1], my[2], my[3]);
+        }
+        if (changed) reinterpret_cast<float4*>(U + 3 * n)[q] = make_float4(e[0], e[1], e[2], e[3]);
+        const float ga[4] = {a.x, a.y, a.z, a.w}, gb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) g2 = fmax(g2, (double)ga[k] * ga[k] + (double)gb[k] * gb[k]);
     }
+    gmax = (float)sqrt(g2);
     __shared__ float sr[32], sg[32];
     __shared__ long long sn[32];
     __shared__ bool last;
@@ -915,8 +954,8 @@ __global__ void dt_finalize_kernel(int nblocks, int channels, const float* part_
 
 int floors_dt_blocks(int w, int h) {
     size_t n = (size_t)w * h;
-    int b = (int)div_up((unsigned)((n + 3) / 4), 256u);
-    return b < 1 ? 1 : (b > 148 * 8 ? 148 * 8 : b);
+    int b = (int)div_up((unsigned)(n / 4), 256u);
+    return b < 1 ? 1 : (b > 148 * 4 ? 148 * 4 : b);
 }
 
 void floors_dt_launch(const HydroConst& H, float* U, const float* gx, const float* gy, int do_floors, float* part_rate,
