@@ -48,6 +48,215 @@ struct HeatConst {
     int ref;  // reference mode: the sides of heat_cells_kernel's reference branch (C = Σ/μ of each cell)
 };
 
+// ---- the implicit step under device control (MG and Jacobi preconditioners)
+//
+// The host-driven step (heat_step's Newton loop, solve_pass's FP64 refinement, inner_pcg's rounds) decides from
+// read-back scalars. Here the same decisions are taken on the device, inside one captured CUDA graph, and steer its
+// conditional nodes: an IF around the step (no gas, pinned temperature or Δt <= 0 leave only the fluxes), a WHILE over
+// the Newton passes, a WHILE over a pass's refinements, an IF around each inner solve, a WHILE over its PCG rounds (the
+// residual tested after every round: no host round trip, no predicted cadence), an IF around the next pass's coarsening,
+// and IFs choosing the commit. A decision is taken by the thread that has just written the sums it reads, the last CTA's
+// of the kernel whose grid sum it is (ctl_run): decisions in one-thread kernels of their own cost 3.5 us each with their
+// launch gap, 250 of them in three 2048² steps and 1,050 in four 512² reference-mode steps. No launch argument changes
+// from step to step: Δt, the scale, δ and the round state live in the device scalars.
+struct HeatCtl {
+    // configuration (host-written)
+    double tol, nheat, ncell, inner_floor;
+    int max_passes, max_rounds, pin;
+    // the step
+    double heat0, n_gas;
+    int passes, rounds, refinements, converged, ok, skipped;
+    double pass_tol, moved_prev, rel;
+    // the pass's refinement and its inner solve
+    int ref, reached, it, max_it;
+    double prev, eta, rr0;
+    // the commit
+    double delta, radiated;
+    // how often each body ran since the host last counted (for the launch count)
+    unsigned long long runs[10];
+};
+enum CtlBody { B_MAIN, B_SKIP, B_PASS, B_REFINE, B_INNER, B_ROUND, B_NSYS, B_COARSEN, B_CONV, B_LIM, B_COUNT };
+
+struct CtlHandles {
+    cudaGraphConditionalHandle h[B_COUNT];
+};
+
+// A kernel's part in the control: the block (null: the host decides), the step's Δt and the conditional handles.
+struct Ctl {
+    HeatCtl* c;
+    const double* dt;
+    CtlHandles hd;
+};
+
+enum CtlPhase { C_BEGIN, C_NEWTON_BEGIN, C_REFINE, C_INNER_BEGIN, C_ROUND, C_NEWTON, C_DELTA, C_LIMITED };
+
+__device__ __forceinline__ void ctl_set(const Ctl& k, int body, bool on, bool count_entry) {
+    cudaGraphSetConditional(k.hd.h[body], on ? 1u : 0u);
+    if (on && count_entry) k.c->runs[body]++;
+}
+
+// The commit follows: the converged one, or past the ceiling (or a breakdown) the limited one.
+__device__ __forceinline__ void ctl_commit(const Ctl& k) {
+    ctl_set(k, B_CONV, k.c->converged != 0, true);
+    ctl_set(k, B_LIM, !k.c->converged, true);
+}
+
+__device__ __forceinline__ void ctl_pass_begin(const Ctl& k) {
+    k.c->runs[B_PASS]++;
+    k.c->passes++;
+    k.c->ref = 0;
+    k.c->prev = INFINITY;
+    ctl_set(k, B_REFINE, true, false);
+}
+
+// The pass's solve is done: its Newton update, unless the solve broke down.
+__device__ __forceinline__ void ctl_refine_end(const Ctl& k) {
+    ctl_set(k, B_REFINE, false, false);
+    ctl_set(k, B_NSYS, k.c->ok != 0, true);
+    if (!k.c->ok) {
+        ctl_set(k, B_PASS, false, false);
+        ctl_commit(k);
+    }
+}
+
+// The inner solve is done (its correction x += scale e follows).
+__device__ __forceinline__ void ctl_inner_end(const Ctl& k) {
+    HeatCtl* c = k.c;
+    bool more = c->ok != 0;
+    if (c->ok) {
+        c->rounds += c->it;
+        c->refinements++;
+        // an intermediate pass (its tolerance far above the FP32 solve's floor) trusts the solve that reached its
+        // reduction; the final pass is always verified by another FP64 residual
+        if (c->reached && c->pass_tol >= kTrustedPassTol) {
+            c->rel *= c->eta;
+            more = false;
+        }
+    }
+    if (++c->ref >= kMaxRefinements) more = false;
+    if (more) ctl_set(k, B_REFINE, true, false);
+    else ctl_refine_end(k);
+}
+
+// One decision, by one thread, after the sums it reads are in the scalars.
+__device__ __noinline__ void ctl_run(const Ctl& k, double* scal, int phase) {
+    HeatCtl* c = k.c;
+    switch (phase) {
+        case C_BEGIN: {  // after Σ C T⁰ and the gas cells
+            scal[S_DT] = *k.dt;
+            c->heat0 = scal[S_HEAT0];
+            c->n_gas = scal[S_NGAS];
+            const bool skip = c->pin || c->n_gas == 0.0 || !(scal[S_DT] > 0.0);
+            c->skipped = skip;
+            c->passes = c->rounds = c->refinements = 0;
+            c->converged = skip ? 1 : 0;
+            c->ok = 1;
+            c->rel = c->delta = c->radiated = 0.0;
+            ctl_set(k, B_MAIN, !skip, true);
+            ctl_set(k, B_SKIP, skip, true);
+            break;
+        }
+        case C_NEWTON_BEGIN: {  // after the first system (its two bounds in S_UB, S_TB)
+            c->pass_tol = fmax(c->tol, kFirstPassTol);
+            c->moved_prev = 0.0;
+            const bool go = c->max_passes > 0 && c->max_rounds > 0;
+            ctl_set(k, B_PASS, go, false);
+            if (go) ctl_pass_begin(k);
+            else ctl_commit(k);
+            break;
+        }
+        case C_REFINE: {  // after the FP64 residual: stop, or scale the residual for an inner solve
+            c->runs[B_REFINE]++;
+            const double rr = scal[S_RR], bb = scal[S_BB], gam = scal[S_GAM], hm = scal[S_HM];
+            bool go = false;
+            if (!isfinite(rr) || !isfinite(bb) || !isfinite(gam) || !isfinite(hm)) {
+                c->ok = 0;
+            } else {
+                c->rel = bb > 0.0 ? sqrt(rr / bb) : 0.0;
+                const double tol = c->pass_tol, ub = scal[S_UB], tb = scal[S_TB];
+                double worst = c->rel / tol;
+                if (ub > 0.0) worst = fmax(worst, sqrt(gam / ub) / tol);
+                if (tb > 0.0) worst = fmax(worst, sqrt(hm / tb) / tol);
+                if (!(worst <= 1.0 || rr == 0.0) && !(worst > 0.5 * c->prev) && c->rounds < c->max_rounds) {
+                    c->prev = worst;
+                    const double scale = sqrt(rr / fmax(1.0, c->n_gas));
+                    scal[S_SCALE] = scale;
+                    scal[S_ISCALE] = 1.0 / scale;
+                    c->eta = fmin(0.5, fmax(c->inner_floor, 0.5 / worst));
+                    c->max_it = c->max_rounds - c->rounds;
+                    go = true;
+                }
+            }
+            ctl_set(k, B_INNER, go, true);
+            if (!go) ctl_refine_end(k);
+            break;
+        }
+        case C_INNER_BEGIN: {  // after the scaled residual
+            scal[S_BETA] = 0.0;
+            scal[S_PAR] = 0.0;
+            c->rr0 = scal[S_R32];
+            c->it = 0;
+            c->reached = 0;
+            const bool go = c->rr0 > 0.0 && c->max_it > 0;
+            ctl_set(k, B_ROUND, go, false);
+            if (!go) ctl_inner_end(k);
+            break;
+        }
+        case C_ROUND: {  // after a round: rotate its state, test the residual
+            c->runs[B_ROUND]++;
+            c->it++;
+            scal[S_RZP] = scal[S_RZN];
+            scal[S_PAR] = scal[S_PAR] != 0.0 ? 0.0 : 1.0;
+            const double pq = scal[S_PQ], rr = scal[S_RRI];
+            bool more = true;
+            if (!(pq > 0.0) || !isfinite(pq) || !isfinite(rr)) {
+                c->ok = 0;  // a breakdown: the solve's correction is dropped
+                scal[S_SCALE] = 0.0;
+                more = false;
+            } else if (rr <= c->eta * c->eta * c->rr0) {
+                c->reached = 1;
+                more = false;
+            } else if (c->it >= c->max_it) {
+                more = false;
+            }
+            ctl_set(k, B_ROUND, more, false);
+            if (!more) ctl_inner_end(k);
+            break;
+        }
+        case C_NEWTON: {  // after the update and the next system: stop, or the next pass's tolerance and coarsening
+            const double rel_moved = c->heat0 > 0.0 ? scal[S_MOVED] / c->heat0 : 0.0;
+            bool more;
+            if (rel_moved <= c->nheat && scal[S_VIOL] == 0.0 && c->pass_tol <= c->tol) {
+                c->converged = 1;
+                more = false;
+            } else {
+                // the next pass is solved to tol once it is expected to move less than nheat (the passes' observed
+                // contraction times this pass's move), since only a pass solved to tol can end them
+                const double ratio = c->moved_prev > 0.0 ? fmin(1.0, fmax(0.01, rel_moved / c->moved_prev)) : 0.1;
+                c->moved_prev = rel_moved;
+                c->pass_tol = fmax(c->tol, fmin(kFirstPassTol, rel_moved));
+                if (ratio * rel_moved <= c->nheat) c->pass_tol = c->tol;
+                more = c->passes < c->max_passes && c->rounds < c->max_rounds;
+            }
+            ctl_set(k, B_COARSEN, more, true);
+            ctl_set(k, B_PASS, more, false);
+            if (more) ctl_pass_begin(k);
+            else ctl_commit(k);
+            break;
+        }
+        case C_DELTA: {  // after the commit's sums (heat.rs:521-531)
+            const double rad = scal[S_RAD], gain = scal[S_GAIN], held = scal[S_HELD];
+            c->delta = -(gain + rad) / held;
+            c->radiated = rad;
+            scal[S_DELTA] = c->delta;
+            break;
+        }
+        case C_LIMITED:
+            c->radiated = scal[S_RAD];
+            break;
+    }
+}
+
 __device__ __forceinline__ double u_of(const HeatConst& K, double t) {
     return K.chi > 0.0 ? t : K.a_r * ((t * t) * (t * t));
 }
@@ -74,7 +283,7 @@ __device__ __forceinline__ double cold_u64(const float* u, const float* d, doubl
 // ---- step set-up: the sides (heat.rs:215-226), the faces' D_f (heat.rs:263-294), Σ_f k and its vacuum part
 __global__ void heat_cells_kernel(HeatConst K, HeatRef RF, const float* __restrict__ U, const float* __restrict__ kappa,
                                   uint8_t* gas, double* t0, double* C, float* kap, float* sig, double* t, double* u,
-                                  Red R) {
+                                  Red R, const __grid_constant__ Ctl ctl) {
     const size_t n = (size_t)K.w * K.h;
     double acc = 0.0, ngas = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -147,7 +356,8 @@ __global__ void heat_cells_kernel(HeatConst K, HeatRef RF, const float* __restri
         ngas += 1.0;
     }
     const double v[2] = {acc, ngas};
-    grid_sum_last<2>(v, R.part, R.counter, R.out);
+    const bool last = grid_sum_last<2>(v, R.part, R.counter, R.out);
+    if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_HEAT0, C_BEGIN);
 }
 
 struct Side {
@@ -273,7 +483,7 @@ __global__ void heat_system_kernel(HeatConst K, const double* __restrict__ scal,
                                    const double* __restrict__ C, const double* __restrict__ t,
                                    const double* __restrict__ u, const double* __restrict__ t0,
                                    const double* __restrict__ kvac, double* c64, double* rhs, float* c0, double* x,
-                                   Red R) {
+                                   Red R, const __grid_constant__ Ctl ctl) {
     const size_t n = (size_t)K.w * K.h;
     const double u_vac = u_of(K, K.t_floor);
     const double dt = scal[S_DT];
@@ -296,7 +506,8 @@ __global__ void heat_system_kernel(HeatConst K, const double* __restrict__ scal,
         tb += heat * t[i] * t[i];
     }
     const double v[2] = {ub, tb};
-    grid_sum_last<2>(v, R.part, R.counter, R.out);
+    const bool last = grid_sum_last<2>(v, R.part, R.counter, R.out);
+    if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_UB, C_NEWTON_BEGIN);
 }
 
 // r = b - A x in FP64, A x = c x + Σ_gas D (x_i - x_j), with partials of <r, r>, <b, b> and the reference's two
@@ -309,7 +520,7 @@ __global__ void heat_residual64_kernel(HeatConst K, const double* __restrict__ s
                                        const double* __restrict__ c64, const double* __restrict__ rhs,
                                        const double* __restrict__ kx, const double* __restrict__ ky,
                                        const double* __restrict__ C, const double* __restrict__ t,
-                                       const double* __restrict__ x, double* __restrict__ r, Red R) {
+                                       const double* __restrict__ x, double* __restrict__ r, Red R, const __grid_constant__ Ctl ctl) {
     const int w = K.w, h = K.h;
     const size_t n = (size_t)w * h, stride = (size_t)gridDim.x * blockDim.x;
     const double dt = scal[S_DT];
@@ -360,11 +571,12 @@ __global__ void heat_residual64_kernel(HeatConst K, const double* __restrict__ s
         }
     }
     const double v[4] = {rr, bb, gg, hh};
-    grid_sum_last<4>(v, R.part, R.counter, R.out);
+    const bool last = grid_sum_last<4>(v, R.part, R.counter, R.out);
+    if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_RR, C_REFINE);
 }
 
 __global__ void scale_kernel(size_t n, const double* __restrict__ r64, const double* __restrict__ scal, float* r32,
-                             float* e32, Red R) {
+                             float* e32, Red R, const __grid_constant__ Ctl ctl) {
     const double inv_scale = scal[S_ISCALE];
     double acc = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -373,7 +585,8 @@ __global__ void scale_kernel(size_t n, const double* __restrict__ r64, const dou
         e32[i] = 0.0f;
         acc += (double)v * v;
     }
-    grid_sum_last1(acc, R.part, R.counter, R.out);
+    const bool last = grid_sum_last1(acc, R.part, R.counter, R.out);
+    if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_R32, C_INNER_BEGIN);
 }
 
 // q = A p on level 0's FP32 operator in difference form, c p_i + Σ d (p_i - p_j); partials of <p, q>. ILP cells per
@@ -569,7 +782,7 @@ __global__ void spmv_dir_kernel(MgLevel L, double* scal, const float* __restrict
 
 // e += α p, r -= α q with 16-byte accesses (four cells per thread), p the round's new direction; partials of <r, r>.
 __global__ void pcg_update4_kernel(size_t n, const double* __restrict__ scal, const float* pa, const float* pb,
-                                   const float* __restrict__ q, float* __restrict__ e, float* __restrict__ r, Red R) {
+                                   const float* __restrict__ q, float* __restrict__ e, float* __restrict__ r, Red R, const __grid_constant__ Ctl ctl) {
     const float alpha = (float)(scal[S_RZN] / scal[S_PQ]);
     const float* __restrict__ p = scal[S_PAR] != 0.0 ? pa : pb;
     const size_t n4 = n / 4, stride = (size_t)gridDim.x * blockDim.x;
@@ -583,7 +796,8 @@ __global__ void pcg_update4_kernel(size_t n, const double* __restrict__ scal, co
         reinterpret_cast<float4*>(r)[t] = rv;
         acc += (double)rv.x * rv.x + (double)rv.y * rv.y + (double)rv.z * rv.z + (double)rv.w * rv.w;
     }
-    grid_sum_last1(acc, R.part, R.counter, R.out);
+    const bool last = grid_sum_last1(acc, R.part, R.counter, R.out);
+    if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_RRI, C_ROUND);
 }
 
 // Flexible CG (the learned preconditioner is not a fixed linear operator): the update keeps the residual it replaces,
@@ -683,7 +897,7 @@ __global__ void newton_system_kernel(HeatConst K, double cell_tol, const double*
                                      const uint8_t* __restrict__ gas,
                                      const double* __restrict__ C, const double* __restrict__ t0,
                                      const double* __restrict__ kvac, double* t, double* u, double* x, double* c64,
-                                     double* rhs, float* c0, Red R) {
+                                     double* rhs, float* c0, Red R, const __grid_constant__ Ctl ctl) {
     const size_t n = (size_t)K.w * K.h, stride = (size_t)gridDim.x * blockDim.x;
     const double u_vac = u_of(K, K.t_floor);
     const double dt = scal[S_DT];
@@ -729,7 +943,8 @@ __global__ void newton_system_kernel(HeatConst K, double cell_tol, const double*
         }
     }
     const double v[4] = {moved, viol, ub, tb};
-    grid_sum_last<4>(v, R.part, R.counter, R.out);
+    const bool last = grid_sum_last<4>(v, R.part, R.counter, R.out);
+    if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_MOVED, C_NEWTON);
 }
 
 // F = -k (v_b - v_a) at every face (heat.rs:338-361), v = u on gas cells, u_vac elsewhere; FP32 out.
@@ -778,7 +993,7 @@ __global__ void heat_flux_kernel(HeatConst K, const uint8_t* __restrict__ gas, c
 __global__ void commit_sums_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
                                    const double* __restrict__ C, const double* __restrict__ t,
                                    const double* __restrict__ t0, const double* __restrict__ u,
-                                   const double* __restrict__ kvac, Red R) {
+                                   const double* __restrict__ kvac, Red R, const __grid_constant__ Ctl ctl) {
     const size_t n = (size_t)K.w * K.h;
     const double u_vac = u_of(K, K.t_floor);
     const double dt = scal[S_DT];
@@ -790,7 +1005,8 @@ __global__ void commit_sums_kernel(HeatConst K, const double* __restrict__ scal,
         held += C[i] * t[i];
     }
     const double v[3] = {rad, gain, held};
-    grid_sum_last<3>(v, R.part, R.counter, R.out);
+    const bool last = grid_sum_last<3>(v, R.part, R.counter, R.out);
+    if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_RAD, C_DELTA);
 }
 
 // E_i += C_i ((1 + δ) T_i - T_i⁰) (heat.rs:532-535), and the cell's rate (T - T⁰)/Δt kept for the next step's first
@@ -856,7 +1072,7 @@ __global__ void limited_scale_kernel(HeatConst K, const double* __restrict__ sca
 __global__ void limited_apply_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
                                      const double* __restrict__ kx, const double* __restrict__ ky,
                                      const double* __restrict__ u, const double* __restrict__ scale, float* U,
-                                     Red R) {
+                                     Red R, const __grid_constant__ Ctl ctl) {
     const int w = K.w, h = K.h;
     const size_t n = (size_t)w * h;
     const double u_vac = u_of(K, K.t_floor);
@@ -887,7 +1103,8 @@ __global__ void limited_apply_kernel(HeatConst K, const double* __restrict__ sca
             if (!(nb[f] >= 0 && gas[nb[f]])) rad += dt * out[f];
         U[3 * n + i] = (float)((double)U[3 * n + i] - dt * (((out[0] + out[1]) + out[2]) + out[3]));
     }
-    grid_sum_last1(rad, R.part, R.counter, R.out);
+    const bool last = grid_sum_last1(rad, R.part, R.counter, R.out);
+    if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_RAD, C_LIMITED);
 }
 
 __global__ void zero_kernel(double* a, size_t n) {
@@ -921,184 +1138,6 @@ __global__ void pcg_rotate_kernel(double* scal) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     scal[S_RZP] = scal[S_RZN];
     scal[S_PAR] = scal[S_PAR] != 0.0 ? 0.0 : 1.0;
-}
-
-// ---- the implicit step under device control (MG and Jacobi preconditioners)
-//
-// The host-driven step (heat_step's Newton loop, solve_pass's FP64 refinement, inner_pcg's rounds) decides from
-// read-back scalars. Here the same decisions are taken by one-thread controller kernels that run between the step's
-// kernels inside one captured CUDA graph and steer its conditional nodes: an IF around the step (no gas, pinned
-// temperature or Δt <= 0 leave only the fluxes), a WHILE over the Newton passes, a WHILE over a pass's refinements, an
-// IF around each inner solve, a WHILE over its PCG rounds (the residual tested after every round: no host round trip,
-// no predicted cadence), an IF around the next pass's coarsening, and IFs choosing the commit. No launch argument
-// changes from step to step: Δt, the scale, δ and the round state live in the device scalars.
-struct HeatCtl {
-    // configuration (host-written)
-    double tol, nheat, ncell, inner_floor;
-    int max_passes, max_rounds, pin;
-    // the step
-    double heat0, n_gas;
-    int passes, rounds, refinements, converged, ok, skipped;
-    double pass_tol, moved_prev, rel;
-    // the pass's refinement and its inner solve
-    int ref, reached, it, max_it;
-    double prev, eta, rr0;
-    // the commit
-    double delta, radiated;
-    // how often each body ran since the host last counted (for the launch count)
-    unsigned long long runs[10];
-};
-enum CtlBody { B_MAIN, B_SKIP, B_PASS, B_REFINE, B_INNER, B_ROUND, B_NSYS, B_COARSEN, B_CONV, B_LIM, B_COUNT };
-
-struct CtlHandles {
-    cudaGraphConditionalHandle h[B_COUNT];
-};
-
-enum CtlPhase { C_BEGIN, C_NEWTON_BEGIN, C_PASS_BEGIN, C_REFINE, C_INNER_BEGIN, C_ROUND, C_AFTER_INNER, C_PASS_END,
-                C_NEWTON, C_COMMIT, C_DELTA, C_LIMITED };
-
-__device__ __forceinline__ void ctl_set(const CtlHandles& hd, HeatCtl* c, int body, bool on, bool count_entry) {
-    cudaGraphSetConditional(hd.h[body], on ? 1u : 0u);
-    if (on && count_entry) c->runs[body]++;
-}
-
-__global__ void heat_ctl_kernel(HeatCtl* c, double* scal, int phase, CtlHandles hd) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    switch (phase) {
-        case C_BEGIN: {  // after the set-up: Σ C T⁰, the gas cells and Δt in the scalars
-            c->heat0 = scal[S_HEAT0];
-            c->n_gas = scal[S_NGAS];
-            const bool skip = c->pin || c->n_gas == 0.0 || !(scal[S_DT] > 0.0);
-            c->skipped = skip;
-            c->passes = c->rounds = c->refinements = 0;
-            c->converged = skip ? 1 : 0;
-            c->ok = 1;
-            c->rel = c->delta = c->radiated = 0.0;
-            ctl_set(hd, c, B_MAIN, !skip, true);
-            ctl_set(hd, c, B_SKIP, skip, true);
-            break;
-        }
-        case C_NEWTON_BEGIN:  // after the first system (its two bounds in S_UB, S_TB)
-            c->pass_tol = fmax(c->tol, kFirstPassTol);
-            c->moved_prev = 0.0;
-            ctl_set(hd, c, B_PASS, c->max_passes > 0 && c->max_rounds > 0, false);
-            break;
-        case C_PASS_BEGIN:
-            c->runs[B_PASS]++;
-            c->passes++;
-            c->ref = 0;
-            c->prev = INFINITY;
-            ctl_set(hd, c, B_REFINE, true, false);
-            break;
-        case C_REFINE: {  // after the FP64 residual: stop, or scale the residual for an inner solve
-            c->runs[B_REFINE]++;
-            const double rr = scal[S_RR], bb = scal[S_BB], gam = scal[S_GAM], hm = scal[S_HM];
-            bool go = false;
-            if (!isfinite(rr) || !isfinite(bb) || !isfinite(gam) || !isfinite(hm)) {
-                c->ok = 0;
-            } else {
-                c->rel = bb > 0.0 ? sqrt(rr / bb) : 0.0;
-                const double tol = c->pass_tol, ub = scal[S_UB], tb = scal[S_TB];
-                double worst = c->rel / tol;
-                if (ub > 0.0) worst = fmax(worst, sqrt(gam / ub) / tol);
-                if (tb > 0.0) worst = fmax(worst, sqrt(hm / tb) / tol);
-                if (!(worst <= 1.0 || rr == 0.0) && !(worst > 0.5 * c->prev) && c->rounds < c->max_rounds) {
-                    c->prev = worst;
-                    const double scale = sqrt(rr / fmax(1.0, c->n_gas));
-                    scal[S_SCALE] = scale;
-                    scal[S_ISCALE] = 1.0 / scale;
-                    c->eta = fmin(0.5, fmax(c->inner_floor, 0.5 / worst));
-                    c->max_it = c->max_rounds - c->rounds;
-                    go = true;
-                }
-            }
-            ctl_set(hd, c, B_INNER, go, true);
-            if (!go) ctl_set(hd, c, B_REFINE, false, false);
-            break;
-        }
-        case C_INNER_BEGIN: {  // after the scaled residual
-            scal[S_BETA] = 0.0;
-            scal[S_PAR] = 0.0;
-            c->rr0 = scal[S_R32];
-            c->it = 0;
-            c->reached = 0;
-            ctl_set(hd, c, B_ROUND, c->rr0 > 0.0 && c->max_it > 0, false);
-            break;
-        }
-        case C_ROUND: {  // after a round: rotate its state, test the residual
-            c->runs[B_ROUND]++;
-            c->it++;
-            scal[S_RZP] = scal[S_RZN];
-            scal[S_PAR] = scal[S_PAR] != 0.0 ? 0.0 : 1.0;
-            const double pq = scal[S_PQ], rr = scal[S_RRI];
-            bool more = true;
-            if (!(pq > 0.0) || !isfinite(pq) || !isfinite(rr)) {
-                c->ok = 0;  // a breakdown: the solve's correction is dropped
-                scal[S_SCALE] = 0.0;
-                more = false;
-            } else if (rr <= c->eta * c->eta * c->rr0) {
-                c->reached = 1;
-                more = false;
-            } else if (c->it >= c->max_it) {
-                more = false;
-            }
-            ctl_set(hd, c, B_ROUND, more, false);
-            break;
-        }
-        case C_AFTER_INNER: {  // after the correction x += scale e
-            bool more = c->ok != 0;
-            if (c->ok) {
-                c->rounds += c->it;
-                c->refinements++;
-                // an intermediate pass (its tolerance far above the FP32 solve's floor) trusts the solve that reached
-                // its reduction; the final pass is always verified by another FP64 residual
-                if (c->reached && c->pass_tol >= kTrustedPassTol) {
-                    c->rel *= c->eta;
-                    more = false;
-                }
-            }
-            if (++c->ref >= kMaxRefinements) more = false;
-            ctl_set(hd, c, B_REFINE, more, false);
-            break;
-        }
-        case C_PASS_END:  // the pass's solve is done: its Newton update, unless the solve broke down
-            ctl_set(hd, c, B_NSYS, c->ok != 0, true);
-            if (!c->ok) ctl_set(hd, c, B_PASS, false, false);
-            break;
-        case C_NEWTON: {  // after the update and the next system: stop, or the next pass's tolerance and coarsening
-            const double rel_moved = c->heat0 > 0.0 ? scal[S_MOVED] / c->heat0 : 0.0;
-            bool more;
-            if (rel_moved <= c->nheat && scal[S_VIOL] == 0.0 && c->pass_tol <= c->tol) {
-                c->converged = 1;
-                more = false;
-            } else {
-                // the next pass is solved to tol once it is expected to move less than nheat (the passes' observed
-                // contraction times this pass's move), since only a pass solved to tol can end them
-                const double ratio = c->moved_prev > 0.0 ? fmin(1.0, fmax(0.01, rel_moved / c->moved_prev)) : 0.1;
-                c->moved_prev = rel_moved;
-                c->pass_tol = fmax(c->tol, fmin(kFirstPassTol, rel_moved));
-                if (ratio * rel_moved <= c->nheat) c->pass_tol = c->tol;
-                more = c->passes < c->max_passes && c->rounds < c->max_rounds;
-            }
-            ctl_set(hd, c, B_COARSEN, more, true);
-            ctl_set(hd, c, B_PASS, more, false);
-            break;
-        }
-        case C_COMMIT:
-            ctl_set(hd, c, B_CONV, c->converged != 0, true);
-            ctl_set(hd, c, B_LIM, !c->converged, true);
-            break;
-        case C_DELTA: {  // after the commit's sums (heat.rs:521-531)
-            const double rad = scal[S_RAD], gain = scal[S_GAIN], held = scal[S_HELD];
-            c->delta = -(gain + rad) / held;
-            c->radiated = rad;
-            scal[S_DELTA] = c->delta;
-            break;
-        }
-        case C_LIMITED:
-            c->radiated = scal[S_RAD];
-            break;
-    }
 }
 
 int grid_for(size_t n) {
@@ -1174,10 +1213,10 @@ void set_scalar(HeatSolver* H, int slot, double value, cudaStream_t s) {
     sr_note_launch();
 }
 
-void setup_step(HeatSolver* H, const float* U, const float* kappa, cudaStream_t s) {
+void setup_step(HeatSolver* H, const float* U, const float* kappa, cudaStream_t s, const Ctl& ctl = Ctl{}) {
     const HeatConst& K = H->K;
     heat_cells_kernel<<<H->grid, RED_THREADS, 0, s>>>(K, H->ref, U, kappa, H->gas, H->t0, H->C, H->kap, H->sig, H->t, H->u,
-                                                      H->red(S_HEAT0));
+                                                      H->red(S_HEAT0), ctl);
     sr_note_launch();
     const size_t nf = (size_t)(H->w + 1) * H->h + (size_t)H->w * (H->h + 1);
     heat_faces_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(K, H->gas, H->t0, H->kap, H->sig, H->C, H->kx, H->ky);
@@ -1244,7 +1283,7 @@ void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s)
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
     sr_note_launch();
     pcg_update4_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, H->p32, H->p2, H->q32, H->e32, H->r32,
-                                                       H->red(S_RRI));
+                                                       H->red(S_RRI), Ctl{});
     sr_note_launch();
     pcg_rotate_kernel<<<1, 32, 0, s>>>(H->scal);
     sr_note_launch();
@@ -1335,7 +1374,7 @@ SolveResult solve_pass(HeatSolver* H, uint32_t precond, double tol, int max_roun
     const double ub = H->hscal[S_UB], tb = H->hscal[S_TB];
     for (int ref = 0; ref < 16; ref++) {
         heat_residual64_kernel<<<H->grid, RED_THREADS, 0, s>>>(K, H->scal, H->gas, H->c64, H->rhs, H->kx, H->ky, H->C,
-                                                               H->t, H->x, H->r64, H->red(S_RR));
+                                                               H->t, H->x, H->r64, H->red(S_RR), Ctl{});
         sr_note_launch();
         H->read(S_RR, 4, s);
         const double rr = H->hscal[S_RR], bb = H->hscal[S_BB], gam = H->hscal[S_GAM], hm = H->hscal[S_HM];
@@ -1353,7 +1392,7 @@ SolveResult solve_pass(HeatSolver* H, uint32_t precond, double tol, int max_roun
         const double scale = sqrt(rr / (double)std::max(1, H->n_gas));
         set_scalar(H, S_SCALE, scale, s);
         set_scalar(H, S_ISCALE, 1.0 / scale, s);
-        scale_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32));
+        scale_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32), Ctl{});
         sr_note_launch();
         const double eta = std::min(0.5, std::max(H->inner_floor, 0.5 / worst));
         bool reached = false;
@@ -1387,7 +1426,7 @@ SolveResult solve_pass(HeatSolver* H, uint32_t precond, double tol, int max_roun
 void build_system(HeatSolver* H, double dt, cudaStream_t s) {
     set_scalar(H, S_DT, dt, s);
     heat_system_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->C, H->t, H->u, H->t0, H->kvac, H->c64,
-                                                       H->rhs, H->mg.L[0].c, H->x, H->red(S_UB));
+                                                       H->rhs, H->mg.L[0].c, H->x, H->red(S_UB), Ctl{});
     sr_note_launch();
     H->mg.coarsen(s);
     H->read(S_UB, 2, s);
@@ -1426,25 +1465,19 @@ long long capture_body(cudaGraph_t g, cudaStream_t cs, F body) {
     return n;
 }
 
-void ctl_launch(HeatSolver* H, int phase, const CtlHandles& hd, cudaStream_t s) {
-    heat_ctl_kernel<<<1, 32, 0, s>>>(H->ctl, H->scal, phase, hd);
-    sr_note_launch();
-}
-
 // The whole implicit step (MG or Jacobi preconditioner) appended to the capture in progress on `s`, whose root graph
 // is `root` (the conditional handles belong to it): set-up, Δt from the device record, the device-controlled Newton
 // passes, refinements and PCG rounds, and the commit. The state buffer `U` and the opacity plane are fixed in it.
 void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev, cudaStream_t s,
                        cudaGraph_t root) {
-    CtlHandles hd;
-    for (int b = 0; b < B_COUNT; b++) SR_CUDA_TRY(cudaGraphConditionalHandleCreate(&hd.h[b], root, 0, 0));
+    Ctl ctl{H->ctl, dt_dev, {}};
+    const CtlHandles& hd = ctl.hd;
+    for (int b = 0; b < B_COUNT; b++) SR_CUDA_TRY(cudaGraphConditionalHandleCreate(&ctl.hd.h[b], root, 0, 0));
     const uint32_t precond = H->precond;
     const size_t nf = (size_t)(H->w + 1) * H->h + (size_t)H->w * (H->h + 1);
     long long* nb = H->body_launches;
     const long long top0 = (long long)sr_launches();
-    setup_step(H, U, kappa, s);
-    SR_CUDA_TRY(cudaMemcpyAsync(H->scal + S_DT, dt_dev, sizeof(double), cudaMemcpyDeviceToDevice, s));
-    ctl_launch(H, C_BEGIN, hd, s);
+    setup_step(H, U, kappa, s, ctl);
     const long long top1 = (long long)sr_launches();
     nb[B_MAIN] = capture_body(capture_conditional(s, hd.h[B_MAIN], cudaGraphCondTypeIf), H->cap[0], [&](cudaStream_t s0) {
         if (precond != SR_PRECOND_JACOBI) {
@@ -1452,24 +1485,20 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
             sr_note_launch();
         }
         heat_system_kernel<<<H->grid, RED_THREADS, 0, s0>>>(H->K, H->scal, H->gas, H->C, H->t, H->u, H->t0, H->kvac,
-                                                            H->c64, H->rhs, H->mg.L[0].c, H->x, H->red(S_UB));
+                                                            H->c64, H->rhs, H->mg.L[0].c, H->x, H->red(S_UB), ctl);
         sr_note_launch();
         H->mg.coarsen(s0);
-        ctl_launch(H, C_NEWTON_BEGIN, hd, s0);
         nb[B_PASS] = capture_body(capture_conditional(s0, hd.h[B_PASS], cudaGraphCondTypeWhile), H->cap[1],
                                   [&](cudaStream_t s1) {
-            ctl_launch(H, C_PASS_BEGIN, hd, s1);
             nb[B_REFINE] = capture_body(capture_conditional(s1, hd.h[B_REFINE], cudaGraphCondTypeWhile), H->cap[2],
                                         [&](cudaStream_t s2) {
                 heat_residual64_kernel<<<H->grid, RED_THREADS, 0, s2>>>(H->K, H->scal, H->gas, H->c64, H->rhs, H->kx,
-                                                                         H->ky, H->C, H->t, H->x, H->r64, H->red(S_RR));
+                                                                         H->ky, H->C, H->t, H->x, H->r64, H->red(S_RR), ctl);
                 sr_note_launch();
-                ctl_launch(H, C_REFINE, hd, s2);
                 nb[B_INNER] = capture_body(capture_conditional(s2, hd.h[B_INNER], cudaGraphCondTypeIf), H->cap[3],
                                            [&](cudaStream_t s3) {
-                    scale_kernel<<<H->grid, RED_THREADS, 0, s3>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32));
+                    scale_kernel<<<H->grid, RED_THREADS, 0, s3>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32), ctl);
                     sr_note_launch();
-                    ctl_launch(H, C_INNER_BEGIN, hd, s3);
                     nb[B_ROUND] = capture_body(capture_conditional(s3, hd.h[B_ROUND], cudaGraphCondTypeWhile), H->cap[4],
                                                [&](cudaStream_t s4) {
                         precondition(H, precond, S_RZN, s4);
@@ -1478,37 +1507,31 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
                         sr_note_launch();
                         pcg_update4_kernel<<<H->grid, RED_THREADS, 0, s4>>>(H->n, H->scal, H->p32, H->p2, H->q32,
-                                                                             H->e32, H->r32, H->red(S_RRI));
+                                                                             H->e32, H->r32, H->red(S_RRI), ctl);
                         sr_note_launch();
-                        ctl_launch(H, C_ROUND, hd, s4);
                     });
                     correction_kernel<<<H->grid, RED_THREADS, 0, s3>>>(H->n, H->gas, H->e32, H->scal, H->x);
                     sr_note_launch();
-                    ctl_launch(H, C_AFTER_INNER, hd, s3);
                 });
             });
-            ctl_launch(H, C_PASS_END, hd, s1);
             nb[B_NSYS] = capture_body(capture_conditional(s1, hd.h[B_NSYS], cudaGraphCondTypeIf), H->cap[2],
                                       [&](cudaStream_t s2) {
                 newton_system_kernel<<<H->grid, RED_THREADS, 0, s2>>>(H->K, H->cfg.newton_cell, H->scal, H->gas, H->C,
                                                                        H->t0, H->kvac, H->t, H->u, H->x, H->c64,
-                                                                       H->rhs, H->mg.L[0].c, H->red(S_MOVED));
+                                                                       H->rhs, H->mg.L[0].c, H->red(S_MOVED), ctl);
                 sr_note_launch();
-                ctl_launch(H, C_NEWTON, hd, s2);
                 nb[B_COARSEN] = capture_body(capture_conditional(s2, hd.h[B_COARSEN], cudaGraphCondTypeIf), H->cap[3],
                                              [&](cudaStream_t s3) { H->mg.coarsen(s3); });
             });
         });
-        ctl_launch(H, C_COMMIT, hd, s0);
         nb[B_CONV] = capture_body(capture_conditional(s0, hd.h[B_CONV], cudaGraphCondTypeIf), H->cap[1],
                                   [&](cudaStream_t s1) {
             heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s1>>>(H->K, H->gas, H->kx, H->ky, H->u, nullptr, H->fx,
                                                                    H->fy);
             sr_note_launch();
             commit_sums_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->C, H->t, H->t0, H->u,
-                                                                H->kvac, H->red(S_RAD));
+                                                                H->kvac, H->red(S_RAD), ctl);
             sr_note_launch();
-            ctl_launch(H, C_DELTA, hd, s1);
             commit_apply_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->C, H->t, H->t0, U, H->rate);
             sr_note_launch();
         });
@@ -1521,11 +1544,10 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                                                                    H->fy);
             sr_note_launch();
             limited_apply_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->u,
-                                                                  H->lscale, U, H->red(S_RAD));
+                                                                  H->lscale, U, H->red(S_RAD), ctl);
             sr_note_launch();
             zero_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->rate, H->n);
             sr_note_launch();
-            ctl_launch(H, C_LIMITED, hd, s1);
         });
     });
     nb[B_SKIP] = capture_body(capture_conditional(s, hd.h[B_SKIP], cudaGraphCondTypeIf), H->cap[0],
@@ -1686,7 +1708,7 @@ int heat_collect(HeatSolver* H, Learner* L, const float* U, const float* kappa, 
     H->n_gas = (int)H->hscal[S_NGAS];
     build_system(H, dt, s);
     heat_residual64_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->c64, H->rhs, H->kx, H->ky, H->C,
-                                                           H->t, H->x, H->r64, H->red(S_RR));
+                                                           H->t, H->x, H->r64, H->red(S_RR), Ctl{});
     sr_note_launch();
     H->read(S_RR, 1, s);
     const double rr = H->hscal[S_RR];
@@ -1694,7 +1716,7 @@ int heat_collect(HeatSolver* H, Learner* L, const float* U, const float* kappa, 
     const double scale = sqrt(rr / (double)std::max(1, H->n_gas));
     set_scalar(H, S_SCALE, scale, s);
     set_scalar(H, S_ISCALE, 1.0 / scale, s);
-    scale_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32));
+    scale_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32), Ctl{});
     sr_note_launch();
     if (!H->ez) SR_CUDA_TRY(cudaMalloc(&H->ez, sizeof(float) * H->n));
     // after each V-cycle z_k = M_mg r_k: the sample (r_k − A z_k, e_k + z_k); q32 is free until the next round's SpMV
@@ -1878,7 +1900,7 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
         if (!S.ok) break;
         newton_system_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, ncell, H->scal, H->gas, H->C, H->t0,
                                                               H->kvac, H->t, H->u, H->x, H->c64, H->rhs,
-                                                              H->mg.L[0].c, H->red(S_MOVED));
+                                                              H->mg.L[0].c, H->red(S_MOVED), Ctl{});
         sr_note_launch();
         H->read(S_MOVED, 4, s);  // moved, violations, and the next system's two bounds
         const double rel_moved = heat0 > 0.0 ? H->hscal[S_MOVED] / heat0 : 0.0;
@@ -1900,7 +1922,7 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
         heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(H->K, H->gas, H->kx, H->ky, H->u, nullptr, H->fx, H->fy);
         sr_note_launch();
         commit_sums_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->C, H->t, H->t0, H->u, H->kvac,
-                                                           H->red(S_RAD));
+                                                           H->red(S_RAD), Ctl{});
         sr_note_launch();
         H->read(S_RAD, 3, s);
         const double rad = H->hscal[S_RAD], gain = H->hscal[S_GAIN], held = H->hscal[S_HELD];
@@ -1919,7 +1941,7 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
                                                                H->fy);
         sr_note_launch();
         limited_apply_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->u, H->lscale, U,
-                                                             H->red(S_RAD));
+                                                             H->red(S_RAD), Ctl{});
         sr_note_launch();
         SR_CUDA_TRY(cudaMemsetAsync(H->rate, 0, sizeof(double) * H->n, s));
         H->read(S_RAD, 1, s);
