@@ -1145,6 +1145,16 @@ int grid_for(size_t n) {
     return (int)(b < 1 ? 1 : (b > (size_t)MAX_PART ? (size_t)MAX_PART : b));
 }
 
+// CTAs for `turns` turns of RED_THREADS threads, at most one wave of them.
+template <class F>
+int whole_waves(F kernel, size_t turns) {
+    int per_sm = 0, dev = 0, sms = 0;
+    SR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, RED_THREADS, 0));
+    SR_CUDA_TRY(cudaGetDevice(&dev));
+    SR_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return std::max(1, std::min(grid_for(turns), per_sm * sms));
+}
+
 }  // namespace
 
 struct RoundGraph {
@@ -1158,7 +1168,11 @@ struct HeatSolver {
     HeatRef ref{};
     int w = 0, h = 0;
     size_t n = 0;
-    int grid = 0;
+    int grid = 0;  // CTAs of the grid-stride kernels
+    // of the solve's heaviest, by the cells a thread takes a turn (two, two, four and four) and by what fits the GPU at
+    // once: a CTA without a turn still takes a sum's ticket (512²: the SpMV 256 CTAs instead of 1,024), and a wave that
+    // does not fill costs a whole one
+    int grid_residual = 0, grid_newton = 0, grid_spmv = 0, grid_update = 0;
     uint32_t precond = SR_PRECOND_MG;
     uint32_t max_passes = 128, max_rounds = 4096;
     double inner_floor = 1e-5;  // the smallest residual reduction asked of one inner FP32 solve
@@ -1278,11 +1292,11 @@ void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s)
     (void)rz_old;
     (void)rz_new;
     precondition(H, precond, S_RZN, s);
-    spmv_dir_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2, H->q32,
+    spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2, H->q32,
                                                     H->red(S_PQ), H->scal + S_BETA, H->rz_part,
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
     sr_note_launch();
-    pcg_update4_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, H->p32, H->p2, H->q32, H->e32, H->r32,
+    pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s>>>(H->n, H->scal, H->p32, H->p2, H->q32, H->e32, H->r32,
                                                        H->red(S_RRI), Ctl{});
     sr_note_launch();
     pcg_rotate_kernel<<<1, 32, 0, s>>>(H->scal);
@@ -1373,7 +1387,7 @@ SolveResult solve_pass(HeatSolver* H, uint32_t precond, double tol, int max_roun
     double prev = INFINITY;
     const double ub = H->hscal[S_UB], tb = H->hscal[S_TB];
     for (int ref = 0; ref < 16; ref++) {
-        heat_residual64_kernel<<<H->grid, RED_THREADS, 0, s>>>(K, H->scal, H->gas, H->c64, H->rhs, H->kx, H->ky, H->C,
+        heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(K, H->scal, H->gas, H->c64, H->rhs, H->kx, H->ky, H->C,
                                                                H->t, H->x, H->r64, H->red(S_RR), Ctl{});
         sr_note_launch();
         H->read(S_RR, 4, s);
@@ -1492,7 +1506,7 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                                   [&](cudaStream_t s1) {
             nb[B_REFINE] = capture_body(capture_conditional(s1, hd.h[B_REFINE], cudaGraphCondTypeWhile), H->cap[2],
                                         [&](cudaStream_t s2) {
-                heat_residual64_kernel<<<H->grid, RED_THREADS, 0, s2>>>(H->K, H->scal, H->gas, H->c64, H->rhs, H->kx,
+                heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s2>>>(H->K, H->scal, H->gas, H->c64, H->rhs, H->kx,
                                                                          H->ky, H->C, H->t, H->x, H->r64, H->red(S_RR), ctl);
                 sr_note_launch();
                 nb[B_INNER] = capture_body(capture_conditional(s2, hd.h[B_INNER], cudaGraphCondTypeIf), H->cap[3],
@@ -1502,11 +1516,11 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                     nb[B_ROUND] = capture_body(capture_conditional(s3, hd.h[B_ROUND], cudaGraphCondTypeWhile), H->cap[4],
                                                [&](cudaStream_t s4) {
                         precondition(H, precond, S_RZN, s4);
-                        spmv_dir_kernel<<<H->grid, RED_THREADS, 0, s4>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2,
+                        spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s4>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2,
                                                                           H->q32, H->red(S_PQ), H->scal + S_BETA, H->rz_part,
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
                         sr_note_launch();
-                        pcg_update4_kernel<<<H->grid, RED_THREADS, 0, s4>>>(H->n, H->scal, H->p32, H->p2, H->q32,
+                        pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s4>>>(H->n, H->scal, H->p32, H->p2, H->q32,
                                                                              H->e32, H->r32, H->red(S_RRI), ctl);
                         sr_note_launch();
                     });
@@ -1516,7 +1530,7 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
             });
             nb[B_NSYS] = capture_body(capture_conditional(s1, hd.h[B_NSYS], cudaGraphCondTypeIf), H->cap[2],
                                       [&](cudaStream_t s2) {
-                newton_system_kernel<<<H->grid, RED_THREADS, 0, s2>>>(H->K, H->cfg.newton_cell, H->scal, H->gas, H->C,
+                newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s2>>>(H->K, H->cfg.newton_cell, H->scal, H->gas, H->C,
                                                                        H->t0, H->kvac, H->t, H->u, H->x, H->c64,
                                                                        H->rhs, H->mg.L[0].c, H->red(S_MOVED), ctl);
                 sr_note_launch();
@@ -1609,6 +1623,10 @@ HeatSolver* heat_create(const sr_config& cfg, cudaStream_t s) {
         K.chi = cfg.chi;
         K.limiter_on = cfg.flux_limiter != 0;
         H->grid = grid_for(H->n);
+        H->grid_residual = whole_waves(heat_residual64_kernel, H->n / 2);
+        H->grid_newton = whole_waves(newton_system_kernel, H->n / 2);
+        H->grid_spmv = whole_waves(spmv_dir_kernel, H->n / 4);
+        H->grid_update = whole_waves(pcg_update4_kernel, H->n / 4);
         const size_t n = H->n, nx = (size_t)(H->w + 1) * H->h, ny = (size_t)H->w * (H->h + 1);
         SR_CUDA_TRY(cudaMalloc(&H->gas, n));
         double** d64[] = {&H->t0, &H->C, &H->t, &H->u, &H->ksum, &H->kvac, &H->c64, &H->rhs, &H->x, &H->r64,
@@ -1707,7 +1725,7 @@ int heat_collect(HeatSolver* H, Learner* L, const float* U, const float* kappa, 
     H->read(S_HEAT0, 2, s);
     H->n_gas = (int)H->hscal[S_NGAS];
     build_system(H, dt, s);
-    heat_residual64_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->c64, H->rhs, H->kx, H->ky, H->C,
+    heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->c64, H->rhs, H->kx, H->ky, H->C,
                                                            H->t, H->x, H->r64, H->red(S_RR), Ctl{});
     sr_note_launch();
     H->read(S_RR, 1, s);
@@ -1898,7 +1916,7 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
         R.rel_residual = S.rel;
         if (S.fallback) R.fallback_used = 1;
         if (!S.ok) break;
-        newton_system_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, ncell, H->scal, H->gas, H->C, H->t0,
+        newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s>>>(H->K, ncell, H->scal, H->gas, H->C, H->t0,
                                                               H->kvac, H->t, H->u, H->x, H->c64, H->rhs,
                                                               H->mg.L[0].c, H->red(S_MOVED), Ctl{});
         sr_note_launch();
