@@ -280,10 +280,10 @@ __device__ __forceinline__ double cold_u64(const float* u, const float* d, doubl
     return (double)u[i] * exp((pos - (double)i) * (double)d[i]);
 }
 
-// ---- step set-up: the sides (heat.rs:215-226), the faces' D_f (heat.rs:263-294), Σ_f k and its vacuum part
+// ---- step set-up: the sides (heat.rs:215-226), the faces' D_f (heat.rs:263-294), Σ_f k over the vacuum faces
 __global__ void heat_cells_kernel(HeatConst K, HeatRef RF, const float* __restrict__ U, const float* __restrict__ kappa,
-                                  uint8_t* gas, double* t0, double* C, float* kap, float* sig, double* t, double* u,
-                                  Red R, const __grid_constant__ Ctl ctl) {
+                                  uint8_t* gas, double* t0, double* C, float* kap, float* sig, double* t, Red R,
+                                  const __grid_constant__ Ctl ctl) {
     const size_t n = (size_t)K.w * K.h;
     double acc = 0.0, ngas = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -322,7 +322,6 @@ __global__ void heat_cells_kernel(HeatConst K, HeatRef RF, const float* __restri
             sig[i] = g ? (float)s : (float)K.sigma_floor;
             C[i] = (g ? s : K.sigma_floor) * inv_mu;
             t[i] = T;
-            u[i] = u_of(K, T);
             if (g) {
                 acc += C[i] * T;
                 ngas += 1.0;
@@ -337,7 +336,6 @@ __global__ void heat_cells_kernel(HeatConst K, HeatRef RF, const float* __restri
             sig[i] = (float)K.sigma_floor;
             C[i] = K.sigma_floor / (K.mu * K.gm1);
             t[i] = K.t_floor;
-            u[i] = u_of(K, K.t_floor);
             continue;
         }
         const double mx = U[n + i], my = U[2 * n + i], e = U[3 * n + i];
@@ -351,7 +349,6 @@ __global__ void heat_cells_kernel(HeatConst K, HeatRef RF, const float* __restri
         sig[i] = (float)s;
         C[i] = s / (K.mu * K.gm1);
         t[i] = T;
-        u[i] = u_of(K, T);
         acc += C[i] * T;
         ngas += 1.0;
     }
@@ -451,12 +448,11 @@ __global__ void heat_faces_kernel(HeatConst K, const uint8_t* __restrict__ gas, 
 }
 
 __global__ void heat_ksum_kernel(HeatConst K, const uint8_t* __restrict__ gas, const double* __restrict__ kx,
-                                 const double* __restrict__ ky, double* ksum, double* kvac) {
+                                 const double* __restrict__ ky, double* kvac) {
     const int w = K.w, h = K.h;
     const size_t n = (size_t)w * h;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         if (!gas[i]) {
-            ksum[i] = 0.0;
             kvac[i] = 0.0;
             continue;
         }
@@ -466,44 +462,51 @@ __global__ void heat_ksum_kernel(HeatConst K, const uint8_t* __restrict__ gas, c
                              ky[(size_t)(y + 1) * w + x]};
         const bool nb[4] = {x > 0 && gas[i - 1], x + 1 < w && gas[i + 1], y > 0 && gas[i - w],
                             y + 1 < h && gas[i + w]};
-        double s = 0.0, v = 0.0;
-        for (int f = 0; f < 4; f++) {
-            s += k[f];
+        double v = 0.0;
+        for (int f = 0; f < 4; f++)
             if (!nb[f]) v += k[f];
-        }
-        ksum[i] = s;
         kvac[i] = v;
     }
 }
 
-// ---- a Newton pass's system at the iterate (heat.rs:476-489), kept as its mass term c = c_i + Σ_vac D_f (the
-// diagonal less the couplings to gas neighbours, f64; FP32 copy as level 0's c) so that A x = c x + Σ D (x_i - x_j)
-// is evaluated without cancellation; partials of the two measures' bounds, Σ c_i u² and Σ (C/Δt) T² (heat.rs:480-487).
+// ---- a Newton pass's system at the iterate (heat.rs:476-489): the mass term c = c_i + Σ_vac D_f (the diagonal less the
+// couplings to gas neighbours, so that A x = c x + Σ D (x_i - x_j) is evaluated without cancellation) and the right-hand
+// side. Both follow from a cell's C, T, T⁰ and Σ_vac D_f: the kernels that need them in f64 form them from those (as
+// many bytes read as the stored pair would take, and none written), and only level 0's FP32 copy of c is stored.
+struct CellSystem {
+    double heat, slope, c, rhs;
+};
+__device__ __forceinline__ CellSystem cell_system(const HeatConst& K, double inv_dt, double u_vac, double C, double t,
+                                                  double t0, double kvac) {
+    CellSystem s;
+    s.heat = C * inv_dt;
+    s.slope = dt_du(K, t);
+    const double ci = s.heat * s.slope;
+    s.c = ci + kvac;
+    s.rhs = ci * u_of(K, t) - s.heat * (t - t0) + kvac * u_vac;
+    return s;
+}
+
+// The first pass's system: level 0's c, the iterate x = u(T), and partials of the two measures' bounds, Σ c_i u² and
+// Σ (C/Δt) T² (heat.rs:480-487).
 __global__ void heat_system_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
                                    const double* __restrict__ C, const double* __restrict__ t,
-                                   const double* __restrict__ u, const double* __restrict__ t0,
-                                   const double* __restrict__ kvac, double* c64, double* rhs, float* c0, double* x,
-                                   Red R, const __grid_constant__ Ctl ctl) {
+                                   const double* __restrict__ kvac, float* c0, double* x, Red R, const __grid_constant__ Ctl ctl) {
     const size_t n = (size_t)K.w * K.h;
-    const double u_vac = u_of(K, K.t_floor);
     const double dt = scal[S_DT];
     double ub = 0.0, tb = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         if (!gas[i]) {
-            c64[i] = 1.0;
-            rhs[i] = 0.0;
             c0[i] = 1.0f;
             x[i] = 0.0;
             continue;
         }
-        const double heat = C[i] / dt;
-        const double ci = heat * dt_du(K, t[i]);
-        c64[i] = ci + kvac[i];
-        rhs[i] = ci * u[i] - heat * (t[i] - t0[i]) + kvac[i] * u_vac;
+        const double heat = C[i] / dt, ti = t[i], ui = u_of(K, ti);
+        const double ci = heat * dt_du(K, ti);
         c0[i] = (float)(ci + kvac[i]);
-        x[i] = u[i];
-        ub += ci * u[i] * u[i];
-        tb += heat * t[i] * t[i];
+        x[i] = ui;
+        ub += ci * ui * ui;
+        tb += heat * ti * ti;
     }
     const double v[2] = {ub, tb};
     const bool last = grid_sum_last<2>(v, R.part, R.counter, R.out);
@@ -517,13 +520,13 @@ __global__ void heat_system_kernel(HeatConst K, const double* __restrict__ scal,
 constexpr int ILP = 4;
 
 __global__ void heat_residual64_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
-                                       const double* __restrict__ c64, const double* __restrict__ rhs,
-                                       const double* __restrict__ kx, const double* __restrict__ ky,
-                                       const double* __restrict__ C, const double* __restrict__ t,
+                                       const double* __restrict__ kvac, const double* __restrict__ kx,
+                                       const double* __restrict__ ky, const double* __restrict__ C,
+                                       const double* __restrict__ t, const double* __restrict__ t0,
                                        const double* __restrict__ x, double* __restrict__ r, Red R, const __grid_constant__ Ctl ctl) {
     const int w = K.w, h = K.h;
     const size_t n = (size_t)w * h, stride = (size_t)gridDim.x * blockDim.x;
-    const double dt = scal[S_DT];
+    const double inv_dt = 1.0 / scal[S_DT], u_vac = u_of(K, K.t_floor);
     double rr = 0.0, bb = 0.0, gg = 0.0, hh = 0.0;
     for (size_t base = (size_t)blockIdx.x * blockDim.x + threadIdx.x; base < n; base += 2 * stride) {
 #pragma unroll
@@ -535,7 +538,7 @@ __global__ void heat_residual64_kernel(HeatConst K, const double* __restrict__ s
             const bool gi = gas[i];
             const bool gl = xx > 0 && gas[i - 1], gr = xx + 1 < w && gas[i + 1];
             const bool gu = y > 0 && gas[i - w], gd = y + 1 < h && gas[i + w];
-            const double xi = x[i], ci = c64[i], bi = rhs[i], Ci = C[i], ti = t[i];
+            const double xi = x[i], kv = kvac[i], t0i = t0[i], Ci = C[i], ti = t[i];
             const double xl = xx > 0 ? x[i - 1] : 0.0, xr = xx + 1 < w ? x[i + 1] : 0.0;
             const double xu = y > 0 ? x[i - w] : 0.0, xd = y + 1 < h ? x[i + w] : 0.0;
             const double kl = kx[(size_t)y * (w + 1) + xx], kr = kx[(size_t)y * (w + 1) + xx + 1];
@@ -544,7 +547,8 @@ __global__ void heat_residual64_kernel(HeatConst K, const double* __restrict__ s
                 r[i] = 0.0;
                 continue;
             }
-            double s = ci * xi, d = ci;
+            const CellSystem S = cell_system(K, inv_dt, u_vac, Ci, ti, t0i, kv);
+            double s = S.c * xi, d = S.c;
             if (gl) {
                 s += kl * (xi - xl);
                 d += kl;
@@ -561,13 +565,14 @@ __global__ void heat_residual64_kernel(HeatConst K, const double* __restrict__ s
                 s += kd * (xi - xd);
                 d += kd;
             }
-            const double ri = bi - s;
+            const double ri = S.rhs - s;
             r[i] = ri;
             rr += ri * ri;
-            bb += bi * bi;
-            gg += ri * ri / d;
-            const double e = ri * dt_du(K, ti) / d;
-            hh += Ci / dt * e * e;
+            bb += S.rhs * S.rhs;
+            const double rd = ri / d;  // FP64 divisions are what this kernel has few of to spend
+            gg += ri * rd;
+            const double e = rd * S.slope;
+            hh += S.heat * e * e;
         }
     }
     const double v[4] = {rr, bb, gg, hh};
@@ -895,9 +900,8 @@ __global__ void correction_kernel(size_t n, const uint8_t* __restrict__ gas, con
 // the system goes unused.
 __global__ void newton_system_kernel(HeatConst K, double cell_tol, const double* __restrict__ scal,
                                      const uint8_t* __restrict__ gas,
-                                     const double* __restrict__ C, const double* __restrict__ t0,
-                                     const double* __restrict__ kvac, double* t, double* u, double* x, double* c64,
-                                     double* rhs, float* c0, Red R, const __grid_constant__ Ctl ctl) {
+                                     const double* __restrict__ C, const double* __restrict__ kvac, double* t, double* x,
+                                     float* c0, Red R, const __grid_constant__ Ctl ctl) {
     const size_t n = (size_t)K.w * K.h, stride = (size_t)gridDim.x * blockDim.x;
     const double u_vac = u_of(K, K.t_floor);
     const double dt = scal[S_DT];
@@ -906,23 +910,21 @@ __global__ void newton_system_kernel(HeatConst K, double cell_tol, const double*
     for (size_t base = (size_t)blockIdx.x * blockDim.x + threadIdx.x; base < n; base += 2 * stride) {
         const size_t i2 = base + stride;
         const bool g1 = gas[base], g2 = i2 < n && gas[i2];
-        double tv[2], xv[2], Cv[2], t0v[2], kv[2];
+        double tv[2], xv[2], Cv[2], kv[2];
         tv[0] = t[base];
         xv[0] = x[base];
         Cv[0] = C[base];
-        t0v[0] = t0[base];
         kv[0] = kvac[base];
         if (i2 < n) {
             tv[1] = t[i2];
             xv[1] = x[i2];
             Cv[1] = C[i2];
-            t0v[1] = t0[i2];
             kv[1] = kvac[i2];
         }
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const size_t i = e ? i2 : base;
-            if (!(e ? g2 : g1)) continue;  // the system's masked rows (c = 1, b = 0, x = 0) are already in place
+            if (!(e ? g2 : g1)) continue;  // the system's masked rows (c = 1, x = 0) are already in place
             const double ti = tv[e];
             double nx = t_of(K, fmax(xv[e], u_vac));
             nx = fmin(fmax(nx, 0.5 * ti), 2.0 * ti);
@@ -931,11 +933,8 @@ __global__ void newton_system_kernel(HeatConst K, double cell_tol, const double*
             if (!(d <= cell_tol * ti)) viol += 1.0;
             const double un = u_of(K, nx);
             t[i] = nx;
-            u[i] = un;
             const double heat = Cv[e] / dt;
             const double ci = heat * dt_du(K, nx);
-            c64[i] = ci + kv[e];
-            rhs[i] = ci * un - heat * (nx - t0v[e]) + kv[e] * u_vac;
             c0[i] = (float)(ci + kv[e]);
             x[i] = un;
             ub += ci * un * un;
@@ -947,17 +946,17 @@ __global__ void newton_system_kernel(HeatConst K, double cell_tol, const double*
     if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_MOVED, C_NEWTON);
 }
 
-// F = -k (v_b - v_a) at every face (heat.rs:338-361), v = u on gas cells, u_vac elsewhere; FP32 out.
-__device__ __forceinline__ double face_flux(const HeatConst& K, const uint8_t* gas, const double* u, double k,
+// F = -k (v_b - v_a) at every face (heat.rs:338-361), v = u(T) on gas cells, u_vac elsewhere; FP32 out.
+__device__ __forceinline__ double face_flux(const HeatConst& K, const uint8_t* gas, const double* t, double k,
                                             long a, long b, double u_vac) {
     if (k == 0.0) return 0.0;
-    const double va = (a >= 0 && gas[a]) ? u[a] : u_vac;
-    const double vb = (b >= 0 && gas[b]) ? u[b] : u_vac;
+    const double va = (a >= 0 && gas[a]) ? u_of(K, t[a]) : u_vac;
+    const double vb = (b >= 0 && gas[b]) ? u_of(K, t[b]) : u_vac;
     return -k * (vb - va);
 }
 
 __global__ void heat_flux_kernel(HeatConst K, const uint8_t* __restrict__ gas, const double* __restrict__ kx,
-                                 const double* __restrict__ ky, const double* __restrict__ u,
+                                 const double* __restrict__ ky, const double* __restrict__ t,
                                  const double* __restrict__ scale, float* fx, float* fy) {
     const int w = K.w, h = K.h;
     const size_t nx = (size_t)(w + 1) * h, ny = (size_t)w * (h + 1);
@@ -979,7 +978,7 @@ __global__ void heat_flux_kernel(HeatConst K, const uint8_t* __restrict__ gas, c
             b = y < h ? (long)y * w + x : -1;
             k = ky[g];
         }
-        double F = face_flux(K, gas, u, k, a, b, u_vac);
+        double F = face_flux(K, gas, t, k, a, b, u_vac);
         if (scale) {
             const long from = F > 0.0 ? a : b;
             F *= from >= 0 ? scale[from] : 1.0;
@@ -992,15 +991,14 @@ __global__ void heat_flux_kernel(HeatConst K, const uint8_t* __restrict__ gas, c
 // The commit's sums (heat.rs:521-531): radiated, gained and held.
 __global__ void commit_sums_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
                                    const double* __restrict__ C, const double* __restrict__ t,
-                                   const double* __restrict__ t0, const double* __restrict__ u,
-                                   const double* __restrict__ kvac, Red R, const __grid_constant__ Ctl ctl) {
+                                   const double* __restrict__ t0, const double* __restrict__ kvac, Red R, const __grid_constant__ Ctl ctl) {
     const size_t n = (size_t)K.w * K.h;
     const double u_vac = u_of(K, K.t_floor);
     const double dt = scal[S_DT];
     double rad = 0.0, gain = 0.0, held = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         if (!gas[i]) continue;
-        rad += dt * kvac[i] * (u[i] - u_vac);
+        rad += dt * kvac[i] * (u_of(K, t[i]) - u_vac);
         gain += C[i] * (t[i] - t0[i]);
         held += C[i] * t[i];
     }
@@ -1025,7 +1023,7 @@ __global__ void commit_apply_kernel(HeatConst K, const double* __restrict__ scal
 // The first iterate on the V-cycle (heat.wgsl:710-722): T⁰ + the last step's rate × Δt, T⁰ where that is off by more
 // than a factor 2 or not finite, floored at T_floor.
 __global__ void warm_start_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
-                                  const double* __restrict__ t0, const double* __restrict__ rate, double* t, double* u) {
+                                  const double* __restrict__ t0, const double* __restrict__ rate, double* t) {
     const size_t n = (size_t)K.w * K.h;
     const double dt = scal[S_DT];
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -1034,14 +1032,13 @@ __global__ void warm_start_kernel(HeatConst K, const double* __restrict__ scal, 
         if (!(tg >= 0.5 * t0[i] && tg <= 2.0 * t0[i])) tg = t0[i];
         tg = fmax(tg, K.t_floor);
         t[i] = tg;
-        u[i] = u_of(K, tg);
     }
 }
 
 // Past the ceiling (heat.rs:545-564): each gas cell's outflow scaled to the heat it holds above its floor.
 __global__ void limited_scale_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
                                      const double* __restrict__ kx, const double* __restrict__ ky,
-                                     const double* __restrict__ u, const double* __restrict__ C,
+                                     const double* __restrict__ t, const double* __restrict__ C,
                                      const double* __restrict__ t0, double* scale) {
     const int w = K.w, h = K.h;
     const size_t n = (size_t)w * h;
@@ -1056,10 +1053,10 @@ __global__ void limited_scale_kernel(HeatConst K, const double* __restrict__ sca
         split_index(i, w, x, y);
         const long L = x > 0 ? (long)i - 1 : -1, R = x + 1 < w ? (long)i + 1 : -1;
         const long Uu = y > 0 ? (long)i - w : -1, D = y + 1 < h ? (long)i + w : -1;
-        const double lv[4] = {-face_flux(K, gas, u, kx[(size_t)y * (w + 1) + x], L, (long)i, u_vac),
-                              face_flux(K, gas, u, kx[(size_t)y * (w + 1) + x + 1], (long)i, R, u_vac),
-                              -face_flux(K, gas, u, ky[(size_t)y * w + x], Uu, (long)i, u_vac),
-                              face_flux(K, gas, u, ky[(size_t)(y + 1) * w + x], (long)i, D, u_vac)};
+        const double lv[4] = {-face_flux(K, gas, t, kx[(size_t)y * (w + 1) + x], L, (long)i, u_vac),
+                              face_flux(K, gas, t, kx[(size_t)y * (w + 1) + x + 1], (long)i, R, u_vac),
+                              -face_flux(K, gas, t, ky[(size_t)y * w + x], Uu, (long)i, u_vac),
+                              face_flux(K, gas, t, ky[(size_t)(y + 1) * w + x], (long)i, D, u_vac)};
         double out = 0.0;
         for (int f = 0; f < 4; f++) out += fmax(lv[f], 0.0);
         out *= dt;
@@ -1071,7 +1068,7 @@ __global__ void limited_scale_kernel(HeatConst K, const double* __restrict__ sca
 // E -= Δt Σ_f F_f with every face's F at the scale of the cell it leaves (heat.rs:565-592); partials of radiated.
 __global__ void limited_apply_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
                                      const double* __restrict__ kx, const double* __restrict__ ky,
-                                     const double* __restrict__ u, const double* __restrict__ scale, float* U,
+                                     const double* __restrict__ t, const double* __restrict__ scale, float* U,
                                      Red R, const __grid_constant__ Ctl ctl) {
     const int w = K.w, h = K.h;
     const size_t n = (size_t)w * h;
@@ -1084,10 +1081,10 @@ __global__ void limited_apply_kernel(HeatConst K, const double* __restrict__ sca
         split_index(i, w, x, y);
         const long nb[4] = {x > 0 ? (long)i - 1 : -1, x + 1 < w ? (long)i + 1 : -1, y > 0 ? (long)i - w : -1,
                             y + 1 < h ? (long)i + w : -1};
-        double F[4] = {face_flux(K, gas, u, kx[(size_t)y * (w + 1) + x], nb[0], (long)i, u_vac),
-                       face_flux(K, gas, u, kx[(size_t)y * (w + 1) + x + 1], (long)i, nb[1], u_vac),
-                       face_flux(K, gas, u, ky[(size_t)y * w + x], nb[2], (long)i, u_vac),
-                       face_flux(K, gas, u, ky[(size_t)(y + 1) * w + x], (long)i, nb[3], u_vac)};
+        double F[4] = {face_flux(K, gas, t, kx[(size_t)y * (w + 1) + x], nb[0], (long)i, u_vac),
+                       face_flux(K, gas, t, kx[(size_t)y * (w + 1) + x + 1], (long)i, nb[1], u_vac),
+                       face_flux(K, gas, t, ky[(size_t)y * w + x], nb[2], (long)i, u_vac),
+                       face_flux(K, gas, t, ky[(size_t)(y + 1) * w + x], (long)i, nb[3], u_vac)};
         // the low cell of faces 0 and 2 is the neighbour, of faces 1 and 3 this cell
         const long low[4] = {nb[0], (long)i, nb[2], (long)i}, high[4] = {(long)i, nb[1], (long)i, nb[3]};
         double out[4];
@@ -1178,8 +1175,8 @@ struct HeatSolver {
     double inner_floor = 1e-5;  // the smallest residual reduction asked of one inner FP32 solve
     bool use_graphs = true;
     uint8_t* gas = nullptr;
-    double *t0 = nullptr, *C = nullptr, *t = nullptr, *u = nullptr, *kx = nullptr, *ky = nullptr;
-    double *ksum = nullptr, *kvac = nullptr, *c64 = nullptr, *rhs = nullptr, *x = nullptr, *r64 = nullptr;
+    double *t0 = nullptr, *C = nullptr, *t = nullptr, *kx = nullptr, *ky = nullptr;
+    double *kvac = nullptr, *x = nullptr, *r64 = nullptr;
     double* lscale = nullptr;
     double* rate = nullptr;      // each cell's P5 rate (T - T⁰)/Δt in the last step, for the next first iterate
     float *kap = nullptr, *sig = nullptr;
@@ -1229,13 +1226,13 @@ void set_scalar(HeatSolver* H, int slot, double value, cudaStream_t s) {
 
 void setup_step(HeatSolver* H, const float* U, const float* kappa, cudaStream_t s, const Ctl& ctl = Ctl{}) {
     const HeatConst& K = H->K;
-    heat_cells_kernel<<<H->grid, RED_THREADS, 0, s>>>(K, H->ref, U, kappa, H->gas, H->t0, H->C, H->kap, H->sig, H->t, H->u,
+    heat_cells_kernel<<<H->grid, RED_THREADS, 0, s>>>(K, H->ref, U, kappa, H->gas, H->t0, H->C, H->kap, H->sig, H->t,
                                                       H->red(S_HEAT0), ctl);
     sr_note_launch();
     const size_t nf = (size_t)(H->w + 1) * H->h + (size_t)H->w * (H->h + 1);
     heat_faces_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(K, H->gas, H->t0, H->kap, H->sig, H->C, H->kx, H->ky);
     sr_note_launch();
-    heat_ksum_kernel<<<H->grid, RED_THREADS, 0, s>>>(K, H->gas, H->kx, H->ky, H->ksum, H->kvac);
+    heat_ksum_kernel<<<H->grid, RED_THREADS, 0, s>>>(K, H->gas, H->kx, H->ky, H->kvac);
     sr_note_launch();
     H->mg.set_couplings(H->kx, H->ky, H->gas, s);
 }
@@ -1387,8 +1384,8 @@ SolveResult solve_pass(HeatSolver* H, uint32_t precond, double tol, int max_roun
     double prev = INFINITY;
     const double ub = H->hscal[S_UB], tb = H->hscal[S_TB];
     for (int ref = 0; ref < 16; ref++) {
-        heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(K, H->scal, H->gas, H->c64, H->rhs, H->kx, H->ky, H->C,
-                                                               H->t, H->x, H->r64, H->red(S_RR), Ctl{});
+        heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(K, H->scal, H->gas, H->kvac, H->kx, H->ky, H->C,
+                                                               H->t, H->t0, H->x, H->r64, H->red(S_RR), Ctl{});
         sr_note_launch();
         H->read(S_RR, 4, s);
         const double rr = H->hscal[S_RR], bb = H->hscal[S_BB], gam = H->hscal[S_GAM], hm = H->hscal[S_HM];
@@ -1439,8 +1436,8 @@ SolveResult solve_pass(HeatSolver* H, uint32_t precond, double tol, int max_roun
 // A pass's system and its measures' bounds (read to the host), then every coarse level and the coarsest inverse.
 void build_system(HeatSolver* H, double dt, cudaStream_t s) {
     set_scalar(H, S_DT, dt, s);
-    heat_system_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->C, H->t, H->u, H->t0, H->kvac, H->c64,
-                                                       H->rhs, H->mg.L[0].c, H->x, H->red(S_UB), Ctl{});
+    heat_system_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->C, H->t, H->kvac,
+                                                       H->mg.L[0].c, H->x, H->red(S_UB), Ctl{});
     sr_note_launch();
     H->mg.coarsen(s);
     H->read(S_UB, 2, s);
@@ -1495,19 +1492,19 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
     const long long top1 = (long long)sr_launches();
     nb[B_MAIN] = capture_body(capture_conditional(s, hd.h[B_MAIN], cudaGraphCondTypeIf), H->cap[0], [&](cudaStream_t s0) {
         if (precond != SR_PRECOND_JACOBI) {
-            warm_start_kernel<<<H->grid, RED_THREADS, 0, s0>>>(H->K, H->scal, H->gas, H->t0, H->rate, H->t, H->u);
+            warm_start_kernel<<<H->grid, RED_THREADS, 0, s0>>>(H->K, H->scal, H->gas, H->t0, H->rate, H->t);
             sr_note_launch();
         }
-        heat_system_kernel<<<H->grid, RED_THREADS, 0, s0>>>(H->K, H->scal, H->gas, H->C, H->t, H->u, H->t0, H->kvac,
-                                                            H->c64, H->rhs, H->mg.L[0].c, H->x, H->red(S_UB), ctl);
+        heat_system_kernel<<<H->grid, RED_THREADS, 0, s0>>>(H->K, H->scal, H->gas, H->C, H->t, H->kvac,
+                                                            H->mg.L[0].c, H->x, H->red(S_UB), ctl);
         sr_note_launch();
         H->mg.coarsen(s0);
         nb[B_PASS] = capture_body(capture_conditional(s0, hd.h[B_PASS], cudaGraphCondTypeWhile), H->cap[1],
                                   [&](cudaStream_t s1) {
             nb[B_REFINE] = capture_body(capture_conditional(s1, hd.h[B_REFINE], cudaGraphCondTypeWhile), H->cap[2],
                                         [&](cudaStream_t s2) {
-                heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s2>>>(H->K, H->scal, H->gas, H->c64, H->rhs, H->kx,
-                                                                         H->ky, H->C, H->t, H->x, H->r64, H->red(S_RR), ctl);
+                heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s2>>>(H->K, H->scal, H->gas, H->kvac, H->kx,
+                                                                         H->ky, H->C, H->t, H->t0, H->x, H->r64, H->red(S_RR), ctl);
                 sr_note_launch();
                 nb[B_INNER] = capture_body(capture_conditional(s2, hd.h[B_INNER], cudaGraphCondTypeIf), H->cap[3],
                                            [&](cudaStream_t s3) {
@@ -1530,9 +1527,7 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
             });
             nb[B_NSYS] = capture_body(capture_conditional(s1, hd.h[B_NSYS], cudaGraphCondTypeIf), H->cap[2],
                                       [&](cudaStream_t s2) {
-                newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s2>>>(H->K, H->cfg.newton_cell, H->scal, H->gas, H->C,
-                                                                       H->t0, H->kvac, H->t, H->u, H->x, H->c64,
-                                                                       H->rhs, H->mg.L[0].c, H->red(S_MOVED), ctl);
+                newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s2>>>(H->K, H->cfg.newton_cell, H->scal, H->gas, H->C, H->kvac, H->t, H->x, H->mg.L[0].c, H->red(S_MOVED), ctl);
                 sr_note_launch();
                 nb[B_COARSEN] = capture_body(capture_conditional(s2, hd.h[B_COARSEN], cudaGraphCondTypeIf), H->cap[3],
                                              [&](cudaStream_t s3) { H->mg.coarsen(s3); });
@@ -1540,10 +1535,10 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
         });
         nb[B_CONV] = capture_body(capture_conditional(s0, hd.h[B_CONV], cudaGraphCondTypeIf), H->cap[1],
                                   [&](cudaStream_t s1) {
-            heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s1>>>(H->K, H->gas, H->kx, H->ky, H->u, nullptr, H->fx,
+            heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s1>>>(H->K, H->gas, H->kx, H->ky, H->t, nullptr, H->fx,
                                                                    H->fy);
             sr_note_launch();
-            commit_sums_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->C, H->t, H->t0, H->u,
+            commit_sums_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->C, H->t, H->t0,
                                                                 H->kvac, H->red(S_RAD), ctl);
             sr_note_launch();
             commit_apply_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->C, H->t, H->t0, U, H->rate);
@@ -1551,13 +1546,13 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
         });
         nb[B_LIM] = capture_body(capture_conditional(s0, hd.h[B_LIM], cudaGraphCondTypeIf), H->cap[1],
                                  [&](cudaStream_t s1) {
-            limited_scale_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->u, H->C,
+            limited_scale_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->t, H->C,
                                                                   H->t0, H->lscale);
             sr_note_launch();
-            heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s1>>>(H->K, H->gas, H->kx, H->ky, H->u, H->lscale, H->fx,
+            heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s1>>>(H->K, H->gas, H->kx, H->ky, H->t, H->lscale, H->fx,
                                                                    H->fy);
             sr_note_launch();
-            limited_apply_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->u,
+            limited_apply_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->t,
                                                                   H->lscale, U, H->red(S_RAD), ctl);
             sr_note_launch();
             zero_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->rate, H->n);
@@ -1566,7 +1561,7 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
     });
     nb[B_SKIP] = capture_body(capture_conditional(s, hd.h[B_SKIP], cudaGraphCondTypeIf), H->cap[0],
                               [&](cudaStream_t s0) {
-        heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s0>>>(H->K, H->gas, H->kx, H->ky, H->u, nullptr, H->fx, H->fy);
+        heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s0>>>(H->K, H->gas, H->kx, H->ky, H->t, nullptr, H->fx, H->fy);
         sr_note_launch();
     });
     nb[B_COUNT] = top1 - top0;
@@ -1629,7 +1624,7 @@ HeatSolver* heat_create(const sr_config& cfg, cudaStream_t s) {
         H->grid_update = whole_waves(pcg_update4_kernel, H->n / 4);
         const size_t n = H->n, nx = (size_t)(H->w + 1) * H->h, ny = (size_t)H->w * (H->h + 1);
         SR_CUDA_TRY(cudaMalloc(&H->gas, n));
-        double** d64[] = {&H->t0, &H->C, &H->t, &H->u, &H->ksum, &H->kvac, &H->c64, &H->rhs, &H->x, &H->r64,
+        double** d64[] = {&H->t0, &H->C, &H->t, &H->kvac, &H->x, &H->r64,
                           &H->lscale, &H->rate};
         for (double** p : d64) SR_CUDA_TRY(cudaMalloc(p, sizeof(double) * n));
         SR_CUDA_TRY(cudaMemset(H->rate, 0, sizeof(double) * n));
@@ -1675,7 +1670,7 @@ void heat_destroy(HeatSolver* H) {
     for (cudaStream_t c : H->cap)
         if (c) cudaStreamDestroy(c);
     cudaFree(H->gas);
-    double* d64[] = {H->t0, H->C, H->t, H->u, H->ksum, H->kvac, H->c64, H->rhs, H->x, H->r64, H->lscale, H->rate,
+    double* d64[] = {H->t0, H->C, H->t, H->kvac, H->x, H->r64, H->lscale, H->rate,
                      H->kx, H->ky};
     for (double* p : d64) cudaFree(p);
     float* d32[] = {H->kap, H->sig, H->r32, H->e32, H->p32, H->q32, H->z32, H->fx, H->fy, H->p2};
@@ -1725,8 +1720,8 @@ int heat_collect(HeatSolver* H, Learner* L, const float* U, const float* kappa, 
     H->read(S_HEAT0, 2, s);
     H->n_gas = (int)H->hscal[S_NGAS];
     build_system(H, dt, s);
-    heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->c64, H->rhs, H->kx, H->ky, H->C,
-                                                           H->t, H->x, H->r64, H->red(S_RR), Ctl{});
+    heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->kvac, H->kx, H->ky, H->C,
+                                                           H->t, H->t0, H->x, H->r64, H->red(S_RR), Ctl{});
     sr_note_launch();
     H->read(S_RR, 1, s);
     const double rr = H->hscal[S_RR];
@@ -1884,7 +1879,7 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
     const double heat0 = H->hscal[S_HEAT0];
     const size_t nf = (size_t)(H->w + 1) * H->h + (size_t)H->w * (H->h + 1);
     if (H->cfg.pin_temperature || H->n_gas == 0 || !(dt > 0.0)) {
-        heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(H->K, H->gas, H->kx, H->ky, H->u, nullptr, H->fx,
+        heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(H->K, H->gas, H->kx, H->ky, H->t, nullptr, H->fx,
                                                                H->fy);
         sr_note_launch();
         R.converged = 1;
@@ -1894,7 +1889,7 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
     }
     R.dt = dt;
     if (H->precond != SR_PRECOND_JACOBI) {
-        warm_start_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->t0, H->rate, H->t, H->u);
+        warm_start_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->t0, H->rate, H->t);
         sr_note_launch();
     }
     uint32_t passes = 0, rounds = 0;
@@ -1916,9 +1911,7 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
         R.rel_residual = S.rel;
         if (S.fallback) R.fallback_used = 1;
         if (!S.ok) break;
-        newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s>>>(H->K, ncell, H->scal, H->gas, H->C, H->t0,
-                                                              H->kvac, H->t, H->u, H->x, H->c64, H->rhs,
-                                                              H->mg.L[0].c, H->red(S_MOVED), Ctl{});
+        newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s>>>(H->K, ncell, H->scal, H->gas, H->C, H->kvac, H->t, H->x, H->mg.L[0].c, H->red(S_MOVED), Ctl{});
         sr_note_launch();
         H->read(S_MOVED, 4, s);  // moved, violations, and the next system's two bounds
         const double rel_moved = heat0 > 0.0 ? H->hscal[S_MOVED] / heat0 : 0.0;
@@ -1937,9 +1930,9 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
     R.passes = passes;
     R.rounds = rounds;
     if (converged) {
-        heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(H->K, H->gas, H->kx, H->ky, H->u, nullptr, H->fx, H->fy);
+        heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(H->K, H->gas, H->kx, H->ky, H->t, nullptr, H->fx, H->fy);
         sr_note_launch();
-        commit_sums_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->C, H->t, H->t0, H->u, H->kvac,
+        commit_sums_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->C, H->t, H->t0, H->kvac,
                                                            H->red(S_RAD), Ctl{});
         sr_note_launch();
         H->read(S_RAD, 3, s);
@@ -1952,13 +1945,13 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
         R.delta = delta;
         R.radiated = rad;
     } else {
-        limited_scale_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->u, H->C, H->t0,
+        limited_scale_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->t, H->C, H->t0,
                                                              H->lscale);
         sr_note_launch();
-        heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(H->K, H->gas, H->kx, H->ky, H->u, H->lscale, H->fx,
+        heat_flux_kernel<<<grid_for(nf), RED_THREADS, 0, s>>>(H->K, H->gas, H->kx, H->ky, H->t, H->lscale, H->fx,
                                                                H->fy);
         sr_note_launch();
-        limited_apply_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->u, H->lscale, U,
+        limited_apply_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->kx, H->ky, H->t, H->lscale, U,
                                                              H->red(S_RAD), Ctl{});
         sr_note_launch();
         SR_CUDA_TRY(cudaMemsetAsync(H->rate, 0, sizeof(double) * H->n, s));
