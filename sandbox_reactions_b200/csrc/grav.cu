@@ -8,8 +8,9 @@
 //   2. columns: each kx column zero-padded to py, forward FFT, times the kernel's real-even spectrum K̂ (the quarter
 //      table, 1/(px py) folded in), inverse FFT, the world's rows and the two ring rows kept, in place;
 //   3. inverse rows: two output rows packed through Hermitian symmetry into one complex inverse FFT, the world's
-//      columns and the ring columns kept;
-//   4. gradient: φ and g = -∇φ.
+//      columns and the ring columns kept; up to 1,024 points the CTA's eight rows give φ and g = -∇φ of the six between
+//      them right away;
+//   4. longer rows: φ and g from the ringed potential, in a kernel of its own.
 // The FFT is a Stockham autosort over radix-16 stages and one radix-2/4/8 stage when log2 N is not a multiple of 4 (last
 // in a forward transform, first in an inverse one), each thread holding 16 points in registers. A transform's first
 // stage takes its points straight from global memory and its last leaves them in natural order in registers, so the
@@ -19,6 +20,7 @@
 // out so that neighbouring threads read neighbouring entries.
 #include <math.h>
 
+#include <algorithm>
 #include <functional>
 #include <map>
 #include <mutex>
@@ -262,21 +264,44 @@ __global__ void __launch_bounds__(column_group<N>() * fft_threads<N>(), N == 409
     }
 }
 
-// ---- pass 3: two output rows per complex inverse FFT, grouped as in pass 1; columns -1..w kept into φ_ring
+// ---- pass 3: two output rows per complex inverse FFT. FUSED (rows of up to 1,024 points): a CTA's 2G rows overlap the
+// next CTA's by two, and it writes φ and g of the rows between its first and last; the third more transforms cost less
+// than the ring's round trip and a launch while the launch is latency (256²: 5.9 + 2.0 us and a launch -> 4.4), and more
+// once it is work (2,048 points, 1024²: 7.8 + 3.7 -> 14.6, so those keep the two kernels). Not FUSED: columns -1..w kept
+// into φ_ring.
 template <int N>
-__global__ void __launch_bounds__(rows_group<N>() * fft_threads<N>()) grav_rows_inverse_kernel(GravArgs A) {
+constexpr bool inverse_fused() { return N <= kRingless; }
+template <int N>
+constexpr int inverse_group() {
+    return !inverse_fused<N>() ? 2 : (fft_threads<N>() < 8 ? 32 / fft_threads<N>() : 4);
+}
+
+template <int N>
+__global__ void __launch_bounds__(inverse_group<N>() * fft_threads<N>()) grav_rows_inverse_kernel(GravArgs A) {
     extern __shared__ float2 sm[];
-    constexpr int T = fft_threads<N>(), G = rows_group<N>();
-    const int rows = A.h + 2, r0 = blockIdx.x * 2 * G;  // rows is even (the world's height is)
+    constexpr int T = fft_threads<N>(), G = inverse_group<N>(), NT = G * T;
+    constexpr bool FUSED = inverse_fused<N>();
+    const int rows = A.h + 2, r0 = blockIdx.x * (FUSED ? 2 * G - 2 : 2 * G);  // rows is even (the world's height is)
     const size_t ld = A.ld;
-    for (int e = threadIdx.x; e < G * (N / 2 + 1); e += G * T) {
-        const int f = e % G, k = e / G, ra = r0 + 2 * f;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);  // X_a[k], X_b[k]
-        if (ra < rows) x = *reinterpret_cast<const float4*>(A.spec + (size_t)k * ld + ra);
+    auto place = [&](int f, int k, const float4& x) {
         // Z[k] = X_a[k] + i X_b[k]; Z[N-k] = conj X_a[k] + i conj X_b[k]
         float2* buf = sm + f * fft_len<N>();
         buf[fpad(k)] = make_float2(x.x - x.w, x.y + x.z);
         if (k > 0 && k < N / 2) buf[fpad(N - k)] = make_float2(x.x + x.w, x.z - x.y);
+    };
+    auto load = [&](int f, int k) {
+        const int ra = r0 + 2 * f;
+        return ra < rows ? *reinterpret_cast<const float4*>(A.spec + (size_t)k * ld + ra) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if constexpr (!FUSED) {  // many CTAs per SM hide each other's loads
+        for (int e = threadIdx.x; e < G * (N / 2 + 1); e += NT) place(e % G, e / G, load(e % G, e / G));
+    } else {
+        float4 x[8];  // X_a[k], X_b[k] of k = 0..N/2-1, all loads in flight together
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = load((threadIdx.x + u * NT) % G, (threadIdx.x + u * NT) / G);
+#pragma unroll
+        for (int u = 0; u < 8; u++) place((threadIdx.x + u * NT) % G, (threadIdx.x + u * NT) / G, x[u]);
+        if (threadIdx.x < G) place(threadIdx.x, N / 2, load(threadIdx.x, N / 2));
     }
     __syncthreads();
     const int f = threadIdx.x / T, t = threadIdx.x % T;
@@ -285,21 +310,54 @@ __global__ void __launch_bounds__(rows_group<N>() * fft_threads<N>()) grav_rows_
     fft_gather<N, true, 0>(v, buf, t);
     fft_sync<N>(1 + f);
     fft_stages<N, true, 0>(v, buf, A.tw_x, t, 1 + f);
-    const int rw = A.w + 2, ra = r0 + 2 * f;
-    if (ra >= rows) return;
-    float* ring = A.phi_ring + (size_t)ra * A.rp + kRingPad;
+    const int w = A.w, rw = w + 2;
+    if constexpr (!FUSED) {
+        const int ra = r0 + 2 * f;
+        if (ra >= rows) return;
+        float* ring = A.phi_ring + (size_t)ra * A.rp + kRingPad;
 #pragma unroll
-    for (int r = 0; r < 16; r++) {
-        const int c = (t + r * T + 1) & (N - 1);
-        if (c < rw) {
-            ring[c] = v[r].x;
-            ring[A.rp + c] = v[r].y;
+        for (int r = 0; r < 16; r++) {
+            const int c = (t + r * T + 1) & (N - 1);
+            if (c < rw) {
+                ring[c] = v[r].x;
+                ring[A.rp + c] = v[r].y;
+            }
+        }
+    } else {
+        // the transform's two ring rows over its own buffer (free since its last gather): N/2 + 2 columns at most each
+        constexpr int RP = fft_len<N>();
+        float* own = reinterpret_cast<float*>(buf);
+#pragma unroll
+        for (int r = 0; r < 16; r++) {
+            const int c = (t + r * T + 1) & (N - 1);
+            if (c < rw) {
+                own[c] = v[r].x;
+                own[RP + c] = v[r].y;
+            }
+        }
+        __syncthreads();
+        const float* ring = reinterpret_cast<const float*>(sm);  // ring row r0 + i at i RP
+        const int w4 = w / 4;
+        for (int e = threadIdx.x; e < (2 * G - 2) * w4; e += NT) {
+            const int i = e / w4, x = 4 * (e - i * w4), y = r0 + i;  // the world's row y is ring row y + 1
+            if (y >= A.h) break;
+            const float* c = ring + (i + 1) * RP + x;  // columns x - 1 on
+            float4 p, gx, gy;
+            p = make_float4(c[1], c[2], c[3], c[4]);
+            gx = make_float4(-(c[2] - c[0]) / 2.0f, -(c[3] - c[1]) / 2.0f, -(c[4] - c[2]) / 2.0f, -(c[5] - c[3]) / 2.0f);
+            const float *u = c - RP, *d = c + RP;
+            gy = make_float4(-(d[1] - u[1]) / 2.0f, -(d[2] - u[2]) / 2.0f, -(d[3] - u[3]) / 2.0f, -(d[4] - u[4]) / 2.0f);
+            const size_t o = (size_t)y * w + x;
+            *reinterpret_cast<float4*>(A.phi + o) = p;
+            *reinterpret_cast<float4*>(A.gx + o) = gx;
+            *reinterpret_cast<float4*>(A.gy + o) = gy;
         }
     }
 }
 
-// ---- pass 4: φ and g = -∇φ by central differences over the ringed potential (grav.rs:55-70), four cells a thread (the
-// world's width is a multiple of 8 and the ring's rows are padded so that its cells lie on 16-byte boundaries)
+// ---- pass 4 (rows past 1,024 points): φ and g = -∇φ by central differences over the ringed potential (grav.rs:55-70),
+// four cells a thread (the world's width is a multiple of 8 and the ring's rows are padded so that its cells lie on
+// 16-byte boundaries)
 __global__ void grav_gradient_kernel(GravArgs A) {
     const int w = A.w, h = A.h, rp = A.rp;
     const int n4 = w * h / 4;
@@ -318,27 +376,40 @@ __global__ void grav_gradient_kernel(GravArgs A) {
     }
 }
 
+// The opt-in past 48 KB of shared memory (per device, so with every launch that needs it: the longest transforms).
+template <class K>
+void allow_smem(K kernel, size_t smem) {
+    if (smem > 48 * 1024)
+        SR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+}
+
 template <int N>
 void launch_rows(const GravArgs& A, cudaStream_t s) {
-    size_t smem = rows_group<N>() * fft_len<N>() * sizeof(float2);
-    cudaFuncSetAttribute(grav_rows_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr size_t smem = rows_group<N>() * fft_len<N>() * sizeof(float2);
+    allow_smem(grav_rows_kernel<N>, smem);
     grav_rows_kernel<N><<<div_up(A.h, 2 * rows_group<N>()), rows_group<N>() * fft_threads<N>(), smem, s>>>(A);
     sr_note_launch();
 }
 
 template <int N>
 void launch_columns(const GravArgs& A, cudaStream_t s) {
-    size_t smem = column_group<N>() * fft_len<N>() * sizeof(float2);
-    cudaFuncSetAttribute(grav_columns_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr size_t smem = column_group<N>() * fft_len<N>() * sizeof(float2);
+    allow_smem(grav_columns_kernel<N>, smem);
     grav_columns_kernel<N><<<div_up(A.px / 2 + 1, column_group<N>()), column_group<N>() * fft_threads<N>(), smem, s>>>(A);
     sr_note_launch();
 }
 
 template <int N>
 void launch_rows_inverse(const GravArgs& A, cudaStream_t s) {
-    size_t smem = rows_group<N>() * fft_len<N>() * sizeof(float2);
-    cudaFuncSetAttribute(grav_rows_inverse_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    grav_rows_inverse_kernel<N><<<div_up(A.h + 2, 2 * rows_group<N>()), rows_group<N>() * fft_threads<N>(), smem, s>>>(A);
+    constexpr int G = inverse_group<N>();
+    constexpr size_t smem = G * fft_len<N>() * sizeof(float2);
+    allow_smem(grav_rows_inverse_kernel<N>, smem);
+    const unsigned grid = inverse_fused<N>() ? div_up(A.h, 2 * G - 2) : div_up(A.h + 2, 2 * G);
+    grav_rows_inverse_kernel<N><<<grid, G * fft_threads<N>(), smem, s>>>(A);
+    sr_note_launch();
+    if (inverse_fused<N>()) return;
+    const int nb = std::min<int>(div_up((unsigned)((size_t)A.w * A.h / 4), 256u), 148 * 8);
+    grav_gradient_kernel<<<nb, 256, 0, s>>>(A);
     sr_note_launch();
 }
 
@@ -491,7 +562,7 @@ void GravPlan::create(int w_, int h_, int kernel, double G, double eps, float si
     sigma_vac = sigma_vac_;
     ld = grav_column_stride(h);
     SR_CUDA_TRY(cudaMalloc(&spec, sizeof(float2) * (size_t)(px / 2 + 1) * ld));
-    SR_CUDA_TRY(cudaMalloc(&phi_ring, sizeof(float) * (size_t)grav_ring_stride(w) * (h + 2)));
+    if (px > kRingless) SR_CUDA_TRY(cudaMalloc(&phi_ring, sizeof(float) * (size_t)grav_ring_stride(w) * (h + 2)));
     const std::vector<float>& q = khat_quarter(px, py, kernel, G, eps);
     SR_CUDA_TRY(cudaMalloc(&khat, sizeof(float) * q.size()));
     SR_CUDA_TRY(cudaMemcpy(khat, q.data(), sizeof(float) * q.size(), cudaMemcpyHostToDevice));
@@ -517,7 +588,8 @@ void GravPlan::destroy() {
 }
 
 size_t GravPlan::bytes() const {
-    return sizeof(float2) * (size_t)(px / 2 + 1) * ld + sizeof(float) * (size_t)grav_ring_stride(w) * (h + 2) +
+    return sizeof(float2) * (size_t)(px / 2 + 1) * ld +
+           (px > kRingless ? sizeof(float) * (size_t)grav_ring_stride(w) * (h + 2) : 0) +
            sizeof(float) * (size_t)(px / 2 + 1) * (py / 2 + 1) +
            sizeof(float2) * (grav_twiddle_count(px) + grav_twiddle_count(py));
 }
@@ -543,9 +615,4 @@ void GravPlan::solve(const float* src, float* phi, float* gx, float* gy, cudaStr
     dispatch_rows(px, A, s);
     dispatch_columns(py, A, s);
     dispatch_rows_inverse(px, A, s);
-    size_t n = (size_t)w * h;
-    int nb = (int)div_up((unsigned)((n + 3) / 4), 256u);
-    nb = nb < 1 ? 1 : (nb > 148 * 8 ? 148 * 8 : nb);
-    grav_gradient_kernel<<<nb, 256, 0, s>>>(A);
-    sr_note_launch();
 }

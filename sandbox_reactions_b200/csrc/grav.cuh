@@ -26,6 +26,8 @@ size_t grav_twiddle_count(int n);
 void grav_twiddles(int n, float2* out);
 // A spectrum column holds the world's h rows, then the ring's h + 2 in their place; columns begin on 32 bytes.
 constexpr int grav_column_stride(int h) { return (h + 2 + 3) & ~3; }
+// Rows of at most this many points need no ringed potential in memory: the inverse pass gives φ and g itself.
+constexpr int kRingless = 1024;
 // A row of the ringed potential: column c of -1..w at kRingPad + 1 + c, so that the world's cells begin on 16 bytes.
 constexpr int kRingPad = 3;
 constexpr int grav_ring_stride(int w) { return w + 8; }

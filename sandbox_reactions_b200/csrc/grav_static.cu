@@ -3,10 +3,10 @@
 // Some hosts own every byte of device memory themselves (a game engine or plug-in host that hands its plug-ins
 // buffers and forbids them cudaMalloc), and some cannot afford cudaMalloc's device-wide synchronisation inside a
 // time-stepping loop. For them, sr_gravity_solve_static runs the same FFT-convolution kernels as a context's P2 on
-// device buffers the caller passes in, with every scratch buffer the solve needs — the half spectrum, the ringed
-// potential, the kernel's spectrum and the twiddle tables — held in file-scope static device arrays sized for worlds
-// of at most kStaticMaxWorld cells a side. Every GPU that loads this library holds those arrays (about 1.1 MB) until
-// the process exits.
+// device buffers the caller passes in, with every scratch buffer the solve needs — the half spectrum, the kernel's
+// spectrum and the twiddle tables — held in file-scope static device arrays sized for worlds of at most
+// kStaticMaxWorld cells a side. Every GPU that loads this library holds those arrays (about 0.8 MB) until the process
+// exits.
 //
 // Host code never hands a static array's name to a kernel: a __device__ array's name is a host-side stand-in, not a
 // device address. Once per device, with that device current, the first call looks up each array's device address with
@@ -28,12 +28,11 @@ namespace {
 
 constexpr int kStaticMaxWorld = 256;                // world axes up to 256 cells
 constexpr int kStaticMaxPadded = 2 * kStaticMaxWorld;  // their padded FFT length
+static_assert(kStaticMaxPadded <= kRingless, "no ringed potential is held here");
 constexpr size_t kSpecCount = (size_t)(kStaticMaxPadded / 2 + 1) * grav_column_stride(kStaticMaxWorld);
-constexpr size_t kRingCount = (size_t)grav_ring_stride(kStaticMaxWorld) * (kStaticMaxWorld + 2);
 constexpr size_t kKhatCount = (size_t)(kStaticMaxPadded / 2 + 1) * (kStaticMaxPadded / 2 + 1);
 
 static __device__ __align__(256) float2 g_spec[kSpecCount];
-static __device__ __align__(256) float g_ring[kRingCount];
 static __device__ __align__(256) float g_khat[kKhatCount];
 constexpr size_t kTwiddleMax = 3 * kStaticMaxPadded;  // an axis's twiddle table at most (grav_twiddle_count)
 static __device__ __align__(256) float2 g_tw[2 * kTwiddleMax];
@@ -49,7 +48,6 @@ constexpr int kMaxDevices = 64;
 struct DeviceSlot {
     bool ready = false;
     float2* spec = nullptr;
-    float* ring = nullptr;
     float* khat = nullptr;
     float2* tw = nullptr;
     // what the uploaded tables were built for
@@ -166,7 +164,6 @@ extern "C" sr_status sr_gravity_solve_static(const sr_config* cfg, const float* 
         if (!d.ready) {
             // the device addresses of the static arrays, looked up with this device current
             check(cudaGetSymbolAddress((void**)&d.spec, g_spec), "cudaGetSymbolAddress(g_spec)");
-            check(cudaGetSymbolAddress((void**)&d.ring, g_ring), "cudaGetSymbolAddress(g_ring)");
             check(cudaGetSymbolAddress((void**)&d.khat, g_khat), "cudaGetSymbolAddress(g_khat)");
             check(cudaGetSymbolAddress((void**)&d.tw, g_tw), "cudaGetSymbolAddress(g_tw)");
             d.ready = true;
@@ -185,7 +182,6 @@ extern "C" sr_status sr_gravity_solve_static(const sr_config* cfg, const float* 
         plan.ld = grav_column_stride(h);
         plan.sigma_vac = (float)cfg->sigma_vac;
         plan.spec = d.spec;
-        plan.phi_ring = d.ring;
         plan.khat = d.khat;
         plan.tw_x = d.tw;
         plan.tw_y = d.tw + kTwiddleMax;
