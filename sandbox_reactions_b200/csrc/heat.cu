@@ -206,6 +206,7 @@ __device__ __noinline__ void ctl_run(const Ctl& k, double* scal, int phase) {
             c->runs[B_ROUND]++;
             c->it++;
             scal[S_RZP] = scal[S_RZN];
+            scal[S_BETA] = 1.0;
             scal[S_PAR] = scal[S_PAR] != 0.0 ? 0.0 : 1.0;
             const double pq = scal[S_PQ], rr = scal[S_RRI];
             bool more = true;
@@ -692,6 +693,20 @@ __global__ void pcg_direction_kernel(size_t n, const double* __restrict__ scal, 
     }
 }
 
+// The block's Σ acc into part[blockIdx.x], in a fixed order.
+__device__ __forceinline__ void block_partial(double acc, double* part) {
+    __shared__ double red[32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
+        part[blockIdx.x] = t;
+    }
+}
+
 // Σ v[0..n) by the block, in an order that depends on n and the block's size alone; valid in thread 0.
 __device__ __forceinline__ double block_sum_ordered(const double* __restrict__ v, int n) {
     __shared__ double red[32];
@@ -714,14 +729,13 @@ __global__ void sum_parts_kernel(const double* __restrict__ v, int n, double* ou
 
 // After a (non-flexible) round's preconditioner: the search direction p_new = z + β p (β = <r,z> / <r,z>_prev, or
 // p_new = z while the S_BETA flag is 0: the first round) and q = A p_new in difference form, with partials of
-// <p_new, q>; the last CTA sets the flag. Four consecutive cells of a row per thread with 16-byte loads (W is a
+// <p_new, q>, left for pcg_update4_kernel to sum. Four consecutive cells of a row per thread with 16-byte loads (W is a
 // multiple of 8); the neighbours' p_new are formed from their z and old p, so p_new goes to the other of the two
 // direction buffers (S_PAR says which holds the old one).
 // <r, z> comes as the preconditioner's `parts` partials, which every CTA sums for itself in the same order (0: it is in
 // S_RZN already); the first CTA leaves it there.
 __global__ void spmv_dir_kernel(MgLevel L, double* scal, const float* __restrict__ z, float* pa, float* pb,
-                                float* __restrict__ q, Red R, double* beta_flag, const double* __restrict__ rz_part,
-                                int parts) {
+                                float* __restrict__ q, double* pq_part, const double* __restrict__ rz_part, int parts) {
     __shared__ double s_rz;
     if (parts > 0) {
         const double v = block_sum_ordered(rz_part, parts);
@@ -781,14 +795,22 @@ __global__ void spmv_dir_kernel(MgLevel L, double* scal, const float* __restrict
         *reinterpret_cast<float4*>(pnew + i) = pc;
         *reinterpret_cast<float4*>(q + i) = make_float4(out[0], out[1], out[2], out[3]);
     }
-    // the last CTA raises the flag: every CTA read it before taking its ticket
-    if (grid_sum_last1(acc, R.part, R.counter, R.out) && threadIdx.x == 0 && beta_flag) *beta_flag = 1.0;
+    block_partial(acc, pq_part);
 }
 
 // e += α p, r -= α q with 16-byte accesses (four cells per thread), p the round's new direction; partials of <r, r>.
-__global__ void pcg_update4_kernel(size_t n, const double* __restrict__ scal, const float* pa, const float* pb,
-                                   const float* __restrict__ q, float* __restrict__ e, float* __restrict__ r, Red R, const __grid_constant__ Ctl ctl) {
-    const float alpha = (float)(scal[S_RZN] / scal[S_PQ]);
+// <p, q> comes as `parts` partials, which every CTA sums in the same order; the first CTA leaves it in S_PQ.
+__global__ void pcg_update4_kernel(size_t n, double* scal, const double* __restrict__ pq_part, int parts,
+                                   const float* pa, const float* pb, const float* __restrict__ q, float* __restrict__ e,
+                                   float* __restrict__ r, Red R, const __grid_constant__ Ctl ctl) {
+    __shared__ double s_pq;
+    const double pq = block_sum_ordered(pq_part, parts);
+    if (threadIdx.x == 0) {
+        s_pq = pq;
+        if (blockIdx.x == 0) scal[S_PQ] = pq;
+    }
+    __syncthreads();
+    const float alpha = (float)(scal[S_RZN] / s_pq);
     const float* __restrict__ p = scal[S_PAR] != 0.0 ? pa : pb;
     const size_t n4 = n / 4, stride = (size_t)gridDim.x * blockDim.x;
     double acc = 0.0;
@@ -1130,10 +1152,11 @@ __global__ void pcg_start_kernel(double* scal) {
     scal[S_PAR] = 0.0;
 }
 
-// A fused PCG round's end: its <r, z> becomes the last one and the new direction buffer the old.
+// A fused PCG round's end: its <r, z> becomes the last one, later directions take β, the new direction buffer is the old.
 __global__ void pcg_rotate_kernel(double* scal) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     scal[S_RZP] = scal[S_RZN];
+    scal[S_BETA] = 1.0;
     scal[S_PAR] = scal[S_PAR] != 0.0 ? 0.0 : 1.0;
 }
 
@@ -1184,7 +1207,7 @@ struct HeatSolver {
     float* p2 = nullptr;  // the fused rounds' second direction buffer (rounds alternate p32 -> p2 -> p32)
     float *fx = nullptr, *fy = nullptr;
     double* part = nullptr;      // grid-sum partials: 4 x PART_CAP
-    double* rz_part = nullptr;   // the preconditioner's partials of <r, z>
+    double *rz_part = nullptr, *pq_part = nullptr;  // the preconditioner's partials of <r, z>, the SpMV's of <p, q>
     unsigned* counter = nullptr;  // grid-sum ticket
     double* scal = nullptr;       // S_COUNT device scalars
     double* hscal = nullptr;      // pinned host copy
@@ -1290,10 +1313,10 @@ void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s)
     (void)rz_new;
     precondition(H, precond, S_RZN, s);
     spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2, H->q32,
-                                                    H->red(S_PQ), H->scal + S_BETA, H->rz_part,
+                                                    H->pq_part, H->rz_part,
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
     sr_note_launch();
-    pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s>>>(H->n, H->scal, H->p32, H->p2, H->q32, H->e32, H->r32,
+    pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s>>>(H->n, H->scal, H->pq_part, H->grid_spmv, H->p32, H->p2, H->q32, H->e32, H->r32,
                                                        H->red(S_RRI), Ctl{});
     sr_note_launch();
     pcg_rotate_kernel<<<1, 32, 0, s>>>(H->scal);
@@ -1514,10 +1537,10 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                                                [&](cudaStream_t s4) {
                         precondition(H, precond, S_RZN, s4);
                         spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s4>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2,
-                                                                          H->q32, H->red(S_PQ), H->scal + S_BETA, H->rz_part,
+                                                                          H->q32, H->pq_part, H->rz_part,
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
                         sr_note_launch();
-                        pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s4>>>(H->n, H->scal, H->p32, H->p2, H->q32,
+                        pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s4>>>(H->n, H->scal, H->pq_part, H->grid_spmv, H->p32, H->p2, H->q32,
                                                                              H->e32, H->r32, H->red(S_RRI), ctl);
                         sr_note_launch();
                     });
@@ -1638,6 +1661,7 @@ HeatSolver* heat_create(const sr_config& cfg, cudaStream_t s) {
         SR_CUDA_TRY(cudaMemset(H->fy, 0, sizeof(float) * ny));
         SR_CUDA_TRY(cudaMalloc(&H->part, sizeof(double) * 4 * PART_CAP));
         SR_CUDA_TRY(cudaMalloc(&H->rz_part, sizeof(double) * PART_CAP));
+        SR_CUDA_TRY(cudaMalloc(&H->pq_part, sizeof(double) * MAX_PART));
         SR_CUDA_TRY(cudaMalloc(&H->counter, sizeof(unsigned)));
         SR_CUDA_TRY(cudaMemset(H->counter, 0, sizeof(unsigned)));
         SR_CUDA_TRY(cudaMalloc(&H->scal, sizeof(double) * S_COUNT));
@@ -1677,6 +1701,7 @@ void heat_destroy(HeatSolver* H) {
     for (float* p : d32) cudaFree(p);
     cudaFree(H->part);
     cudaFree(H->rz_part);
+    cudaFree(H->pq_part);
     cudaFree(H->counter);
     cudaFree(H->scal);
     cudaFree(H->r_old);
