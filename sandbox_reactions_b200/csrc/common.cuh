@@ -149,3 +149,26 @@ void sr_note_launch();
 void sr_note_launches(long long n);
 unsigned long long sr_launches();
 static inline unsigned div_up(unsigned a, unsigned b) { return (a + b - 1) / b; }
+
+// ---- overlapped launches: a kernel launched with `overlap` may start while the one before it on the stream still runs.
+// It must call pdl_wait (which returns once that kernel, and so everything before it, is complete and visible) before
+// it reads anything the kernels since the last plain launch wrote, and before it writes global memory at all; what it
+// does earlier (barrier set-up, loads of planes no recent kernel writes) hides the launch and the ramp. A kernel lets
+// the next one start with pdl_launch. Both are no-ops where the launch is plain.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+void launch_kernel(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    SR_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}

@@ -186,6 +186,7 @@ __global__ void __launch_bounds__(rows_group<N>() * fft_threads<N>()) grav_rows_
     const int w = A.w, h = A.h, y0 = blockIdx.x * 2 * G;
     const float sv = A.sigma_vac;
     float2* buf = sm + f * fft_len<N>();
+    pdl_launch();
     {
         const int ya = y0 + 2 * f;
         const float* ra = A.src + (size_t)ya * w;
@@ -240,6 +241,8 @@ __global__ void __launch_bounds__(column_group<N>() * fft_threads<N>(), N == 409
     float2* buf = sm + f * fft_len<N>();
     float2* col = A.spec + (size_t)(on ? kx : 0) * A.ld;
     float2 v[16];
+    pdl_launch();
+    pdl_wait();
 #pragma unroll
     for (int r = 0; r < 16; r++) {
         const int y = t + r * T;
@@ -293,6 +296,8 @@ __global__ void __launch_bounds__(inverse_group<N>() * fft_threads<N>()) grav_ro
         const int ra = r0 + 2 * f;
         return ra < rows ? *reinterpret_cast<const float4*>(A.spec + (size_t)k * ld + ra) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
+    pdl_launch();
+    pdl_wait();
     if constexpr (!FUSED) {  // many CTAs per SM hide each other's loads
         for (int e = threadIdx.x; e < G * (N / 2 + 1); e += NT) place(e % G, e / G, load(e % G, e / G));
     } else {
@@ -383,6 +388,9 @@ void allow_smem(K kernel, size_t smem) {
         SR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 }
 
+// Short transforms (the inverse takes the gradient too) overlap: their kernels are a fraction of a wave, and a launch is
+// as long as they are (256², solve and read: 18.2 -> 12.3 us). Past that an early CTA takes a slot on whichever SM is
+// free first, the next kernel's load is uneven, and a 1024² disk's step got 1.3 % slower.
 template <int N>
 void launch_rows(const GravArgs& A, cudaStream_t s) {
     constexpr size_t smem = rows_group<N>() * fft_len<N>() * sizeof(float2);
@@ -395,7 +403,8 @@ template <int N>
 void launch_columns(const GravArgs& A, cudaStream_t s) {
     constexpr size_t smem = column_group<N>() * fft_len<N>() * sizeof(float2);
     allow_smem(grav_columns_kernel<N>, smem);
-    grav_columns_kernel<N><<<div_up(A.px / 2 + 1, column_group<N>()), column_group<N>() * fft_threads<N>(), smem, s>>>(A);
+    launch_kernel(N <= kRingless, grav_columns_kernel<N>, dim3(div_up(A.px / 2 + 1, column_group<N>())),
+                  dim3(column_group<N>() * fft_threads<N>()), smem, s, A);
     sr_note_launch();
 }
 
@@ -405,7 +414,7 @@ void launch_rows_inverse(const GravArgs& A, cudaStream_t s) {
     constexpr size_t smem = G * fft_len<N>() * sizeof(float2);
     allow_smem(grav_rows_inverse_kernel<N>, smem);
     const unsigned grid = inverse_fused<N>() ? div_up(A.h, 2 * G - 2) : div_up(A.h + 2, 2 * G);
-    grav_rows_inverse_kernel<N><<<grid, G * fft_threads<N>(), smem, s>>>(A);
+    launch_kernel(N <= kRingless, grav_rows_inverse_kernel<N>, dim3(grid), dim3(G * fft_threads<N>()), smem, s, A);
     sr_note_launch();
     if (inverse_fused<N>()) return;
     const int nb = std::min<int>(div_up((unsigned)((size_t)A.w * A.h / 4), 256u), 148 * 8);
