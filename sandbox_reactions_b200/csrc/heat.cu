@@ -1260,8 +1260,12 @@ void setup_step(HeatSolver* H, const float* U, const float* kappa, cudaStream_t 
     H->mg.set_couplings(H->kx, H->ky, H->gas, s);
 }
 
+// `overlap`: multigrid's launches start while the one before still runs. In the host's rounds (one graph each) that takes
+// the launch gaps out (learned preconditioner at 512²: 6.84 -> 6.54 ms a step); in the device-controlled step's
+// conditional bodies it gave 0.6 to 1.4 %, and a batch, whose other worlds want the SMs that an early kernel waits on,
+// lost 10 %.
 // z = M r, and <r, z> into scalar `rz_slot` (into S_RZN, multigrid's: as partials, for spmv_dir_kernel to sum).
-void precondition(HeatSolver* H, uint32_t precond, int rz_slot, cudaStream_t s) {
+void precondition(HeatSolver* H, uint32_t precond, int rz_slot, bool overlap, cudaStream_t s) {
     if (precond == SR_PRECOND_JACOBI) {
         jacobi_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->mg.L[0], H->r32, H->z32, H->red(rz_slot));
         sr_note_launch();
@@ -1270,17 +1274,17 @@ void precondition(HeatSolver* H, uint32_t precond, int rz_slot, cudaStream_t s) 
         // smooth error the first cycle leaves; the second cycle removes the rounding noise of its BF16 output (high
         // frequencies, which the smoothers take out) and what remains of the smooth error.
         const MgLevel& L0 = H->mg.L[0];
-        H->mg.apply(H->r32, H->z32, nullptr, s);
+        H->mg.apply(H->r32, H->z32, nullptr, overlap, s);
         vcycle_residual_kernel<<<H->grid, RED_THREADS, 0, s>>>(L0, H->r32, H->z32, nullptr, H->q32, nullptr);
         sr_note_launch();
         learned_apply(H->lapply, L0, H->q32, H->z32, H->r32, H->z32, H->part, H->counter, H->scal + S_MGRZ, s);
         vcycle_residual_kernel<<<H->grid, RED_THREADS, 0, s>>>(L0, H->r32, H->z32, nullptr, H->q32, nullptr);
         sr_note_launch();
-        H->mg.apply(H->q32, H->vz, nullptr, s);
+        H->mg.apply(H->q32, H->vz, nullptr, overlap, s);
         add_dot_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->r32, H->vz, H->z32, H->red(rz_slot));
         sr_note_launch();
     } else {
-        H->mg.apply(H->r32, H->z32, H->rz_part, s);
+        H->mg.apply(H->r32, H->z32, H->rz_part, overlap, s);
         if (rz_slot != S_RZN) {  // a round outside the fused loop: its kernels read the sum
             sum_parts_kernel<<<1, RED_THREADS, 0, s>>>(H->rz_part, H->mg.parts(), H->scal + rz_slot);
             sr_note_launch();
@@ -1300,7 +1304,7 @@ void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s)
         pcg_update_flex_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, rz_old, H->p32, H->q32, H->e32, H->r32,
                                                                H->r_old, H->red(S_RRI));
         sr_note_launch();
-        precondition(H, precond, rz_new, s);
+        precondition(H, precond, rz_new, true, s);
         dot_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->z32, H->r_old, H->red(S_ZRO));
         sr_note_launch();
         pcg_direction_flex_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, rz_old, rz_new, H->z32, H->p32);
@@ -1311,7 +1315,7 @@ void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s)
     // one captured graph serves every round
     (void)rz_old;
     (void)rz_new;
-    precondition(H, precond, S_RZN, s);
+    precondition(H, precond, S_RZN, true, s);
     spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2, H->q32,
                                                     H->pq_part, H->rz_part,
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
@@ -1362,7 +1366,7 @@ constexpr int kStallRounds = 24;  // learned: rounds after which a solve that ha
 int inner_pcg(HeatSolver* H, uint32_t precond, double eta, int max_it, cudaStream_t s, bool* reached = nullptr) {
     if (reached) *reached = false;
     if (precond == SR_PRECOND_LEARNED) {  // flexible CG forms its direction at the end of a round
-        precondition(H, precond, S_RZ0, s);
+        precondition(H, precond, S_RZ0, true, s);
         pcg_direction_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, -1, S_RZ0, H->z32, H->p32);
         sr_note_launch();
     } else {  // the first round's fused direction is p = z
@@ -1535,7 +1539,7 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                     sr_note_launch();
                     nb[B_ROUND] = capture_body(capture_conditional(s3, hd.h[B_ROUND], cudaGraphCondTypeWhile), H->cap[4],
                                                [&](cudaStream_t s4) {
-                        precondition(H, precond, S_RZN, s4);
+                        precondition(H, precond, S_RZN, false, s4);
                         spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s4>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2,
                                                                           H->q32, H->pq_part, H->rz_part,
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
@@ -1765,7 +1769,7 @@ int heat_collect(HeatSolver* H, Learner* L, const float* U, const float* kappa, 
     };
     const int before = learned_samples(L);
     learned_begin_collect(L, H->w, H->h, crops, seed);
-    precondition(H, SR_PRECOND_MG, S_RZ0, s);
+    precondition(H, SR_PRECOND_MG, S_RZ0, true, s);
     snapshot();
     pcg_direction_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, -1, S_RZ0, H->z32, H->p32);
     sr_note_launch();
@@ -1781,7 +1785,7 @@ int heat_collect(HeatSolver* H, Learner* L, const float* U, const float* kappa, 
         H->read(S_PQ, 2, s);
         // solve on to a 1e-6 residual reduction; samples only while the remaining error is large against that
         if (!(H->hscal[S_PQ] > 0.0) || H->hscal[S_RRI] <= 1e-12 * rr0) break;
-        precondition(H, SR_PRECOND_MG, rz_new, s);
+        precondition(H, SR_PRECOND_MG, rz_new, true, s);
         if (H->hscal[S_RRI] > 1e-8 * rr0) snapshot();
         pcg_direction_kernel<<<H->grid, RED_THREADS, 0, s>>>(H->n, H->scal, rz_old, rz_new, H->z32, H->p32);
         sr_note_launch();

@@ -577,14 +577,20 @@ __global__ void __launch_bounds__(RB_NT, 2)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    // the operator's boxes (fixed over a solve) while the kernel before still runs, the iterates' after it
+    pdl_launch();
+    const int xs = X0 - XO, ys = Y0 - 1;
     if (tid == 0) {
         tma::expect_tx(mbar, (uint32_t)(NA * RB_TMA_X * RB_TMA_Y * sizeof(float)));
-        const int xs = X0 - XO, ys = Y0 - 1;
-        tma::load_3d(sarr, &mb, xs, ys, 0, mbar);
         tma::load_3d(sarr + AB, &mc, xs, ys, 0, mbar);
         tma::load_3d(sarr + 2 * AB, &mdx, xs, ys, 0, mbar);
         tma::load_3d(sarr + 3 * AB, &mdy, xs, ys, 0, mbar);
-        if constexpr (NA == 5) tma::load_3d(sarr + 4 * AB, &mx, xs, ys, 0, mbar);
+        if constexpr (PRE && NA == 5) tma::load_3d(sarr + 4 * AB, &mx, xs, ys, 0, mbar);
+    }
+    pdl_wait();
+    if (tid == 0) {
+        tma::load_3d(sarr, &mb, xs, ys, 0, mbar);
+        if constexpr (!PRE) tma::load_3d(sarr + 4 * AB, &mx, xs, ys, 0, mbar);
     }
     const int gx = X0 + 2 * lane;
     const bool xin = gx >= 0 && gx < w;
@@ -1007,6 +1013,8 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1) mg_tail_kernel(const __grid_c
     float* f = reinterpret_cast<float*>(tail_smem_raw + 2 * sizeof(TailEdge));
     TailEdge* e = reinterpret_cast<TailEdge*>(tail_smem_raw);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_launch();
+    pdl_wait();
     // the level table, read by run-time index below, out of the constant bank once; the lower levels' image (b and x 0)
     // into shared memory while the top level's loads are in flight
     __shared__ TailLevel sT[kTailLevels];
@@ -1349,7 +1357,8 @@ constexpr int tile_sy() {
 }
 
 template <int NS, bool PRE>
-void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, cudaStream_t s) {
+void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, bool overlap,
+                    cudaStream_t s) {
     constexpr int H = rb_halo<NS, PRE>();
     const dim3 grid(div_up(L.w, RB_RX - 2 * H), div_up(L.h, RB_RY - 2 * H));
     // rows of 16 bytes and 16-byte bases: the region staged by TMA
@@ -1369,7 +1378,7 @@ void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float o
                 SR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 attr = true;
             }
-            kernel<<<grid, RB_NT, smem, s>>>(mb, mc, mdx, mdy, mx, L, C, xc, omega, part);
+            launch_kernel(overlap, kernel, grid, dim3(RB_NT), smem, s, mb, mc, mdx, mdy, mx, L, C, xc, omega, part);
         };
         static bool attr_w = false, attr_u = false;
         if (L.t) go(mg_rowband_tma_kernel<NS, PRE, true>, rb_tma_smem<PRE, true>(), attr_w);
@@ -1386,9 +1395,10 @@ void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float o
 // shared-memory tiles at every size (level 0 of a 512² world under V(4,4): pre 11.9 -> 4.7 us, post 12.5 -> 7.0). Levels
 // of odd width take the shared-memory tiles, the small one where the big one leaves fewer than 2 CTAs per SM.
 template <int NS, bool PRE>
-void launch_smooth(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, cudaStream_t s) {
+void launch_smooth(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, bool overlap,
+                   cudaStream_t s) {
     if (L.w % 2 == 0)
-        launch_rowband<NS, PRE>(L, C, xc, omega, part, s);
+        launch_rowband<NS, PRE>(L, C, xc, omega, part, overlap, s);
     else if (small_tiles(L))
         launch_smooth_t<NS, PRE, SMALL_SX, tile_sy<NS, PRE, SMALL_SX, SMALL_SY, SMALL_NT>(), SMALL_NT>(
             L, C, xc, omega, s);
@@ -1396,18 +1406,19 @@ void launch_smooth(const MgLevel& L, const MgLevel& C, const float* xc, float om
         launch_smooth_t<NS, PRE, BIG_SX, tile_sy<NS, PRE, BIG_SX, BIG_SY, BIG_NT>(), BIG_NT>(L, C, xc, omega, s);
 }
 
+// `overlap`: the launch before on the stream is a kernel of the same V-cycle.
 void smooth(int nu, bool pre, const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part,
-            cudaStream_t s) {
+            bool overlap, cudaStream_t s) {
     if (pre) {
-        if (nu == 1) launch_smooth<2, true>(L, C, xc, omega, part, s);
-        else if (nu == 2) launch_smooth<4, true>(L, C, xc, omega, part, s);
-        else if (nu == 3) launch_smooth<6, true>(L, C, xc, omega, part, s);
-        else launch_smooth<8, true>(L, C, xc, omega, part, s);
+        if (nu == 1) launch_smooth<2, true>(L, C, xc, omega, part, overlap, s);
+        else if (nu == 2) launch_smooth<4, true>(L, C, xc, omega, part, overlap, s);
+        else if (nu == 3) launch_smooth<6, true>(L, C, xc, omega, part, overlap, s);
+        else launch_smooth<8, true>(L, C, xc, omega, part, overlap, s);
     } else {
-        if (nu == 1) launch_smooth<2, false>(L, C, xc, omega, part, s);
-        else if (nu == 2) launch_smooth<4, false>(L, C, xc, omega, part, s);
-        else if (nu == 3) launch_smooth<6, false>(L, C, xc, omega, part, s);
-        else launch_smooth<8, false>(L, C, xc, omega, part, s);
+        if (nu == 1) launch_smooth<2, false>(L, C, xc, omega, part, overlap, s);
+        else if (nu == 2) launch_smooth<4, false>(L, C, xc, omega, part, overlap, s);
+        else if (nu == 3) launch_smooth<6, false>(L, C, xc, omega, part, overlap, s);
+        else launch_smooth<8, false>(L, C, xc, omega, part, overlap, s);
     }
 }
 
@@ -1554,17 +1565,17 @@ int Multigrid::parts() const {
     return (int)(div_up(L[0].w, out) * div_up(L[0].h, out));
 }
 
-void Multigrid::apply(const float* r, float* z, double* rz_part, cudaStream_t s) {
+void Multigrid::apply(const float* r, float* z, double* rz_part, bool overlap, cudaStream_t s) {
     L[0].b = const_cast<float*>(r);
     L[0].x2 = z;
-    for (int l = 0; l < tail; l++) smooth(pre, true, L[l], L[l + 1], nullptr, omega, nullptr, s);
+    for (int l = 0; l < tail; l++) smooth(pre, true, L[l], L[l + 1], nullptr, omega, nullptr, overlap && l > 0, s);
     TailArgs T;
     const size_t ts = tail_args(*this, T);
     T.out = tail == 0 ? rz_part : nullptr;
-    mg_tail_kernel<<<1, TAIL_THREADS, ts, s>>>(T);
+    launch_kernel(overlap && tail > 0, mg_tail_kernel, dim3(1), dim3(TAIL_THREADS), ts, s, T);
     sr_note_launch();
     for (int l = tail - 1; l >= 0; l--)
-        smooth(post, false, L[l], L[l + 1], L[l + 1].x2, omega, l == 0 ? rz_part : nullptr, s);
+        smooth(post, false, L[l], L[l + 1], L[l + 1].x2, omega, l == 0 ? rz_part : nullptr, overlap, s);
 }
 
 void Multigrid::time_level0(int reps, void* flush, size_t flush_bytes, cudaStream_t s, double* pre_ms,
@@ -1580,9 +1591,9 @@ void Multigrid::time_level0(int reps, void* flush, size_t flush_bytes, cudaStrea
             SR_CUDA_TRY(cudaMemsetAsync(flush, k & 0xff, flush_bytes, s));
             SR_CUDA_TRY(cudaEventRecord(a, s));
             if (which == 0)
-                smooth(pre, true, L[0], L[1], nullptr, omega, nullptr, s);
+                smooth(pre, true, L[0], L[1], nullptr, omega, nullptr, false, s);
             else
-                smooth(post, false, L[0], L[1], L[1].x2, omega, nullptr, s);
+                smooth(post, false, L[0], L[1], L[1].x2, omega, nullptr, false, s);
             SR_CUDA_TRY(cudaEventRecord(b, s));
             SR_CUDA_TRY(cudaEventSynchronize(b));
             float t = 0.0f;

@@ -53,8 +53,9 @@ struct Multigrid {
     void set_couplings(const double* kx, const double* ky, const uint8_t* gas, cudaStream_t s);
     // Every coarse level's operator, once level 0's c (written by the caller, per Newton pass) is in place.
     void coarsen(cudaStream_t s);
+    // (`overlap`: its launches overlap one another, the first only plainly follows what came before.)
     // z = M r (level-0 b := r, x2 := z), and (rz_part not null) <r, z> as parts() partials, to be summed in order.
-    void apply(const float* r, float* z, double* rz_part, cudaStream_t s);
+    void apply(const float* r, float* z, double* rz_part, bool overlap, cudaStream_t s);
     int parts() const;
     // The device time (ms) of one launch of level 0's pre- and post-smoother on the last applied system, each
     // averaged over `reps` launches with `flush` (flush_bytes, larger than L2) rewritten before each: a timing hook.
