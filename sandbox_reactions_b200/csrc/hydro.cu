@@ -533,8 +533,6 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
     const int w = H.w, h = H.h;
     const size_t n = (size_t)w * h;
     const int tid = threadIdx.x, lane = tid & 31, row = tid >> 5;
-    const float dt = (float)(*A.dt);
-    const float half = 0.5f * dt;
     const bool grav = A.gx != nullptr;
     const int ntx = (w + HB_TX - 1) / HB_TX, tiles = ntx * ((h + HB_TY - 1) / HB_TY);
 
@@ -544,7 +542,11 @@ __global__ void __launch_bounds__(HB_NT, 2) hydro_band_kernel(const __grid_const
         tc::mbar_init(&sh.mbar[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    pdl_launch();
     __syncthreads();
+    pdl_wait();
+    const float dt = (float)(*A.dt);
+    const float half = 0.5f * dt;
     auto request = [&](int tile, int buf) {
         const int ty = tile / ntx, tx = tile - ty * ntx;
         tma::expect_tx(&sh.mbar[buf], (uint32_t)sizeof(sh.raw2[0]));
@@ -802,7 +804,7 @@ void hydro_launch_t(const CUtensorMap& map, const HydroArgs& A, cudaStream_t s) 
         attr = true;
     }
     const unsigned grid = std::min(div_up(A.H.w, HB_TX) * div_up(A.H.h, HB_TY), 2u * 148u);
-    hydro_band_kernel<MODE, LIM, BRACKET><<<grid, HB_NT, sizeof(BandShared), s>>>(map, A);
+    launch_kernel(MODE == kHydroStep, hydro_band_kernel<MODE, LIM, BRACKET>, dim3(grid), dim3(HB_NT), sizeof(BandShared), s, map, A);
     sr_note_launch();
 }
 
