@@ -43,6 +43,22 @@ def test_the_v_cycle_solves_over_the_level_shapes(w, h, sweeps):
     assert np.abs(x - ref).max() <= 1e-6 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("sweeps", [1, 4])
+@pytest.mark.parametrize("w,h", [(1048, 904), (2056, 1800)])
+def test_levels_of_more_regions_than_fit_the_gpu_at_once(w, h, sweeps):
+    """Level 0 (and, in the larger world, the weighted level 1) has more smoother regions than CTAs, so a CTA walks over
+    several, and the SpMV's threads take several rows. Against the Jacobi-preconditioned solve, which has no smoother:
+    each solution is within 1e-6 of the true one (above), so within 2e-6 of the other."""
+    cfg, P, kappa = world(w, h, 31 * w + h)
+    with Step(cfg.replace(mg_pre=sweeps, mg_post=sweeps)) as s:
+        s.upload(P)
+        s.upload_opacity(kappa)
+        _, rounds, rel, x = s.heat_first_solve(1e-4, "mg", want_x=True)
+        _, plain, plain_rel, ref = s.heat_first_solve(1e-4, "jacobi", want_x=True)
+    assert rel <= 1e-8 and plain_rel <= 1e-8 and 0 < rounds < plain, (rounds, plain)
+    assert np.abs(x - ref).max() <= 2e-6 * np.abs(ref).max()
+
+
 def test_worlds_made_later_leave_the_larger_tails_of_earlier_ones_alone():
     specs = [(128, 128), (80, 40), (16, 24)]
     worlds = [world(w, h, 7 + w) for w, h in specs]
