@@ -376,13 +376,13 @@ __device__ __forceinline__ void cta_partial(double acc, double* part) {
         double t = 0.0;
 #pragma unroll
         for (int q = 0; q < RB_WARPS; q++) t += red[q];
-        part[blockIdx.y * gridDim.x + blockIdx.x] = t;
+        part[blockIdx.x] = t;
     }
 }
 
 template <int NS, bool PRE, bool WT>
 __global__ void __launch_bounds__(RB_NT, 2) mg_rowband_kernel(MgLevel L, MgLevel C, const float* __restrict__ xc,
-                                                            float omega, double* part) {
+                                                            float omega) {
     constexpr int H = rb_halo<NS, PRE>(), SX = RB_RX - 2 * H, SY = RB_RY - 2 * H;
     static_assert(H % 2 == 0 && NS % 2 == 0, "the region starts on an even column and row");
     __shared__ float2 edge[2][2][RB_WARPS][32];  // [buffer][top row / bottom row][warp][lane]: (x of 2j, x of 2j+1)
@@ -516,39 +516,40 @@ __global__ void __launch_bounds__(RB_NT, 2) mg_rowband_kernel(MgLevel L, MgLevel
             }
         }
     } else {
-        double acc = 0.0;
 #pragma unroll
         for (int r = 0; r < RB_R; r++) {
             const int gy = gy0 + r, ly = RB_R * warp + r;
             if (xout && ly >= H && ly < RB_RY - H && gy < h) {
                 const size_t i = (size_t)gy * w + gx;
                 *reinterpret_cast<float2*>(L.x2 + i) = make_float2(xA[r], xB[r]);
-                if (part) acc += (double)bA[r] * (double)xA[r] + (double)bB[r] * (double)xB[r];
             }
         }
-        if (part) cta_partial(acc, part);
     }
     (void)SX;
     (void)SY;
 }
 
-// The row-band smoother of level 0 with its region staged by TMA: the same smoother as mg_rowband_kernel (unweighted
-// levels only), its coefficients (b, c, dx, dy) and, after the coarse correction, the iterate x read from shared memory
-// where one thread's bulk tensor copies put them — the region's 64 rows and the row above it, 72 columns from a
-// 16-byte boundary left of the region (the pair's left coupling included), zero past the level's edges — so a CTA's
-// loads are all in flight at once instead of four row-dependent rounds per thread. Every wait is bounded: a wait that
-// gives up sets the level's error flag and the CTA leaves without its stores.
-constexpr int RB_TMA_X = 72, RB_TMA_Y = RB_RY + 1;
+// The row-band smoother with its regions staged by TMA: the same smoother as mg_rowband_kernel, its coefficients (b, c,
+// dx, dy), after the coarse correction the iterate x, and before the restriction of a weighted level the weights read
+// from shared memory where one thread's bulk tensor copies put them: the region's 64 rows and the row above it, 68
+// columns from a 16-byte boundary left of the region (the pair's left coupling included), zero past the level's edges.
+// A CTA walks over regions: once a region's coefficients are in registers its boxes are free, and the next region's
+// land behind this one's sweeps. (A region a CTA, two CTAs an SM: the loads of a pair of CTAs, 3.8 us of the memory's
+// rate, and their sweeps came one after the other, 6.7 us a wave at 2048².) Level 0 at 2048² under V(4,4): pre-smoother
+// 35.3 -> 31.7 us, post-smoother 37.9 -> 32.2. The pre-smoother reads c again for the residual, so its c alternates between
+// two boxes; a weighted level has no room for that and asks for c and the weights once its residual is done. Every
+// wait is bounded: a wait that gives up sets the level's error flag and the CTA leaves without its stores.
+constexpr int RB_TMA_X = 68, RB_TMA_Y = RB_RY + 1;
 constexpr uint32_t kMgWaitPolls = 1u << 24;
-// b, c, dx, dy, then x after the coarse correction (post) or the weights the restriction takes (pre, weighted levels);
-// the post-smoother of a weighted level reads its weights while the boxes land
-template <bool PRE, bool WT>
-constexpr int rb_tma_arrays() { return PRE ? (WT ? 5 : 4) : 5; }
-constexpr size_t rb_tma_array_bytes() { return ((size_t)RB_TMA_X * RB_TMA_Y * sizeof(float) + 127) / 128 * 128; }
-template <bool PRE, bool WT>
-constexpr size_t rb_tma_smem() {
-    return rb_tma_arrays<PRE, WT>() * rb_tma_array_bytes() + sizeof(float2) * 2 * 2 * RB_WARPS * 32 + 16;
-}
+// b, dx, dy, c, then x (post), the other c (pre) or the weights (pre of a weighted level); the post-smoother of a
+// weighted level reads its weights while the boxes land
+constexpr int RB_BOXES = 5;
+constexpr size_t kRbBox = ((size_t)RB_TMA_X * RB_TMA_Y * sizeof(float) + 127) / 128 * 128;
+constexpr size_t kRbEdges = sizeof(float2) * 2 * 2 * RB_WARPS * 32, kRbCoarse = sizeof(float) * RB_NT * (RB_R / 2);
+constexpr size_t kRbSmem = RB_BOXES * kRbBox + kRbEdges + kRbCoarse + 16;
+// two CTAs an SM and no more than there are regions
+inline unsigned rb_regions(const MgLevel& L, int halo) { return div_up(L.w, RB_RX - 2 * halo) * div_up(L.h, RB_RY - 2 * halo); }
+inline unsigned rb_grid(const MgLevel& L, int halo) { return std::min(rb_regions(L, halo), 2u * 148u); }
 
 template <int NS, bool PRE, bool WT>
 __global__ void __launch_bounds__(RB_NT, 2)
@@ -556,204 +557,253 @@ __global__ void __launch_bounds__(RB_NT, 2)
                           const __grid_constant__ CUtensorMap mdx, const __grid_constant__ CUtensorMap mdy,
                           const __grid_constant__ CUtensorMap mx, MgLevel L, MgLevel C, const float* __restrict__ xc,
                           float omega, double* part) {
-    constexpr int H = rb_halo<NS, PRE>(), SX = RB_RX - 2 * H;
+    constexpr int H = rb_halo<NS, PRE>(), SX = RB_RX - 2 * H, SY = RB_RY - 2 * H;
     constexpr int XO = (H % 4 == 2) ? 2 : 4;  // the region's first column within the box (X0 - XO on a 16-byte boundary)
-    constexpr int NA = rb_tma_arrays<PRE, WT>();
-    constexpr size_t AB = rb_tma_array_bytes() / sizeof(float);
+    constexpr bool TWO_C = PRE && !WT, LATE = PRE && WT;
+    constexpr size_t AB = kRbBox / sizeof(float);
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* sarr = reinterpret_cast<float*>(smem_raw);
-    float2(*edge)[2][RB_WARPS][32] = reinterpret_cast<float2(*)[2][RB_WARPS][32]>(smem_raw + NA * rb_tma_array_bytes());
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + NA * rb_tma_array_bytes() + sizeof(float2) * 2 * 2 * RB_WARPS * 32);
+    float2(*edge)[2][RB_WARPS][32] = reinterpret_cast<float2(*)[2][RB_WARPS][32]>(smem_raw + RB_BOXES * kRbBox);
+    float* sxc = reinterpret_cast<float*>(smem_raw + RB_BOXES * kRbBox + kRbEdges);
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + RB_BOXES * kRbBox + kRbEdges + kRbCoarse);
     const float* sb = sarr;
-    const float* sc = sarr + AB;
-    const float* sdx = sarr + 2 * AB;
-    const float* sdy = sarr + 3 * AB;
+    const float* sdx = sarr + AB;
+    const float* sdy = sarr + 2 * AB;
     const float* sx = sarr + 4 * AB;  // post: the iterate; pre of a weighted level: the weights
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int w = L.w, h = L.h;
-    const int X0 = blockIdx.x * SX - H, Y0 = blockIdx.y * (RB_RY - 2 * H) - H;
+    const int nx = (w + SX - 1) / SX, regions = nx * ((h + SY - 1) / SY);
     if (tid == 0) {
         tc::mbar_init(mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // the operator's boxes (fixed over a solve) while the kernel before still runs, the iterates' after it
     pdl_launch();
-    const int xs = X0 - XO, ys = Y0 - 1;
+    auto arm = [&] { tma::expect_tx(mbar, (uint32_t)((PRE && !WT ? 4 : 5) * RB_TMA_X * RB_TMA_Y * sizeof(float))); };
+    // (x, y): a region's corner on the level
+    auto request_couplings = [&](int x, int y) {
+        tma::load_3d(sarr + AB, &mdx, x - XO, y - 1, 0, mbar);
+        tma::load_3d(sarr + 2 * AB, &mdy, x - XO, y - 1, 0, mbar);
+    };
+    auto request_c = [&](int x, int y, int it) {  // c, and what a weighted level's restriction takes
+        tma::load_3d(sarr + (TWO_C ? 3 + (it & 1) : 3) * AB, &mc, x - XO, y - 1, 0, mbar);
+        if constexpr (PRE && WT) tma::load_3d(sarr + 4 * AB, &mx, x - XO, y - 1, 0, mbar);
+    };
+    auto request_iterate = [&](int x, int y) {
+        tma::load_3d(sarr, &mb, x - XO, y - 1, 0, mbar);
+        if constexpr (!PRE) tma::load_3d(sarr + 4 * AB, &mx, x - XO, y - 1, 0, mbar);
+    };
+    // the post-smoother's coarse values, one per aggregate of the thread's rows, by a copy that only the thread reads
+    auto request_coarse = [&](int x, int y) {
+        if constexpr (!PRE) {
+            const int X = (x + 2 * lane) >> 1, Y = (y + RB_R * warp) >> 1;
+#pragma unroll
+            for (int k = 0; k < RB_R / 2; k++) {
+                const bool in = X >= 0 && X < C.w && Y + k >= 0 && Y + k < C.h;
+                const float* src = in ? xc + (size_t)(Y + k) * C.w + X : xc;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(tc::smem_addr(sxc + k * RB_NT + tid)), "l"(src),
+                             "r"(in ? 4 : 0) : "memory");
+            }
+        }
+    };
+    int yt = blockIdx.x / nx, xt = blockIdx.x - yt * nx;  // the region
+    int X0 = xt * SX - H, Y0 = yt * SY - H;
+    // the operator's boxes (fixed over a solve) while the kernel before still runs, the iterates' after it
     if (tid == 0) {
-        tma::expect_tx(mbar, (uint32_t)(NA * RB_TMA_X * RB_TMA_Y * sizeof(float)));
-        tma::load_3d(sarr + AB, &mc, xs, ys, 0, mbar);
-        tma::load_3d(sarr + 2 * AB, &mdx, xs, ys, 0, mbar);
-        tma::load_3d(sarr + 3 * AB, &mdy, xs, ys, 0, mbar);
-        if constexpr (PRE && NA == 5) tma::load_3d(sarr + 4 * AB, &mx, xs, ys, 0, mbar);
+        arm();
+        request_couplings(X0, Y0);
+        request_c(X0, Y0, 0);
     }
     pdl_wait();
-    if (tid == 0) {
-        tma::load_3d(sarr, &mb, xs, ys, 0, mbar);
-        if constexpr (!PRE) tma::load_3d(sarr + 4 * AB, &mx, xs, ys, 0, mbar);
-    }
-    const int gx = X0 + 2 * lane;
-    const bool xin = gx >= 0 && gx < w;
-    const int gy0 = Y0 + RB_R * warp;
-    // read while the boxes land: the post-smoother's coarse correction, the pre-smoother's coarse mask (global, half
-    // resolution)
-    float corrA[RB_R], corrB[RB_R];
-    uint8_t cmask[RB_R / 2];
+    if (tid == 0) request_iterate(X0, Y0);
+    request_coarse(X0, Y0);
+    double acc = 0.0;
+    int it = 0;
+    for (int t = blockIdx.x; t < regions; t += gridDim.x, it++) {
+        const int next = t + (int)gridDim.x;
+        int Xn = 0, Yn = 0;  // the next region's corner
+        const int gx = X0 + 2 * lane;
+        const bool xin = gx >= 0 && gx < w;
+        const int gy0 = Y0 + RB_R * warp;
+        // read while the boxes land: a weighted level's prolongation weights, the pre-smoother's coarse mask
+        float2 t2[RB_R];
+        uint8_t cmask[RB_R / 2];
+        if constexpr (WT && !PRE) {
 #pragma unroll
-    for (int r = 0; r < RB_R; r++) {
-        const int gy = gy0 + r;
-        const bool in = !PRE && xin && gy >= 0 && gy < h;
-        const float cr = in ? omega * xc[(size_t)(gy >> 1) * C.w + (gx >> 1)] : 0.0f;
-        corrA[r] = cr;
-        corrB[r] = cr;
-        if constexpr (WT && !PRE) {  // the prolongation's weights
-            if (in) {
-                const float2 t2 = *reinterpret_cast<const float2*>(L.t + (size_t)gy * w + gx);
-                corrA[r] = cr * t2.x;
-                corrB[r] = cr * t2.y;
+            for (int r = 0; r < RB_R; r++) {
+                const int gy = gy0 + r;
+                t2[r] = xin && gy >= 0 && gy < h ? *reinterpret_cast<const float2*>(L.t + (size_t)gy * w + gx) : make_float2(0.f, 0.f);
             }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < RB_R / 2; k++) {
-        const int X = gx >> 1, Y = (gy0 + 2 * k) >> 1;
-        cmask[k] = (PRE && xin && gy0 + 2 * k >= 0 && X < C.w && Y < C.h) ? C.mask[(size_t)Y * C.w + X] : 0;
-    }
-    const bool landed = tc::mbar_wait(mbar, 0, kMgWaitPolls);
-    if (__syncthreads_or(!landed)) {
-        if (tid == 0 && L.err) atomicOr(L.err, 1);
-        tc::mbar_wait(mbar, 0, kMgWaitPolls);  // copies still in flight land before the CTA leaves
-        return;
-    }
-    float bA[RB_R], bB[RB_R], iA[RB_R], iB[RB_R], dl[RB_R], dm[RB_R], dr[RB_R], dA[RB_R], dB[RB_R];
-    float xA[RB_R], xB[RB_R], cA[RB_R], cB[RB_R];
-    float uA = 0.0f, uB = 0.0f;
-    const int col0 = XO + 2 * lane;  // the pair's first column within the box
-#pragma unroll
-    for (int r = 0; r < RB_R; r++) {
-        const int gy = gy0 + r;
-        const bool in = xin && gy >= 0 && gy < h;
-        const int q = (RB_R * warp + r + 1) * RB_TMA_X + col0;  // the box's row 0 is the region's row -1
-        float2 b2 = make_float2(0.f, 0.f), c2 = make_float2(1.f, 1.f), dx2 = b2, dy2 = b2;
-        float left = 0.0f;
-        if (in) {
-            b2 = *reinterpret_cast<const float2*>(sb + q);
-            c2 = *reinterpret_cast<const float2*>(sc + q);
-            dx2 = *reinterpret_cast<const float2*>(sdx + q);
-            dy2 = *reinterpret_cast<const float2*>(sdy + q);
-            left = sdx[q - 1];  // zero past the level's left edge
-            if (r == 0) {
-                const float2 u2 = *reinterpret_cast<const float2*>(sdy + q - RB_TMA_X);  // zero above row 0
-                uA = u2.x;
-                uB = u2.y;
-            }
-        }
-        bA[r] = b2.x;
-        bB[r] = b2.y;
-        cA[r] = c2.x;
-        cB[r] = c2.y;
-        dm[r] = dx2.x;
-        dr[r] = dx2.y;
-        dA[r] = dy2.x;
-        dB[r] = dy2.y;
-        dl[r] = left;
-        const float upA = r ? dA[r - 1] : uA, upB = r ? dB[r - 1] : uB;
-        iA[r] = in ? __fdividef(1.0f, c2.x + dl[r] + dx2.x + upA + dy2.x) : 0.0f;
-        iB[r] = in ? __fdividef(1.0f, c2.y + dx2.x + dx2.y + upB + dy2.y) : 0.0f;
-        float x0 = 0.0f, x1 = 0.0f;
-        if (!PRE && in) {
-            const float2 xv = *reinterpret_cast<const float2*>(sx + q);
-            x0 = xv.x + corrA[r];
-            x1 = xv.y + corrB[r];
-        }
-        xA[r] = x0;
-        xB[r] = x1;
-    }
-    edge[0][0][warp][lane] = make_float2(xA[0], xB[0]);
-    edge[0][1][warp][lane] = make_float2(xA[RB_R - 1], xB[RB_R - 1]);
-    __syncthreads();
-    const int wu = warp > 0 ? warp - 1 : warp, wd = warp + 1 < RB_WARPS ? warp + 1 : warp;
-#pragma unroll
-    for (int s = 0; s < NS; s++) {
-        const int col = PRE ? (s & 1) : 1 - (s & 1);
-        const int rd = s & 1, wr = (s + 1) & 1;
-        const float2 above = edge[rd][1][wu][lane], below = edge[rd][0][wd][lane];
-#pragma unroll
-        for (int r = 0; r < RB_R; r++) {
-            if (PRE && s == 0) {  // the pre-smoother starts from x = 0: its first half-sweep is b times the inverse
-                if ((r & 1) == col) xA[r] = bA[r] * iA[r];
-                else xB[r] = bB[r] * iB[r];
-                continue;
-            }
-            if ((r & 1) == col) {
-                const float left = __shfl_up_sync(0xffffffffu, xB[r], 1);
-                const float up = r ? xA[r - 1] : above.x, down = r + 1 < RB_R ? xA[r + 1] : below.x;
-                const float cu = r ? dA[r - 1] : uA;
-                xA[r] = (bA[r] + dl[r] * left + dm[r] * xB[r] + cu * up + dA[r] * down) * iA[r];
-            } else {
-                const float right = __shfl_down_sync(0xffffffffu, xA[r], 1);
-                const float up = r ? xB[r - 1] : above.y, down = r + 1 < RB_R ? xB[r + 1] : below.y;
-                const float cu = r ? dB[r - 1] : uB;
-                xB[r] = (bB[r] + dm[r] * xA[r] + dr[r] * right + cu * up + dB[r] * down) * iB[r];
-            }
-        }
-        edge[wr][0][warp][lane] = make_float2(xA[0], xB[0]);
-        edge[wr][1][warp][lane] = make_float2(xA[RB_R - 1], xB[RB_R - 1]);
-        __syncthreads();
-    }
-    const bool xout = xin && 2 * lane >= H && 2 * lane < RB_RX - H;
-    if constexpr (PRE) {
-        const float2 above = edge[NS & 1][1][wu][lane], below = edge[NS & 1][0][wd][lane];
-        float ragg[RB_R / 2] = {};
-#pragma unroll
-        for (int r = 0; r < RB_R; r++) {
-            const int gy = gy0 + r, ly = RB_R * warp + r;
-            const bool o = xout && ly >= H && ly < RB_RY - H && gy < h;
-            const size_t i = (size_t)gy * w + gx;
-            if (o) *reinterpret_cast<float2*>(L.x + i) = make_float2(xA[r], xB[r]);
-            const float left = __shfl_up_sync(0xffffffffu, xB[r], 1);
-            const float right = __shfl_down_sync(0xffffffffu, xA[r], 1);
-            const float upA = r ? xA[r - 1] : above.x, dnA = r + 1 < RB_R ? xA[r + 1] : below.x;
-            const float upB = r ? xB[r - 1] : above.y, dnB = r + 1 < RB_R ? xB[r + 1] : below.y;
-            const float cuA = r ? dA[r - 1] : uA, cuB = r ? dB[r - 1] : uB;
-            float axA = cA[r] * xA[r];
-            axA += dl[r] * (xA[r] - left);
-            axA += dm[r] * (xA[r] - xB[r]);
-            axA += cuA * (xA[r] - upA);
-            axA += dA[r] * (xA[r] - dnA);
-            float axB = cB[r] * xB[r];
-            axB += dm[r] * (xB[r] - xA[r]);
-            axB += dr[r] * (xB[r] - right);
-            axB += cuB * (xB[r] - upB);
-            axB += dB[r] * (xB[r] - dnB);
-            float rA = bA[r] - axA, rB = bB[r] - axB;
-            if constexpr (WT) {  // the restriction's weights, zero past the level (the box's fill)
-                const float2 t2 = *reinterpret_cast<const float2*>(sx + (RB_R * warp + r + 1) * RB_TMA_X + col0);
-                rA *= t2.x;
-                rB *= t2.y;
-            }
-            ragg[r >> 1] += rA + rB;
         }
 #pragma unroll
         for (int k = 0; k < RB_R / 2; k++) {
-            const int ly = RB_R * warp + 2 * k;
             const int X = gx >> 1, Y = (gy0 + 2 * k) >> 1;
-            if (xout && ly >= H && ly < RB_RY - H && X < C.w && Y < C.h && gy0 + 2 * k >= 0)
-                C.b[(size_t)Y * C.w + X] = cmask[k] ? ragg[k] : 0.0f;
+            cmask[k] = (PRE && xin && gy0 + 2 * k >= 0 && X < C.w && Y < C.h) ? C.mask[(size_t)Y * C.w + X] : 0;
         }
-    } else {
-        double acc = 0.0;
+        const bool landed = tc::mbar_wait(mbar, it & 1, kMgWaitPolls);
+        if (__syncthreads_or(!landed)) {
+            if (tid == 0 && L.err) atomicOr(L.err, 1);
+            tc::mbar_wait(mbar, it & 1, kMgWaitPolls);  // copies still in flight land before the CTA leaves
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            return;
+        }
+        const float* sc = sarr + (TWO_C ? 3 + (it & 1) : 3) * AB;
+        if constexpr (!PRE) asm volatile("cp.async.wait_all;" ::: "memory");
+        float bA[RB_R], bB[RB_R], iA[RB_R], iB[RB_R], dl[RB_R], dm[RB_R], dr[RB_R], dA[RB_R], dB[RB_R];
+        float xA[RB_R], xB[RB_R];
+        float uA = 0.0f, uB = 0.0f;
+        const int col0 = XO + 2 * lane;  // the pair's first column within the box
 #pragma unroll
         for (int r = 0; r < RB_R; r++) {
-            const int gy = gy0 + r, ly = RB_R * warp + r;
-            if (xout && ly >= H && ly < RB_RY - H && gy < h) {
+            const int gy = gy0 + r;
+            const bool in = xin && gy >= 0 && gy < h;
+            const int q = (RB_R * warp + r + 1) * RB_TMA_X + col0;  // the box's row 0 is the region's row -1
+            float2 b2 = make_float2(0.f, 0.f), c2 = make_float2(1.f, 1.f), dx2 = b2, dy2 = b2;
+            float left = 0.0f;
+            if (in) {
+                b2 = *reinterpret_cast<const float2*>(sb + q);
+                c2 = *reinterpret_cast<const float2*>(sc + q);
+                dx2 = *reinterpret_cast<const float2*>(sdx + q);
+                dy2 = *reinterpret_cast<const float2*>(sdy + q);
+                left = sdx[q - 1];  // zero past the level's left edge
+                if (r == 0) {
+                    const float2 u2 = *reinterpret_cast<const float2*>(sdy + q - RB_TMA_X);  // zero above row 0
+                    uA = u2.x;
+                    uB = u2.y;
+                }
+            }
+            bA[r] = b2.x;
+            bB[r] = b2.y;
+            dm[r] = dx2.x;
+            dr[r] = dx2.y;
+            dA[r] = dy2.x;
+            dB[r] = dy2.y;
+            dl[r] = left;
+            const float upA = r ? dA[r - 1] : uA, upB = r ? dB[r - 1] : uB;
+            iA[r] = in ? __fdividef(1.0f, c2.x + dl[r] + dx2.x + upA + dy2.x) : 0.0f;
+            iB[r] = in ? __fdividef(1.0f, c2.y + dx2.x + dx2.y + upB + dy2.y) : 0.0f;
+            float x0 = 0.0f, x1 = 0.0f;
+            if (!PRE && in) {
+                const float2 xv = *reinterpret_cast<const float2*>(sx + q);
+                const float corr = omega * sxc[(r >> 1) * RB_NT + tid];
+                if constexpr (WT) {
+                    x0 = xv.x + corr * t2[r].x;
+                    x1 = xv.y + corr * t2[r].y;
+                } else {
+                    x0 = xv.x + corr;
+                    x1 = xv.y + corr;
+                }
+            }
+            xA[r] = x0;
+            xB[r] = x1;
+        }
+        edge[0][0][warp][lane] = make_float2(xA[0], xB[0]);
+        edge[0][1][warp][lane] = make_float2(xA[RB_R - 1], xB[RB_R - 1]);
+        __syncthreads();
+        if (next < regions) {  // this region's boxes are read
+            yt = next / nx;
+            xt = next - yt * nx;
+            Xn = xt * SX - H;
+            Yn = yt * SY - H;
+            if (tid == 0) {
+                arm();
+                request_couplings(Xn, Yn);
+                if constexpr (!LATE) request_c(Xn, Yn, it + 1);
+                request_iterate(Xn, Yn);
+            }
+            request_coarse(Xn, Yn);
+        }
+        const int wu = warp > 0 ? warp - 1 : warp, wd = warp + 1 < RB_WARPS ? warp + 1 : warp;
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            const int col = PRE ? (s & 1) : 1 - (s & 1);
+            const int rd = s & 1, wr = (s + 1) & 1;
+            const float2 above = edge[rd][1][wu][lane], below = edge[rd][0][wd][lane];
+#pragma unroll
+            for (int r = 0; r < RB_R; r++) {
+                if (PRE && s == 0) {  // the pre-smoother starts from x = 0: its first half-sweep is b times the inverse
+                    if ((r & 1) == col) xA[r] = bA[r] * iA[r];
+                    else xB[r] = bB[r] * iB[r];
+                    continue;
+                }
+                if ((r & 1) == col) {
+                    const float left = __shfl_up_sync(0xffffffffu, xB[r], 1);
+                    const float up = r ? xA[r - 1] : above.x, down = r + 1 < RB_R ? xA[r + 1] : below.x;
+                    const float cu = r ? dA[r - 1] : uA;
+                    xA[r] = (bA[r] + dl[r] * left + dm[r] * xB[r] + cu * up + dA[r] * down) * iA[r];
+                } else {
+                    const float right = __shfl_down_sync(0xffffffffu, xA[r], 1);
+                    const float up = r ? xB[r - 1] : above.y, down = r + 1 < RB_R ? xB[r + 1] : below.y;
+                    const float cu = r ? dB[r - 1] : uB;
+                    xB[r] = (bB[r] + dm[r] * xA[r] + dr[r] * right + cu * up + dB[r] * down) * iB[r];
+                }
+            }
+            edge[wr][0][warp][lane] = make_float2(xA[0], xB[0]);
+            edge[wr][1][warp][lane] = make_float2(xA[RB_R - 1], xB[RB_R - 1]);
+            __syncthreads();
+        }
+        const bool xout = xin && 2 * lane >= H && 2 * lane < RB_RX - H;
+        if constexpr (PRE) {
+            const float2 above = edge[NS & 1][1][wu][lane], below = edge[NS & 1][0][wd][lane];
+            float ragg[RB_R / 2] = {};
+#pragma unroll
+            for (int r = 0; r < RB_R; r++) {
+                const int gy = gy0 + r, ly = RB_R * warp + r;
+                const bool o = xout && ly >= H && ly < RB_RY - H && gy < h;
                 const size_t i = (size_t)gy * w + gx;
-                *reinterpret_cast<float2*>(L.x2 + i) = make_float2(xA[r], xB[r]);
-                if (part) acc += (double)bA[r] * (double)xA[r] + (double)bB[r] * (double)xB[r];
+                if (o) *reinterpret_cast<float2*>(L.x + i) = make_float2(xA[r], xB[r]);
+                const float left = __shfl_up_sync(0xffffffffu, xB[r], 1);
+                const float right = __shfl_down_sync(0xffffffffu, xA[r], 1);
+                const float upA = r ? xA[r - 1] : above.x, dnA = r + 1 < RB_R ? xA[r + 1] : below.x;
+                const float upB = r ? xB[r - 1] : above.y, dnB = r + 1 < RB_R ? xB[r + 1] : below.y;
+                const float cuA = r ? dA[r - 1] : uA, cuB = r ? dB[r - 1] : uB;
+                const float2 c2 = *reinterpret_cast<const float2*>(sc + (RB_R * warp + r + 1) * RB_TMA_X + col0);
+                float axA = c2.x * xA[r];
+                axA += dl[r] * (xA[r] - left);
+                axA += dm[r] * (xA[r] - xB[r]);
+                axA += cuA * (xA[r] - upA);
+                axA += dA[r] * (xA[r] - dnA);
+                float axB = c2.y * xB[r];
+                axB += dm[r] * (xB[r] - xA[r]);
+                axB += dr[r] * (xB[r] - right);
+                axB += cuB * (xB[r] - upB);
+                axB += dB[r] * (xB[r] - dnB);
+                float rA = bA[r] - axA, rB = bB[r] - axB;
+                if constexpr (WT) {  // the restriction's weights, zero past the level (the box's fill)
+                    const float2 wt = *reinterpret_cast<const float2*>(sx + (RB_R * warp + r + 1) * RB_TMA_X + col0);
+                    rA *= wt.x;
+                    rB *= wt.y;
+                }
+                ragg[r >> 1] += rA + rB;
+            }
+#pragma unroll
+            for (int k = 0; k < RB_R / 2; k++) {
+                const int ly = RB_R * warp + 2 * k;
+                const int X = gx >> 1, Y = (gy0 + 2 * k) >> 1;
+                if (xout && ly >= H && ly < RB_RY - H && X < C.w && Y < C.h && gy0 + 2 * k >= 0)
+                    C.b[(size_t)Y * C.w + X] = cmask[k] ? ragg[k] : 0.0f;
+            }
+            if constexpr (LATE) {
+                if (next < regions) {
+                    __syncthreads();
+                    if (tid == 0) request_c(Xn, Yn, it + 1);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < RB_R; r++) {
+                const int gy = gy0 + r, ly = RB_R * warp + r;
+                if (xout && ly >= H && ly < RB_RY - H && gy < h) {
+                    const size_t i = (size_t)gy * w + gx;
+                    *reinterpret_cast<float2*>(L.x2 + i) = make_float2(xA[r], xB[r]);
+                    if (part) acc += (double)bA[r] * (double)xA[r] + (double)bB[r] * (double)xB[r];
+                }
             }
         }
-        if (part) cta_partial(acc, part);
+        X0 = Xn;
+        Y0 = Yn;
     }
+    if (!PRE && part) cta_partial(acc, part);
 }
 
 // ---- the coarse tail: every level of at most 64 x 64 cells, inside one CTA
@@ -1360,7 +1410,7 @@ template <int NS, bool PRE>
 void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float omega, double* part, bool overlap,
                     cudaStream_t s) {
     constexpr int H = rb_halo<NS, PRE>();
-    const dim3 grid(div_up(L.w, RB_RX - 2 * H), div_up(L.h, RB_RY - 2 * H));
+    // Level 0 (a world's axes are multiples of 8, its planes allocations of their own) and every other level with
     // rows of 16 bytes and 16-byte bases: the region staged by TMA
     auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
     if (L.w % 4 == 0 && aligned(L.b) && aligned(L.c) && aligned(L.dx) && aligned(L.dy) && aligned(L.x) &&
@@ -1373,21 +1423,23 @@ void launch_rowband(const MgLevel& L, const MgLevel& C, const float* xc, float o
         if (!PRE) tma_encode_planes(&mx, L.x, L.w, L.h, 1, RB_TMA_X, RB_TMA_Y);
         else if (L.t) tma_encode_planes(&mx, L.t, L.w, L.h, 1, RB_TMA_X, RB_TMA_Y);
         else mx = mb;
-        auto go = [&](auto kernel, size_t smem, bool& attr) {
+        auto go = [&](auto kernel, bool& attr) {
             if (!attr) {  // the instance's shared-memory attribute, once per process
-                SR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                SR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRbSmem));
                 attr = true;
             }
-            launch_kernel(overlap, kernel, grid, dim3(RB_NT), smem, s, mb, mc, mdx, mdy, mx, L, C, xc, omega, part);
+            launch_kernel(overlap, kernel, dim3(rb_grid(L, H)), dim3(RB_NT), kRbSmem, s, mb, mc, mdx, mdy, mx, L, C, xc, omega, part);
         };
         static bool attr_w = false, attr_u = false;
-        if (L.t) go(mg_rowband_tma_kernel<NS, PRE, true>, rb_tma_smem<PRE, true>(), attr_w);
-        else go(mg_rowband_tma_kernel<NS, PRE, false>, rb_tma_smem<PRE, false>(), attr_u);
+        if (L.t) go(mg_rowband_tma_kernel<NS, PRE, true>, attr_w);
+        else go(mg_rowband_tma_kernel<NS, PRE, false>, attr_u);
         sr_note_launch();
         return;
     }
-    if (L.t) mg_rowband_kernel<NS, PRE, true><<<grid, RB_NT, 0, s>>>(L, C, xc, omega, part);
-    else mg_rowband_kernel<NS, PRE, false><<<grid, RB_NT, 0, s>>>(L, C, xc, omega, part);
+    if (part) throw SrError{SR_E_CUDA, "multigrid: level 0 is not laid out in 16-byte rows"};
+    const dim3 grid(div_up(L.w, RB_RX - 2 * H), div_up(L.h, RB_RY - 2 * H));
+    if (L.t) mg_rowband_kernel<NS, PRE, true><<<grid, RB_NT, 0, s>>>(L, C, xc, omega);
+    else mg_rowband_kernel<NS, PRE, false><<<grid, RB_NT, 0, s>>>(L, C, xc, omega);
     sr_note_launch();
 }
 
@@ -1561,8 +1613,7 @@ void Multigrid::coarsen(cudaStream_t s) {
 
 int Multigrid::parts() const {
     if (tail == 0) return 1;
-    const unsigned out = RB_RX - 2 * (2 * post);  // the post-smoother's halo is its half-sweeps
-    return (int)(div_up(L[0].w, out) * div_up(L[0].h, out));
+    return (int)rb_grid(L[0], 2 * post);  // the post-smoother's halo is its half-sweeps
 }
 
 void Multigrid::apply(const float* r, float* z, double* rz_part, bool overlap, cudaStream_t s) {
