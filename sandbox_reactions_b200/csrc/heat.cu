@@ -729,14 +729,40 @@ __global__ void sum_parts_kernel(const double* __restrict__ v, int n, double* ou
 
 // After a (non-flexible) round's preconditioner: the search direction p_new = z + β p (β = <r,z> / <r,z>_prev, or
 // p_new = z while the S_BETA flag is 0: the first round) and q = A p_new in difference form, with partials of
-// <p_new, q>, left for pcg_update4_kernel to sum. Four consecutive cells of a row per thread with 16-byte loads (W is a
-// multiple of 8); the neighbours' p_new are formed from their z and old p, so p_new goes to the other of the two
-// direction buffers (S_PAR says which holds the old one).
+// <p_new, q>, left for pcg_update4_kernel to sum. The neighbours' p_new are formed from their z and old p, so p_new goes
+// to the other of the two direction buffers (S_PAR says which holds the old one).
 // <r, z> comes as the preconditioner's `parts` partials, which every CTA sums for itself in the same order (0: it is in
 // S_RZN already); the first CTA leaves it there.
-__global__ void spmv_dir_kernel(MgLevel L, double* scal, const float* __restrict__ z, float* pa, float* pb,
-                                float* __restrict__ q, double* pq_part, const double* __restrict__ rz_part, int parts) {
+// A thread takes four consecutive columns (W is a multiple of 8) of `rows` rows and walks down them: the row above and
+// its own stay in registers, its side neighbours come from the next lanes, so a row costs one 16-byte load of each plane
+// (a thread a row: three of z and of p, two of dy, and six words at its sides; 2048²: 28.0 -> 20.2 us; 512²: 6.2 -> 4.4). `rows` is what
+// puts all threads on the GPU at once (1 up to some 600,000 cells); the next row's operands are in flight behind this
+// row's arithmetic.
+__global__ void __launch_bounds__(RED_THREADS, 3)
+    spmv_dir_kernel(MgLevel L, int rows, double* scal, const float* __restrict__ z, float* pa, float* pb,
+                    float* __restrict__ q, double* pq_part, const double* __restrict__ rz_part, int parts) {
     __shared__ double s_rz;
+    const int w = L.w, h = L.h, w4 = w / 4, lane = threadIdx.x & 31;
+    const int t = blockIdx.x * RED_THREADS + threadIdx.x, bands = (h + rows - 1) / rows;
+    const bool live = t < w4 * bands;
+    const int band = live ? t / w4 : 0, x = 4 * (live ? t - band * w4 : 0), y0 = band * rows;
+    struct Op {
+        float4 c, dx, dy;
+        float dl;  // the coupling to the left of lane 0's columns
+        uchar4 m;
+    };
+    auto op_at = [&](int y) {
+        const size_t i = (size_t)y * w + x;
+        Op o;
+        o.c = *reinterpret_cast<const float4*>(L.c + i);
+        o.dx = *reinterpret_cast<const float4*>(L.dx + i);
+        o.dy = *reinterpret_cast<const float4*>(L.dy + i);
+        o.dl = lane == 0 && x > 0 ? L.dx[i - 1] : 0.0f;
+        o.m = *reinterpret_cast<const uchar4*>(L.mask + i);
+        return o;
+    };
+    Op o = op_at(y0);
+    float4 dyu = y0 > 0 ? *reinterpret_cast<const float4*>(L.dy + (size_t)(y0 - 1) * w + x) : make_float4(0.f, 0.f, 0.f, 0.f);
     if (parts > 0) {
         const double v = block_sum_ordered(rz_part, parts);
         if (threadIdx.x == 0) {
@@ -752,35 +778,62 @@ __global__ void spmv_dir_kernel(MgLevel L, double* scal, const float* __restrict
     const bool par = scal[S_PAR] != 0.0;
     const float* __restrict__ p = par ? pb : pa;
     float* __restrict__ pnew = par ? pa : pb;
-    const int w = L.w, h = L.h;
-    const size_t n4 = (size_t)w * h / 4, stride = (size_t)gridDim.x * blockDim.x;
+    struct Raw {
+        float4 z, p;
+        float ze, pe;  // the column beside the warp's, lane 0's left and lane 31's right
+    };
+    const int side = lane == 0 ? (x > 0 ? -1 : 0) : (lane == 31 && x + 4 < w ? 4 : 0);
+    auto raw_at = [&](int y) {
+        const size_t i = (size_t)y * w + x;
+        Raw a;
+        a.z = *reinterpret_cast<const float4*>(z + i);
+        a.ze = side ? z[i + side] : 0.0f;
+        a.p = make_float4(0.f, 0.f, 0.f, 0.f);
+        a.pe = 0.0f;
+        if (!first) {
+            a.p = *reinterpret_cast<const float4*>(p + i);
+            a.pe = side ? p[i + side] : 0.0f;
+        }
+        return a;
+    };
+    auto dir4 = [&](const Raw& a) {
+        if (first) return a.z;
+        return make_float4(a.z.x + beta * a.p.x, a.z.y + beta * a.p.y, a.z.z + beta * a.p.z, a.z.w + beta * a.p.w);
+    };
+    auto dir_side = [&](const Raw& a) { return first ? a.ze : a.ze + beta * a.pe; };
+    Raw ra = raw_at(max(y0 - 1, 0)), rc = raw_at(y0), rd = raw_at(min(y0 + 1, h - 1));
+    float4 pu = dir4(ra), pc = dir4(rc);
+    float pe = dir_side(rc);
     double acc = 0.0;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n4; t += stride) {
-        const size_t i = 4 * t;
-        int x, y;
-        split_index(i, w, x, y);
-        auto pn4 = [&](size_t j) {
-            const float4 zz = *reinterpret_cast<const float4*>(z + j);
-            if (first) return zz;
-            const float4 pp = *reinterpret_cast<const float4*>(p + j);
-            return make_float4(zz.x + beta * pp.x, zz.y + beta * pp.y, zz.z + beta * pp.z, zz.w + beta * pp.w);
-        };
-        auto pn1 = [&](size_t j) { return first ? z[j] : z[j] + beta * p[j]; };
-        const float4 pc = pn4(i);
-        const float4 pu = y > 0 ? pn4(i - w) : pc, pd = y + 1 < h ? pn4(i + w) : pc;
-        const float pl = x > 0 ? pn1(i - 1) : pc.x;
-        const float pr = x + 4 < w ? pn1(i + 4) : pc.w;
-        const float4 c = *reinterpret_cast<const float4*>(L.c + i);
-        const float4 dx = *reinterpret_cast<const float4*>(L.dx + i), dy = *reinterpret_cast<const float4*>(L.dy + i);
-        const float dxl = x > 0 ? L.dx[i - 1] : 0.0f;
-        const float4 dyu = y > 0 ? *reinterpret_cast<const float4*>(L.dy + i - w) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const uchar4 m = *reinterpret_cast<const uchar4*>(L.mask + i);
+    for (int r = 0; r < rows; r++) {
+        const int y = y0 + r;
+        const float4 pd = dir4(rd);
+        const float pde = dir_side(rd);
+        Op on = o;
+        if (r + 1 < rows) {  // rows past the last are the last again, and leave nothing
+            on = op_at(min(y + 1, h - 1));
+            rd = raw_at(min(y + 2, h - 1));
+        }
+        float pl = __shfl_up_sync(0xffffffffu, pc.w, 1), pr = __shfl_down_sync(0xffffffffu, pc.x, 1);
+        float dl = __shfl_up_sync(0xffffffffu, o.dx.w, 1);
+        if (lane == 0) {
+            pl = pe;
+            dl = o.dl;
+        }
+        if (lane == 31) pr = pe;
+        if (x == 0) {
+            pl = pc.x;
+            dl = 0.0f;
+        }
+        if (x + 4 >= w) pr = pc.w;
+        const float4 up = y > 0 ? pu : pc, dn = y + 1 < h ? pd : pc;
         const float P[6] = {pl, pc.x, pc.y, pc.z, pc.w, pr};
-        const float U[4] = {pu.x, pu.y, pu.z, pu.w}, D[4] = {pd.x, pd.y, pd.z, pd.w};
-        const float CC[4] = {c.x, c.y, c.z, c.w}, DXs[5] = {dxl, dx.x, dx.y, dx.z, dx.w};
-        const float DYu[4] = {dyu.x, dyu.y, dyu.z, dyu.w}, DYd[4] = {dy.x, dy.y, dy.z, dy.w};
-        const unsigned char M[4] = {m.x, m.y, m.z, m.w};
+        const float U[4] = {up.x, up.y, up.z, up.w}, D[4] = {dn.x, dn.y, dn.z, dn.w};
+        const float CC[4] = {o.c.x, o.c.y, o.c.z, o.c.w}, DXs[5] = {dl, o.dx.x, o.dx.y, o.dx.z, o.dx.w};
+        const float DYu[4] = {dyu.x, dyu.y, dyu.z, dyu.w}, DYd[4] = {o.dy.x, o.dy.y, o.dy.z, o.dy.w};
+        const unsigned char M[4] = {o.m.x, o.m.y, o.m.z, o.m.w};
         float out[4];
+        const bool on_row = live && y < h;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const float pi = P[k + 1];
@@ -790,10 +843,18 @@ __global__ void spmv_dir_kernel(MgLevel L, double* scal, const float* __restrict
             a += DYu[k] * (pi - U[k]);
             a += DYd[k] * (pi - D[k]);
             out[k] = M[k] ? a : 0.0f;
-            acc += (double)pi * out[k];
+            if (on_row) acc += (double)pi * out[k];
         }
-        *reinterpret_cast<float4*>(pnew + i) = pc;
-        *reinterpret_cast<float4*>(q + i) = make_float4(out[0], out[1], out[2], out[3]);
+        if (on_row) {
+            const size_t i = (size_t)y * w + x;
+            *reinterpret_cast<float4*>(pnew + i) = pc;
+            *reinterpret_cast<float4*>(q + i) = make_float4(out[0], out[1], out[2], out[3]);
+        }
+        dyu = o.dy;
+        pu = pc;
+        pc = pd;
+        pe = pde;
+        o = on;
     }
     block_partial(acc, pq_part);
 }
@@ -1193,6 +1254,7 @@ struct HeatSolver {
     // once: a CTA without a turn still takes a sum's ticket (512²: the SpMV 256 CTAs instead of 1,024), and a wave that
     // does not fill costs a whole one
     int grid_residual = 0, grid_newton = 0, grid_spmv = 0, grid_update = 0;
+    int spmv_rows = 1;
     uint32_t precond = SR_PRECOND_MG;
     uint32_t max_passes = 128, max_rounds = 4096;
     double inner_floor = 1e-5;  // the smallest residual reduction asked of one inner FP32 solve
@@ -1316,7 +1378,7 @@ void round_launches(HeatSolver* H, uint32_t precond, int parity, cudaStream_t s)
     (void)rz_old;
     (void)rz_new;
     precondition(H, precond, S_RZN, true, s);
-    spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2, H->q32,
+    spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s>>>(H->mg.L[0], H->spmv_rows, H->scal, H->z32, H->p32, H->p2, H->q32,
                                                     H->pq_part, H->rz_part,
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
     sr_note_launch();
@@ -1540,7 +1602,7 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                     nb[B_ROUND] = capture_body(capture_conditional(s3, hd.h[B_ROUND], cudaGraphCondTypeWhile), H->cap[4],
                                                [&](cudaStream_t s4) {
                         precondition(H, precond, S_RZN, false, s4);
-                        spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s4>>>(H->mg.L[0], H->scal, H->z32, H->p32, H->p2,
+                        spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s4>>>(H->mg.L[0], H->spmv_rows, H->scal, H->z32, H->p32, H->p2,
                                                                           H->q32, H->pq_part, H->rz_part,
                                                     precond == SR_PRECOND_MG ? H->mg.parts() : 0);
                         sr_note_launch();
@@ -1647,7 +1709,10 @@ HeatSolver* heat_create(const sr_config& cfg, cudaStream_t s) {
         H->grid = grid_for(H->n);
         H->grid_residual = whole_waves(heat_residual64_kernel, H->n / 2);
         H->grid_newton = whole_waves(newton_system_kernel, H->n / 2);
-        H->grid_spmv = whole_waves(spmv_dir_kernel, H->n / 4);
+        // rows a thread of the SpMV: as few as leave its threads room on the GPU all at once
+        const int w4 = H->w / 4, most = whole_waves(spmv_dir_kernel, H->n) * RED_THREADS;
+        H->spmv_rows = (H->h + std::max(1, most / w4) - 1) / std::max(1, most / w4);
+        H->grid_spmv = grid_for((size_t)w4 * ((H->h + H->spmv_rows - 1) / H->spmv_rows));
         H->grid_update = whole_waves(pcg_update4_kernel, H->n / 4);
         const size_t n = H->n, nx = (size_t)(H->w + 1) * H->h, ny = (size_t)H->w * (H->h + 1);
         SR_CUDA_TRY(cudaMalloc(&H->gas, n));
