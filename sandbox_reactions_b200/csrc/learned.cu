@@ -439,24 +439,37 @@ __global__ void __launch_bounds__(DW_NT) dw_kernel(ConvArgs A, const float* __re
     }
 }
 
-// dW and db from the partials into the gradient vector (the parameter layout W[cout][3][3][cin], b[cout]).
-__global__ void dw_reduce_kernel(const float* __restrict__ part, int chunks, int cin, int cout, int cin_p, int cout_p,
-                                 float* gw, float* gb, const float* __restrict__ bpart) {
-    const int kt = 9 * cin_p;
-    const int n = cout * 9 * cin;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n + cout; e += gridDim.x * blockDim.x) {
-        if (e < n) {
-            const int co = e / (9 * cin), rem = e % (9 * cin), tap = rem / cin, ci = rem % cin;
-            const int k = tap * cin_p + ci;
-            double s = 0.0;
-            for (int c = 0; c < chunks; c++) s += part[((size_t)c * cout_p + co) * kt + k];
-            gw[e] = (float)s;
-        } else {
-            const int co = e - n;
-            double s = 0.0;
-            for (int c = 0; c < chunks; c++) s += bpart[(size_t)c * cout_p + co];
-            gb[co] = (float)s;
-        }
+// dW and db from the partials into the gradient vector (the parameter layout W[cout][3][3][cin], b[cout]). A sum of up
+// to 128 partials is 128 dependent steps of a load's latency for one thread, so each parameter's are dealt to RD_S threads
+// in runs, and the runs' sums added in order: 8.7 -> 3.2 us a layer.
+constexpr int RD_E = 32, RD_S = 8;  // parameters and runs of a CTA
+__global__ void __launch_bounds__(RD_E * RD_S) dw_reduce_kernel(const float* __restrict__ part, int chunks, int cin,
+                                                               int cout, int cin_p, int cout_p, float* gw, float* gb,
+                                                               const float* __restrict__ bpart) {
+    __shared__ double run[RD_S][RD_E];
+    const int kt = 9 * cin_p, n = cout * 9 * cin;
+    const int e = blockIdx.x * RD_E + threadIdx.x, k = threadIdx.y;
+    const float* src = bpart;  // the parameter's first partial; the next ones `step` apart
+    size_t step = (size_t)cout_p;
+    if (e < n) {
+        const int co = e / (9 * cin), rem = e % (9 * cin), tap = rem / cin, ci = rem % cin;
+        src = part + (size_t)co * kt + tap * cin_p + ci;
+        step = (size_t)cout_p * kt;
+    } else if (e < n + cout) {
+        src = bpart + (e - n);
+    }
+    const int len = (chunks + RD_S - 1) / RD_S, c0 = k * len, c1 = min(chunks, c0 + len);
+    double s = 0.0;
+    if (e < n + cout) {
+#pragma unroll 4
+        for (int c = c0; c < c1; c++) s += src[c * step];
+    }
+    run[k][threadIdx.x] = s;
+    __syncthreads();
+    if (k == 0 && e < n + cout) {
+#pragma unroll
+        for (int q = 1; q < RD_S; q++) s += run[q][threadIdx.x];
+        (e < n ? gw[e] : gb[e - n]) = (float)s;
     }
 }
 
@@ -906,7 +919,7 @@ void backward(Learner* Lr, Net& N, cudaStream_t s) {
         ConvArgs A = layer_args(Lr, N, l);
         const int chunks = dw_chunks(A.B, A.H, A.W);
         launch_dw(ci, co, A, N.gact[l], N.act[l], d.relu, N.wpart, N.bpart, s);
-        dw_reduce_kernel<<<grid_of((size_t)d.cout * 9 * d.cin + d.cout), RT, 0, s>>>(
+        dw_reduce_kernel<<<(d.cout * 9 * d.cin + d.cout + RD_E - 1) / RD_E, dim3(RD_E, RD_S), 0, s>>>(
             N.wpart, chunks, d.cin, d.cout, ci, co, Lr->grad + Lr->woff[l], Lr->grad + Lr->boff[l], N.bpart);
         sr_note_launch();
         if (l == 0) break;
