@@ -833,10 +833,12 @@ void hydro_gravity_launch(const HydroArgs& A, cudaStream_t s) {
 
 // ------------------------------------------------------------------------------------------------ P8 + P9
 // P8's floors, then P9's per-cell Δt terms of the floored state and |g| of the step's P2 field; per-CTA partials, the
-// last CTA to arrive (a ticket) reduces them (max and min are exact in any order) and closes the step's Δt record.
-__global__ void __launch_bounds__(256) floors_dt_kernel(HydroConst H, float* __restrict__ U, const float* __restrict__ gx,
-                                                        const float* __restrict__ gy, int do_floors, float* part_rate,
-                                                        float* part_g, long long* part_nf, unsigned* ticket, DtRule rule) {
+// last CTA to arrive (a ticket) reduces them (max and min are exact in any order) and closes the step's Δt record. Four CTAs
+// an SM (63 registers), as many as the grid has for each: with three the grid was a wave and a third (1024²: 13.8 -> 11.9
+// us).
+__global__ void __launch_bounds__(256, 4)
+    floors_dt_kernel(HydroConst H, float* __restrict__ U, const float* __restrict__ gx, const float* __restrict__ gy,
+                     int do_floors, float* part_rate, float* part_g, long long* part_nf, unsigned* ticket, DtRule rule) {
     const size_t n = (size_t)H.w * H.h, n4 = n / 4;  // the world's axes are multiples of 8
     float rate = 0.0f, gmax = 0.0f;
     double g2 = 0.0;  // |g|²: no square of an f32 leaves f64's range
