@@ -30,6 +30,14 @@ __device__ __forceinline__ void load_3d(void* dst, const CUtensorMap* map, int x
         : "memory");
 }
 
+// `bytes` (a multiple of 16) from `src` to shared memory at `dst`, both on 16-byte boundaries, completing on `mbar`.
+__device__ __forceinline__ void load_bytes(void* dst, const void* src, uint32_t bytes, uint64_t* mbar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     tc::smem_addr(dst)),
+                 "l"(src), "r"(bytes), "r"(tc::smem_addr(mbar))
+                 : "memory");
+}
+
 }  // namespace tma
 
 // Host: the tensor map of `planes` f32 planes of w x h at `base` (16-byte aligned), box bx x by x planes.
