@@ -160,6 +160,7 @@ __device__ __noinline__ void ctl_run(const Ctl& k, double* scal, int phase) {
             c->pass_tol = fmax(c->tol, kFirstPassTol);
             c->moved_prev = 0.0;
             const bool go = c->max_passes > 0 && c->max_rounds > 0;
+            ctl_set(k, B_COARSEN, go, true);
             ctl_set(k, B_PASS, go, false);
             if (go) ctl_pass_begin(k);
             else ctl_commit(k);
@@ -192,6 +193,7 @@ __device__ __noinline__ void ctl_run(const Ctl& k, double* scal, int phase) {
             break;
         }
         case C_INNER_BEGIN: {  // after the scaled residual
+            ctl_set(k, B_COARSEN, false, true);  // this pass's is done
             scal[S_BETA] = 0.0;
             scal[S_PAR] = 0.0;
             c->rr0 = scal[S_R32];
@@ -1287,7 +1289,8 @@ struct HeatSolver {
     HeatCtl* ctl = nullptr;
     HeatCtl* hctl = nullptr;      // pinned host copy
     std::map<const float*, cudaGraphExec_t> step_graphs;
-    cudaStream_t cap[6] = {};
+    cudaStream_t cap[6] = {};  // [5]: the captured pass's branch
+    cudaEvent_t fork[2] = {};  // its start and its end
     long long body_launches[B_COUNT + 1] = {};  // [B_COUNT]: the graph's own top-level kernels
     bool report_pending = false;  // the last step ran as a graph: its report is in ctl
     cudaStream_t stream = nullptr;  // the owning context's stream
@@ -1587,14 +1590,21 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
         heat_system_kernel<<<H->grid, RED_THREADS, 0, s0>>>(H->K, H->scal, H->gas, H->C, H->t, H->kvac,
                                                             H->mg.L[0].c, H->x, H->red(S_UB), ctl);
         sr_note_launch();
-        H->mg.coarsen(s0);
         nb[B_PASS] = capture_body(capture_conditional(s0, hd.h[B_PASS], cudaGraphCondTypeWhile), H->cap[1],
                                   [&](cudaStream_t s1) {
             nb[B_REFINE] = capture_body(capture_conditional(s1, hd.h[B_REFINE], cudaGraphCondTypeWhile), H->cap[2],
                                         [&](cudaStream_t s2) {
+                // a new system's coarse levels beside its first FP64 residual: a chain of small kernels (39 us of
+                // latency at 512², 95 at 2048²) and one that takes the whole GPU, neither of which the other needs
+                SR_CUDA_TRY(cudaEventRecord(H->fork[0], s2));
+                SR_CUDA_TRY(cudaStreamWaitEvent(H->cap[5], H->fork[0], 0));
+                nb[B_COARSEN] = capture_body(capture_conditional(H->cap[5], hd.h[B_COARSEN], cudaGraphCondTypeIf),
+                                             H->cap[3], [&](cudaStream_t s3) { H->mg.coarsen(s3); });
+                SR_CUDA_TRY(cudaEventRecord(H->fork[1], H->cap[5]));
                 heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s2>>>(H->K, H->scal, H->gas, H->kvac, H->kx,
                                                                          H->ky, H->C, H->t, H->t0, H->x, H->r64, H->red(S_RR), ctl);
                 sr_note_launch();
+                SR_CUDA_TRY(cudaStreamWaitEvent(s2, H->fork[1], 0));
                 nb[B_INNER] = capture_body(capture_conditional(s2, hd.h[B_INNER], cudaGraphCondTypeIf), H->cap[3],
                                            [&](cudaStream_t s3) {
                     scale_kernel<<<H->grid, RED_THREADS, 0, s3>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32), ctl);
@@ -1618,8 +1628,6 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                                       [&](cudaStream_t s2) {
                 newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s2>>>(H->K, H->cfg.newton_cell, H->scal, H->gas, H->C, H->kvac, H->t, H->x, H->mg.L[0].c, H->red(S_MOVED), ctl);
                 sr_note_launch();
-                nb[B_COARSEN] = capture_body(capture_conditional(s2, hd.h[B_COARSEN], cudaGraphCondTypeIf), H->cap[3],
-                                             [&](cudaStream_t s3) { H->mg.coarsen(s3); });
             });
         });
         nb[B_CONV] = capture_body(capture_conditional(s0, hd.h[B_CONV], cudaGraphCondTypeIf), H->cap[1],
@@ -1740,6 +1748,7 @@ HeatSolver* heat_create(const sr_config& cfg, cudaStream_t s) {
         SR_CUDA_TRY(cudaMemset(H->ctl, 0, sizeof(HeatCtl)));
         SR_CUDA_TRY(cudaMallocHost(&H->hctl, sizeof(HeatCtl)));
         for (cudaStream_t& c : H->cap) SR_CUDA_TRY(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking));
+        for (cudaEvent_t& e : H->fork) SR_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         H->mg.create(H->w, H->h, (int)cfg.mg_pre, (int)cfg.mg_post);
         H->mg.omega = cfg.mg_omega > 0.0 ? (float)cfg.mg_omega : 1.0f;
         H->inner_floor = cfg.inner_tol > 0.0 ? cfg.inner_tol : 1e-5;
@@ -1760,6 +1769,8 @@ void heat_destroy(HeatSolver* H) {
     drop_step_graphs(H);
     cudaFree(H->ctl);
     if (H->hctl) cudaFreeHost(H->hctl);
+    for (cudaEvent_t e : H->fork)
+        if (e) cudaEventDestroy(e);
     for (cudaStream_t c : H->cap)
         if (c) cudaStreamDestroy(c);
     cudaFree(H->gas);
