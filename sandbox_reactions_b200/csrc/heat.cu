@@ -517,66 +517,120 @@ __global__ void heat_system_kernel(HeatConst K, const double* __restrict__ scal,
 }
 
 // r = b - A x in FP64, A x = c x + Σ_gas D (x_i - x_j), with partials of <r, r>, <b, b> and the reference's two
-// measures (heat.rs:413-447): rᵀD⁻¹r and the heat measure Σ (C/Δt)(r (dT/du) / D_ii)². Each thread takes ILP cells a
-// grid stride apart and issues all of their loads before the arithmetic (the loads do not depend on the gas flags:
-// the flags select afterwards), so a thread keeps several DRAM requests in flight.
-constexpr int ILP = 4;
-
-__global__ void heat_residual64_kernel(HeatConst K, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
-                                       const double* __restrict__ kvac, const double* __restrict__ kx,
-                                       const double* __restrict__ ky, const double* __restrict__ C,
-                                       const double* __restrict__ t, const double* __restrict__ t0,
-                                       const double* __restrict__ x, double* __restrict__ r, Red R, const __grid_constant__ Ctl ctl) {
-    const int w = K.w, h = K.h;
-    const size_t n = (size_t)w * h, stride = (size_t)gridDim.x * blockDim.x;
+// measures (heat.rs:413-447): rᵀD⁻¹r and the heat measure Σ (C/Δt)(r (dT/du) / D_ii)².
+// A thread walks down `rows` rows of a column (as spmv_dir_kernel does, and by the same rule): the iterate above and below
+// and the couplings between rows stay in registers, those across come from the next lanes, and the next row's operands
+// are in flight behind this row's arithmetic (a thread a cell: five loads of x and of the mask and two of each coupling;
+// 512²: 12.9 -> 11.0 us; 2048², beside the coarsening: 75).
+__global__ void __launch_bounds__(RED_THREADS, 2)
+    heat_residual64_kernel(HeatConst K, int rows, const double* __restrict__ scal, const uint8_t* __restrict__ gas,
+                           const double* __restrict__ kvac, const double* __restrict__ kx,
+                           const double* __restrict__ ky, const double* __restrict__ C, const double* __restrict__ t,
+                           const double* __restrict__ t0, const double* __restrict__ x, double* __restrict__ r, Red R,
+                           const __grid_constant__ Ctl ctl) {
+    const int w = K.w, h = K.h, lane = threadIdx.x & 31;
+    const int at = blockIdx.x * RED_THREADS + threadIdx.x, bands = (h + rows - 1) / rows;
+    const bool live = at < w * bands;
+    const int band = live ? at / w : 0, xx = live ? at - band * w : 0, y0 = band * rows;
     const double inv_dt = 1.0 / scal[S_DT], u_vac = u_of(K, K.t_floor);
     double rr = 0.0, bb = 0.0, gg = 0.0, hh = 0.0;
-    for (size_t base = (size_t)blockIdx.x * blockDim.x + threadIdx.x; base < n; base += 2 * stride) {
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const size_t i = base + u * stride;
-            if (i >= n) break;
-            int xx, y;
-            split_index(i, w, xx, y);
-            const bool gi = gas[i];
-            const bool gl = xx > 0 && gas[i - 1], gr = xx + 1 < w && gas[i + 1];
-            const bool gu = y > 0 && gas[i - w], gd = y + 1 < h && gas[i + w];
-            const double xi = x[i], kv = kvac[i], t0i = t0[i], Ci = C[i], ti = t[i];
-            const double xl = xx > 0 ? x[i - 1] : 0.0, xr = xx + 1 < w ? x[i + 1] : 0.0;
-            const double xu = y > 0 ? x[i - w] : 0.0, xd = y + 1 < h ? x[i + w] : 0.0;
-            const double kl = kx[(size_t)y * (w + 1) + xx], kr = kx[(size_t)y * (w + 1) + xx + 1];
-            const double ku = ky[(size_t)y * w + xx], kd = ky[(size_t)(y + 1) * w + xx];
-            if (!gi) {
-                r[i] = 0.0;
-                continue;
-            }
-            const CellSystem S = cell_system(K, inv_dt, u_vac, Ci, ti, t0i, kv);
-            double s = S.c * xi, d = S.c;
-            if (gl) {
-                s += kl * (xi - xl);
-                d += kl;
-            }
-            if (gr) {
-                s += kr * (xi - xr);
-                d += kr;
-            }
-            if (gu) {
-                s += ku * (xi - xu);
-                d += ku;
-            }
-            if (gd) {
-                s += kd * (xi - xd);
-                d += kd;
-            }
-            const double ri = S.rhs - s;
-            r[i] = ri;
-            rr += ri * ri;
-            bb += S.rhs * S.rhs;
-            const double rd = ri / d;  // FP64 divisions are what this kernel has few of to spend
-            gg += ri * rd;
-            const double e = rd * S.slope;
-            hh += S.heat * e * e;
+    // what lane 0 lacks on its left and lane 31 on its right
+    const int side = lane == 0 ? (xx > 0 ? -1 : 0) : (lane == 31 && xx + 1 < w ? 1 : 0);
+    struct Below {  // of the row below the one in work
+        double x, xs;
+        int g, gs;
+    };
+    auto below_at = [&](int y) {
+        const size_t i = (size_t)min(y, h - 1) * w + xx;
+        Below b;
+        b.x = x[i];
+        b.g = gas[i];
+        b.xs = side ? x[i + side] : 0.0;
+        b.gs = side ? gas[i + side] : 0;
+        return b;
+    };
+    struct Cell {
+        double kv, t0, C, t, kl, kr, kd;
+    };
+    auto cell_at = [&](int y) {
+        const size_t i = (size_t)min(y, h - 1) * w + xx, f = (size_t)min(y, h - 1) * (w + 1) + xx;
+        Cell c;
+        c.kv = kvac[i];
+        c.t0 = t0[i];
+        c.C = C[i];
+        c.t = t[i];
+        c.kl = kx[f];
+        c.kr = lane == 31 || xx + 1 == w ? kx[f + 1] : 0.0;
+        c.kd = ky[i + w];
+        return c;
+    };
+    double xu = y0 > 0 ? x[(size_t)(y0 - 1) * w + xx] : 0.0, ku = ky[(size_t)y0 * w + xx];
+    int gu = y0 > 0 && gas[(size_t)(y0 - 1) * w + xx];
+    Below c = below_at(y0), dn = below_at(y0 + 1);
+    Cell k = cell_at(y0);
+    for (int q = 0; q < rows; q++) {
+        const int y = y0 + q;
+        Below nb = dn;
+        Cell nk = k;
+        if (q + 1 < rows) {  // rows past the last are the last again, and leave nothing
+            nb = below_at(y + 2);
+            nk = cell_at(y + 1);
         }
+        double xl = __shfl_up_sync(0xffffffffu, c.x, 1), xr = __shfl_down_sync(0xffffffffu, c.x, 1);
+        double kr = __shfl_down_sync(0xffffffffu, k.kl, 1);
+        int gl = __shfl_up_sync(0xffffffffu, c.g, 1), gr = __shfl_down_sync(0xffffffffu, c.g, 1);
+        if (lane == 0) {
+            xl = c.xs;
+            gl = c.gs;
+        }
+        if (lane == 31) {
+            xr = c.xs;
+            gr = c.gs;
+        }
+        if (lane == 31 || xx + 1 == w) kr = k.kr;
+        if (xx == 0) gl = 0;
+        if (xx + 1 == w) gr = 0;
+        const bool gd = y + 1 < h && dn.g;
+        if (live && y < h) {
+            const size_t i = (size_t)y * w + xx;
+            if (!c.g) {
+                r[i] = 0.0;
+            } else {
+                const double xi = c.x;
+                const CellSystem S = cell_system(K, inv_dt, u_vac, k.C, k.t, k.t0, k.kv);
+                double s = S.c * xi, d = S.c;
+                if (gl) {
+                    s += k.kl * (xi - xl);
+                    d += k.kl;
+                }
+                if (gr) {
+                    s += kr * (xi - xr);
+                    d += kr;
+                }
+                if (gu) {
+                    s += ku * (xi - xu);
+                    d += ku;
+                }
+                if (gd) {
+                    s += k.kd * (xi - dn.x);
+                    d += k.kd;
+                }
+                const double ri = S.rhs - s;
+                r[i] = ri;
+                rr += ri * ri;
+                bb += S.rhs * S.rhs;
+                const double rd = ri / d;  // FP64 divisions are what this kernel has few of to spend
+                gg += ri * rd;
+                const double e = rd * S.slope;
+                hh += S.heat * e * e;
+            }
+        }
+        xu = c.x;
+        gu = c.g;
+        ku = k.kd;
+        c = dn;
+        dn = nb;
+        k = nk;
     }
     const double v[4] = {rr, bb, gg, hh};
     const bool last = grid_sum_last<4>(v, R.part, R.counter, R.out);
@@ -596,6 +650,8 @@ __global__ void scale_kernel(size_t n, const double* __restrict__ r64, const dou
     const bool last = grid_sum_last1(acc, R.part, R.counter, R.out);
     if (last && threadIdx.x == 0 && ctl.c) ctl_run(ctl, R.out - S_R32, C_INNER_BEGIN);
 }
+
+constexpr int ILP = 4;  // cells a thread takes a grid stride apart, all of their loads issued before the arithmetic
 
 // q = A p on level 0's FP32 operator in difference form, c p_i + Σ d (p_i - p_j); partials of <p, q>. ILP cells per
 // thread, loads first (masked cells have c = 1 and no couplings; the mask selects afterwards).
@@ -1256,7 +1312,7 @@ struct HeatSolver {
     // once: a CTA without a turn still takes a sum's ticket (512²: the SpMV 256 CTAs instead of 1,024), and a wave that
     // does not fill costs a whole one
     int grid_residual = 0, grid_newton = 0, grid_spmv = 0, grid_update = 0;
-    int spmv_rows = 1;
+    int spmv_rows = 1, residual_rows = 1;
     uint32_t precond = SR_PRECOND_MG;
     uint32_t max_passes = 128, max_rounds = 4096;
     double inner_floor = 1e-5;  // the smallest residual reduction asked of one inner FP32 solve
@@ -1476,7 +1532,7 @@ SolveResult solve_pass(HeatSolver* H, uint32_t precond, double tol, int max_roun
     double prev = INFINITY;
     const double ub = H->hscal[S_UB], tb = H->hscal[S_TB];
     for (int ref = 0; ref < 16; ref++) {
-        heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(K, H->scal, H->gas, H->kvac, H->kx, H->ky, H->C,
+        heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(K, H->residual_rows, H->scal, H->gas, H->kvac, H->kx, H->ky, H->C,
                                                                H->t, H->t0, H->x, H->r64, H->red(S_RR), Ctl{});
         sr_note_launch();
         H->read(S_RR, 4, s);
@@ -1601,7 +1657,7 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
                 nb[B_COARSEN] = capture_body(capture_conditional(H->cap[5], hd.h[B_COARSEN], cudaGraphCondTypeIf),
                                              H->cap[3], [&](cudaStream_t s3) { H->mg.coarsen(s3); });
                 SR_CUDA_TRY(cudaEventRecord(H->fork[1], H->cap[5]));
-                heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s2>>>(H->K, H->scal, H->gas, H->kvac, H->kx,
+                heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s2>>>(H->K, H->residual_rows, H->scal, H->gas, H->kvac, H->kx,
                                                                          H->ky, H->C, H->t, H->t0, H->x, H->r64, H->red(S_RR), ctl);
                 sr_note_launch();
                 SR_CUDA_TRY(cudaStreamWaitEvent(s2, H->fork[1], 0));
@@ -1715,12 +1771,15 @@ HeatSolver* heat_create(const sr_config& cfg, cudaStream_t s) {
         K.chi = cfg.chi;
         K.limiter_on = cfg.flux_limiter != 0;
         H->grid = grid_for(H->n);
-        H->grid_residual = whole_waves(heat_residual64_kernel, H->n / 2);
         H->grid_newton = whole_waves(newton_system_kernel, H->n / 2);
-        // rows a thread of the SpMV: as few as leave its threads room on the GPU all at once
-        const int w4 = H->w / 4, most = whole_waves(spmv_dir_kernel, H->n) * RED_THREADS;
-        H->spmv_rows = (H->h + std::max(1, most / w4) - 1) / std::max(1, most / w4);
-        H->grid_spmv = grid_for((size_t)w4 * ((H->h + H->spmv_rows - 1) / H->spmv_rows));
+        // rows a thread of the kernels that walk: as few as leave their threads room on the GPU all at once
+        auto walk = [&](auto kernel, int columns, int& rows, int& grid) {
+            const int bands = std::max(1, whole_waves(kernel, H->n) * RED_THREADS / columns);
+            rows = (H->h + bands - 1) / bands;
+            grid = grid_for((size_t)columns * ((H->h + rows - 1) / rows));
+        };
+        walk(spmv_dir_kernel, H->w / 4, H->spmv_rows, H->grid_spmv);
+        walk(heat_residual64_kernel, H->w, H->residual_rows, H->grid_residual);
         H->grid_update = whole_waves(pcg_update4_kernel, H->n / 4);
         const size_t n = H->n, nx = (size_t)(H->w + 1) * H->h, ny = (size_t)H->w * (H->h + 1);
         SR_CUDA_TRY(cudaMalloc(&H->gas, n));
@@ -1825,7 +1884,7 @@ int heat_collect(HeatSolver* H, Learner* L, const float* U, const float* kappa, 
     H->read(S_HEAT0, 2, s);
     H->n_gas = (int)H->hscal[S_NGAS];
     build_system(H, dt, s);
-    heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(H->K, H->scal, H->gas, H->kvac, H->kx, H->ky, H->C,
+    heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s>>>(H->K, H->residual_rows, H->scal, H->gas, H->kvac, H->kx, H->ky, H->C,
                                                            H->t, H->t0, H->x, H->r64, H->red(S_RR), Ctl{});
     sr_note_launch();
     H->read(S_RR, 1, s);
