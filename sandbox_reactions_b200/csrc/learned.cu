@@ -123,6 +123,13 @@ struct ConvShape {
     static constexpr size_t SMEM = SB + SI + 32 + 4 * COUT_P;
 };
 
+// A CTA takes tiles in turn once there are more than ten an SM: a CTA a tile was bound by the rate at which the GPU starts
+// CTAs (512², 8 -> 8 channels: 2,048 CTAs of 2.7 us, of which 3.7 an SM ran at a time where 12 fit; with six an SM 12.5 ->
+// 11.1 us). A layer's launch overlaps the one before (the network's fifteen are 6 to 12 us each): both together, a 512²
+// world with the learned preconditioner 5.94 -> 5.65 ms a step, a 16 x 64² batch's loss_grad 600 -> 581 us; six, eight and
+// twelve an SM are within 1 % of ten.
+constexpr int CONV_CTAS = 10 * 148;
+
 template <int CIN_P, int COUT_P>
 __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
     using S = ConvShape<CIN_P, COUT_P>;
@@ -137,9 +144,12 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
     const int tid = threadIdx.x, warp = tid >> 5;
     constexpr uint32_t IDESC = tc::idesc_bf16_f32(128, S::NM);
 
+    // The next convolution may start (its own set-up and weights, fixed here, then wait for this one's output) once this
+    // one's CTAs hold their TMEM: one of its CTAs never keeps the columns that one of these waits for.
     if (warp == 0) {
         tc::tmem_alloc(tbase, S::NCOLS);
         tc::tmem_relinquish();
+        pdl_launch();
     }
     // the weight image by one bulk copy, behind the halo's loads (by the threads' own loads and stores, up to 36 a thread
     // before the first of the halo: 64 -> 64 channels at 64², 18.6 -> 10.4 us; 32 -> 32 at 128², 10.8 -> 6.8)
@@ -155,13 +165,26 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
         for (int i = tid; i < (int)((S::SB - S::SBG) / 16); i += 128) d[i] = make_int4(0, 0, 0, 0);
     }
     if (tid < COUT_P) sbias[tid] = A.bias && tid < A.cout_real ? A.bias[tid] : 0.0f;
-    const int img = blockIdx.z, X0 = blockIdx.x * TW, Y0 = blockIdx.y * TH;
+    const int tx = (A.W + TW - 1) / TW, ty = (A.H + TH - 1) / TH, tiles = tx * ty * A.B;
+    int img = 0, X0 = 0, Y0 = 0;  // where the tile last gathered lies
+    auto place = [&](int tile) {
+        img = 0;
+        int rem = tile;
+        if (A.B > 1) {
+            img = tile / (tx * ty);
+            rem = tile - img * (tx * ty);
+        }
+        const int row = rem / tx;
+        X0 = (rem - row * tx) * TW;
+        Y0 = row * TH;
+    };
     // the halo tile, through the input transform (zero outside the image), as BF16; a thread's items in batches of
-    // six, all of a batch's loads issued before any conversion
+    // six, all of a batch's loads issued before any conversion; where one batch is all, the next tile's are issued before
+    // this tile's product is waited for
     constexpr int NI = (HP * G + 127) / 128, NB = NI < 6 ? NI : 6;
-#pragma unroll
-    for (int i0 = 0; i0 < NI; i0 += NB) {
-        float v[NB][8];
+    constexpr bool AHEAD = NI <= 3;
+    float v[NB][8];
+    auto gather = [&](int i0) {
 #pragma unroll
         for (int u = 0; u < NB; u++) {
             const int e = tid + (i0 + u) * 128;
@@ -171,6 +194,8 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
                 conv_input<CIN_P>(A, img, Y0 + hy - 1, X0 + hx - 1, g * 8, v[u]);
             }
         }
+    };
+    auto put = [&](int i0) {
 #pragma unroll
         for (int u = 0; u < NB; u++) {
             const int e = tid + (i0 + u) * 128;
@@ -186,70 +211,91 @@ __global__ void __launch_bounds__(128) conv_tc_kernel(ConvArgs A) {
                 *reinterpret_cast<uint4*>(sIn + g * HPLANE + hp * 16) = packed;
             }
         }
-    }
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tmem = *tbase;
-    bool weights = true;
-    if (tid == 0) {
-        weights = tc::mbar_wait(wbar, 0u, kWaitLimit);
-        if (!weights) {  // no commit follows: every thread's wait below gives up
-            atomicExch(A.err, 1);
-            tc::mbar_wait(wbar, 0u, kWaitLimit);  // a copy still in flight lands before the CTA leaves
-        }
-    }
-    if (tid == 0 && weights) {
-        const uint32_t a0 = tc::smem_addr(sIn), b0 = tc::smem_addr(sB);
+    };
+    pdl_wait();
+    place(blockIdx.x);
+    if (AHEAD) gather(0);
+    uint32_t tmem = 0;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, it++) {
+        if constexpr (AHEAD) {
+            put(0);
+        } else {
 #pragma unroll
-        for (int ks = 0; ks < S::KT / 16; ks++) {
-            uint32_t at, lbo;  // the A operand's first core matrix, and the distance to the one 8 of K on
-            if constexpr (CIN_P == 8) {
-                // taps 2 ks and 2 ks + 1; the last MMA is tap 7 again, against zero weights, and tap 8
-                const int t0 = ks < 4 ? 2 * ks : 7, t1 = t0 + 1;
-                const int p0 = (t0 / 3) * HW_ + t0 % 3, p1 = (t1 / 3) * HW_ + t1 % 3;
-                at = a0 + 16 * p0;
-                lbo = 16 * (p1 - p0);
-            } else {
-                const int tap = ks / (CIN_P / 16), g = 2 * (ks % (CIN_P / 16));
-                at = a0 + g * HPLANE + 16 * ((tap / 3) * HW_ + tap % 3);
-                lbo = HPLANE;
+            for (int i0 = 0; i0 < NI; i0 += NB) {
+                gather(i0);
+                put(i0);
             }
-            const uint64_t ad = tc::desc_kmajor(at, lbo, 16 * HW_);
-            const uint64_t bd = tc::desc_kmajor(b0 + 2 * ks * 128, 128, S::KT * 16);
-            tc::mma_bf16(tmem, ad, bd, IDESC, ks > 0);
         }
-        tc::mma_commit(mbar);
-    }
-    const bool ok = tc::mbar_wait(mbar, 0u, kWaitLimit);
-    tc::fence_after_sync();
-    const int x = X0 + tid % TW, y = Y0 + tid / TW;
-    const bool valid = x < A.W && y < A.H;
-    float acc[COUT_P];
-#pragma unroll
-    for (int c0 = 0; c0 < COUT_P; c0 += 8) tc::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc + c0);
-    tc::tmem_wait_ld();
-    if (!ok) atomicExch(A.err, 1);
-    if (valid && ok) {
-        const size_t at = ((((size_t)img * A.H + y) * A.W) + x) * COUT_P;
-#pragma unroll
-        for (int c0 = 0; c0 < COUT_P; c0 += 4) {
-            float4 q;
-            float* qq = reinterpret_cast<float*>(&q);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int co = c0 + j;
-                float v = acc[co] + sbias[co];
-                if (A.relu) v = fmaxf(v, 0.0f);
-                qq[j] = v;
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        __syncthreads();
+        tc::fence_after_sync();
+        tmem = *tbase;
+        bool weights = true;
+        if (tid == 0 && it == 0) {
+            weights = tc::mbar_wait(wbar, 0u, kWaitLimit);
+            if (!weights) {  // no commit follows: every thread's wait below gives up
+                atomicExch(A.err, 1);
+                tc::mbar_wait(wbar, 0u, kWaitLimit);  // a copy still in flight lands before the CTA leaves
             }
-            *reinterpret_cast<float4*>(A.out + at + c0) = q;
-            if (A.out2) *reinterpret_cast<float4*>(A.out2 + at + c0) = q;
         }
+        if (tid == 0 && weights) {
+            const uint32_t a0 = tc::smem_addr(sIn), b0 = tc::smem_addr(sB);
+#pragma unroll
+            for (int ks = 0; ks < S::KT / 16; ks++) {
+                uint32_t at, lbo;  // the A operand's first core matrix, and the distance to the one 8 of K on
+                if constexpr (CIN_P == 8) {
+                    // taps 2 ks and 2 ks + 1; the last MMA is tap 7 again, against zero weights, and tap 8
+                    const int t0 = ks < 4 ? 2 * ks : 7, t1 = t0 + 1;
+                    const int p0 = (t0 / 3) * HW_ + t0 % 3, p1 = (t1 / 3) * HW_ + t1 % 3;
+                    at = a0 + 16 * p0;
+                    lbo = 16 * (p1 - p0);
+                } else {
+                    const int tap = ks / (CIN_P / 16), g = 2 * (ks % (CIN_P / 16));
+                    at = a0 + g * HPLANE + 16 * ((tap / 3) * HW_ + tap % 3);
+                    lbo = HPLANE;
+                }
+                const uint64_t ad = tc::desc_kmajor(at, lbo, 16 * HW_);
+                const uint64_t bd = tc::desc_kmajor(b0 + 2 * ks * 128, 128, S::KT * 16);
+                tc::mma_bf16(tmem, ad, bd, IDESC, ks > 0);
+            }
+            tc::mma_commit(mbar);
+        }
+        const int at_img = img, x = X0 + tid % TW, y = Y0 + tid / TW, next = tile + (int)gridDim.x;
+        if (next < tiles) {
+            place(next);
+            if (AHEAD) gather(0);
+        }
+        const bool ok = tc::mbar_wait(mbar, it & 1, kWaitLimit);
+        tc::fence_after_sync();
+        const bool valid = x < A.W && y < A.H;
+        float acc[COUT_P];
+#pragma unroll
+        for (int c0 = 0; c0 < COUT_P; c0 += 8) tc::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc + c0);
+        tc::tmem_wait_ld();
+        if (!ok) atomicExch(A.err, 1);
+        if (valid && ok) {
+            const size_t at = ((((size_t)at_img * A.H + y) * A.W) + x) * COUT_P;
+#pragma unroll
+            for (int c0 = 0; c0 < COUT_P; c0 += 4) {
+                float4 q;
+                float* qq = reinterpret_cast<float*>(&q);
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int co = c0 + j;
+                    float r = acc[co] + sbias[co];
+                    if (A.relu) r = fmaxf(r, 0.0f);
+                    qq[j] = r;
+                }
+                *reinterpret_cast<float4*>(A.out + at + c0) = q;
+                if (A.out2) *reinterpret_cast<float4*>(A.out2 + at + c0) = q;
+            }
+        }
+        tc::fence_before_sync();
+        // the product is read and the halo free; a CTA one of whose waits gave up takes no further tile
+        if (__syncthreads_or(!ok)) break;
     }
-    tc::fence_before_sync();
-    __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, S::NCOLS);
 }
 
@@ -276,8 +322,9 @@ void conv_attributes() {
 template <int CI, int CO>
 void launch_conv_t(const ConvArgs& A, cudaStream_t s) {
     using S = ConvShape<CI, CO>;
-    const dim3 grid((unsigned)((A.W + TW - 1) / TW), (unsigned)((A.H + TH - 1) / TH), (unsigned)A.B);
-    conv_tc_kernel<CI, CO><<<grid, 128, S::SMEM, s>>>(A);
+    const int tiles = ((A.W + TW - 1) / TW) * ((A.H + TH - 1) / TH) * A.B;
+    const int each = (tiles + CONV_CTAS - 1) / CONV_CTAS;  // tiles a CTA, as evenly as they go
+    launch_kernel(true, conv_tc_kernel<CI, CO>, dim3((tiles + each - 1) / each), dim3(128), S::SMEM, s, A);
     sr_note_launch();
 }
 

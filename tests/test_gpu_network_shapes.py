@@ -1,5 +1,6 @@
-"""The network's kernels at batches and crops whose tiles are ragged at some level: the forward pass and every gradient
-against the f64 network with the same BF16 rounding of the convolutions' operands.
+"""The network's kernels at batches and crops whose tiles are ragged at some level, and at one with more tiles than run
+at once: the forward pass and every gradient against the f64 network with the same BF16 rounding of the convolutions'
+operands.
 
 The bound: the kernels accumulate in FP32, so an activation near a rounding boundary may round to the other BF16
 neighbour. It then lies one spacing from the oracle's operand, twice the half spacing that a rounding moves an operand at
@@ -20,7 +21,7 @@ def rel_l2(a, b):
     return np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-300)
 
 
-@pytest.mark.parametrize("crop,n", [(16, 1), (40, 3), (88, 2), (136, 1)])
+@pytest.mark.parametrize("crop,n", [(16, 1), (40, 3), (88, 2), (136, 1), (360, 2)])
 def test_the_network_at_ragged_tiles(crop, n):
     rng = np.random.default_rng(crop + n)
     theta = unet.init_params(3)
