@@ -53,12 +53,20 @@ struct HeatConst {
 // The host-driven step (heat_step's Newton loop, solve_pass's FP64 refinement, inner_pcg's rounds) decides from
 // read-back scalars. Here the same decisions are taken on the device, inside one captured CUDA graph, and steer its
 // conditional nodes: an IF around the step (no gas, pinned temperature or Δt <= 0 leave only the fluxes), a WHILE over
-// the Newton passes, a WHILE over a pass's refinements, an IF around each inner solve, a WHILE over its PCG rounds (the
-// residual tested after every round: no host round trip, no predicted cadence), an IF around the next pass's coarsening,
-// and IFs choosing the commit. A decision is taken by the thread that has just written the sums it reads, the last CTA's
-// of the kernel whose grid sum it is (ctl_run): decisions in one-thread kernels of their own cost 3.5 us each with their
-// launch gap, 250 of them in three 2048² steps and 1,050 in four 512² reference-mode steps. No launch argument changes
-// from step to step: Δt, the scale, δ and the round state live in the device scalars.
+// the refinements of all Newton passes (an FP64 residual, an inner solve, and after a pass's last the Newton update), a
+// WHILE over an inner solve's PCG rounds (the residual tested after every round: no host round trip, no predicted
+// cadence), an IF around a new system's coarsening, and IFs choosing the commit. Entering a body costs 4 to 8 us, more
+// than most of its kernels, so a kernel that may have nothing to do this time (the inner solve's scaling and correction,
+// the Newton update) reads that and leaves instead of having a body of its own (a WHILE of passes around a WHILE of
+// refinements, an IF around each inner solve and each Newton update: 2048², three steps, 30.5 -> 29.9 ms). A decision is
+// taken by the thread that has just written the sums it reads, the last CTA's of the kernel whose grid sum it is
+// (ctl_run): decisions in one-thread kernels of their own cost 3.5 us each with their launch gap, 250 of them in three
+// 2048² steps and 1,050 in four 512² reference-mode steps. No launch argument changes from step to step: Δt, the scale, δ
+// and the round state live in the device scalars.
+
+// The graph's conditional bodies.
+enum CtlBody { B_MAIN, B_SKIP, B_LOOP, B_ROUND, B_COARSEN, B_CONV, B_LIM, B_COUNT };
+
 struct HeatCtl {
     // configuration (host-written)
     double tol, nheat, ncell, inner_floor;
@@ -70,12 +78,12 @@ struct HeatCtl {
     // the pass's refinement and its inner solve
     int ref, reached, it, max_it;
     double prev, eta, rr0;
+    int newton;  // the loop body's Newton update has work this time
     // the commit
     double delta, radiated;
     // how often each body ran since the host last counted (for the launch count)
-    unsigned long long runs[10];
+    unsigned long long runs[B_COUNT];
 };
-enum CtlBody { B_MAIN, B_SKIP, B_PASS, B_REFINE, B_INNER, B_ROUND, B_NSYS, B_COARSEN, B_CONV, B_LIM, B_COUNT };
 
 struct CtlHandles {
     cudaGraphConditionalHandle h[B_COUNT];
@@ -102,19 +110,17 @@ __device__ __forceinline__ void ctl_commit(const Ctl& k) {
 }
 
 __device__ __forceinline__ void ctl_pass_begin(const Ctl& k) {
-    k.c->runs[B_PASS]++;
     k.c->passes++;
     k.c->ref = 0;
     k.c->prev = INFINITY;
-    ctl_set(k, B_REFINE, true, false);
+    ctl_set(k, B_LOOP, true, false);
 }
 
 // The pass's solve is done: its Newton update, unless the solve broke down.
 __device__ __forceinline__ void ctl_refine_end(const Ctl& k) {
-    ctl_set(k, B_REFINE, false, false);
-    ctl_set(k, B_NSYS, k.c->ok != 0, true);
+    k.c->newton = k.c->ok;
     if (!k.c->ok) {
-        ctl_set(k, B_PASS, false, false);
+        ctl_set(k, B_LOOP, false, false);
         ctl_commit(k);
     }
 }
@@ -134,7 +140,7 @@ __device__ __forceinline__ void ctl_inner_end(const Ctl& k) {
         }
     }
     if (++c->ref >= kMaxRefinements) more = false;
-    if (more) ctl_set(k, B_REFINE, true, false);
+    if (more) ctl_set(k, B_LOOP, true, false);
     else ctl_refine_end(k);
 }
 
@@ -161,13 +167,14 @@ __device__ __noinline__ void ctl_run(const Ctl& k, double* scal, int phase) {
             c->moved_prev = 0.0;
             const bool go = c->max_passes > 0 && c->max_rounds > 0;
             ctl_set(k, B_COARSEN, go, true);
-            ctl_set(k, B_PASS, go, false);
+            ctl_set(k, B_LOOP, go, false);
             if (go) ctl_pass_begin(k);
             else ctl_commit(k);
             break;
         }
         case C_REFINE: {  // after the FP64 residual: stop, or scale the residual for an inner solve
-            c->runs[B_REFINE]++;
+            c->runs[B_LOOP]++;
+            c->newton = 0;
             const double rr = scal[S_RR], bb = scal[S_BB], gam = scal[S_GAM], hm = scal[S_HM];
             bool go = false;
             if (!isfinite(rr) || !isfinite(bb) || !isfinite(gam) || !isfinite(hm)) {
@@ -188,8 +195,11 @@ __device__ __noinline__ void ctl_run(const Ctl& k, double* scal, int phase) {
                     go = true;
                 }
             }
-            ctl_set(k, B_INNER, go, true);
-            if (!go) ctl_refine_end(k);
+            if (!go) {
+                scal[S_SCALE] = scal[S_ISCALE] = 0.0;
+                ctl_set(k, B_ROUND, false, false);
+                ctl_refine_end(k);
+            }
             break;
         }
         case C_INNER_BEGIN: {  // after the scaled residual
@@ -242,7 +252,7 @@ __device__ __noinline__ void ctl_run(const Ctl& k, double* scal, int phase) {
                 more = c->passes < c->max_passes && c->rounds < c->max_rounds;
             }
             ctl_set(k, B_COARSEN, more, true);
-            ctl_set(k, B_PASS, more, false);
+            ctl_set(k, B_LOOP, more, false);
             if (more) ctl_pass_begin(k);
             else ctl_commit(k);
             break;
@@ -640,6 +650,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2)
 __global__ void scale_kernel(size_t n, const double* __restrict__ r64, const double* __restrict__ scal, float* r32,
                              float* e32, Red R, const __grid_constant__ Ctl ctl) {
     const double inv_scale = scal[S_ISCALE];
+    if (inv_scale == 0.0) return;  // the captured loop: no inner solve this time
     double acc = 0.0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float v = (float)(r64[i] * inv_scale);
@@ -1031,6 +1042,7 @@ __global__ void add_dot_kernel(size_t n, const float* __restrict__ r, const floa
 __global__ void correction_kernel(size_t n, const uint8_t* __restrict__ gas, const float* __restrict__ e,
                                   const double* __restrict__ scal, double* x) {
     const double scale = scal[S_SCALE];
+    if (scale == 0.0) return;  // no inner solve, or one that broke down
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         if (gas[i]) x[i] += scale * (double)e[i];
 }
@@ -1043,6 +1055,7 @@ __global__ void newton_system_kernel(HeatConst K, double cell_tol, const double*
                                      const uint8_t* __restrict__ gas,
                                      const double* __restrict__ C, const double* __restrict__ kvac, double* t, double* x,
                                      float* c0, Red R, const __grid_constant__ Ctl ctl) {
+    if (ctl.c && !ctl.c->newton) return;
     const size_t n = (size_t)K.w * K.h, stride = (size_t)gridDim.x * blockDim.x;
     const double u_vac = u_of(K, K.t_floor);
     const double dt = scal[S_DT];
@@ -1646,45 +1659,40 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
         heat_system_kernel<<<H->grid, RED_THREADS, 0, s0>>>(H->K, H->scal, H->gas, H->C, H->t, H->kvac,
                                                             H->mg.L[0].c, H->x, H->red(S_UB), ctl);
         sr_note_launch();
-        nb[B_PASS] = capture_body(capture_conditional(s0, hd.h[B_PASS], cudaGraphCondTypeWhile), H->cap[1],
+        nb[B_LOOP] = capture_body(capture_conditional(s0, hd.h[B_LOOP], cudaGraphCondTypeWhile), H->cap[1],
                                   [&](cudaStream_t s1) {
-            nb[B_REFINE] = capture_body(capture_conditional(s1, hd.h[B_REFINE], cudaGraphCondTypeWhile), H->cap[2],
-                                        [&](cudaStream_t s2) {
-                // a new system's coarse levels beside its first FP64 residual: a chain of small kernels (39 us of
-                // latency at 512², 95 at 2048²) and one that takes the whole GPU, neither of which the other needs
-                SR_CUDA_TRY(cudaEventRecord(H->fork[0], s2));
-                SR_CUDA_TRY(cudaStreamWaitEvent(H->cap[5], H->fork[0], 0));
-                nb[B_COARSEN] = capture_body(capture_conditional(H->cap[5], hd.h[B_COARSEN], cudaGraphCondTypeIf),
-                                             H->cap[3], [&](cudaStream_t s3) { H->mg.coarsen(s3); });
-                SR_CUDA_TRY(cudaEventRecord(H->fork[1], H->cap[5]));
-                heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s2>>>(H->K, H->residual_rows, H->scal, H->gas, H->kvac, H->kx,
-                                                                         H->ky, H->C, H->t, H->t0, H->x, H->r64, H->red(S_RR), ctl);
+            // a new system's coarse levels beside its first FP64 residual: a chain of small kernels (39 us of latency at
+            // 512², 95 at 2048²) and one that takes the whole GPU, neither of which the other needs
+            SR_CUDA_TRY(cudaEventRecord(H->fork[0], s1));
+            SR_CUDA_TRY(cudaStreamWaitEvent(H->cap[5], H->fork[0], 0));
+            nb[B_COARSEN] = capture_body(capture_conditional(H->cap[5], hd.h[B_COARSEN], cudaGraphCondTypeIf),
+                                         H->cap[2], [&](cudaStream_t s2) { H->mg.coarsen(s2); });
+            SR_CUDA_TRY(cudaEventRecord(H->fork[1], H->cap[5]));
+            heat_residual64_kernel<<<H->grid_residual, RED_THREADS, 0, s1>>>(
+                H->K, H->residual_rows, H->scal, H->gas, H->kvac, H->kx, H->ky, H->C, H->t, H->t0, H->x, H->r64,
+                H->red(S_RR), ctl);
+            sr_note_launch();
+            SR_CUDA_TRY(cudaStreamWaitEvent(s1, H->fork[1], 0));
+            scale_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32), ctl);
+            sr_note_launch();
+            nb[B_ROUND] = capture_body(capture_conditional(s1, hd.h[B_ROUND], cudaGraphCondTypeWhile), H->cap[2],
+                                       [&](cudaStream_t s2) {
+                precondition(H, precond, S_RZN, false, s2);
+                spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s2>>>(
+                    H->mg.L[0], H->spmv_rows, H->scal, H->z32, H->p32, H->p2, H->q32, H->pq_part, H->rz_part,
+                    precond == SR_PRECOND_MG ? H->mg.parts() : 0);
                 sr_note_launch();
-                SR_CUDA_TRY(cudaStreamWaitEvent(s2, H->fork[1], 0));
-                nb[B_INNER] = capture_body(capture_conditional(s2, hd.h[B_INNER], cudaGraphCondTypeIf), H->cap[3],
-                                           [&](cudaStream_t s3) {
-                    scale_kernel<<<H->grid, RED_THREADS, 0, s3>>>(H->n, H->r64, H->scal, H->r32, H->e32, H->red(S_R32), ctl);
-                    sr_note_launch();
-                    nb[B_ROUND] = capture_body(capture_conditional(s3, hd.h[B_ROUND], cudaGraphCondTypeWhile), H->cap[4],
-                                               [&](cudaStream_t s4) {
-                        precondition(H, precond, S_RZN, false, s4);
-                        spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s4>>>(H->mg.L[0], H->spmv_rows, H->scal, H->z32, H->p32, H->p2,
-                                                                          H->q32, H->pq_part, H->rz_part,
-                                                    precond == SR_PRECOND_MG ? H->mg.parts() : 0);
-                        sr_note_launch();
-                        pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s4>>>(H->n, H->scal, H->pq_part, H->grid_spmv, H->p32, H->p2, H->q32,
-                                                                             H->e32, H->r32, H->red(S_RRI), ctl);
-                        sr_note_launch();
-                    });
-                    correction_kernel<<<H->grid, RED_THREADS, 0, s3>>>(H->n, H->gas, H->e32, H->scal, H->x);
-                    sr_note_launch();
-                });
-            });
-            nb[B_NSYS] = capture_body(capture_conditional(s1, hd.h[B_NSYS], cudaGraphCondTypeIf), H->cap[2],
-                                      [&](cudaStream_t s2) {
-                newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s2>>>(H->K, H->cfg.newton_cell, H->scal, H->gas, H->C, H->kvac, H->t, H->x, H->mg.L[0].c, H->red(S_MOVED), ctl);
+                pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s2>>>(H->n, H->scal, H->pq_part, H->grid_spmv,
+                                                                          H->p32, H->p2, H->q32, H->e32, H->r32,
+                                                                          H->red(S_RRI), ctl);
                 sr_note_launch();
             });
+            correction_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->n, H->gas, H->e32, H->scal, H->x);
+            sr_note_launch();
+            newton_system_kernel<<<H->grid_newton, RED_THREADS, 0, s1>>>(H->K, H->cfg.newton_cell, H->scal, H->gas, H->C,
+                                                                        H->kvac, H->t, H->x, H->mg.L[0].c,
+                                                                        H->red(S_MOVED), ctl);
+            sr_note_launch();
         });
         nb[B_CONV] = capture_body(capture_conditional(s0, hd.h[B_CONV], cudaGraphCondTypeIf), H->cap[1],
                                   [&](cudaStream_t s1) {
