@@ -42,9 +42,9 @@ sys.path.insert(0, ROOT)
 METRIC = "Mcell-steps/s hydro+grav+FLD @2048²; FLD time-to-1e-8: learned vs MG-PCG"
 UNIT = "Mcell-steps/s"
 BREAKDOWN_STEPS = 2  # steps of the per-pass timing leg (passes launched one by one) after the timed steps
-# algorithmic bytes per cell of the fused hydro update kernel with gravity: state in 16 + out 16, P2's g 8,
-# the half-step source 4, φ_mid 4 and g_mid 8
-HYDRO_UPDATE_BYTES_PER_CELL = 56
+# algorithmic bytes per cell of the hydro kernel of a step with gravity: state in 16 + out 16, P2's g 8, the half step's
+# source 4 and its Σ, Σu, Σv 12, the mass fluxes 8
+HYDRO_UPDATE_BYTES_PER_CELL = 64
 # the multigrid's level-0 smoothers, the step's dominant kernels (per cell of level 0): the pre-smoother reads
 # b, c, dx, dy (16) and the mask (1) and writes x (4) and the coarse right-hand side (4 per 2x2 aggregate: 1);
 # the post-smoother reads x, b, c, dx, dy (20), the mask (1) and the coarse correction (1) and writes x2 (4)
@@ -389,7 +389,7 @@ def fld_system_checks(cfg, P, kappa, x_mg) -> dict:
 def config_runs(peak_gbs: float):
     """The other single-GPU configurations as side measurements (device time of the steps, library events): C1, the
     Sod tube at 512² with minmod (hydro only, 200 steps), and C2, the disk at 1024² with its FFT gravity (100 steps);
-    each with its hydro update kernel's HBM roofline (32 B/cell without gravity, 56 B/cell with) and its parity: one
+    each with its hydro update kernel's HBM roofline (32 B/cell without gravity, 64 B/cell with) and its parity: one
     GPU step against the oracle's step from the same f32 start (bar 1e-5 per field); for C1 also the 200 steps against
     the twin's (the reference's G-REF band, 1e-3), for C2 the start state's potential against an f64 direct sum on a
     128² subsample of target cells."""
@@ -402,7 +402,7 @@ def config_runs(peak_gbs: float):
     O.set_threads(os.cpu_count() or 1)
     out = {}
     for name, (cfg, P), steps, bpc in (("C1_sod_512_minmod", scenes.sod(512), 200, 32),
-                                       ("C2_disk_hydro_grav_1024", scenes.disk(1024), 100, 56)):
+                                       ("C2_disk_hydro_grav_1024", scenes.disk(1024), 100, HYDRO_UPDATE_BYTES_PER_CELL)):
         with Step(cfg) as s:
             s.upload(P)
             phi = s.gravity_field()[0] if cfg.gravity else None
@@ -737,10 +737,10 @@ def main():
                     "algorithmic_bytes_per_cell": {"pre": SMOOTH_PRE_BYTES_PER_CELL,
                                                    "post": SMOOTH_POST_BYTES_PER_CELL},
                     "peak_kind": "burst copy bandwidth (kernels timed alone)",
-                    "other": {"hydro_band_kernel<kHydroUpdateGrav>": {
+                    "other": {"hydro_band_kernel<kHydroPredict>": {
                         "achieved": upd_gbs, "frac": upd_gbs / peak, "ms_per_launch": upd_ms,
                         "algorithmic_bytes_per_cell": HYDRO_UPDATE_BYTES_PER_CELL,
-                        "traffic": committed_traffic("hydro_update", n * n)}}}
+                        "traffic": committed_traffic("hydro_predict", n * n)}}}
         clocks = sampler.summary()
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,

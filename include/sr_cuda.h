@@ -227,8 +227,8 @@ typedef struct sr_box_report {
 sr_status sr_read_box(sr_ctx* ctx, sr_box_report* out);
 
 /* Step::set_timing / read_cost (step/mod.rs:722-777). `on`: 0 off; 1 each step's device time (total_ms) as the steps
- * normally run — after the first step, one captured graph per step — with the per-pass fields left 0; 2 the per-pass
- * breakdown, the passes launched one by one (the implicit step still one captured graph after the first step). */
+ * normally run — one captured graph per step, or a gas-only step's one kernel — with the per-pass fields left 0; 2 the
+ * per-pass breakdown, the passes launched one by one (the implicit step still one captured graph). */
 sr_status sr_set_timing(sr_ctx* ctx, int32_t on);
 sr_status sr_read_cost(sr_ctx* ctx, sr_cost* out);
 
