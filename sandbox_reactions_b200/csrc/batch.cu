@@ -4,9 +4,8 @@
 // batch's stream it forks to every world's stream, each branch holds that world's whole step — P1 to P9, the implicit
 // step under device control with its conditional loops — and the branches join again. The graph is captured once per
 // combination of the worlds' state buffers (two, as the worlds alternate them in step) and replayed; the worlds'
-// kernels interleave on the device with no host decision between them. Until then (the first step, or a world whose
-// step cannot be captured: the learned preconditioner) the worlds step on a pool of host threads, one context per
-// world, balanced by cell count.
+// kernels interleave on the device with no host decision between them. With a world whose step cannot be captured (the
+// learned preconditioner) the worlds step on a pool of host threads, one context per world, balanced by cell count.
 #include <map>
 #include <algorithm>
 #include <condition_variable>
@@ -36,7 +35,7 @@ struct sr_batch {
 };
 
 extern "C" cudaStream_t sr_ctx_stream(sr_ctx* c);
-long long sr_ctx_capture_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t root);
+long long sr_ctx_capture_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t root, bool alone);
 bool sr_ctx_prepare_capture(sr_ctx* c);
 void sr_ctx_graph_steps_done(sr_ctx* c, uint32_t steps, long long launches_per_step);
 sr_status sr_ctx_after_steps(sr_ctx* c);
@@ -93,7 +92,7 @@ BatchGraph* batch_graph(sr_batch* b) {
         for (size_t i = 0; i < b->ctx.size(); i++) {
             cudaStream_t ws = sr_ctx_stream(b->ctx[i]);
             SR_CUDA_TRY(cudaStreamWaitEvent(ws, b->start_fork, 0));
-            bg.launches.push_back(sr_ctx_capture_step(b->ctx[i], key[i], ws, g));
+            bg.launches.push_back(sr_ctx_capture_step(b->ctx[i], key[i], ws, g, false));
             bg.generation.push_back(sr_ctx_generation(b->ctx[i]));
             SR_CUDA_TRY(cudaEventRecord(b->done[i], ws));
             SR_CUDA_TRY(cudaStreamWaitEvent(b->join, b->done[i], 0));

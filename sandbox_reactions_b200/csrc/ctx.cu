@@ -347,10 +347,10 @@ static HydroArgs hydro_args(sr_ctx* c, int cur) {
 
 // One step's launches on `s` from state buffer `cur`, in the reference's pass order P1 → P2 → P4 → P5 → P8 → P9
 // (reference/mod.rs:264-297). With `root` the launches are captured into that graph and P5 is the device-controlled
-// step (heat_capture_step); otherwise they run now, P5 by heat_step. `mark(slot)` is called at the pass boundaries
+// step (heat_capture_step; `alone`: not among a batch's worlds); otherwise they run now, P5 by heat_step. `mark(slot)` is called at the pass boundaries
 // (0 start, 1 after P2, 2 hydro update start, 3 its end, 4 after P4, 5 after P5, 6 after P8/P9).
 template <class Mark>
-static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t root, Mark mark) {
+static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t root, bool alone, Mark mark) {
     long long heat_top = 0;  // kernels of a captured implicit step outside its loops
     const sr_config& k = c->cfg;
     float* U = c->U[cur];
@@ -377,7 +377,7 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
         }
         mark(4);
         if (k.heat) {
-            if (root) heat_top = heat_capture_step(c->heat, U, nullptr, &c->rec->dt_next, s, root);
+            if (root) heat_top = heat_capture_step(c->heat, U, nullptr, &c->rec->dt_next, s, root, alone);
             else heat_step(c->heat, U, nullptr, &c->rec->dt_next, s, &c->heat_report);
             const float *fx, *fy;
             heat_flux_planes(c->heat, &fx, &fy);
@@ -417,7 +417,7 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
     mark(4);
     if (k.heat) {
         const float* kappa = k.opacity_plane ? c->kappa : nullptr;
-        if (root) heat_top = heat_capture_step(c->heat, U, kappa, &c->rec->dt_next, s, root);
+        if (root) heat_top = heat_capture_step(c->heat, U, kappa, &c->rec->dt_next, s, root, alone);
         else heat_step(c->heat, U, kappa, &c->rec->dt_next, s, &c->heat_report);
     }
     mark(5);
@@ -432,9 +432,9 @@ static bool capturable(sr_ctx* c) { return !c->cfg.heat || heat_capturable(c->he
 
 // Appends one whole step from state buffer `cur` to the capture in progress on `s` (root graph `root`); returns the
 // kernels one replay launches outside the implicit step's loops.
-long long sr_ctx_capture_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t root) {
+long long sr_ctx_capture_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t root, bool alone) {
     const long long before = (long long)sr_launches();
-    const long long heat_top = enqueue_step(c, cur, s, root, [](int) {});
+    const long long heat_top = enqueue_step(c, cur, s, root, alone, [](int) {});
     const long long n = (long long)sr_launches() - before;
     sr_note_launches(-n);  // captured, not launched
     return n + heat_top;
@@ -601,7 +601,7 @@ static void capture_step_graph(sr_ctx* c) {
     SR_CUDA_TRY(cudaStreamBeginCaptureToGraph(c->stream, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
     long long n = 0;
     try {
-        n = sr_ctx_capture_step(c, c->cur, c->stream, g);
+        n = sr_ctx_capture_step(c, c->cur, c->stream, g, true);
     } catch (...) {
         cudaGraph_t dead;
         cudaStreamEndCapture(c->stream, &dead);
@@ -631,7 +631,7 @@ static void run_steps(sr_ctx* c, uint32_t steps) {
         for (uint32_t s = 0; s < steps; s++) {
             if (!one && !c->step_graph[c->cur]) capture_step_graph(c);  // before the step's start event
             if (c->timing) SR_CUDA_TRY(cudaEventRecord(event_at(c, 2 * (size_t)s), c->stream));
-            if (one) enqueue_step(c, c->cur, c->stream, nullptr, [](int) {});
+            if (one) enqueue_step(c, c->cur, c->stream, nullptr, true, [](int) {});
             else SR_CUDA_TRY(cudaGraphLaunch(c->step_graph[c->cur], c->stream));
             if (c->timing) SR_CUDA_TRY(cudaEventRecord(event_at(c, 2 * (size_t)s + 1), c->stream));
             sr_ctx_graph_steps_done(c, 1, one ? 0 : c->step_launches);
@@ -658,7 +658,7 @@ static void run_steps(sr_ctx* c, uint32_t steps) {
         auto mark = [&](int slot) {
             if (c->timing) SR_CUDA_TRY(cudaEventRecord(event_at(c, (size_t)s * E + slot), c->stream));
         };
-        enqueue_step(c, c->cur, c->stream, nullptr, mark);
+        enqueue_step(c, c->cur, c->stream, nullptr, true, mark);
         if (c->cfg.hydro) c->cur = 1 - c->cur;
         SR_CUDA_TRY(cudaGetLastError());
     }

@@ -811,6 +811,7 @@ __global__ void __launch_bounds__(RED_THREADS, 3)
     spmv_dir_kernel(MgLevel L, int rows, double* scal, const float* __restrict__ z, float* pa, float* pb,
                     float* __restrict__ q, double* pq_part, const double* __restrict__ rz_part, int parts) {
     __shared__ double s_rz;
+    pdl_launch();
     const int w = L.w, h = L.h, w4 = w / 4, lane = threadIdx.x & 31;
     const int t = blockIdx.x * RED_THREADS + threadIdx.x, bands = (h + rows - 1) / rows;
     const bool live = t < w4 * bands;
@@ -832,6 +833,7 @@ __global__ void __launch_bounds__(RED_THREADS, 3)
     };
     Op o = op_at(y0);
     float4 dyu = y0 > 0 ? *reinterpret_cast<const float4*>(L.dy + (size_t)(y0 - 1) * w + x) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();
     if (parts > 0) {
         const double v = block_sum_ordered(rz_part, parts);
         if (threadIdx.x == 0) {
@@ -934,6 +936,7 @@ __global__ void pcg_update4_kernel(size_t n, double* scal, const double* __restr
                                    const float* pa, const float* pb, const float* __restrict__ q, float* __restrict__ e,
                                    float* __restrict__ r, Red R, const __grid_constant__ Ctl ctl) {
     __shared__ double s_pq;
+    pdl_wait();
     const double pq = block_sum_ordered(pq_part, parts);
     if (threadIdx.x == 0) {
         s_pq = pq;
@@ -1394,10 +1397,10 @@ void setup_step(HeatSolver* H, const float* U, const float* kappa, cudaStream_t 
     H->mg.set_couplings(H->kx, H->ky, H->gas, s);
 }
 
-// `overlap`: multigrid's launches start while the one before still runs. In the host's rounds (one graph each) that takes
-// the launch gaps out (learned preconditioner at 512²: 6.84 -> 6.54 ms a step); in the device-controlled step's
-// conditional bodies it gave 0.6 to 1.4 %, and a batch, whose other worlds want the SMs that an early kernel waits on,
-// lost 10 %.
+// `overlap`: multigrid's launches start while the one before still runs, which takes the launch gaps out of the host's
+// rounds (learned preconditioner at 512²: 6.84 -> 6.54 ms a step) and of the captured step of a world alone (with the
+// SpMV's and the update's; 512² reference mode, four steps: 39.98 -> 38.60 ms; 2048², three: 29.87 -> 29.75). Not of a
+// batch's step: its other worlds want the SMs that an early kernel waits on (10 % slower).
 // z = M r, and <r, z> into scalar `rz_slot` (into S_RZN, multigrid's: as partials, for spmv_dir_kernel to sum).
 void precondition(HeatSolver* H, uint32_t precond, int rz_slot, bool overlap, cudaStream_t s) {
     if (precond == SR_PRECOND_JACOBI) {
@@ -1641,7 +1644,7 @@ long long capture_body(cudaGraph_t g, cudaStream_t cs, F body) {
 // is `root` (the conditional handles belong to it): set-up, Δt from the device record, the device-controlled Newton
 // passes, refinements and PCG rounds, and the commit. The state buffer `U` and the opacity plane are fixed in it.
 void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev, cudaStream_t s,
-                       cudaGraph_t root) {
+                       cudaGraph_t root, bool alone) {
     Ctl ctl{H->ctl, dt_dev, {}};
     const CtlHandles& hd = ctl.hd;
     for (int b = 0; b < B_COUNT; b++) SR_CUDA_TRY(cudaGraphConditionalHandleCreate(&ctl.hd.h[b], root, 0, 0));
@@ -1677,14 +1680,13 @@ void capture_heat_step(HeatSolver* H, float* U, const float* kappa, const double
             sr_note_launch();
             nb[B_ROUND] = capture_body(capture_conditional(s1, hd.h[B_ROUND], cudaGraphCondTypeWhile), H->cap[2],
                                        [&](cudaStream_t s2) {
-                precondition(H, precond, S_RZN, false, s2);
-                spmv_dir_kernel<<<H->grid_spmv, RED_THREADS, 0, s2>>>(
-                    H->mg.L[0], H->spmv_rows, H->scal, H->z32, H->p32, H->p2, H->q32, H->pq_part, H->rz_part,
-                    precond == SR_PRECOND_MG ? H->mg.parts() : 0);
+                precondition(H, precond, S_RZN, alone, s2);
+                launch_kernel(alone && precond == SR_PRECOND_MG, spmv_dir_kernel, dim3(H->grid_spmv), dim3(RED_THREADS), 0,
+                              s2, H->mg.L[0], H->spmv_rows, H->scal, H->z32, H->p32, H->p2, H->q32, H->pq_part,
+                              H->rz_part, precond == SR_PRECOND_MG ? H->mg.parts() : 0);
                 sr_note_launch();
-                pcg_update4_kernel<<<H->grid_update, RED_THREADS, 0, s2>>>(H->n, H->scal, H->pq_part, H->grid_spmv,
-                                                                          H->p32, H->p2, H->q32, H->e32, H->r32,
-                                                                          H->red(S_RRI), ctl);
+                launch_kernel(alone, pcg_update4_kernel, dim3(H->grid_update), dim3(RED_THREADS), 0, s2, H->n, H->scal,
+                              H->pq_part, H->grid_spmv, H->p32, H->p2, H->q32, H->e32, H->r32, H->red(S_RRI), ctl);
                 sr_note_launch();
             });
             correction_kernel<<<H->grid, RED_THREADS, 0, s1>>>(H->n, H->gas, H->e32, H->scal, H->x);
@@ -2019,7 +2021,7 @@ void heat_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev
             SR_CUDA_TRY(cudaGraphCreate(&g, 0));
             SR_CUDA_TRY(cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
             try {
-                capture_heat_step(H, U, kappa, dt_dev, s, g);
+                capture_heat_step(H, U, kappa, dt_dev, s, g, true);
             } catch (...) {
                 cudaGraph_t dead;
                 cudaStreamEndCapture(s, &dead);
@@ -2154,8 +2156,8 @@ void heat_prepare_capture(HeatSolver* H, cudaStream_t s) {
 }
 
 long long heat_capture_step(HeatSolver* H, float* U, const float* kappa, const double* dt_dev, cudaStream_t s,
-                            cudaGraph_t root) {
-    capture_heat_step(H, U, kappa, dt_dev, s, root);
+                            cudaGraph_t root, bool alone) {
+    capture_heat_step(H, U, kappa, dt_dev, s, root, alone);
     return H->body_launches[B_COUNT];
 }
 
