@@ -73,7 +73,8 @@ struct HeatCtl {
     int max_passes, max_rounds, pin;
     // the step
     double heat0, n_gas;
-    int passes, rounds, refinements, converged, ok, skipped;
+    double dt;  // the Δt it covers; 0 where there was nothing to solve
+    int passes, rounds, refinements, converged, ok;
     double pass_tol, moved_prev, rel;
     // the pass's refinement and its inner solve
     int ref, reached, it, max_it;
@@ -153,7 +154,7 @@ __device__ __noinline__ void ctl_run(const Ctl& k, double* scal, int phase) {
             c->heat0 = scal[S_HEAT0];
             c->n_gas = scal[S_NGAS];
             const bool skip = c->pin || c->n_gas == 0.0 || !(scal[S_DT] > 0.0);
-            c->skipped = skip;
+            c->dt = skip ? 0.0 : scal[S_DT];
             c->passes = c->rounds = c->refinements = 0;
             c->converged = skip ? 1 : 0;
             c->ok = 1;
@@ -1997,7 +1998,7 @@ void heat_sync_report(HeatSolver* H, cudaStream_t s) {
     sr_note_launches(n);
     sr_heat_report R{};
     R.precond = H->precond;
-    R.dt = c.skipped ? 0.0 : H->hscal[S_DT];
+    R.dt = c.dt;
     R.passes = (uint32_t)c.passes;
     R.rounds = (uint32_t)c.rounds;
     R.refinements = (uint32_t)c.refinements;
