@@ -298,8 +298,8 @@ sr_ctx* sr_batch_ctx(sr_batch* b, uint32_t index);
 /* P2's gravity solve (φ and g = -∇φ of Σ, as a context's) with no device allocation — no counterpart in the
  * reference. For callers that cannot allocate device memory: hosts that own every byte of device memory and hand their
  * plug-ins buffers (no cudaMalloc allowed), or loops that cannot afford cudaMalloc's device-wide synchronisation. The
- * caller passes device buffers: `sigma` (W*H) in, `phi`, `gx`, `gy` (W*H each) out, and the CUDA stream (NULL: the
- * default stream) as `stream`. The scratch lives in static device arrays sized for worlds up to 256 x 256 cells, held
+ * caller passes device buffers: `sigma` (W*H) in, `phi`, `gx`, `gy` (W*H each) out, each on a float's boundary (outputs
+ * that all begin on 16 bytes are written 16 bytes at a time), and the CUDA stream (NULL: the default stream) as `stream`. The scratch lives in static device arrays sized for worlds up to 256 x 256 cells, held
  * by every GPU that loads the library until exit; a larger world is refused with SR_E_INVALID. The first call on a
  * device looks up the arrays and uploads the kernel's spectrum; so does every call whose padded FFT size, kernel, G or
  * (softened kernel only) softening differs from the previous call's on that device. Such a call copies from the host

@@ -19,6 +19,7 @@
 // stage through shared memory took 16 passes over it. Stage twiddles come from a table built in f64 on the host, laid
 // out so that neighbouring threads read neighbouring entries.
 #include <math.h>
+#include <stdint.h>
 
 #include <algorithm>
 #include <functional>
@@ -353,16 +354,26 @@ __global__ void __launch_bounds__(inverse_group<N>() * fft_threads<N>()) grav_ro
             const float *u = c - RP, *d = c + RP;
             gy = make_float4(-(d[1] - u[1]) / 2.0f, -(d[2] - u[2]) / 2.0f, -(d[3] - u[3]) / 2.0f, -(d[4] - u[4]) / 2.0f);
             const size_t o = (size_t)y * w + x;
-            *reinterpret_cast<float4*>(A.phi + o) = p;
-            *reinterpret_cast<float4*>(A.gx + o) = gx;
-            *reinterpret_cast<float4*>(A.gy + o) = gy;
+            auto store = [&](float* a, const float4& v) {
+                if (A.vec) {
+                    *reinterpret_cast<float4*>(a + o) = v;
+                } else {
+                    a[o] = v.x;
+                    a[o + 1] = v.y;
+                    a[o + 2] = v.z;
+                    a[o + 3] = v.w;
+                }
+            };
+            store(A.phi, p);
+            store(A.gx, gx);
+            store(A.gy, gy);
         }
     }
 }
 
 // ---- pass 4 (rows past 1,024 points): φ and g = -∇φ by central differences over the ringed potential (grav.rs:55-70),
 // four cells a thread (the world's width is a multiple of 8 and the ring's rows are padded so that its cells lie on
-// 16-byte boundaries)
+// 16-byte boundaries; a context's planes, the only ones that come here, are allocations of their own)
 __global__ void grav_gradient_kernel(GravArgs A) {
     const int w = A.w, h = A.h, rp = A.rp;
     const int n4 = w * h / 4;
@@ -621,6 +632,7 @@ void GravPlan::solve(const float* src, float* phi, float* gx, float* gy, cudaStr
     A.phi = phi;
     A.gx = gx;
     A.gy = gy;
+    A.vec = (((uintptr_t)phi | (uintptr_t)gx | (uintptr_t)gy) & 15) == 0;
     dispatch_rows(px, A, s);
     dispatch_columns(py, A, s);
     dispatch_rows_inverse(px, A, s);
