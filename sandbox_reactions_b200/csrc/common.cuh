@@ -153,8 +153,10 @@ static inline unsigned div_up(unsigned a, unsigned b) { return (a + b - 1) / b; 
 // ---- overlapped launches: a kernel launched with `overlap` may start while the one before it on the stream still runs.
 // It must call pdl_wait (which returns once that kernel, and so everything before it, is complete and visible) before
 // it reads anything the kernels since the last plain launch wrote, and before it writes global memory at all; what it
-// does earlier (barrier set-up, loads of planes no recent kernel writes) hides the launch and the ramp. A kernel lets
-// the next one start with pdl_launch. Both are no-ops where the launch is plain.
+// does earlier (barrier set-up, loads of planes no recent kernel writes) hides the launch and the ramp. What those
+// kernels wrote it takes as plain pointers: as `const T* __restrict__` (or by __ldg) it would be promised to be read-only
+// for the kernel's whole life, and the compiler could load it before the wait. A kernel lets the next one start with
+// pdl_launch. Both are no-ops where the launch is plain.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

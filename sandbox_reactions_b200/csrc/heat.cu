@@ -778,7 +778,7 @@ __device__ __forceinline__ void block_partial(double acc, double* part) {
 }
 
 // Σ v[0..n) by the block, in an order that depends on n and the block's size alone; valid in thread 0.
-__device__ __forceinline__ double block_sum_ordered(const double* __restrict__ v, int n) {
+__device__ __forceinline__ double block_sum_ordered(const double* v, int n) {
     __shared__ double red[32];
     double x = 0.0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) x += v[i];
@@ -792,7 +792,7 @@ __device__ __forceinline__ double block_sum_ordered(const double* __restrict__ v
     return t;
 }
 
-__global__ void sum_parts_kernel(const double* __restrict__ v, int n, double* out) {
+__global__ void sum_parts_kernel(const double* v, int n, double* out) {
     const double t = block_sum_ordered(v, n);
     if (threadIdx.x == 0) *out = t;
 }
@@ -809,8 +809,8 @@ __global__ void sum_parts_kernel(const double* __restrict__ v, int n, double* ou
 // puts all threads on the GPU at once (1 up to some 600,000 cells); the next row's operands are in flight behind this
 // row's arithmetic.
 __global__ void __launch_bounds__(RED_THREADS, 3)
-    spmv_dir_kernel(MgLevel L, int rows, double* scal, const float* __restrict__ z, float* pa, float* pb,
-                    float* __restrict__ q, double* pq_part, const double* __restrict__ rz_part, int parts) {
+    spmv_dir_kernel(MgLevel L, int rows, double* scal, const float* z, float* pa, float* pb, float* __restrict__ q,
+                    double* pq_part, const double* rz_part, int parts) {
     __shared__ double s_rz;
     pdl_launch();
     const int w = L.w, h = L.h, w4 = w / 4, lane = threadIdx.x & 31;
@@ -933,9 +933,9 @@ __global__ void __launch_bounds__(RED_THREADS, 3)
 
 // e += α p, r -= α q with 16-byte accesses (four cells per thread), p the round's new direction; partials of <r, r>.
 // <p, q> comes as `parts` partials, which every CTA sums in the same order; the first CTA leaves it in S_PQ.
-__global__ void pcg_update4_kernel(size_t n, double* scal, const double* __restrict__ pq_part, int parts,
-                                   const float* pa, const float* pb, const float* __restrict__ q, float* __restrict__ e,
-                                   float* __restrict__ r, Red R, const __grid_constant__ Ctl ctl) {
+__global__ void pcg_update4_kernel(size_t n, double* scal, const double* pq_part, int parts, const float* pa,
+                                   const float* pb, const float* q, float* __restrict__ e, float* __restrict__ r, Red R,
+                                   const __grid_constant__ Ctl ctl) {
     __shared__ double s_pq;
     pdl_wait();
     const double pq = block_sum_ordered(pq_part, parts);
@@ -945,7 +945,7 @@ __global__ void pcg_update4_kernel(size_t n, double* scal, const double* __restr
     }
     __syncthreads();
     const float alpha = (float)(scal[S_RZN] / s_pq);
-    const float* __restrict__ p = scal[S_PAR] != 0.0 ? pa : pb;
+    const float* p = scal[S_PAR] != 0.0 ? pa : pb;
     const size_t n4 = n / 4, stride = (size_t)gridDim.x * blockDim.x;
     double acc = 0.0;
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n4; t += stride) {

@@ -555,8 +555,8 @@ template <int NS, bool PRE, bool WT>
 __global__ void __launch_bounds__(RB_NT, 2)
     mg_rowband_tma_kernel(const __grid_constant__ CUtensorMap mb, const __grid_constant__ CUtensorMap mc,
                           const __grid_constant__ CUtensorMap mdx, const __grid_constant__ CUtensorMap mdy,
-                          const __grid_constant__ CUtensorMap mx, MgLevel L, MgLevel C, const float* __restrict__ xc,
-                          float omega, double* part) {
+                          const __grid_constant__ CUtensorMap mx, MgLevel L, MgLevel C, const float* xc, float omega,
+                          double* part) {
     constexpr int H = rb_halo<NS, PRE>(), SX = RB_RX - 2 * H, SY = RB_RY - 2 * H;
     constexpr int XO = (H % 4 == 2) ? 2 : 4;  // the region's first column within the box (X0 - XO on a 16-byte boundary)
     constexpr bool TWO_C = PRE && !WT, LATE = PRE && WT;
