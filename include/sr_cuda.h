@@ -146,8 +146,9 @@ typedef struct sr_cost {
     double floors_ms;    /* P8 */
     double dt_ms;        /* P9 */
     double total_ms;
-    double hydro_update_ms; /* the fused hydro update kernel alone (the roofline kernel) */
-    uint32_t hydro_update_launches;
+    double hydro_update_ms; /* of P4, the kernels of the gas update alone: with gravity the predictor and the kick (the
+                             * half step's solve between them left out), without it the fused update */
+    uint32_t hydro_update_launches; /* the updates it covers, one a step */
     uint32_t pad2;
     uint64_t kernel_launches; /* this library's kernel launches during the call */
 } sr_cost;

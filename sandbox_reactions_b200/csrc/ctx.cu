@@ -345,18 +345,22 @@ static HydroArgs hydro_args(sr_ctx* c, int cur) {
     return A;
 }
 
+// The events of a step under the per-pass timing: its start, after P2, the gas update's start and end (with gravity the
+// predictor's, and the kick's start once the half step's field is solved: it ends P4), after P4, after P5, after P8/P9.
+enum StepMark { kStart, kP2, kUpdate, kUpdated, kKick, kP4, kP5, kP9, kMarks };
+
 // One step's launches on `s` from state buffer `cur`, in the reference's pass order P1 → P2 → P4 → P5 → P8 → P9
 // (reference/mod.rs:264-297). With `root` the launches are captured into that graph and P5 is the device-controlled
-// step (heat_capture_step; `alone`: not among a batch's worlds); otherwise they run now, P5 by heat_step. `mark(slot)` is called at the pass boundaries
-// (0 start, 1 after P2, 2 hydro update start, 3 its end, 4 after P4, 5 after P5, 6 after P8/P9).
+// step (heat_capture_step; `alone`: not among a batch's worlds); otherwise they run now, P5 by heat_step. `mark(m)` is
+// called at the pass boundaries; with the per-pass timing (2) a gas-only step's floors and Δt are a pass of their own.
 template <class Mark>
 static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t root, bool alone, Mark mark) {
     long long heat_top = 0;  // kernels of a captured implicit step outside its loops
     const sr_config& k = c->cfg;
     float* U = c->U[cur];
-    mark(0);
+    mark(kStart);
     if (k.gravity) c->grav.solve(U, c->phi, c->gx, c->gy, s);
-    mark(1);
+    mark(kP2);
     if (ref_mode(c)) {
         // reference mode: P4 (step_held), P8's floors, the hold and P9 (reference/mod.rs:264-297; P5 is off)
         if (k.hydro) {
@@ -366,16 +370,16 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
                 c->grav.solve(c->src, c->phim, c->gxm, c->gym, s);
                 c->grav.solve(c->src_free, c->phip, c->gxp, c->gyp, s);
             }
-            mark(2);
+            mark(kUpdate);
             ref_hydro_update_launch(A, k.gravity, s);
-            mark(3);
+            mark(kUpdated);
             ref_hydro_finalize_launch(A, s);
             U = c->U[1 - cur];
         } else {
-            mark(2);
-            mark(3);
+            mark(kUpdate);
+            mark(kUpdated);
         }
-        mark(4);
+        mark(kP4);
         if (k.heat) {
             if (root) heat_top = heat_capture_step(c->heat, U, nullptr, &c->rec->dt_next, s, root, alone);
             else heat_step(c->heat, U, nullptr, &c->rec->dt_next, s, &c->heat_report);
@@ -383,47 +387,49 @@ static long long enqueue_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t ro
             heat_flux_planes(c->heat, &fx, &fy);
             ref_cell_flux_launch(fx, fy, c->radx, c->rady, c->w, c->h, s);
         }
-        mark(5);
+        mark(kP5);
         ref_floors_launch(c->R, U, s);
         ref_hold_dt_launch(c->R, U, c->held, k.gravity ? c->gx : nullptr, k.gravity ? c->gy : nullptr, 1, 1,
                            c->part_rate, c->part_g, c->part_nf, dt_rule(c, 1), s);
-        mark(6);
+        mark(kP9);
         return heat_top;
     }
     if (k.hydro) {
         HydroArgs A = hydro_args(c, cur);
         if (k.gravity) {
-            mark(2);
+            mark(kUpdate);
             hydro_launch(kHydroPredict, A, s);
-            mark(3);
+            mark(kUpdated);
             c->grav.solve(c->src, c->phim, c->gxm, c->gym, s);
+            mark(kKick);
             hydro_gravity_launch(A, s);
         } else {
-            mark(2);
-            hydro_launch(k.heat ? kHydroUpdate : kHydroStep, A, s);
-            mark(3);
-            if (!k.heat) {  // the floors and Δt rode along: the step is done
-                mark(4);
-                mark(5);
-                mark(6);
+            const bool whole = !k.heat && (root || c->timing != 2);
+            mark(kUpdate);
+            hydro_launch(whole ? kHydroStep : kHydroUpdate, A, s);
+            mark(kUpdated);
+            if (whole) {  // the floors and Δt rode along: the step is done
+                mark(kP4);
+                mark(kP5);
+                mark(kP9);
                 return 0;
             }
         }
         U = c->U[1 - cur];
     } else {
-        mark(2);
-        mark(3);
+        mark(kUpdate);
+        mark(kUpdated);
     }
-    mark(4);
+    mark(kP4);
     if (k.heat) {
         const float* kappa = k.opacity_plane ? c->kappa : nullptr;
         if (root) heat_top = heat_capture_step(c->heat, U, kappa, &c->rec->dt_next, s, root, alone);
         else heat_step(c->heat, U, kappa, &c->rec->dt_next, s, &c->heat_report);
     }
-    mark(5);
+    mark(kP5);
     floors_dt_launch(c->H, U, k.gravity ? c->gx : nullptr, k.gravity ? c->gy : nullptr, 1, c->part_rate, c->part_g,
                      c->part_nf, c->tickets, dt_rule(c, 1), s);
-    mark(6);
+    mark(kP9);
     return heat_top;
 }
 
@@ -434,7 +440,7 @@ static bool capturable(sr_ctx* c) { return !c->cfg.heat || heat_capturable(c->he
 // kernels one replay launches outside the implicit step's loops.
 long long sr_ctx_capture_step(sr_ctx* c, int cur, cudaStream_t s, cudaGraph_t root, bool alone) {
     const long long before = (long long)sr_launches();
-    const long long heat_top = enqueue_step(c, cur, s, root, alone, [](int) {});
+    const long long heat_top = enqueue_step(c, cur, s, root, alone, [](StepMark) {});
     const long long n = (long long)sr_launches() - before;
     sr_note_launches(-n);  // captured, not launched
     return n + heat_top;
@@ -631,7 +637,7 @@ static void run_steps(sr_ctx* c, uint32_t steps) {
         for (uint32_t s = 0; s < steps; s++) {
             if (!one && !c->step_graph[c->cur]) capture_step_graph(c);  // before the step's start event
             if (c->timing) SR_CUDA_TRY(cudaEventRecord(event_at(c, 2 * (size_t)s), c->stream));
-            if (one) enqueue_step(c, c->cur, c->stream, nullptr, true, [](int) {});
+            if (one) enqueue_step(c, c->cur, c->stream, nullptr, true, [](StepMark) {});
             else SR_CUDA_TRY(cudaGraphLaunch(c->step_graph[c->cur], c->stream));
             if (c->timing) SR_CUDA_TRY(cudaEventRecord(event_at(c, 2 * (size_t)s + 1), c->stream));
             sr_ctx_graph_steps_done(c, 1, one ? 0 : c->step_launches);
@@ -651,12 +657,10 @@ static void run_steps(sr_ctx* c, uint32_t steps) {
         }
         return;
     }
-    // event slots per step: 0 start, 1 after P2, 2 hydro update start, 3 hydro update end, 4 after P4, 5 after P5,
-    // 6 after P8/P9
-    const int E = 7;
+    const bool kick = c->cfg.hydro && c->cfg.gravity && !ref_mode(c);
     for (uint32_t s = 0; s < steps; s++) {
-        auto mark = [&](int slot) {
-            if (c->timing) SR_CUDA_TRY(cudaEventRecord(event_at(c, (size_t)s * E + slot), c->stream));
+        auto mark = [&](StepMark m) {
+            if (c->timing) SR_CUDA_TRY(cudaEventRecord(event_at(c, (size_t)s * kMarks + m), c->stream));
         };
         enqueue_step(c, c->cur, c->stream, nullptr, true, mark);
         if (c->cfg.hydro) c->cur = 1 - c->cur;
@@ -669,19 +673,17 @@ static void run_steps(sr_ctx* c, uint32_t steps) {
         memset(&t, 0, sizeof t);
         t.steps = steps;
         for (uint32_t s = 0; s < steps; s++) {
-            float ms[6];
-            for (int q = 0; q < 6; q++) {
-                int a = q, b = q + 1;
-                SR_CUDA_TRY(cudaEventElapsedTime(&ms[q], c->events[(size_t)s * E + a], c->events[(size_t)s * E + b]));
-            }
-            t.gravity_ms += ms[0];
-            t.hydro_ms += ms[1] + ms[2] + ms[3];
-            t.hydro_update_ms += ms[2];
-            t.heat_ms += ms[4];
-            t.dt_ms += ms[5];
-            float total;
-            SR_CUDA_TRY(cudaEventElapsedTime(&total, c->events[(size_t)s * E], c->events[(size_t)s * E + 6]));
-            t.total_ms += total;
+            auto between = [&](StepMark a, StepMark b) {
+                float ms;
+                SR_CUDA_TRY(cudaEventElapsedTime(&ms, c->events[(size_t)s * kMarks + a], c->events[(size_t)s * kMarks + b]));
+                return (double)ms;
+            };
+            t.gravity_ms += between(kStart, kP2);
+            t.hydro_ms += between(kP2, kP4);
+            t.hydro_update_ms += between(kUpdate, kUpdated) + (kick ? between(kKick, kP4) : 0.0);
+            t.heat_ms += between(kP4, kP5);
+            t.dt_ms += between(kP5, kP9);
+            t.total_ms += between(kStart, kP9);
         }
         t.hydro_update_launches = c->cfg.hydro ? steps : 0;
         t.kernel_launches = sr_launches() - launches0;
