@@ -376,7 +376,9 @@ __global__ void pack_weights_kernel(const float* __restrict__ theta, int cin, in
 // fifteen layers: 2.8 -> 0.2 ms against one output channel's 2,048 pixels per thread with a shared-memory load for
 // nearly every multiply-add, and 8 threads a channel for the bias.
 constexpr int DW_W = 16, DW_H = 8, DW_HW = DW_W + 2, DW_HH = DW_H + 2, DW_NT = 192;
-constexpr int DW_CHUNKS = 128;  // partials at most
+// A partial is FP32 over at most 2,048 pixels (16 tiles), and the partials are summed in FP64: the error does not grow
+// with the batch. Up to 2,048 tiles that leaves 128 CTAs, or one a tile.
+constexpr int DW_CHUNKS = 128, DW_TILES = 2048 / (DW_W * DW_H);
 
 template <int CIN_P, int COUT_P>
 struct DwShape {
@@ -392,7 +394,7 @@ struct DwShape {
 
 int dw_chunks(int B, int H, int W) {
     const long long tiles = (long long)B * ((H + DW_H - 1) / DW_H) * ((W + DW_W - 1) / DW_W);
-    return (int)std::min<long long>(tiles, DW_CHUNKS);
+    return (int)std::min<long long>(tiles, std::max<long long>(DW_CHUNKS, (tiles + DW_TILES - 1) / DW_TILES));
 }
 
 template <int CIN_P, int COUT_P>
@@ -502,8 +504,8 @@ __global__ void __launch_bounds__(DW_NT) dw_kernel(ConvArgs A, const float* __re
     }
 }
 
-// dW and db from the partials into the gradient vector (the parameter layout W[cout][3][3][cin], b[cout]). A sum of up
-// to 128 partials is 128 dependent steps of a load's latency for one thread, so each parameter's are dealt to RD_S threads
+// dW and db from the partials into the gradient vector (the parameter layout W[cout][3][3][cin], b[cout]). A sum of 128
+// partials is 128 dependent steps of a load's latency for one thread, so each parameter's are dealt to RD_S threads
 // in runs, and the runs' sums added in order: 8.7 -> 3.2 us a layer.
 constexpr int RD_E = 32, RD_S = 8;  // parameters and runs of a CTA
 __global__ void __launch_bounds__(RD_E * RD_S) dw_reduce_kernel(const float* __restrict__ part, int chunks, int cin,
