@@ -549,7 +549,7 @@ constexpr size_t kRbEdges = sizeof(float2) * 2 * 2 * RB_WARPS * 32, kRbCoarse = 
 constexpr size_t kRbSmem = RB_BOXES * kRbBox + kRbEdges + kRbCoarse + 16;
 // two CTAs an SM and no more than there are regions
 inline unsigned rb_regions(const MgLevel& L, int halo) { return div_up(L.w, RB_RX - 2 * halo) * div_up(L.h, RB_RY - 2 * halo); }
-inline unsigned rb_grid(const MgLevel& L, int halo) { return std::min(rb_regions(L, halo), 2u * 148u); }
+inline unsigned rb_grid(const MgLevel& L, int halo) { return std::min(rb_regions(L, halo), (unsigned)kMgMaxParts); }
 
 template <int NS, bool PRE, bool WT>
 __global__ void __launch_bounds__(RB_NT, 2)
@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(RB_NT, 2)
 // through shared memory; the next level (at most 32 x 32) by up to 4 warps of two 16-pair row groups; every level of at
 // most 16 x 16 by warp 0 alone, 8 pairs x 4 row groups, neighbours by shuffles and no barrier at all. The top level's
 // coefficients stay in registers from its pre- to its post-smoother; the lower levels are read from the image
-// mg_tail_pack_kernel writes once per Newton pass, whose rows are padded to even pitches and heights so that no access
+// mg_tail_setup_kernel writes once per Newton pass, whose rows are padded to even pitches and heights so that no access
 // has an edge case. 64 x 64 top under V(4,4): 27 -> 15.5 us a V-cycle against the whole CTA of 1,024 threads meeting at
 // every half-sweep of every level.
 extern __shared__ __align__(16) unsigned char tail_smem_raw[];
@@ -1499,11 +1499,6 @@ int grid_for(size_t n) {
 }
 
 }  // namespace
-
-size_t mg_smooth_ctas(int w, int h) {
-    constexpr unsigned out = RB_RX - 2 * rb_halo<8, false>();  // the smallest output tile
-    return (size_t)div_up(w, out) * div_up(h, out);
-}
 
 void Multigrid::create(int w, int h, int pre_, int post_) {
     SR_REQUIRE(pre_ >= 1 && pre_ <= 4 && post_ >= 1 && post_ <= 4, "V-cycle sweeps must be 1..4");

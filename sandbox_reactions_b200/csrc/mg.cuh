@@ -33,8 +33,7 @@ struct MgLevel {
     int* err = nullptr;   // set to 1 when a bounded wait of a smoother gave up (its TMA boxes never landed)
 };
 
-// At most this many CTAs in a post-smoother launch on a w x h level 0 (each leaves one partial of <r, z>).
-size_t mg_smooth_ctas(int w, int h);
+constexpr int kMgMaxParts = 2 * 148;  // at most this many CTAs in a row-band launch: two an SM, which walk over the regions
 
 struct Multigrid {
     int nlevels = 0;
@@ -54,7 +53,8 @@ struct Multigrid {
     // Every coarse level's operator, once level 0's c (written by the caller, per Newton pass) is in place.
     void coarsen(cudaStream_t s);
     // (`overlap`: its launches overlap one another, the first only plainly follows what came before.)
-    // z = M r (level-0 b := r, x2 := z), and (rz_part not null) <r, z> as parts() partials, to be summed in order.
+    // z = M r (level-0 b := r, x2 := z), and (rz_part not null) <r, z> as parts() (at most kMgMaxParts) partials, to be summed in
+    // order.
     void apply(const float* r, float* z, double* rz_part, bool overlap, cudaStream_t s);
     int parts() const;
     // The device time (ms) of one launch of level 0's pre- and post-smoother on the last applied system, each
