@@ -37,8 +37,8 @@ def test_a_refused_world_is_named():
 
 
 def test_a_captured_step_matches_the_launched_one():
-    # after the first step (which tunes the multigrid) a context runs each whole step as one captured graph, the
-    # implicit step under device control; with timing on the passes are launched one by one: the same state either way
+    # a context runs each whole step as one captured graph, the implicit step under device control; with timing on the
+    # passes are launched one by one: the same state either way
     cfg, P, kappa = scenes.full_step(96, scene=5)
     out = []
     for timed in (False, True):
