@@ -17,7 +17,6 @@ struct GravArgs {
     float* phi;
     float* gx;
     float* gy;
-    bool vec;  // φ and g begin on 16 bytes (a context's own always; sr_gravity_solve_static's are the caller's)
 };
 
 // The smallest power of two >= 2 len, at least 32, at most 8192 (0: refused).
