@@ -5,13 +5,13 @@
 // tile's and the one-cell ring around it), the faces meet for the HLL fluxes by warp shuffles (x) and shared memory
 // (y), and the per-cell epilogue of the pass finishes:
 //   - kHydroStep:       U' = U - Δt ΔF, then P8's floors and P9's Δt on U' (no gravity, no heat: the whole step);
-//   - kHydroUpdate:     U' = U - Δt ΔF (no gravity; heat follows);
+//   - kHydroUpdate:     U' = U - Δt ΔF (no gravity; heat follows, or the passes are timed one by one);
 //   - kHydroPredict:    with gravity: U - Δt ΔF, the half step's source ½(Σⁿ + Σⁿ⁺¹), masked (reference
 //                       hydro.rs:815-836), and what gravity's work reads — the half-step (Σ, Σu, Σv) and the faces'
 //                       mass fluxes. Once φ_mid is solved, hydro_gravity_kernel adds the half-step kick and the faces'
 //                       work across it (hydro.rs:871-947) and takes the net kick back from the densest cell.
 // The predictor runs once a step: it is what the step costs (FP32 issue), and a second run of it after the solve, to
-// recompute fluxes that 20 B a cell can carry over, took 172 + 331 us at 2048² where predict and gravity take 198 + 90.
+// recompute fluxes that 20 B a cell can carry over, took 172 + 331 us at 2048² where predict and gravity take 208 + 89.
 // The scheme follows crates/sr-physics/src/reference/hydro.rs (step_held without held cells, sinks or radiation).
 #include "hydro.cuh"
 
@@ -398,7 +398,9 @@ __device__ __forceinline__ void take_back(KickPart kp, KickPart* red, const Hydr
 // Gravity's part of the step, after the half step's solve: each cell's kick Δt Σ_src g_mid and its four faces' work.
 // A thread takes four neighbouring columns (16-byte accesses: the world's width is a multiple of 8) of HG_R rows,
 // works out the faces to the right of and below each of its cells once, and hands the right one to the next lane; a
-// cell with no gas around it (its source stored as -0) takes nothing but lends its faces. Bound by HBM: 68 B a cell.
+// cell with no gas around it (its source stored as -0) takes nothing but lends its faces. Bound by latency: 60 B a cell at
+// 2.8 TB/s (2048²: 89 us, DRAM at 32 %, issue 42 %) with the 16 warps an SM that 125 registers leave, each waiting on its
+// row's loads and on the faces' divisions and square roots in turn.
 constexpr int HG_R = 4, HG_WARPS = 4, HG_COLS = 128;
 
 __global__ void __launch_bounds__(32 * HG_WARPS, 4) hydro_gravity_kernel(HydroArgs A) {
