@@ -281,8 +281,9 @@ sr_status sr_attach_learner(sr_ctx* ctx, sr_learner* learner);
 
 /* ---- Batches: many independent worlds of uneven sizes advanced together (the reference runs one world per Step,
  * crates/sr-engine/src/step/mod.rs:367-718; a batch is N such Steps whose kernels overlap on one GPU). Each world keeps
- * its own context and stream; sr_batch_step hands the worlds to a pool of host threads balanced by cell count, so the
- * worlds' kernels (and their implicit solves' host decisions) interleave on the device. */
+ * its own context and stream; a batch step is one captured graph with a branch a world, so the worlds' kernels interleave
+ * on the device with no host decision between them. With a world on the learned preconditioner the worlds step on a pool
+ * of host threads balanced by cell count. */
 typedef struct sr_batch sr_batch;
 /* `count` configurations; `threads` host threads (0: one per world, at most 16). */
 sr_status sr_batch_create(const sr_config* cfgs, uint32_t count, uint32_t threads, sr_batch** out);

@@ -36,3 +36,26 @@ def test_buffers_on_any_float(w, h, at):
     sigma = np.random.default_rng(w + h).random((h, w), np.float32) + np.float32(0.05)
     for got, want in zip(solve(cfg, sigma, at), solve(cfg, sigma, (0, 0, 0, 0))):
         assert np.isfinite(want).all() and np.array_equal(got, want)
+
+
+def test_a_steady_call_can_be_captured():
+    """A call that uploads nothing (the last call's sizes and kernel), captured and replayed on another density."""
+    import torch
+
+    lib, rng = load_library(), np.random.default_rng(5)
+    cfg = Config(width=136, height=104, gravity=True, hydro=False)
+    first, second = (rng.random((104, 136), np.float32) + np.float32(0.05) for _ in range(2))
+    want = solve(cfg, second, (0, 0, 0, 0))
+    c = cfg.to_c()
+    sigma = torch.from_numpy(first).cuda()
+    outs = [torch.zeros((104, 136), device="cuda") for _ in range(3)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        st = lib.sr_gravity_solve_static(C.byref(c), sigma.data_ptr(), *(o.data_ptr() for o in outs),
+                                         C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0, lib.sr_last_error(None).decode()
+    sigma.copy_(torch.from_numpy(second))
+    graph.replay()
+    torch.cuda.synchronize()
+    for o, w in zip(outs, want):
+        assert np.array_equal(o.cpu().numpy().ravel(), w)
